@@ -4,18 +4,44 @@
 // reduced-precision inputs when T = float) and the fallback for bf16 shapes the
 // tensor-core kernel refuses.  W is [out, in] row-major as the reference stores it
 // (include/llmi/model/kernels.hpp:15-17; src/model/kernels.cpp:97-113), x is [rows, in].
-// Every output element is one thread's running sum over k = 0..K-1 in ascending order, so
-// the value of y[r, o] does not depend on how many rows are in the call or where r lies.
+//
+// The order of additions, the same in every kernel of this file: k is cut into segments of SEG places anchored at 0; a
+// segment's sum is one running fmaf chain from 0 in ascending k; an output is the sum of its segments' sums in ascending
+// order.  So the value of y[r, o] does not depend on how many rows are in the call, where r lies or which of the kernels a
+// call's size selects — and the segments of an output can be worked on at the same time.  (One chain over all of k, as
+// before, left a decode step of the 32-bit path nothing to do in parallel but its outputs; against 64 bits the sum of
+// segments is the nearer one.)
+//
+// Three kernels:
+//  * linear_simt_kernel: any type, pitch and alignment (a tile of 64 x 64 outputs, scalar loads);
+//  * linear_f32_tile_kernel: fp32, 16-byte rows, many tokens: four segments of a 64 x 64 tile at a time;
+//  * linear_f32_rows_kernel: fp32, 16-byte rows, few tokens: bound by reading w once.
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace llmi {
 
 constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int SEG = 256;          // k places of a segment (a multiple of BK)
 
 // Output modes of the product.
 constexpr int OUT_STORE = 0;      // y (type T) = acc
 constexpr int OUT_STORE_F32 = 1;  // y (float) = acc
 constexpr int OUT_ADD_F32 = 2;    // y (float) += acc       (residual sum kept in fp32)
+
+template <typename T, int MODE>
+__device__ __forceinline__ void put_output(void* yv, long at, int n, float v, const float* bias, const float* oscale) {
+  if (bias) v = __fadd_rn(v, bias[n]);
+  if (oscale) v = __fmul_rn(v, oscale[n]);
+  if (MODE == OUT_STORE) {
+    ((T*)yv)[at] = from_f32<T>(v);
+  } else if (MODE == OUT_STORE_F32) {
+    ((float*)yv)[at] = v;
+  } else {
+    float* p = (float*)yv + at;
+    *p = __fadd_rn(*p, v);
+  }
+}
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
@@ -34,11 +60,11 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
   const int lr = tid >> 2;        // row of the tile this thread loads
   const int lk = (tid & 3) * 4;   // first of its four k
 
-  float acc[4][4];
+  float acc[4][4], total[4][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0.f;
 
   // The next k block is fetched into registers while the current one is multiplied, so that a block pays the
   // latency of global memory once, not once per k block.  The order of the additions is untouched.
@@ -73,6 +99,15 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
     }
+    if ((k0 + BK) % SEG == 0 || k0 + BK >= K) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          total[i][j] = __fadd_rn(total[i][j], acc[i][j]);
+          acc[i][j] = 0.f;
+        }
+    }
     __syncthreads();
   }
 
@@ -84,39 +119,284 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
       if (n >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[n];
-      if (oscale) v *= oscale[n];
-      if (MODE == OUT_STORE) {
-        ((T*)yv)[(long)m * ldy + n] = from_f32<T>(v);
-      } else if (MODE == OUT_STORE_F32) {
-        ((float*)yv)[(long)m * ldy + n] = v;
-      } else {
-        float* p = (float*)yv + (long)m * ldy + n;
-        *p = *p + v;
-      }
+      put_output<T, MODE>(yv, (long)m * ldy + n, n, total[i][j], bias, oscale);
     }
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Many tokens.  Bound by the FMA pipes (128 a clock and SM).  A block makes a tile of 64 x 64 outputs; its four groups of 64
+// threads take segments 4r, 4r + 1, .. of round r, each thread 8 x 8 outputs in registers (two 16-byte shared loads per 16
+// FMAs where 4 x 4 outputs need four).  With the segments side by side a block keeps four warps' worth of independent chains
+// on every scheduler though its tile is small, and small tiles fill the 148 SMs at the widths of small models (600 tokens x
+// 960 outputs are 150 tiles).  Operands go to shared memory as they lie (rows of 16 k places, 20 floats apart: a quarter
+// warp's 16-byte loads touch 32 different banks) by cp.async, three stages a group.
+constexpr int TILE_STAGES = 3;
+constexpr int TILE_PITCH = BK + 4;
+constexpr int TILE_STAGE_FLOATS = (BM + BN) * TILE_PITCH;
+constexpr int TOTAL_PITCH = BN + 8;
+constexpr int TILE_SMEM = (4 * TILE_STAGES * TILE_STAGE_FLOATS + BM * TOTAL_PITCH) * (int)sizeof(float);
+
+__device__ __forceinline__ void cp_async_16(float* dst, const float* src, bool real) {
+  const int bytes = real ? 16 : 0;               // 0: the place is filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void group_barrier(int group) { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); }
+
+template <int MODE>
+__global__ void __launch_bounds__(256, 1)
+linear_f32_tile_kernel(const float* __restrict__ x, long ldx, const float* __restrict__ w, long ldw, const float* __restrict__ bias,
+                       const float* __restrict__ oscale, float* __restrict__ y, long ldy, int M, int N, int K, long bx, long bw, long by) {
+  extern __shared__ __align__(16) float tile_smem[];
+  x += (long)blockIdx.z * bx;
+  w += (long)blockIdx.z * bw;
+  y += (long)blockIdx.z * by;
+  const int group = threadIdx.x >> 6, t = threadIdx.x & 63;
+  const int tx = t & 7, ty = t >> 3;             // outputs (ty + 8 i, tx + 8 j)
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  float* stages = tile_smem + group * TILE_STAGES * TILE_STAGE_FLOATS;
+  float* total = tile_smem + 4 * TILE_STAGES * TILE_STAGE_FLOATS;
+  for (int i = threadIdx.x; i < BM * TOTAL_PITCH; i += 256) total[i] = 0.f;
+
+  const int n_seg = (K + SEG - 1) / SEG;
+  for (int round = 0; round * 4 < n_seg; ++round) {
+    const int seg = round * 4 + group;
+    const int k_begin = seg * SEG, k_end = min(K, k_begin + SEG);
+    const int steps = seg < n_seg ? (k_end - k_begin + BK - 1) / BK : 0;
+    auto load = [&](int step) {
+      float* s = stages + (step % TILE_STAGES) * TILE_STAGE_FLOATS;
+      const int k = k_begin + step * BK + (t & 3) * 4;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {              // rows 0..63 of x, then 64 rows of w
+        const int r = (t >> 2) + e * 16;
+        const bool of_x = e < 4;
+        const int row = of_x ? m0 + r : n0 + r - BM;
+        const bool real = k < k_end && row < (of_x ? M : N);
+        const float* src = of_x ? x + (long)row * ldx + k : w + (long)row * ldw + k;
+        cp_async_16(s + r * TILE_PITCH + (t & 3) * 4, real ? src : x, real);
+      }
+    };
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+#pragma unroll
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+      if (s < steps) load(s);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int step = 0; step < steps; ++step) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(TILE_STAGES - 2) : "memory");
+      group_barrier(group);                      // this step's rows are here, and everybody is done with the step before's
+      if (step + TILE_STAGES - 1 < steps) load(step + TILE_STAGES - 1);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      const float* s = stages + (step % TILE_STAGES) * TILE_STAGE_FLOATS;
+#pragma unroll
+      for (int q = 0; q < BK / 4; ++q) {
+        float4 a[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(s + (ty + 8 * i) * TILE_PITCH + 4 * q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 b = *reinterpret_cast<const float4*>(s + (BM + tx + 8 * j) * TILE_PITCH + 4 * q);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+        }
+      }
+    }
+    // the segments join the total one after another, in ascending order
+    for (int g = 0; g < 4; ++g) {
+      __syncthreads();
+      if (g == group && seg < n_seg) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float* p = total + (ty + 8 * i) * TOTAL_PITCH + tx + 8 * j;
+            *p = __fadd_rn(*p, acc[i][j]);
+          }
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < BM * BN; i += 256) {
+    const int m = m0 + i / BN, n = n0 + i % BN;
+    if (m < M && n < N) put_output<float, MODE>(y, (long)m * ldy + n, n, total[(i / BN) * TOTAL_PITCH + i % BN], bias, oscale);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Few tokens.  Bound by reading w once, and by latency: a decode step of a small model is a chain of such products.  A block
+// takes ROWS rows of w; every (row, segment) is a bulk copy of at most 1 KB into a place 260 floats from the next (16-byte
+// shared loads of a quarter warp's eight rows touch 32 different banks), all of them asked for at once and before the kernel
+// before has ended (w does not depend on it).  A thread makes the segment sums of one (row, segment) for four tokens: a chain
+// of 256 FMAs is 1,024 clocks, half a microsecond, whatever K is, where one chain over K = 2,560 is 5 us.  x comes through L1
+// (the lanes of a warp share a handful of addresses).
+constexpr int ROWS = 8;
+constexpr int SEG_PITCH = SEG + 4;
+constexpr int MAX_STAGED = 16;        // segments of a row in shared memory at a time (16 x 8 rows: 133 KB)
+constexpr int ROWS_TOKENS = 4;        // tokens a thread takes at a time
+constexpr int ROWS_MAX_TOKENS = 64;
+constexpr int ROWS_OUTPUTS = 4;       // outputs a thread ends with: there are at least 2 M threads, or 193 of the 8 x 64 outputs
+
+template <int MODE>
+__global__ void __launch_bounds__(256)
+linear_f32_rows_kernel(const float* __restrict__ x, long ldx, const float* __restrict__ w, long ldw, const float* __restrict__ bias,
+                       const float* __restrict__ oscale, float* __restrict__ y, long ldy, int M, int N, int K, int staged, int* error_flag,
+                       long bx, long bw, long by) {
+  extern __shared__ __align__(16) float rows_smem[];
+  __shared__ __align__(8) uint64_t bar_store;
+  x += (long)blockIdx.z * bx;
+  w += (long)blockIdx.z * bw;
+  y += (long)blockIdx.z * by;
+  float* w_s = rows_smem;                                             // [staged][ROWS][SEG_PITCH]
+  float* part = w_s + staged * ROWS * SEG_PITCH;                      // [staged][token of the pass][ROWS]
+  const uint32_t bar = smem_u32(&bar_store);
+  const int tid = threadIdx.x, n_threads = blockDim.x;
+  const int n0 = blockIdx.x * ROWS, n_rows = min(ROWS, N - n0);
+  const int n_seg = (K + SEG - 1) / SEG;
+  const int lanes = ROWS * min(staged, 8);                            // threads that share a group of tokens
+  const int groups = n_threads / lanes;                               // groups of tokens at a time
+  const int tg = tid / lanes, row = tid % ROWS, seg_lane = (tid % lanes) / ROWS;
+  const int pass_tokens = groups * ROWS_TOKENS;
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_launch_dependents();
+  uint32_t phase = 0;
+  bool waited = false, ok = true;
+  float total[ROWS_OUTPUTS];                                          // outputs of this thread over the rounds
+#pragma unroll
+  for (int o = 0; o < ROWS_OUTPUTS; ++o) total[o] = 0.f;
+
+  for (int s0 = 0; s0 < n_seg; s0 += staged) {
+    const int here = min(staged, n_seg - s0);
+    if (tid == 0) {                                                   // one thread asks: at most 128 copies
+      const long k_bytes = (long)(min(K, (s0 + here) * SEG) - s0 * SEG) * 4;
+      mbar_expect_tx(bar, (uint32_t)(k_bytes * n_rows));
+      for (int s = 0; s < here; ++s) {
+        const int k = (s0 + s) * SEG;
+        const uint32_t bytes = (uint32_t)(min(SEG, K - k) * 4);
+        for (int r = 0; r < n_rows; ++r)
+          bulk_load(smem_u32(w_s + (s * ROWS + r) * SEG_PITCH), w + (long)(n0 + r) * ldw + k, bytes, bar);
+      }
+    }
+    if (!waited) {
+      pdl_wait();
+      waited = true;
+    }
+    if (!mbar_wait(bar, phase, error_flag, 910)) ok = false;
+    phase ^= 1;
+    for (int t0 = 0; t0 < M; t0 += pass_tokens) {
+      const int tok = t0 + tg * ROWS_TOKENS;
+      for (int s = seg_lane; s < here && tg < groups; s += lanes / ROWS) {
+        const int k0 = (s0 + s) * SEG, len = min(SEG, K - k0);
+        const float* wr = w_s + (s * ROWS + row) * SEG_PITCH;
+        const float* xr[ROWS_TOKENS];
+#pragma unroll
+        for (int e = 0; e < ROWS_TOKENS; ++e) xr[e] = x + (long)min(tok + e, M - 1) * ldx + k0;
+        float acc[ROWS_TOKENS] = {};
+        if (tok < M && row < n_rows) {
+#pragma unroll 4
+          for (int k = 0; k < len; k += 4) {
+            const float4 wv = *reinterpret_cast<const float4*>(wr + k);
+#pragma unroll
+            for (int e = 0; e < ROWS_TOKENS; ++e) {
+              const float4 xv = *reinterpret_cast<const float4*>(xr[e] + k);
+              acc[e] = fmaf(xv.x, wv.x, acc[e]);
+              acc[e] = fmaf(xv.y, wv.y, acc[e]);
+              acc[e] = fmaf(xv.z, wv.z, acc[e]);
+              acc[e] = fmaf(xv.w, wv.w, acc[e]);
+            }
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < ROWS_TOKENS; ++e) part[(s * pass_tokens + tg * ROWS_TOKENS + e) * ROWS + row] = acc[e];
+      }
+      __syncthreads();
+      // outputs of this pass: (token, row), their segments in ascending order
+#pragma unroll
+      for (int o = 0; o < ROWS_OUTPUTS; ++o) {
+        const int at = tid + o * n_threads;                           // place in [M][ROWS]
+        const int m = at / ROWS;
+        if (m >= t0 && m < min(M, t0 + pass_tokens))
+          for (int s = 0; s < here; ++s) total[o] = __fadd_rn(total[o], part[(s * pass_tokens + m - t0) * ROWS + at % ROWS]);
+      }
+      __syncthreads();
+    }
+    if (s0 + staged < n_seg) fence_reads_before_async_writes();
+    __syncthreads();
+  }
+  if (!ok) return;
+#pragma unroll
+  for (int o = 0; o < ROWS_OUTPUTS; ++o) {
+    const int at = tid + o * n_threads, m = at / ROWS, r = at % ROWS;
+    if (m < M && r < n_rows) put_output<float, MODE>(y, (long)m * ldy + n0 + r, n0 + r, total[o], bias, oscale);
+  }
+}
+
+// Which kernel: fp32 rows that 16-byte copies can take go to the two fast ones.  Up to ROWS_MAX_TOKENS tokens the rows kernel
+// (every row of w is read once and by one block), beyond the tiles.
+template <int MODE>
+int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const float* bias, const float* oscale, float* y, long ldy,
+                      int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by, int* error_flag) {
+  if (M <= ROWS_MAX_TOKENS) {
+    const int n_seg = (K + SEG - 1) / SEG;
+    const int staged = n_seg < MAX_STAGED ? n_seg : MAX_STAGED;
+    const int lanes = ROWS * (staged < 8 ? staged : 8);
+    int groups = (M + ROWS_TOKENS - 1) / ROWS_TOKENS;
+    if (groups > 256 / lanes) groups = 256 / lanes;
+    int threads = lanes * groups;
+    while (threads < 32) threads += lanes;         // at least a warp
+    const size_t smem = ((size_t)staged * ROWS * SEG_PITCH + (size_t)staged * (threads / lanes) * ROWS_TOKENS * ROWS) * sizeof(float);
+    static PerDevice<bool> configured;
+    if (!configured.here()) {
+      if (cudaFuncSetAttribute(linear_f32_rows_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+        return LLMI_ERR_LAUNCH;
+      configured.here() = true;
+    }
+    return launch_pdl(PDL_GEMM, linear_f32_rows_kernel<MODE>, dim3((N + ROWS - 1) / ROWS, 1, batch), dim3(threads), smem, stream, x, ldx, w,
+                      ldw, bias, oscale, y, ldy, M, N, K, staged, error_flag, bx, bw, by);
+  }
+  static PerDevice<bool> configured;
+  if (!configured.here()) {
+    if (cudaFuncSetAttribute(linear_f32_tile_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM) != cudaSuccess)
+      return LLMI_ERR_LAUNCH;
+    configured.here() = true;
+  }
+  linear_f32_tile_kernel<MODE><<<dim3((N + BN - 1) / BN, (M + BM - 1) / BM, batch), 256, TILE_SMEM, stream>>>(
+      x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by);
+  return launch_status();
+}
+
 template <typename T>
 int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale, void* y, long ldy, int M,
-                       int N, int K, int mode, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
+                       int N, int K, int mode, int* error_flag, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
   if (grid.y > 65535 || batch < 1 || batch > 65535) return LLMI_ERR_BAD_SIZE;
+  pairs_may_start_early = false;
+  const bool rows_of_16 = (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && ((ldx | ldw | bx | bw | (long)K) & 3) == 0;
+#define LLMI_LAUNCH(MODE)                                                                                                     \
+  if (sizeof(T) == 4 && rows_of_16)                                                                                           \
+    return launch_linear_f32<MODE>((const float*)x, ldx, (const float*)w, ldw, bias, oscale, (float*)y, ldy, M, N, K, stream, \
+                                   batch, bx, bw, by, error_flag);                                                            \
+  linear_simt_kernel<T, MODE><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by)
   switch (mode) {
-    case OUT_STORE:
-      linear_simt_kernel<T, OUT_STORE><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by);
-      break;
-    case OUT_STORE_F32:
-      linear_simt_kernel<T, OUT_STORE_F32><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by);
-      break;
-    case OUT_ADD_F32:
-      linear_simt_kernel<T, OUT_ADD_F32><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by);
-      break;
-    default:
-      return LLMI_ERR_UNSUPPORTED;
+    case OUT_STORE: LLMI_LAUNCH(OUT_STORE); break;
+    case OUT_STORE_F32: LLMI_LAUNCH(OUT_STORE_F32); break;
+    case OUT_ADD_F32: LLMI_LAUNCH(OUT_ADD_F32); break;
+    default: return LLMI_ERR_UNSUPPORTED;
   }
+#undef LLMI_LAUNCH
   return launch_status();
 }
 
@@ -125,13 +405,13 @@ int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const f
 using namespace llmi;
 
 // x [M, K] (row pitch ldx), w [N, K] (row pitch ldw), y [M, N] (row pitch ldy), pitches in elements; y takes
-// (x · wᵀ + bias) * oscale, both [N] or null.
+// (x · wᵀ + bias) * oscale, both [N] or null.  `error_flag` (null or a device int) takes the code of a bounded wait that gave up.
 LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale,
-                                 void* y, long ldy, int M, int N, int K, int mode, cudaStream_t stream) {
+                                 void* y, long ldy, int M, int N, int K, int mode, int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
-  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
+  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, error_flag, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, error_flag, stream);
   return LLMI_ERR_BAD_DTYPE;
 }
 
@@ -140,11 +420,11 @@ LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void*
 // Arithmetic and order of additions are those of llmi_linear_simt.
 LLMI_EXPORT int llmi_linear_simt_batched(int dtype, const void* x, long ldx, long bx, const void* w, long ldw, long bw,
                                          void* y, long ldy, long by, int batch, int M, int N, int K, int mode,
-                                         cudaStream_t stream) {
+                                         int* error_flag, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
   if (dtype == LLMI_DTYPE_F32)
-    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
+    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, error_flag, stream, batch, bx, bw, by);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, error_flag, stream, batch, bx, bw, by);
   return LLMI_ERR_BAD_DTYPE;
 }

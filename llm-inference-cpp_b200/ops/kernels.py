@@ -150,7 +150,7 @@ def lib():
     l = library.load()
     if not _configured:
         for name in ("llmi_embed", "llmi_rmsnorm", "llmi_swiglu", "llmi_linear_simt", "llmi_rope_store",
-                     "llmi_attention_generic", "llmi_argmax", "llmi_sample", "llmi_gemm_tc", "llmi_gemm_tc_splits",
+                     "llmi_attention_generic", "llmi_attention_f32", "llmi_attention_f32_supported", "llmi_argmax", "llmi_sample", "llmi_gemm_tc", "llmi_gemm_tc_splits",
                      "llmi_attention_decode", "llmi_attention_decode_supported", "llmi_attention_decode_resident",
                      "llmi_attention_decode_fused", "llmi_attention_decode_mma", "llmi_attention_decode_mma_supported",
                      "llmi_attention_decode_mma_resident", "llmi_attention_decode_clusters_resident",
@@ -300,7 +300,7 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch
         assert bias.dtype == torch.float32 and bias.numel() == N
     _check("linear_simt", lib().llmi_linear_simt(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), _ptr(w), c_long(w.stride(0)), _ptr(bias), _ptr(oscale), _ptr(out),
-        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
+        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), _ptr(tc_scratch(x.device).error), _stream()))
 
 
 class _TcScratch:
@@ -530,6 +530,31 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, tok_
         c_int(_dtype_code(q)), _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache),
         _ptr(v_cache), _ptr(tok_seq), _ptr(tok_pos), _ptr(seq_pages), c_int(seq_pages.stride(0)), c_int(page_size),
         c_int(T), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), _stream()))
+
+
+def attention_f32(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_pages, n_heads: int, n_kv_heads: int, head_dim: int,
+                  scale: float, window: int = 0) -> None:
+    """The same in the 32-bit path, for the sizes that :func:`attention_f32_applies` takes: a step's tokens by 32 queries and
+    head, a decode step by sequence and kv head with the pages side by side; both give the same bits for a position."""
+    _need_cuda(q, out, k_cache, v_cache, ctx.tok_seq, ctx.tok_pos, seq_pages)
+    T = q.shape[0]
+    assert q.dtype == out.dtype == k_cache.dtype == v_cache.dtype == torch.float32 and q.stride(1) == 1 and out.stride(1) == 1
+    assert out.shape == (T, n_heads * head_dim) and k_cache.is_contiguous() and v_cache.is_contiguous()
+    _check("attention_f32", lib().llmi_attention_f32(
+        _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(ctx.tok_seq),
+        _ptr(ctx.tok_pos), _ptr(seq_pages), c_int(seq_pages.stride(0)), c_int(k_cache.shape[-2]), _ptr(ctx.seq_q_start),
+        c_int(seq_pages.shape[0]), c_int(T), c_int(1 if ctx.decode else 0), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),
+        c_float(scale), c_int(window), _stream()))
+
+
+def attention_f32_applies(q: torch.Tensor, out: torch.Tensor, ctx, page_size: int, n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    """Whether a step's attention goes to :func:`attention_f32`: fp32, pages of 64, heads of whole 16-byte pieces up to 128 entries.
+    The answer is the same for a model's prompt and decode steps (so its positions are computed one way), but for a prompt step
+    padded to a shape, which the 32-bit path does not make."""
+    return bool(q.dtype == torch.float32 and page_size == 64 and not _FORCE_GENERIC_ATTENTION
+                and (ctx.decode or getattr(ctx, "host_q_lens", None) is not None) and (not ctx.decode or q.shape[0] <= 65535)
+                and q.stride(0) % 4 == 0 and out.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
+                and lib().llmi_attention_f32_supported(c_int(head_dim), c_int(n_heads // n_kv_heads)))
 
 
 def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
@@ -886,7 +911,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
     """Attention of a step's tokens over the cache; q is the first n_heads*head_dim columns of ``qkv``.
 
     In bf16, a decode step goes to the split kernel and a prompt step to the flash kernel when they
-    have the head size; everything else (the 32-bit path, other head sizes) goes to the generic kernel.
+    have the head size; the 32-bit path has kernels of its own (``attention_f32``); other head sizes go to the generic kernel.
     ``rope=(inv_freq, rotary_dim, write_kv)``: q, k are not rotated yet and k, v not appended — the kernel
     does it (only where :func:`attention_fuses_rotation` says so).
     """
@@ -927,6 +952,9 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             return
         attention_prefill(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, ctx.n_q_blocks,
                           n_heads, n_kv_heads, head_dim, scale, window)
+        return
+    if attention_f32_applies(qkv, out, ctx, page_size, n_heads, n_kv_heads, head_dim):
+        attention_f32(qkv, out, k_cache, v_cache, ctx, seq_pages, n_heads, n_kv_heads, head_dim, scale, window)
         return
     attention_generic(qkv, out, k_cache, v_cache, ctx.tok_seq, ctx.tok_pos, seq_pages, page_size, n_heads,
                       n_kv_heads, head_dim, scale, window)
@@ -1290,7 +1318,7 @@ def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor,
         return
     _check("linear_batched", lib().llmi_linear_simt_batched(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), c_long(bx), _ptr(w), c_long(K), c_long(N * K), _ptr(out),
-        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
+        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode), _ptr(tc_scratch(x.device).error), _stream()))
 
 
 # ---------------------------------------------------------------------------------------------

@@ -1,0 +1,124 @@
+"""The 32-bit path's product and attention at the edges of their tiles: against 64 bits, and bit for bit between the kernels
+that a call's size selects (a position must not depend on how many others are in the step) (GPU)."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def K():
+    from llmi_b200.ops import kernels
+    return kernels
+
+
+@pytest.mark.parametrize("N,K_", [(8, 4), (7, 256), (65, 260), (129, 576), (200, 1020), (71, 1028), (64, 2560), (9, 4100), (17, 8192)])
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 17, 64, 65, 130])
+def test_linear_f32_every_kernel_same_bits(M, N, K_):
+    k = K()
+    torch.manual_seed(M * 7 + N + K_)
+    x = torch.randn(M, K_ + 8, device="cuda")[:, :K_]
+    w, b, s = torch.randn(N, K_, device="cuda") / K_ ** 0.5, torch.randn(N, device="cuda"), torch.rand(N, device="cuda") + 0.5
+    y = torch.full((M, N + 3), 7.0, device="cuda")
+    k.linear_simt(x, w, y[:, :N], b, k.OUT_STORE, s)
+    ref = (x.double() @ w.double().T + b.double()) * s.double()
+    # a chain of 256 additions and one of K / 256: (256 + K / 256 + 2) roundings of 6e-8 of the terms' root sum of squares, at most
+    bound = 6e-8 * (258 + K_ / 256) * float((x.double().abs() @ w.double().abs().T).max()) * 1.5
+    assert float((y[:, :N].double() - ref).abs().max()) < bound
+    assert float((y[:, :N].double() - ref).norm() / ref.norm()) < 1e-6
+    assert bool((y[:, N:] == 7.0).all())
+    # the same rows one by one, and through the kernel that takes any alignment
+    one = torch.empty(1, N, device="cuda")
+    for r in {0, M // 2, M - 1}:
+        k.linear_simt(x[r:r + 1], w, one, b, k.OUT_STORE, s)
+        assert torch.equal(one, y[r:r + 1, :N])
+    odd = torch.empty(M * (K_ + 5) + 1, device="cuda")[1:].view(M, K_ + 5)[:, :K_]
+    odd.copy_(x)
+    z = torch.empty(M, N, device="cuda")
+    k.linear_simt(odd, w, z, b, k.OUT_STORE, s)
+    assert torch.equal(z, y[:, :N])
+    acc = torch.randn(M, N, device="cuda")
+    both = acc.clone()
+    k.linear_simt(x, w, acc, None, k.OUT_ADD_F32)
+    k.linear_simt(odd, w, both, None, k.OUT_ADD_F32)
+    assert torch.equal(acc, both)
+    k.check_device_errors("cuda:0")
+
+
+def test_linear_f32_batched_same_bits():
+    k = K()
+    for M in (2, 70):
+        x, w = torch.randn(M, 3 * 300, device="cuda"), torch.randn(3, 50, 300, device="cuda")
+        out = torch.empty(M, 150, device="cuda")
+        k.linear_batched(x, 300, w, out, 50, 300)
+        for b in range(3):
+            one = torch.empty(M, 50, device="cuda")
+            k.linear_simt(x[:, 300 * b:300 * b + 300], w[b], one)
+            assert torch.equal(out[:, 50 * b:50 * b + 50], one)
+    k.check_device_errors("cuda:0")
+
+
+def _context(q_lens, kv_lens, decode):
+    lens = torch.tensor(q_lens)
+    start = torch.cat([torch.zeros(1, dtype=torch.long), lens.cumsum(0)])
+    seq = torch.repeat_interleave(torch.arange(len(q_lens)), lens)
+    pos = torch.cat([torch.arange(k - q, k) for q, k in zip(q_lens, kv_lens)])
+    i32 = lambda t: t.to(torch.int32).cuda()      # noqa: E731
+    return types.SimpleNamespace(decode=decode, host_q_lens=list(q_lens), host_kv_lens=list(kv_lens), tok_seq=i32(seq), tok_pos=i32(pos),
+                                 seq_q_start=i32(start), seq_kv_len=i32(torch.tensor(kv_lens)))
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(3, 1, 64), (4, 4, 64), (6, 2, 36), (8, 2, 128), (10, 2, 8), (2, 2, 100)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_f32_prompt_and_decode(nh, nkv, hd, window):
+    """Prompts of unequal lengths on top of what is there, against 64 bits; every query alone as a decode step gives the same bits.
+    What no query sees is NaN."""
+    k = K()
+    torch.manual_seed(nh * hd + window)
+    q_lens, kv_lens = [1, 31, 32, 33, 70, 64], [1, 31, 96, 700, 70, 65]
+    ctx = _context(q_lens, kv_lens, False)
+    T, scale = sum(q_lens), hd ** -0.5
+    P = max((n + 63) // 64 for n in kv_lens)
+    pages = torch.full((len(q_lens), P), -1, dtype=torch.int32)
+    order = torch.randperm(64)
+    kc = torch.full((64, nkv, 64, hd), float("nan"), device="cuda")
+    vc = kc.clone()
+    n = 0
+    refs = []
+    q = torch.randn(T, nh * hd + 4, device="cuda")[:, :nh * hd]
+    at = 0
+    for i, (ql, kl) in enumerate(zip(q_lens, kv_lens)):
+        keys, vals = torch.randn(kl, nkv, hd, device="cuda") * 2, torch.randn(kl, nkv, hd, device="cuda")
+        for p in range((kl + 63) // 64):
+            pages[i, p] = order[n]
+            rows = slice(64 * p, min(kl, 64 * p + 64))
+            kc[order[n], :, :rows.stop - rows.start] = keys[rows].transpose(0, 1)
+            vc[order[n], :, :rows.stop - rows.start] = vals[rows].transpose(0, 1)
+            n += 1
+        qi = q[at:at + ql].double().view(ql, nh, hd)
+        s = torch.einsum("qhd,khd->hqk", qi, keys.double().repeat_interleave(nh // nkv, 1)) * scale
+        qp, kp = torch.arange(kl - ql, kl, device="cuda")[:, None], torch.arange(kl, device="cuda")[None]
+        s.masked_fill_((kp > qp) | ((kp <= qp - window) if window else torch.zeros_like(kp > qp)), -float("inf"))
+        refs.append(torch.einsum("hqk,khd->qhd", s.softmax(-1), vals.double().repeat_interleave(nh // nkv, 1)).reshape(ql, -1))
+        at += ql
+    pages = pages.cuda()
+    out = torch.full((T, nh * hd), 7.0, device="cuda")
+    assert k.attention_f32_applies(q, out, ctx, 64, nh, nkv, hd)
+    k.attention(q, out, kc, vc, ctx, pages, 64, nh, nkv, hd, scale, window)
+    ref = torch.cat(refs)
+    assert float((out.double() - ref).norm() / ref.norm()) < 1e-6
+    # token j of every sequence that has one, as a decode step, with a padding row between
+    for j in (0, 17, 31, 32, 69):
+        who = [i for i, ql in enumerate(q_lens) if ql > j]
+        if not who:
+            continue
+        rows = [sum(q_lens[:i]) + j for i in who]
+        one = _context([1] * len(who), [kv_lens[i] - q_lens[i] + j + 1 for i in who], True)
+        one.tok_seq = torch.cat([one.tok_seq, torch.tensor([-1], dtype=torch.int32, device="cuda")])
+        one.tok_pos = torch.cat([one.tok_pos, torch.tensor([0], dtype=torch.int32, device="cuda")])
+        qd = torch.cat([q[rows], q[:1]]).contiguous()
+        got = torch.full((len(who) + 1, nh * hd), 7.0, device="cuda")
+        k.attention(qd, got, kc, vc, one, pages[who].contiguous(), 64, nh, nkv, hd, scale, window)
+        assert torch.equal(got[:-1], out[rows]) and bool((got[-1] == 0).all())
+    k.check_device_errors("cuda:0")
