@@ -22,6 +22,16 @@ import torch
 from ..cache.pages import CacheError, pages_for
 
 
+# Most tokens that a sequence of a prompt step brings, as the launches of the attention of short messages know it: what a
+# recorded prompt step's launches may depend on beside its padded shape
+SHORT_MESSAGES = (4, 8, 16, 32, 48, 64)
+
+
+def short_message(max_q_len: int) -> int:
+    """The entry of SHORT_MESSAGES that covers ``max_q_len``, 0 if none does."""
+    return next((n for n in SHORT_MESSAGES if max_q_len <= n), 0)
+
+
 class StepError(ValueError):
     pass
 
@@ -229,6 +239,7 @@ def plan_step(cache, seqs, vocab_size: int, buffers: StepBuffers, pad_seqs_to: i
     ctx.n_q_blocks = (n_tokens // 128 + n_seqs) if pad_prompt else sum((n + 127) // 128 for n in lens)
     # for kernels that plan on the host (a padded step's launches must not depend on its lengths)
     ctx.host_q_lens, ctx.host_kv_lens = (None, None) if (decode or pad_prompt) else (list(lens), list(kv_lens))
+    ctx.short_message = 0 if decode else short_message(ctx.max_q_len)
     ctx.h2d_bytes = cur * 4
 
     def view(name):

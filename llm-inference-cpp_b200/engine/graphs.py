@@ -224,6 +224,7 @@ class PromptGraphs:
         P = max(need_pages, min(bucket(need_pages), cache.max_pages_per_seq))
         ctx = plan_step(cache, seqs, m.spec.vocab_size, m.buffers, pad_seqs_to=S, pad_pages_to=P, pad_tokens_to=T, pad_want_to=W)
         m._last_h2d = ctx.h2d_bytes
+        P = (P, ctx.short_message)                  # (the attention's launches follow both)
         key = self._key(T, S, W, P, cache)
         entry = self.graphs.get(key)
         if entry is not None:

@@ -155,7 +155,8 @@ def lib():
                      "llmi_attention_decode_fused", "llmi_attention_decode_mma", "llmi_attention_decode_mma_supported",
                      "llmi_attention_decode_mma_resident", "llmi_attention_decode_clusters_resident",
                      "llmi_attention_prefill", "llmi_attention_prefill_supported", "llmi_gemm_skinny",
-                     "llmi_gemm_skinny_max_tokens", "llmi_attention_prefill_tc", "llmi_attention_prefill_tc_supported",
+                     "llmi_gemm_skinny_max_tokens", "llmi_attention_prefill_tc", "llmi_attention_prefill_tc_supported", "llmi_attention_short",
+                     "llmi_attention_short_supported",
                      "llmi_sm_count", "llmi_dyt", "llmi_dyt_add", "llmi_stream_add", "llmi_linear_simt_batched",
                      "llmi_latent_prepare", "llmi_latent_q_rotate", "llmi_attention_latent", "llmi_delta_prepare",
                      "llmi_delta_conv_carry", "llmi_delta_recurrence", "llmi_delta_finish", "llmi_moe_route", "llmi_moe_up",
@@ -862,6 +863,40 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, s
         _addr(gate), gate.stride(0) if gate is not None else 0, _addr(r1), _addr(r2), _addr(sink), _stream_int()))
 
 
+def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int) -> int:
+    """Blocks of a cluster that share the pages of a (sequence, kv head, row tile) in attention_short, or 0 where the prompt
+    kernel of 128-query tiles (attention_prefill_tc) is the faster one.
+
+    Both read a page per tile and head; a tile of 64 rows costs 1.17 times one of 128 queries (measured at 8 x 32
+    sequence-heads of 3,900 positions: 89 against 76 us), but covers all the group's heads at once; up to 32 rows 0.8 times
+    (61 us).  With few pages both are all start-up, and the prompt kernel's single block per head wins earlier (32
+    sequence-heads of 300 positions, heads of 128 in groups of 4, 32 tokens: 20.5 against 18.5 us).
+    A cluster is worth its barriers only while SMs are idle: 256 items 59 us alone, 66 in fours; 40 items of 2,000
+    positions 43 alone, 20.5 in eights; 160 items 45 alone, 37 in pairs, 41 in fours."""
+    rows = max_q * group
+    tiles = -(-rows // 64)
+    if rows > 32 and 1.17 * tiles >= group * (1.0 if n_pages > 8 else 0.55):
+        return 0
+    items, parts = n_seqs * n_kv_heads * tiles, 1
+    while parts < 8 and 2 * items * parts <= 2.2 * sm_count() and 2 * n_pages >= 3 * parts:
+        parts *= 2
+    return parts
+
+
+def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
+                    n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1) -> None:
+    """Causal attention of at most ``max_q`` tokens a sequence over its cache pages (bf16, head size 64 or 128, page 64):
+    arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head."""
+    _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)
+    assert q.dtype == out.dtype == k_cache.dtype == torch.bfloat16 and q.stride(1) == 1 and out.stride(1) == 1
+    assert k_cache.shape[-2] == 64 and k_cache.is_contiguous() and v_cache.is_contiguous()
+    _check("attention_short", lib().llmi_attention_short(
+        _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache), _ptr(v_cache), c_long(k_cache.shape[0]),
+        _ptr(seq_pages), c_int(seq_pages.stride(0)), _ptr(seq_q_start), _ptr(seq_kv_len), c_int(seq_pages.shape[0]), c_int(max_q),
+        c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), c_int(parts),
+        _ptr(tc_scratch(q.device).error), _stream()))
+
+
 # Which prompt-attention kernel runs: "tc" (tcgen05: about 43 us for a 2,048-token prompt of 32 heads of 64) or
 # "mma" (mma.sync: 95 us).
 _PREFILL_ATTENTION = os.environ.get("LLMI_PREFILL_ATTENTION", "tc")     # "mma": the mma.sync kernel for every head size
@@ -940,6 +975,13 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             # longest job: then the key ranges are cut (see the kernel's head).  Measured: 2,048 tokens x 8 heads 28.0 ->
             # 22.2 us, x 4 heads 27.5 -> 21.0 us; with 256 jobs and more the cut gains nothing or costs (4,096 x 8:
             # 49.3 -> 50.5 us; 2,048 x 32: 42.1 -> 49.6 us).
+            max_q = getattr(ctx, "short_message", 0)
+            parts = attention_short_parts(seq_pages.shape[0], n_kv_heads, max_q, n_heads // n_kv_heads,
+                                          seq_pages.shape[1]) if max_q else 0
+            if parts:
+                attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, max_q, n_heads, n_kv_heads,
+                                head_dim, scale, window, parts)
+                return
             split = None
             q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)
             if _PREFILL_SPLIT and rt is not None and q_lens is not None and ctx.n_q_blocks * n_heads < sm_count():
