@@ -125,7 +125,9 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Many tokens.  Bound by the FMA pipes (128 a clock and SM).  A block makes a tile of 64 x 64 outputs; its four groups of 64
+// Many tokens.  Bound by the FMA pipes (128 a clock and SM; 74 TFLOP/s, of which 8 x 8 products out of registers alone reach
+// 55).  800 tokens x 960 -> 5,120: 252 us, 31 TFLOP/s: a block takes 30 us for its 4 segments and the last of 7.03 waves is
+// nearly empty.  (Two blocks of half the stages on an SM: 282 us.)  A block makes a tile of 64 x 64 outputs; its four groups of 64
 // threads take segments 4r, 4r + 1, .. of round r, each thread 8 x 8 outputs in registers (two 16-byte shared loads per 16
 // FMAs where 4 x 4 outputs need four).  With the segments side by side a block keeps four warps' worth of independent chains
 // on every scheduler though its tile is small, and small tiles fill the 148 SMs at the widths of small models (600 tokens x
@@ -234,138 +236,137 @@ linear_f32_tile_kernel(const float* __restrict__ x, long ldx, const float* __res
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Few tokens.  Bound by reading w once, and by latency: a decode step of a small model is a chain of such products.  A block
-// takes ROWS rows of w; every (row, segment) is a bulk copy of at most 1 KB into a place 260 floats from the next (16-byte
-// shared loads of a quarter warp's eight rows touch 32 different banks), all of them asked for at once and before the kernel
-// before has ended (w does not depend on it).  A thread makes the segment sums of one (row, segment) for four tokens: a chain
-// of 256 FMAs is 1,024 clocks, half a microsecond, whatever K is, where one chain over K = 2,560 is 5 us.  x comes through L1
-// (the lanes of a warp share a handful of addresses).
+// takes ROWS rows of w; rows and tokens go to shared memory in segments of 256 places (places 260 floats apart: a quarter
+// warp's 16-byte loads of its four rows touch different banks), w before the kernel before has ended (it does not depend on
+// it).  A thread makes the sums of one segment for two rows and two (or four) tokens: 4 (6) shared loads of 16 bytes per 16
+// (32) FMAs, which is what a block spends its time on: with one row a thread it is 1.5 (1.7) times as many.  A chain of 256
+// FMAs is 1,024 clocks, half a microsecond, whatever K is, where one chain over K = 2,560 is 5 us.
+// Four tokens, as they follow one another in a step (rows of w x K): 960 x 960 22.3 -> 6.0 us, 5,120 x 960 23.4 -> 11.3, 960 x
+// 2,560 41.9 -> 7.1 against the form whose threads had one row, four tokens and x through L1.
 constexpr int ROWS = 8;
 constexpr int SEG_PITCH = SEG + 4;
-constexpr int MAX_STAGED = 16;        // segments of a row in shared memory at a time (16 x 8 rows: 133 KB)
-constexpr int ROWS_TOKENS = 4;        // tokens a thread takes at a time
+constexpr int ROWS_PASS = 16;         // tokens in shared memory at a time
 constexpr int ROWS_MAX_TOKENS = 64;
-constexpr int ROWS_OUTPUTS = 4;       // outputs a thread ends with: there are at least 2 M threads, or 193 of the 8 x 64 outputs
+constexpr int ROWS_THREADS = 128;     // at least: an output of a pass per thread
 
-template <int MODE>
-__global__ void __launch_bounds__(256)
+template <int MODE, int TOKENS>
+__global__ void __launch_bounds__(512)
 linear_f32_rows_kernel(const float* __restrict__ x, long ldx, const float* __restrict__ w, long ldw, const float* __restrict__ bias,
-                       const float* __restrict__ oscale, float* __restrict__ y, long ldy, int M, int N, int K, int staged, int* error_flag,
+                       const float* __restrict__ oscale, float* __restrict__ y, long ldy, int M, int N, int K, int staged, int pass,
                        long bx, long bw, long by) {
   extern __shared__ __align__(16) float rows_smem[];
-  __shared__ __align__(8) uint64_t bar_store;
   x += (long)blockIdx.z * bx;
   w += (long)blockIdx.z * bw;
   y += (long)blockIdx.z * by;
   float* w_s = rows_smem;                                             // [staged][ROWS][SEG_PITCH]
-  float* part = w_s + staged * ROWS * SEG_PITCH;                      // [staged][token of the pass][ROWS]
-  const uint32_t bar = smem_u32(&bar_store);
+  float* x_s = w_s + staged * ROWS * SEG_PITCH;                       // [staged][pass][SEG_PITCH]
+  float* part = x_s + staged * pass * SEG_PITCH;                      // [staged][pass][ROWS]
   const int tid = threadIdx.x, n_threads = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, n_warps = n_threads >> 5;
   const int n0 = blockIdx.x * ROWS, n_rows = min(ROWS, N - n0);
   const int n_seg = (K + SEG - 1) / SEG;
-  const int lanes = ROWS * min(staged, 8);                            // threads that share a group of tokens
-  const int groups = n_threads / lanes;                               // groups of tokens at a time
-  const int tg = tid / lanes, row = tid % ROWS, seg_lane = (tid % lanes) / ROWS;
-  const int pass_tokens = groups * ROWS_TOKENS;
-  if (tid == 0) {
-    mbar_init(bar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
+  const int groups = pass / TOKENS;                                   // groups of tokens of a pass
+  const int row = tid & 3, tg = (tid >> 2) % groups, seg_lane = (tid >> 2) / groups;      // rows `row` and `row` + 4
+  const int seg_lanes = (n_threads >> 2) / groups;
   pdl_launch_dependents();
-  uint32_t phase = 0;
-  bool waited = false, ok = true;
-  float total[ROWS_OUTPUTS];                                          // outputs of this thread over the rounds
-#pragma unroll
-  for (int o = 0; o < ROWS_OUTPUTS; ++o) total[o] = 0.f;
+  bool waited = false;
+  float total[ROWS_MAX_TOKENS / ROWS_PASS] = {};                      // this thread's output of every pass, over the rounds
 
   for (int s0 = 0; s0 < n_seg; s0 += staged) {
     const int here = min(staged, n_seg - s0);
-    if (tid == 0) {                                                   // one thread asks: at most 128 copies
-      const long k_bytes = (long)(min(K, (s0 + here) * SEG) - s0 * SEG) * 4;
-      mbar_expect_tx(bar, (uint32_t)(k_bytes * n_rows));
-      for (int s = 0; s < here; ++s) {
-        const int k = (s0 + s) * SEG;
-        const uint32_t bytes = (uint32_t)(min(SEG, K - k) * 4);
-        for (int r = 0; r < n_rows; ++r)
-          bulk_load(smem_u32(w_s + (s * ROWS + r) * SEG_PITCH), w + (long)(n0 + r) * ldw + k, bytes, bar);
-      }
+    const int k0 = s0 * SEG, pieces = (min(K, (s0 + here) * SEG) - k0) / 4;      // pieces of 16 bytes of a row
+    // (rows that do not exist repeat the last one: their sums go nowhere)
+    for (int r = warp; r < ROWS; r += n_warps) {
+      const float* src = w + (long)(n0 + min(r, n_rows - 1)) * ldw + k0;
+      for (int q = lane; q < pieces; q += 32) cp_async_16(w_s + ((q / (SEG / 4)) * ROWS + r) * SEG_PITCH + (q % (SEG / 4)) * 4, src + 4 * q, true);
     }
     if (!waited) {
       pdl_wait();
       waited = true;
     }
-    if (!mbar_wait(bar, phase, error_flag, 910)) ok = false;
-    phase ^= 1;
-    for (int t0 = 0; t0 < M; t0 += pass_tokens) {
-      const int tok = t0 + tg * ROWS_TOKENS;
-      for (int s = seg_lane; s < here && tg < groups; s += lanes / ROWS) {
-        const int k0 = (s0 + s) * SEG, len = min(SEG, K - k0);
+#pragma unroll
+    for (int turn = 0; turn < ROWS_MAX_TOKENS / ROWS_PASS; ++turn) {
+      const int t0 = turn * pass;
+      if (t0 >= M) break;
+      for (int m = warp; m < pass; m += n_warps) {
+        const float* src = x + (long)min(t0 + m, M - 1) * ldx + k0;
+        for (int q = lane; q < pieces; q += 32) cp_async_16(x_s + ((q / (SEG / 4)) * pass + m) * SEG_PITCH + (q % (SEG / 4)) * 4, src + 4 * q, true);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      for (int s = seg_lane; s < here; s += seg_lanes) {
+        const int len = min(SEG, K - k0 - s * SEG);
         const float* wr = w_s + (s * ROWS + row) * SEG_PITCH;
-        const float* xr[ROWS_TOKENS];
-#pragma unroll
-        for (int e = 0; e < ROWS_TOKENS; ++e) xr[e] = x + (long)min(tok + e, M - 1) * ldx + k0;
-        float acc[ROWS_TOKENS] = {};
-        if (tok < M && row < n_rows) {
+        const float* xr = x_s + (s * pass + tg * TOKENS) * SEG_PITCH;
+        float acc[2][TOKENS] = {};
 #pragma unroll 4
-          for (int k = 0; k < len; k += 4) {
-            const float4 wv = *reinterpret_cast<const float4*>(wr + k);
+        for (int k = 0; k < len; k += 4) {
+          const float4 w0 = *reinterpret_cast<const float4*>(wr + k), w1 = *reinterpret_cast<const float4*>(wr + 4 * SEG_PITCH + k);
 #pragma unroll
-            for (int e = 0; e < ROWS_TOKENS; ++e) {
-              const float4 xv = *reinterpret_cast<const float4*>(xr[e] + k);
-              acc[e] = fmaf(xv.x, wv.x, acc[e]);
-              acc[e] = fmaf(xv.y, wv.y, acc[e]);
-              acc[e] = fmaf(xv.z, wv.z, acc[e]);
-              acc[e] = fmaf(xv.w, wv.w, acc[e]);
-            }
+          for (int e = 0; e < TOKENS; ++e) {
+            const float4 xv = *reinterpret_cast<const float4*>(xr + e * SEG_PITCH + k);
+            acc[0][e] = fmaf(xv.x, w0.x, acc[0][e]);
+            acc[1][e] = fmaf(xv.x, w1.x, acc[1][e]);
+            acc[0][e] = fmaf(xv.y, w0.y, acc[0][e]);
+            acc[1][e] = fmaf(xv.y, w1.y, acc[1][e]);
+            acc[0][e] = fmaf(xv.z, w0.z, acc[0][e]);
+            acc[1][e] = fmaf(xv.z, w1.z, acc[1][e]);
+            acc[0][e] = fmaf(xv.w, w0.w, acc[0][e]);
+            acc[1][e] = fmaf(xv.w, w1.w, acc[1][e]);
           }
         }
 #pragma unroll
-        for (int e = 0; e < ROWS_TOKENS; ++e) part[(s * pass_tokens + tg * ROWS_TOKENS + e) * ROWS + row] = acc[e];
+        for (int e = 0; e < TOKENS; ++e) {
+          part[(s * pass + tg * TOKENS + e) * ROWS + row] = acc[0][e];
+          part[(s * pass + tg * TOKENS + e) * ROWS + row + 4] = acc[1][e];
+        }
       }
       __syncthreads();
-      // outputs of this pass: (token, row), their segments in ascending order
-#pragma unroll
-      for (int o = 0; o < ROWS_OUTPUTS; ++o) {
-        const int at = tid + o * n_threads;                           // place in [M][ROWS]
-        const int m = at / ROWS;
-        if (m >= t0 && m < min(M, t0 + pass_tokens))
-          for (int s = 0; s < here; ++s) total[o] = __fadd_rn(total[o], part[(s * pass_tokens + m - t0) * ROWS + at % ROWS]);
-      }
-      __syncthreads();
+      // this pass's outputs (token, row), a thread each: their segments in ascending order
+      if (tid < pass * ROWS)
+        for (int s = 0; s < here; ++s) total[turn] = __fadd_rn(total[turn], part[s * pass * ROWS + tid]);
     }
-    if (s0 + staged < n_seg) fence_reads_before_async_writes();
     __syncthreads();
   }
-  if (!ok) return;
 #pragma unroll
-  for (int o = 0; o < ROWS_OUTPUTS; ++o) {
-    const int at = tid + o * n_threads, m = at / ROWS, r = at % ROWS;
-    if (m < M && r < n_rows) put_output<float, MODE>(y, (long)m * ldy + n0 + r, n0 + r, total[o], bias, oscale);
+  for (int turn = 0; turn < ROWS_MAX_TOKENS / ROWS_PASS; ++turn) {
+    const int m = turn * pass + tid / ROWS, r = tid % ROWS;
+    if (tid < pass * ROWS && m < M && r < n_rows) put_output<float, MODE>(y, (long)m * ldy + n0 + r, n0 + r, total[turn], bias, oscale);
   }
 }
 
-// Which kernel: fp32 rows that 16-byte copies can take go to the two fast ones.  Up to ROWS_MAX_TOKENS tokens the rows kernel
-// (every row of w is read once and by one block), beyond the tiles.
+template <int MODE, int TOKENS>
+int launch_linear_f32_rows(const float* x, long ldx, const float* w, long ldw, const float* bias, const float* oscale, float* y, long ldy,
+                           int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by) {
+  static PerDevice<bool> configured;
+  if (!configured.here()) {
+    if (cudaFuncSetAttribute(linear_f32_rows_kernel<MODE, TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+      return LLMI_ERR_LAUNCH;
+    configured.here() = true;
+  }
+  const int pass = M >= ROWS_PASS ? ROWS_PASS : (M + TOKENS - 1) / TOKENS * TOKENS;
+  const int n_seg = (K + SEG - 1) / SEG, blocks = (N + ROWS - 1) / ROWS;
+  // as many segments at a time as shared memory takes, in rounds of equal size: all of it where every block has an SM of
+  // its own, else half, so that one block loads while another multiplies
+  const int seg_bytes = ((ROWS + pass) * SEG_PITCH + pass * ROWS) * (int)sizeof(float);
+  const int most = ((long)blocks * batch <= sm_count() ? 216 : 108) * 1024 / seg_bytes;
+  const int rounds = (n_seg + most - 1) / most, staged = (n_seg + rounds - 1) / rounds;
+  int threads = 4 * (pass / TOKENS) * staged;
+  threads = threads < ROWS_THREADS ? ROWS_THREADS : (threads > 512 ? 512 : (threads + 31) / 32 * 32);
+  return launch_pdl(PDL_GEMM, linear_f32_rows_kernel<MODE, TOKENS>, dim3(blocks, 1, batch), dim3(threads), (size_t)staged * seg_bytes, stream,
+                    x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, staged, pass, bx, bw, by);
+}
+
+// Which kernel: fp32 rows that 16-byte copies can take go to the two fast ones.  Up to 8 tokens the rows kernel; up to 64 while
+// the outputs are so few that the tiles leave SMs idle (rows / tiles: 64 x 1,600 of K = 960: 28.7 / 33.5 us, 64 x 960 of
+// K = 2,560: 45 / 83, 32 x 3,072 of K = 576: 15.7 / 21.9; 48 x 3,072: 21.8 / 22.2, 24 x 5,120 of K = 960: 42 / 32).
+constexpr long ROWS_MAX_OUTPUTS = 104 * 1024;
 template <int MODE>
 int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const float* bias, const float* oscale, float* y, long ldy,
-                      int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by, int* error_flag) {
-  if (M <= ROWS_MAX_TOKENS) {
-    const int n_seg = (K + SEG - 1) / SEG;
-    const int staged = n_seg < MAX_STAGED ? n_seg : MAX_STAGED;
-    const int lanes = ROWS * (staged < 8 ? staged : 8);
-    int groups = (M + ROWS_TOKENS - 1) / ROWS_TOKENS;
-    if (groups > 256 / lanes) groups = 256 / lanes;
-    int threads = lanes * groups;
-    while (threads < 32) threads += lanes;         // at least a warp
-    const size_t smem = ((size_t)staged * ROWS * SEG_PITCH + (size_t)staged * (threads / lanes) * ROWS_TOKENS * ROWS) * sizeof(float);
-    static PerDevice<bool> configured;
-    if (!configured.here()) {
-      if (cudaFuncSetAttribute(linear_f32_rows_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
-        return LLMI_ERR_LAUNCH;
-      configured.here() = true;
-    }
-    return launch_pdl(PDL_GEMM, linear_f32_rows_kernel<MODE>, dim3((N + ROWS - 1) / ROWS, 1, batch), dim3(threads), smem, stream, x, ldx, w,
-                      ldw, bias, oscale, y, ldy, M, N, K, staged, error_flag, bx, bw, by);
+                      int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by) {
+  if (M <= 8 || (M <= ROWS_MAX_TOKENS && (long)M * N * batch <= ROWS_MAX_OUTPUTS)) {
+    if (M <= 8) return launch_linear_f32_rows<MODE, 2>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, stream, batch, bx, bw, by);
+    return launch_linear_f32_rows<MODE, 4>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, stream, batch, bx, bw, by);
   }
   static PerDevice<bool> configured;
   if (!configured.here()) {
@@ -380,7 +381,7 @@ int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const 
 
 template <typename T>
 int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale, void* y, long ldy, int M,
-                       int N, int K, int mode, int* error_flag, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
+                       int N, int K, int mode, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
   if (grid.y > 65535 || batch < 1 || batch > 65535) return LLMI_ERR_BAD_SIZE;
   pairs_may_start_early = false;
@@ -388,7 +389,7 @@ int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const f
 #define LLMI_LAUNCH(MODE)                                                                                                     \
   if (sizeof(T) == 4 && rows_of_16)                                                                                           \
     return launch_linear_f32<MODE>((const float*)x, ldx, (const float*)w, ldw, bias, oscale, (float*)y, ldy, M, N, K, stream, \
-                                   batch, bx, bw, by, error_flag);                                                            \
+                                   batch, bx, bw, by);                                                                        \
   linear_simt_kernel<T, MODE><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by)
   switch (mode) {
     case OUT_STORE: LLMI_LAUNCH(OUT_STORE); break;
@@ -405,13 +406,13 @@ int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const f
 using namespace llmi;
 
 // x [M, K] (row pitch ldx), w [N, K] (row pitch ldw), y [M, N] (row pitch ldy), pitches in elements; y takes
-// (x · wᵀ + bias) * oscale, both [N] or null.  `error_flag` (null or a device int) takes the code of a bounded wait that gave up.
+// (x · wᵀ + bias) * oscale, both [N] or null.
 LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale,
-                                 void* y, long ldy, int M, int N, int K, int mode, int* error_flag, cudaStream_t stream) {
+                                 void* y, long ldy, int M, int N, int K, int mode, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
-  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, error_flag, stream);
+  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, error_flag, stream);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
   return LLMI_ERR_BAD_DTYPE;
 }
 
@@ -420,11 +421,11 @@ LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void*
 // Arithmetic and order of additions are those of llmi_linear_simt.
 LLMI_EXPORT int llmi_linear_simt_batched(int dtype, const void* x, long ldx, long bx, const void* w, long ldw, long bw,
                                          void* y, long ldy, long by, int batch, int M, int N, int K, int mode,
-                                         int* error_flag, cudaStream_t stream) {
+                                         cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
   if (dtype == LLMI_DTYPE_F32)
-    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, error_flag, stream, batch, bx, bw, by);
+    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, error_flag, stream, batch, bx, bw, by);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
   return LLMI_ERR_BAD_DTYPE;
 }

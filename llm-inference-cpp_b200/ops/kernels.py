@@ -301,7 +301,7 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch
         assert bias.dtype == torch.float32 and bias.numel() == N
     _check("linear_simt", lib().llmi_linear_simt(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), _ptr(w), c_long(w.stride(0)), _ptr(bias), _ptr(oscale), _ptr(out),
-        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), _ptr(tc_scratch(x.device).error), _stream()))
+        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
 
 
 class _TcScratch:
@@ -1360,7 +1360,7 @@ def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor,
         return
     _check("linear_batched", lib().llmi_linear_simt_batched(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), c_long(bx), _ptr(w), c_long(K), c_long(N * K), _ptr(out),
-        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode), _ptr(tc_scratch(x.device).error), _stream()))
+        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
 
 
 # ---------------------------------------------------------------------------------------------

@@ -13,8 +13,8 @@ def K():
     return kernels
 
 
-@pytest.mark.parametrize("N,K_", [(8, 4), (7, 256), (65, 260), (129, 576), (200, 1020), (71, 1028), (64, 2560), (9, 4100), (17, 8192)])
-@pytest.mark.parametrize("M", [1, 3, 4, 5, 17, 64, 65, 130])
+@pytest.mark.parametrize("N,K_", [(8, 4), (2000, 520), (7, 256), (65, 260), (129, 576), (200, 1020), (71, 1028), (64, 2560), (9, 4100), (17, 8192)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 15, 17, 33, 64, 65, 130])
 def test_linear_f32_every_kernel_same_bits(M, N, K_):
     k = K()
     torch.manual_seed(M * 7 + N + K_)
