@@ -10,7 +10,8 @@ Per token the layer computes, from its input h:
 
 Only [c | r] is cached: one row of kv_rank + rot_dim entries per token (a key-only cache group with one head).  The
 expansions are folded into the query and the output, (Uk_hᵀ q_plain) . c and Uv_h (Σ p c), so that attention runs over
-the cached rows directly, the same way for a prompt and for a single token.  Norms, scores, softmax and the rotation's
+the cached rows directly; a prompt of many tokens multiplies the rows out into keys and values instead, which its queries
+share (``kernels.latent_expanded_pages`` says which step does).  Norms, scores, softmax and the rotation's
 angles are fp32; the rotation turns the first ``rot_dims`` entries of the rotated part, pair i by the angle
 pos * base^(-2i/dims): neighbouring entries (2i, 2i+1) (``pairing`` 1) or entries (i, i + dims/2) (``pairing`` 0) — or as a
 position part says (its frequencies, pairing and amplitude).  With a
@@ -84,6 +85,11 @@ class LatentAttention:
         self.w_uk_t = rt.to_compute(tensors["uk"].reshape(self.H, self.D, self.C).transpose(1, 2).contiguous())
         self.w_uv = rt.to_compute(tensors["uv"].reshape(self.H, self.Dv, self.C).contiguous())
         self.w_o = rt.to_compute(tensors["o"])
+        # prompts multiply the rows out into keys and values where that kernel takes the sizes: per head [Uk_h; Uv_h]
+        self.w_kv = None
+        if self.Q and not self.window and kernels.attention_expanded_supported(rt, self.D, self.Dv, self.R, self.C, self.scale):
+            self.w_kv = rt.to_compute(torch.cat([tensors["uk"].reshape(self.H, self.D, self.C), tensors["uv"].reshape(self.H, self.Dv, self.C)],
+                                                dim=1).reshape(self.H * (self.D + self.Dv), self.C))
 
     def cache_request(self):
         return KVRequest(1, self.C + self.R, self.window, values=False)
@@ -106,16 +112,29 @@ class LatentAttention:
         cache = g.k[binding.index]
         down = rt.scratch("latent_down", (T, self.w_down.shape[0]), torch.float32)
         kernels.linear(h, self.w_down, down, None, kernels.OUT_STORE_F32)
-        qa = rt.scratch("latent_qa", (T, H * (C + R)))
         if Q:
             cq = rt.scratch("latent_cq", (T, Q))
             kernels.latent_prepare(down, Q, C, R, self.w_qnorm, self.w_cnorm, self.eps, self.inv_freq, self.rot_dims, ctx, pages,
                                    g.page_size, cache, cq, write_kv=binding.writes, pairing=self.pairing, amplitude=self.amplitude)
             q = rt.scratch("latent_q", (T, H * (D + R)))
             kernels.linear(cq, self.w_uq, q)
+            n_pages = kernels.latent_expanded_pages(ctx, T, pages, H, D) if self.w_kv is not None else 0
+            if n_pages:
+                rows = 64 * n_pages
+                xc, xr, qr = rt.scratch("latent_xc", (rows, C)), rt.scratch("latent_xr", (rows, 64)), rt.scratch("latent_qr", (T, H * 64))
+                kernels.latent_expand_prepare(cache, ctx, pages, xc, xr, q, qr, H, D, R, self.inv_freq, self.rot_dims, self.pairing,
+                                              self.amplitude)
+                kv = rt.scratch("latent_kv", (rows, H * 2 * D))
+                kernels.linear(xc, self.w_kv, kv)
+                heads = rt.scratch("attn_out", (T, H * Dv))
+                kernels.attention_expanded(q, qr, kv, xr, heads, ctx, H, D, R, self.scale)
+                return kernels.linear(heads, self.w_o, x, None, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,
+                                      None if store else then_norm, out_scale)
+            qa = rt.scratch("latent_qa", (T, H * (C + R)))
             kernels.linear_batched(q, D + R, self.w_uk_t, qa, C + R, D)
             kernels.latent_q_rotate(q, D, qa, C, R, H, self.inv_freq, self.rot_dims, ctx, self.pairing, self.amplitude)
         else:
+            qa = rt.scratch("latent_qa", (T, H * (C + R)))
             qn = rt.scratch("latent_q", (T, H * D))
             kernels.latent_prepare_direct(down, H, D, C, R, self.w_cnorm, self.eps, self.inv_freq, self.rot_dims, self.pairing, ctx,
                                           pages, g.page_size, cache, qn, qa, write_kv=binding.writes, amplitude=self.amplitude)
