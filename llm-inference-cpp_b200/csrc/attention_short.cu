@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <math.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "mma_sync.cuh"
@@ -267,12 +268,28 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive(empty_bar(s));
     }
-    // this warp's rows to shared memory, where the ring was: every page that was asked for has been read by all warps
-    asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 1);
       lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 2);
+    }
+    if (WK == 1 && parts == 1) {                            // a row's only piece: straight out
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = wr * 16 + gq + 8 * h, x = row0 + r, tok = x / G;
+        if (r >= rows) continue;
+        __nv_bfloat16* dst = p.out + (size_t)(q_start + tok) * p.ldo + (size_t)(kvh * G + x - tok * G) * HD + 2 * t;
+        const float inv = 1.0f / lrow[h];
+#pragma unroll
+        for (int dc = 0; dc < HD / 8; ++dc)
+          *reinterpret_cast<uint32_t*>(dst + dc * 8) = sh_pack(o[dc][2 * h] * inv, o[dc][2 * h + 1] * inv);
+      }
+      return;                                               // (nobody waits behind: the barriers below are skipped by all)
+    }
+    // this warp's rows to shared memory, where the ring was: every page that was asked for has been read by all warps
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
       float* mine = results + (size_t)(wk * ROWS + wr * 16 + gq + 8 * h) * C::OUT_PITCH;
 #pragma unroll
       for (int dc = 0; dc < HD / 8; ++dc)
@@ -283,36 +300,60 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
     }
   }
+  if (WK == 1 && parts == 1) return;           // (the producer)
   if (parts > 1) cluster.sync(); else __syncthreads();
 
-  // ---- a row a warp, the cluster's rows dealt out over its warps: the pieces (block, key group) in that order ----
+  // ---- the cluster's rows dealt out over its warps, up to four rows of a warp at a time (a row is a chain of reads from
+  // another SM and shuffles: one by one the 16 rows of a warp were 4 us); the pieces (block, key group) in that order ----
   if (warp < SH_CONSUMERS) {
-    const int n_pieces = parts * WK;                        // <= 32
-    for (int r = part + parts * warp; r < rows; r += parts * SH_CONSUMERS) {
-      const int z = min(lane, n_pieces - 1);
-      const float* mine = cluster.map_shared_rank(results, z / WK) + (size_t)((z % WK) * ROWS + r) * C::OUT_PITCH;
-      const float mz = lane < n_pieces ? mine[HD] : -INFINITY;
-      const float M = warp_max(mz);
-      const float w = (mz == -INFINITY) ? 0.f : fast_exp2(mz - M);
-      const float lw = lane < n_pieces ? mine[HD + 1] * w : 0.f;
-      float L = 0.f, acc[HD / 32];
+    const int n_pieces = parts * WK, step = parts * SH_CONSUMERS;      // (at most 32 pieces)
+    const int z = min(lane, n_pieces - 1);
+    const float* mine = cluster.map_shared_rank(results, z / WK) + (size_t)(z % WK) * ROWS * C::OUT_PITCH;
+    auto merge = [&](int r0, auto batch) {                             // rows r0, r0 + step, ..
+      constexpr int RB = decltype(batch)::value;
+      float w[RB], lw[RB], L[RB], acc[RB][HD / 32];
 #pragma unroll
-      for (int u = 0; u < HD / 32; ++u) acc[u] = 0.f;
-      for (int b = 0; b < parts; ++b) {
-        const float* from = cluster.map_shared_rank(results, b) + (size_t)r * C::OUT_PITCH;
+      for (int i = 0; i < RB; ++i) {
+        const float* at = mine + (size_t)(r0 + i * step) * C::OUT_PITCH;
+        w[i] = lane < n_pieces ? at[HD] : -INFINITY;
+        lw[i] = lane < n_pieces ? at[HD + 1] : 0.f;
+        L[i] = 0.f;
 #pragma unroll
-        for (int g = 0; g < WK; ++g) {
-          const float wz = __shfl_sync(0xffffffffu, w, b * WK + g);
-          L += __shfl_sync(0xffffffffu, lw, b * WK + g);
-#pragma unroll
-          for (int u = 0; u < HD / 32; ++u) acc[u] = fmaf(wz, from[(size_t)g * ROWS * C::OUT_PITCH + lane + 32 * u], acc[u]);
-        }
+        for (int u = 0; u < HD / 32; ++u) acc[i][u] = 0.f;
       }
-      const int x = row0 + r, i = x / G;
-      __nv_bfloat16* dst = p.out + (size_t)(q_start + i) * p.ldo + (size_t)(kvh * G + x - i * G) * HD;
 #pragma unroll
-      for (int u = 0; u < HD / 32; ++u) dst[lane + 32 * u] = __float2bfloat16_rn(acc[u] / L);
-    }
+      for (int i = 0; i < RB; ++i) {
+        const float M = warp_max(w[i]);
+        w[i] = (w[i] == -INFINITY) ? 0.f : fast_exp2(w[i] - M);
+        lw[i] *= w[i];
+      }
+#pragma unroll 2
+      for (int b = 0; b < parts; ++b) {
+        const float* from = cluster.map_shared_rank(results, b) + lane;
+#pragma unroll
+        for (int g = 0; g < WK; ++g)
+#pragma unroll
+          for (int i = 0; i < RB; ++i) {
+            const float* at = from + (size_t)(g * ROWS + r0 + i * step) * C::OUT_PITCH;
+            const float wz = __shfl_sync(0xffffffffu, w[i], b * WK + g);
+            L[i] += __shfl_sync(0xffffffffu, lw[i], b * WK + g);
+#pragma unroll
+            for (int u = 0; u < HD / 32; ++u) acc[i][u] = fmaf(wz, at[32 * u], acc[i][u]);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < RB; ++i) {
+        const int x = row0 + r0 + i * step, tok = x / G;
+        __nv_bfloat16* dst = p.out + (size_t)(q_start + tok) * p.ldo + (size_t)(kvh * G + x - tok * G) * HD + lane;
+        const float inv = 1.0f / L[i];
+#pragma unroll
+        for (int u = 0; u < HD / 32; ++u) dst[32 * u] = __float2bfloat16_rn(acc[i][u] * inv);
+      }
+    };
+    int r0 = part + parts * warp;
+    for (; r0 + 3 * step < rows; r0 += 4 * step) merge(r0, std::integral_constant<int, 4>());
+    for (; r0 + step < rows; r0 += 2 * step) merge(r0, std::integral_constant<int, 2>());
+    if (r0 < rows) merge(r0, std::integral_constant<int, 1>());
   }
   if (parts > 1) cluster.sync();               // nobody's shared memory goes while it is read
 }
@@ -393,7 +434,7 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
   if (n_seqs <= 0 || max_q <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return LLMI_ERR_BAD_SIZE;
   if (!llmi_attention_short_supported(head_dim)) return LLMI_ERR_UNSUPPORTED;
-  if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
+  if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)out & 3) || (ldo & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
   const int group = n_heads / n_kv_heads;
   const long rows = n_cache_pages * n_kv_heads * SH_PAGE, tile_rows = (long)max_q * group;
   const long tiles = (tile_rows + SH_MAX_ROWS - 1) / SH_MAX_ROWS, items = (long)n_seqs * n_kv_heads * tiles;

@@ -864,24 +864,48 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, s
         _addr(gate), gate.stride(0) if gate is not None else 0, _addr(r1), _addr(r2), _addr(sink), _stream_int()))
 
 
-def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int) -> int:
+# attention_short, by head size and rows of a tile: (us of a block alone, us a page of it, us a page and item when every SM is
+# busy); a tile's share of that when it is one block, and one of several; the prompt kernel of 128-query tiles likewise (us of a
+# block alone, a page of it, a block, a page and block when every SM is busy).  Fitted to 1 to 64 sequences of 20 to 1,500 positions,
+# messages of 8 to 48 tokens, 32 x 64, 3 x 3 x 64 and 8 x 4 x 128 (kv heads x group x head size).
+_SHORT_US = {64: {16: (2.4, 0.42, 0.0021), 32: (2.9, 0.55, 0.0022), 64: (2.5, 0.93, 0.0034)},
+             128: {16: (3.5, 0.6, 0.004), 32: (4.1, 0.95, 0.0048), 64: (3.2, 1.42, 0.0072)}}
+_SHORT_BLOCK_US = {64: (0.009, 0.02), 128: (0.02, 0.04)}
+_PREFILL_US = {64: (3.3, 0.7, 0.048, 0.0025), 128: (3.4, 1.15, 0.048, 0.0047)}
+_short_plans: dict = {}
+
+
+def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int, head_dim: int) -> int:
     """Blocks of a cluster that share the pages of a (sequence, kv head, row tile) in attention_short, or 0 where the prompt
     kernel of 128-query tiles (attention_prefill_tc) is the faster one.
 
-    Both read a page per tile and head; a tile of 64 rows costs 1.17 times one of 128 queries (measured at 8 x 32
-    sequence-heads of 3,900 positions: 89 against 76 us), but covers all the group's heads at once; up to 32 rows 0.8 times
-    (61 us).  With few pages both are all start-up, and the prompt kernel's single block per head wins earlier (32
-    sequence-heads of 300 positions, heads of 128 in groups of 4, 32 tokens: 20.5 against 18.5 us).
-    A cluster is worth its barriers only while SMs are idle: 256 items 59 us alone, 66 in fours; 40 items of 2,000
-    positions 43 alone, 20.5 in eights; 160 items 45 alone, 37 in pairs, 41 in fours."""
-    rows = max_q * group
-    tiles = -(-rows // 64)
-    if rows > 32 and 1.17 * tiles >= group * (1.0 if n_pages > 8 else 0.55):
-        return 0
-    items, parts = n_seqs * n_kv_heads * tiles, 1
-    while parts < 8 and 2 * items * parts <= 2.2 * sm_count() and 2 * n_pages >= 3 * parts:
-        parts *= 2
-    return parts
+    A tile of 64 rows is slower a page than one of 128 queries, but covers all heads of a group, and up to 32 rows it is the
+    faster one; a block of the prompt kernel costs 48 ns however short its sequence (tensor memory, barriers), one of this
+    kernel 9.  A cluster is worth its barriers and its reads from other SMs only while SMs are idle.  Measured, this kernel in
+    1 / 2 / 4 / 8 blocks against the prompt kernel (us): 3 x 3 x 64, 4 sequences of 1,500, 16 tokens 24.4 / 16.2 / 11.0 / 8.8
+    against 22.0; 64 of 150 8.0 / 9.0 against 35.9; 16 of 250, 48 tokens 10.4 / 11.0 against 7.6; 32 x 64, 64 of 500, 16 tokens
+    55 / 85 / 157 / 346 against 138; 4 of 1,500, 48 tokens 34.6 / 25.4 / 27.3 / 31.9 against 25.6."""
+    key = (n_seqs, n_kv_heads, max_q, group, n_pages, head_dim)
+    best = _short_plans.get(key)
+    if best is None:
+        rows = max_q * group
+        tiles, tile = -(-rows // 64), 16 if rows <= 16 else (32 if rows <= 32 else 64)
+        items, (fixed, page, busy) = n_seqs * n_kv_heads * tiles, _SHORT_US[head_dim][tile]
+        alone, a_page, block, busy_page = _PREFILL_US[head_dim]
+        cost = max(alone + a_page * n_pages, n_seqs * n_kv_heads * group * (block + busy_page * n_pages))
+        best, cost = 0, 0.92 * cost             # (near the line the prompt kernel: the fit is good to a tenth)
+        for parts in (1, 2, 4, 8):
+            if parts > max(1, n_pages // 2):
+                break
+            of_block = _SHORT_BLOCK_US[head_dim][parts > 1]
+            c = max(fixed + (1.2 + 0.15 * parts if parts > 1 else 0.0) + page * -(-n_pages // parts),
+                    items * (parts * of_block + n_pages * busy))
+            if c < cost:
+                best, cost = parts, c
+        if len(_short_plans) >= 4096:
+            _short_plans.clear()
+        _short_plans[key] = best
+    return best
 
 
 def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
@@ -978,7 +1002,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             # 49.3 -> 50.5 us; 2,048 x 32: 42.1 -> 49.6 us).
             max_q = getattr(ctx, "short_message", 0)
             parts = attention_short_parts(seq_pages.shape[0], n_kv_heads, max_q, n_heads // n_kv_heads,
-                                          seq_pages.shape[1]) if max_q else 0
+                                          seq_pages.shape[1], head_dim) if max_q else 0
             if parts:
                 attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, max_q, n_heads, n_kv_heads,
                                 head_dim, scale, window, parts)
