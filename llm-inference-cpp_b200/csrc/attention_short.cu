@@ -48,6 +48,12 @@ struct ShortParams {
   float scale_log2;
   int window;
   int* error_flag;
+  // a decode step whose position encoding is done here (FUSE): `q` holds the un-rotated [q | k | v] rows
+  const float* inv_freq;      // [HD / 2] when rotary_dim > 0
+  int rotary_dim;             // HD or 0
+  int n_heads, write_kv;
+  __nv_bfloat16* k_cache_w;
+  __nv_bfloat16* v_cache_w;
 };
 
 template <int HD>
@@ -66,6 +72,7 @@ __device__ __forceinline__ uint32_t sh_pack(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
+__device__ __forceinline__ float2 sh_unpack(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
 __device__ __forceinline__ void sh_tma(uint32_t dst, const CUtensorMap* map, int col, int row, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -73,7 +80,9 @@ __device__ __forceinline__ void sh_tma(uint32_t dst, const CUtensorMap* map, int
       : "memory");
 }
 
-template <int HD, int ROWS>
+// FUSE: one token a sequence; its q is rotated as it is read, its k (rotated) and v are appended to the cache by the block that
+// has the newest page, before it asks for that page (rope_store.cu's arithmetic: the same bits).
+template <int HD, int ROWS, bool FUSE>
 __global__ void __launch_bounds__(SH_THREADS, HD == 64 ? 3 : 2)
 attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, ShortParams p) {
   using C = ShCfg<HD>;
@@ -95,7 +104,7 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   item /= p.row_tiles;
   const int kvh = item % p.n_kv_heads, seq = item / p.n_kv_heads;
   const int G = p.group;
-  const int q_start = p.seq_q_start[seq], q_len = p.seq_q_start[seq + 1] - q_start, kv_len = p.seq_kv_len[seq];
+  const int q_start = p.seq_q_start[seq], q_len = FUSE ? 1 : p.seq_q_start[seq + 1] - q_start, kv_len = p.seq_kv_len[seq];
   const int row0 = tile * ROWS, rows = min(ROWS, q_len * G - row0);
   if (rows <= 0 || kv_len <= 0) return;
   const int pos0 = kv_len - q_len;
@@ -107,6 +116,12 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int32_t* pages = p.seq_pages + (size_t)seq * p.pages_stride;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ float s_rot[FUSE ? HD : 1];                     // sines, then cosines, of the step's position
+  const bool rotate = FUSE && p.rotary_dim > 0;
+  if (rotate && threadIdx.x >= 32 && threadIdx.x < 32 + HD / 2) {
+    const int j = threadIdx.x - 32;
+    sincosf((float)pos0 * p.inv_freq[j], &s_rot[j], &s_rot[HD / 2 + j]);
+  }
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
@@ -119,24 +134,53 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   __syncthreads();
 
   if (warp == SH_CONSUMERS) {
-    // ---- producer ----
-    if (lane == 0) {
-      bool waited = false;
-      for (int i = 0; i < n_pages; ++i) {
-        const int s = i % C::STAGES;
-        if (!waited && (pg0 + i + 1) * SH_PAGE > pos0) {     // a page with rows of this step: written by the kernel before
-          pdl_wait();
-          waited = true;
-        }
-        if (i >= C::STAGES && !mbar_wait(empty_bar(s), ((i / C::STAGES) - 1) & 1, p.error_flag, 77)) break;
-        const int row = (pages[pg0 + i] * p.n_kv_heads + kvh) * SH_PAGE;
-        mbar_expect_tx(full_bar(s), C::STAGE_BYTES);
+    // ---- producer (lane 0 asks for the pages; with FUSE the whole warp appends the new k and v) ----
+    bool waited = false, ok = true;
+    for (int i = 0; i < n_pages && ok; ++i) {
+      const int s = i % C::STAGES;
+      const int page = pages[pg0 + i];
+      if (!waited && (pg0 + i + 1) * SH_PAGE > pos0) {       // a page with rows of this step: written by the kernel before
+        pdl_wait();
+        waited = true;
+        if (FUSE && p.write_kv) {                            // (the newest page: the only one that comes here)
+          const __nv_bfloat16* row = p.q + (size_t)q_start * p.ldq;
+          const __nv_bfloat16* ksrc = row + (size_t)(p.n_heads + kvh) * HD;
+          const __nv_bfloat16* vsrc = row + (size_t)(p.n_heads + p.n_kv_heads + kvh) * HD;
+          const size_t dst = (((size_t)page * p.n_kv_heads + kvh) * SH_PAGE + pos0 % SH_PAGE) * HD;
 #pragma unroll
-        for (int u = 0; u < C::NSUB; ++u) {
-          sh_tma(base + s * C::STAGE_BYTES + u * C::SUB_BYTES, &map_k, u * 64, row, full_bar(s));
-          sh_tma(base + s * C::STAGE_BYTES + C::TILE_BYTES + u * C::SUB_BYTES, &map_v, u * 64, row, full_bar(s));
+          for (int j = lane; j < HD / 2; j += 32) {
+            const __nv_bfloat16 a = ksrc[j], b = ksrc[j + HD / 2];
+            if (rotate) {
+              const float fa = __bfloat162float(a), fb = __bfloat162float(b), sn = s_rot[j], cs = s_rot[HD / 2 + j];
+              p.k_cache_w[dst + j] = __float2bfloat16_rn(rot_lo(fa, fb, cs, sn));
+              p.k_cache_w[dst + j + HD / 2] = __float2bfloat16_rn(rot_hi(fa, fb, cs, sn));
+            } else {
+              p.k_cache_w[dst + j] = a;
+              p.k_cache_w[dst + j + HD / 2] = b;
+            }
+            p.v_cache_w[dst + j] = vsrc[j];
+            p.v_cache_w[dst + j + HD / 2] = vsrc[j + HD / 2];
+          }
+          __threadfence();                                    // the copy below reads these rows through the async proxy
+          asm volatile("fence.proxy.async;" ::: "memory");
+          __syncwarp();
         }
       }
+      if (lane == 0) {
+        if (i >= C::STAGES && !mbar_wait(empty_bar(s), ((i / C::STAGES) - 1) & 1, p.error_flag, 77)) {
+          ok = false;
+        } else {
+          const int row = (page * p.n_kv_heads + kvh) * SH_PAGE;
+          mbar_expect_tx(full_bar(s), C::STAGE_BYTES);
+#pragma unroll
+          for (int u = 0; u < C::NSUB; ++u) {
+            sh_tma(base + s * C::STAGE_BYTES + u * C::SUB_BYTES, &map_k, u * 64, row, full_bar(s));
+            sh_tma(base + s * C::STAGE_BYTES + C::TILE_BYTES + u * C::SUB_BYTES, &map_v, u * 64, row, full_bar(s));
+          }
+        }
+      }
+      if (FUSE) __syncwarp();
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     }
   } else {
     // ---- consumers: warp (wr, wk) has rows 16 wr .. and keys KEYS wk .. of every page ----
@@ -161,6 +205,18 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           qa[kc][e] = live[e & 1] ? *reinterpret_cast<const uint32_t*>(src[e & 1] + kc * 16 + (e >> 1) * 8 + 2 * t) : 0u;
+      if (rotate) {                                          // both entries of a pair are this thread's, HD / 32 chunks apart
+#pragma unroll
+        for (int kc = 0; kc < HD / 32; ++kc)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int dim = kc * 16 + (e >> 1) * 8 + 2 * t;
+            const float2 a = sh_unpack(qa[kc][e]), b = sh_unpack(qa[kc + HD / 32][e]);
+            const float s0 = s_rot[dim], c0 = s_rot[HD / 2 + dim], s1 = s_rot[dim + 1], c1 = s_rot[HD / 2 + dim + 1];
+            qa[kc][e] = sh_pack(rot_lo(a.x, b.x, c0, s0), rot_lo(a.y, b.y, c1, s1));
+            qa[kc + HD / 32][e] = sh_pack(rot_hi(a.x, b.x, c0, s0), rot_hi(a.y, b.y, c1, s1));
+          }
+      }
     }
     float o[HD / 8][4];
 #pragma unroll
@@ -384,13 +440,13 @@ static int sh_cache_map(CUtensorMap* map, const void* ptr, long rows, int head_d
              : LLMI_ERR_DRIVER;
 }
 
-template <int HD, int ROWS>
+template <int HD, int ROWS, bool FUSE>
 static int sh_launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShortParams& p, int n_items, int parts, cudaStream_t stream) {
   using C = ShCfg<HD>;
   static PerDevice<bool> configured_on;
   bool& configured = configured_on.here();
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_short_kernel<HD, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_short_kernel<HD, ROWS, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
       return LLMI_ERR_LAUNCH;
     configured = true;
   }
@@ -408,15 +464,16 @@ static int sh_launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShortPa
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   pairs_may_start_early = false;
-  return cudaLaunchKernelEx(&cfg, attention_short_kernel<HD, ROWS>, mk, mv, p) == cudaSuccess ? LLMI_OK : LLMI_ERR_LAUNCH;
+  return cudaLaunchKernelEx(&cfg, attention_short_kernel<HD, ROWS, FUSE>, mk, mv, p) == cudaSuccess ? LLMI_OK : LLMI_ERR_LAUNCH;
 }
 
 template <int HD>
 static int sh_launch_rows(const CUtensorMap& mk, const CUtensorMap& mv, const ShortParams& p, int n_items, int rows, int parts,
                           cudaStream_t stream) {
-  if (rows <= 16) return sh_launch<HD, 16>(mk, mv, p, n_items, parts, stream);
-  if (rows <= 32) return sh_launch<HD, 32>(mk, mv, p, n_items, parts, stream);
-  return sh_launch<HD, 64>(mk, mv, p, n_items, parts, stream);
+  if (p.k_cache_w) return sh_launch<HD, 16, true>(mk, mv, p, n_items, parts, stream);
+  if (rows <= 16) return sh_launch<HD, 16, false>(mk, mv, p, n_items, parts, stream);
+  if (rows <= 32) return sh_launch<HD, 32, false>(mk, mv, p, n_items, parts, stream);
+  return sh_launch<HD, 64, false>(mk, mv, p, n_items, parts, stream);
 }
 
 }  // namespace llmi
@@ -427,15 +484,19 @@ LLMI_EXPORT int llmi_attention_short_supported(int head_dim) { return head_dim =
 
 // q: [tokens, >= n_heads * head_dim] rotated queries, the cache complete; otherwise as llmi_attention_prefill.  max_q: the most
 // tokens a sequence brings; parts: blocks that share a (sequence, kv head, row tile): 1, 2, 4 or 8.
-LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ldo, const void* k_cache, const void* v_cache,
+// fuse = 1 (max_q 1, groups up to 16): a decode step as for llmi_attention_decode_fused — `q` is the step's un-rotated
+// [q | k | v] rows, rotary_dim is head_dim or 0, the new k (rotated) and v are appended with write_kv.
+LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ldo, void* k_cache, void* v_cache,
                                      long n_cache_pages, const int32_t* seq_pages, int pages_stride, const int32_t* seq_q_start,
                                      const int32_t* seq_kv_len, int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim,
-                                     float scale, int window, int parts, int* error_flag, cudaStream_t stream) {
+                                     float scale, int window, int parts, int fuse, const float* inv_freq, int rotary_dim,
+                                     int write_kv, int* error_flag, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return LLMI_ERR_BAD_SIZE;
   if (!llmi_attention_short_supported(head_dim)) return LLMI_ERR_UNSUPPORTED;
   if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)out & 3) || (ldo & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
   const int group = n_heads / n_kv_heads;
+  if (fuse && (max_q != 1 || group > 16 || (rotary_dim != 0 && (rotary_dim != head_dim || !inv_freq)))) return LLMI_ERR_UNSUPPORTED;
   const long rows = n_cache_pages * n_kv_heads * SH_PAGE, tile_rows = (long)max_q * group;
   const long tiles = (tile_rows + SH_MAX_ROWS - 1) / SH_MAX_ROWS, items = (long)n_seqs * n_kv_heads * tiles;
   if (rows > 0x7fffffffL || items * parts > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;
@@ -445,7 +506,8 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
   rc = sh_cache_map(&mv, v_cache, rows, head_dim);
   if (rc != LLMI_OK) return rc;
   ShortParams p{(const __nv_bfloat16*)q, ldq, (__nv_bfloat16*)out, ldo, seq_pages, seq_q_start, seq_kv_len, pages_stride, n_kv_heads,
-                group, (int)tiles, scale * 1.4426950408889634f, window, error_flag};
+                group, (int)tiles, scale * 1.4426950408889634f, window, error_flag, inv_freq, fuse ? rotary_dim : 0, n_heads,
+                write_kv ? 1 : 0, fuse ? (__nv_bfloat16*)k_cache : nullptr, fuse ? (__nv_bfloat16*)v_cache : nullptr};
   const int per_tile = (int)(tile_rows < SH_MAX_ROWS ? tile_rows : SH_MAX_ROWS);
   return head_dim == 64 ? sh_launch_rows<64>(mk, mv, p, (int)items, per_tile, parts, stream)
                         : sh_launch_rows<128>(mk, mv, p, (int)items, per_tile, parts, stream);

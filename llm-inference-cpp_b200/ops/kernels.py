@@ -712,9 +712,41 @@ def decode_cluster(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int, gr
     return 0
 
 
+def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int, group: int) -> int:
+    """Blocks of a cluster that share a (sequence, kv head) in attention_short for a decode step, or 0 where one of the
+    persistent kernels (attention_decode_mma, attention_decode) is as fast or faster.
+
+    Those are bound by the chain behind an item's last page — the four warps' results merged, to memory, a fence, a ticket,
+    the last split's loads of all parts — and, ungrouped with heads of 128, by their arithmetic; here the parts meet in shared
+    memory.  A cluster of up to eight blocks takes an item while all of them are resident at once; so a few sequences of very
+    many pages, which the persistent kernels cut finer, stay with them, as do ungrouped heads of 64 up to that point, and
+    items that need a second, nearly empty wave.  Measured, persistent -> this (us, with the position encoding; kv heads x
+    group x size, sequences, positions): 3 x 3 x 64, 1, 1,000 8.0 -> 5.1, 8, 4,000 11.2 -> 10.0, 1, 8,000 10.4 -> 10.6; 8 x 4 x
+    128, 1, 1,000 9.8 -> 6.1, 24, 2,200 39.5 -> 38.5; 16 x 128, 4, 4,000 31.9 -> 24.3, 64, 2,200 228 -> 172; 32 x 64, 64, 2,200 191
+    -> 171, 16, 2,200 51 -> 58, 4, 2,200 16.4 -> 15.9."""
+    if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma":
+        return 0
+    resident, items = (3 if head_dim == 64 else 2) * sm_count(), n_live * n_kv_heads
+    if items > resident:
+        if head_dim == 64:
+            return 1 if n_pages >= 12 and 10 * items >= 17 * resident else 0
+        return 1 if group == 1 or n_pages >= 4 else 0
+    if group == 1 and (head_dim == 64 or (n_pages < 12 and 5 * items < 4 * resident)):
+        return 0
+    parts = 1
+    while parts < 8 and 2 * items * parts <= resident and n_pages >= (4 if parts == 1 and head_dim == 128 else 8 * parts):
+        parts *= 2
+    if parts == 8 and 2 * 8 * items <= resident and n_pages > (100 if head_dim == 64 else 256):
+        return 0
+    return parts
+
+
 def decode_plan_token(ctx, n_seqs: int, n_pages: int, page_size: int, n_kv_heads: int, head_dim: int, group: int):
     """What tells two recorded decode steps of the same padded shape apart: the split and the kernel's variant."""
     pps, n_live, cluster = decode_plan(ctx, n_seqs, n_pages, page_size, n_kv_heads, head_dim, group)
+    parts = decode_short_parts(n_live, n_kv_heads, n_pages, head_dim, group)
+    if parts:
+        return ("short", parts)
     if decode_uses_mma(head_dim, group):
         return (pps,)
     key = (head_dim, group, n_live, n_kv_heads)
@@ -909,9 +941,12 @@ def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, 
 
 
 def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
-                    n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1) -> None:
+                    n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1, rope=None) -> None:
     """Causal attention of at most ``max_q`` tokens a sequence over its cache pages (bf16, head size 64 or 128, page 64):
-    arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head."""
+    arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head.  ``rope``
+    (``max_q`` 1): see :func:`attention_decode_mma`."""
+    inv_freq, rotary_dim, write_kv = rope if rope is not None else (None, 0, False)
+    assert rotary_dim == 0 or (inv_freq is not None and inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2)
     _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)
     assert q.dtype == out.dtype == k_cache.dtype == torch.bfloat16 and q.stride(1) == 1 and out.stride(1) == 1
     assert k_cache.shape[-2] == 64 and k_cache.is_contiguous() and v_cache.is_contiguous()
@@ -919,6 +954,7 @@ def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pa
         _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache), _ptr(v_cache), c_long(k_cache.shape[0]),
         _ptr(seq_pages), c_int(seq_pages.stride(0)), _ptr(seq_q_start), _ptr(seq_kv_len), c_int(seq_pages.shape[0]), c_int(max_q),
         c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), c_int(parts),
+        c_int(0 if rope is None else 1), _ptr(inv_freq) if rotary_dim else None, c_int(rotary_dim), c_int(1 if write_kv else 0),
         _ptr(tc_scratch(q.device).error), _stream()))
 
 
@@ -978,6 +1014,11 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
     if _decode_kernel_applies(qkv, ctx, seq_pages, page_size, n_heads, n_kv_heads, head_dim, rt):
         S, P = seq_pages.shape
         pps, n_live, cluster = decode_plan(ctx, S, P, page_size, n_kv_heads, head_dim, n_heads // n_kv_heads)
+        parts = decode_short_parts(n_live, n_kv_heads, P, head_dim, n_heads // n_kv_heads)
+        if parts:
+            attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, 1, n_heads, n_kv_heads, head_dim,
+                            scale, window, parts, rope)
+            return
         partials = rt.scratch("attn_partials", (attention_decode_workspace(S, n_heads, head_dim, P, pps),), torch.float32)
         if decode_uses_mma(head_dim, n_heads // n_kv_heads):
             attention_decode_mma(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_kv_len, ctx.seq_q_start, n_heads,

@@ -55,3 +55,45 @@ def test_attention_short(hd, group, window):
         k.attention_short(q, out, kc, vc, table.to(dev), i32(starts), i32(kv_lens), max(q_lens), nh, nkv, hd, scale, window, parts)
         assert float((out.double() - ref).norm() / ref.norm()) < 1.2 * 2 ** -9 * 2 ** 0.5, parts
     k.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("hd,group", [(64, 1), (64, 3), (128, 4), (128, 16)])
+@pytest.mark.parametrize("window,rot,write", [(0, True, True), (200, True, True), (0, False, True), (0, True, False)])
+def test_attention_short_decode_same_bits(hd, group, window, rot, write):
+    """A decode step with the position encoding inside gives, however the pages are shared, the bits and the cache of the
+    kernels it replaces: lengths at the edges of pages, a padding sequence, positions of nobody NaN."""
+    k = K()
+    nkv = 2
+    nh, dev = nkv * group, "cuda"
+    torch.manual_seed(hd * group)
+    lens, P = [1, 64, 65, 700, 0, 129, 1000, 128], 16                     # lengths after the step (0: padding)
+    S, n_pages = len(lens), 48
+    order = torch.randperm(n_pages)
+    table, at = torch.full((S, P), -1, dtype=torch.int32), 0
+    kc = torch.full((n_pages, nkv, 64, hd), float("nan"), device=dev, dtype=torch.bfloat16)
+    vc = kc.clone()
+    for s, n in enumerate(lens):
+        for p in range((n + 63) // 64):
+            table[s, p] = order[at]
+            there = min(64, n - (1 if write else 0) - 64 * p)
+            if there > 0:
+                kc[order[at], :, :there] = torch.randn(nkv, there, hd, device=dev).bfloat16()
+                vc[order[at], :, :there] = torch.randn(nkv, there, hd, device=dev).bfloat16()
+            at += 1
+    qkv = torch.randn(S, (nh + 2 * nkv) * hd, device=dev).bfloat16()
+    inv = torch.rand(hd // 2, device=dev)
+    i32 = lambda x: torch.as_tensor(x).to(torch.int32).to(dev)      # noqa: E731
+    pages, kvlen, starts = table.to(dev), i32(lens), i32(list(range(S + 1)))
+    seq, pos = i32([i if n else -1 for i, n in enumerate(lens)]), i32([max(n - 1, 0) for n in lens])
+    q_rot, kr, vr = qkv.clone(), kc.clone(), vc.clone()
+    k.rope_store(q_rot, inv, hd if rot else 0, seq, pos, pages, 64, kr, vr, nh, nkv, hd, write)
+    for parts in (1, 2, 4, 8):
+        outs = [torch.full((S, nh * hd), 7.0, device=dev, dtype=torch.bfloat16) for _ in range(2)]
+        k.attention_short(q_rot, outs[0], kr, vr, pages, starts, kvlen, 1, nh, nkv, hd, hd ** -0.5, window, parts)
+        k1, v1 = kc.clone(), vc.clone()
+        k.attention_short(qkv, outs[1], k1, v1, pages, starts, kvlen, 1, nh, nkv, hd, hd ** -0.5, window, parts,
+                          (inv, hd if rot else 0, write))
+        assert torch.equal(outs[0], outs[1]) and bool((outs[1][4] == 7.0).all()) and bool(torch.isfinite(outs[1].float()).all())
+        for a, b in ((kr, k1), (vr, v1)):
+            assert torch.equal(torch.nan_to_num(a.float(), nan=-7.0), torch.nan_to_num(b.float(), nan=-7.0))
+    k.check_device_errors("cuda:0")
