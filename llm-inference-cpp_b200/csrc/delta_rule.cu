@@ -21,6 +21,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "recurrence.cuh"
 
 namespace llmi {
 
@@ -339,34 +340,23 @@ delta_recurrence_kernel(const float* __restrict__ prep, long ldp, DeltaDims m, f
 }
 
 // The form for D = 32, 64, 128 and Dv a multiple of 16.  A thread holds TWO neighbouring columns of S and a
-// sixteenth of their entries (lane `sub` of sixteen: d = 64 i + 4 sub + 0..3, while d < D), in registers; partial sums
-// over d are joined by four shuffles.  The recurrence is a chain over the tokens — the time of a prompt is tokens x
-// (time of one token), and a token costs one warp's instructions (each warp has a scheduler to itself) — so the
-// work of a token is spread thin: 16 columns a warp.  Columns are independent: a head's columns are cut into slices
-// of 32 (or 16) and every slice is a block of its own (blockIdx.z).
+// sixteenth of their entries (lane `sub` of sixteen: d = 64 i + 4 sub + 0..3, while d < D), in registers, as pairs of
+// entries; partial sums over d are joined by join_four, a token's Sᵀ k beside the token before's Sᵀ q.  The recurrence is a
+// chain over the tokens — the time of a prompt is tokens x (time of one token), and a token costs one warp's
+// instructions — so the work of a token is spread thin: 16 columns a warp.  Columns are independent: a head's columns are
+// cut into slices of 32 (or 16) and every slice is a block of its own (blockIdx.z).
 //
-// What a token needs — k, q of the head's key head, the slice's v, beta, g — is copied into a ring of DELTA_RING
-// entries DELTA_RING - 1 tokens ahead (cp.async, 16 bytes a copy, no registers in between), so that no load's latency
-// lies on the chain from token to token; one barrier per token.
-constexpr int DELTA_RING = 8;
-
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16_ca(void* dst, const void* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
+// What a token needs — k, q of the head's key head, the slice's v, beta, g — is copied into a ring of REC_STAGES batches
+// of REC_BATCH tokens (cp.async, 16 bytes a copy, each thread's places worked out once), so that no load's latency lies on
+// the chain from token to token; one barrier per batch.
+// 1,000 to 1,900 tokens, two sequences, 16 heads of 128: 478 -> 281 ns a token (a decay per channel 510 -> 299); 8 heads of 64 477 ->
+// 245.  (One barrier a token, two columns a pair, eight shuffles for each of the two sums before.)
 template <int D, bool CH>
 __global__ void __launch_bounds__(256)
 delta_recurrence_quad_kernel(const float* __restrict__ prep, long ldp, DeltaDims m, float* __restrict__ state,
                              const int32_t* __restrict__ seq_q_start, const int32_t* __restrict__ seq_slot,
                              float* __restrict__ o_raw, long ldo, int write_state) {
   extern __shared__ __align__(16) float sm[];
-  pdl_wait();
-  pdl_launch_dependents();
   const int h = blockIdx.x, seq = blockIdx.y;
   const int slot = seq_slot[seq];
   if (slot < 0) return;
@@ -380,119 +370,137 @@ delta_recurrence_quad_kernel(const float* __restrict__ prep, long ldp, DeltaDims
   const bool holds = 4 * sub < D;                            // (D = 32 only: half of the lanes carry zeros)
   const int kh = h / (m.H / m.Hk);
   float* S_g = state + (size_t)slot * m.state_floats() + (size_t)h * D * Dv + (size_t)col0 * D;    // [column][entry]
-  float2 S_r[NI][4];                                         // [chunk][entry of the chunk] . (x, y) = the two columns
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const float4 c0 = holds ? *reinterpret_cast<const float4*>(S_g + 64 * i + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 c1 = holds ? *reinterpret_cast<const float4*>(S_g + D + 64 * i + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-    S_r[i][0] = make_float2(c0.x, c1.x);
-    S_r[i][1] = make_float2(c0.y, c1.y);
-    S_r[i][2] = make_float2(c0.z, c1.z);
-    S_r[i][3] = make_float2(c0.w, c1.w);
-  }
-  // ring entry: [k (D) | q (D) | v of the slice (CB) | beta, g, 0, 0], or, with a decay per channel,
+  // a token's place in the ring: [k (D) | q (D) | v of the slice (CB) | beta, g, 0, 0], or, with a decay per channel,
   // [k (D) | q (D) | v (CB) | g (D) | beta, 0, 0, 0]; all parts are whole 16-byte pieces
   constexpr int NG = CH ? D : 0;
-  const int n16 = (2 * D + CB + NG) / 4, pitch = 2 * D + CB + NG + 4;
-  const float* k_src = prep + (size_t)m.Hk * D + (size_t)kh * D;
-  const float* q_src = prep + (size_t)kh * D;
-  const float* v_src = prep + (size_t)m.n_qk() + (size_t)h * Dv + blockIdx.z * CB;
-  auto issue = [&](int i) {
-    float* dst = sm + (size_t)(i % DELTA_RING) * pitch;
-    const size_t row = (size_t)(r0 + i) * ldp;
-    for (int e = threadIdx.x; e < n16 + (CH ? 1 : 2); e += blockDim.x) {
-      if (e < D / 4) cp_async16_ca(dst + 4 * e, k_src + row + 4 * e);
-      else if (e < D / 2) cp_async16_ca(dst + 4 * e, q_src + row + 4 * (e - D / 4));
-      else if (e < (2 * D + CB) / 4) cp_async16_ca(dst + 4 * e, v_src + row + 4 * (e - D / 2));
-      else if (CH && e < n16) cp_async16_ca(dst + 4 * e, prep + row + m.decay_at() + h * D + 4 * (e - (2 * D + CB) / 4));
-      else cp_async4(dst + 4 * n16 + (e - n16), prep + row + (e == n16 ? m.beta_at() + h : m.decay_at() + h));
-    }
-  };
+  const int n16 = (2 * D + CB + NG) / 4, pitch = 2 * D + CB + NG + 4, pieces = n16 + (CH ? 1 : 2);
+  // My copies: piece (threadIdx.x + r blockDim.x) of a batch, counted over its tokens.  (CB = 16, D = 128, CH: 4 x 105 pieces
+  // for 128 threads.)
+  constexpr int COPIES = 4;
+  const float* src[COPIES];
+  int dst[COPIES], of_token[COPIES];
 #pragma unroll
-  for (int s = 0; s < DELTA_RING - 1; ++s) {
-    if (s < n) issue(s);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int r = 0; r < COPIES; ++r) {
+    const int x = threadIdx.x + r * blockDim.x, u = x / pieces, e = x - u * pieces;
+    of_token[r] = u < REC_BATCH ? u : 0x7fffffff / 2;        // (behind every sequence's end: never copied)
+    const float* row = prep + (size_t)(r0 + (u < REC_BATCH ? u : 0)) * ldp;
+    dst[r] = (u < REC_BATCH ? u : 0) * pitch + (e < n16 ? 4 * e : 4 * n16 + (e - n16));
+    if (e < D / 4) src[r] = row + (size_t)m.Hk * D + (size_t)kh * D + 4 * e;
+    else if (e < D / 2) src[r] = row + (size_t)kh * D + 4 * (e - D / 4);
+    else if (e < (2 * D + CB) / 4) src[r] = row + m.n_qk() + (size_t)h * Dv + blockIdx.z * CB + 4 * (e - D / 2);
+    else if (CH && e < n16) src[r] = row + m.decay_at() + h * D + 4 * (e - (2 * D + CB) / 4);
+    else src[r] = row + (e == n16 ? m.beta_at() + h : m.decay_at() + h);
+    if (e >= n16) dst[r] |= 1 << 30;                         // a copy of four bytes
   }
-  for (int i = 0; i < n; ++i) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(DELTA_RING - 2) : "memory");
-    __syncthreads();                                         // token i's entry is there; token i-1's entry is read out
-    if (i + DELTA_RING - 1 < n) issue(i + DELTA_RING - 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* in = sm + (size_t)(i % DELTA_RING) * pitch;
-    float4 kk[NI], qq[NI];
+  const int stage_floats = REC_BATCH * pitch;
+  const size_t advance = (size_t)REC_BATCH * ldp;
+  int asked = 0;                                             // tokens asked for so far (whole batches)
+  auto issue = [&](int stage) {
+    float* base = sm + stage * stage_floats;
 #pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      kk[c] = holds ? *reinterpret_cast<const float4*>(in + 64 * c + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-      qq[c] = holds ? *reinterpret_cast<const float4*>(in + D + 64 * c + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < COPIES; ++r) {
+      if (asked + of_token[r] < n) {
+        float* to = base + (dst[r] & ~(1 << 30));
+        if (dst[r] >> 30) rec_copy4(to, src[r]);
+        else rec_copy16(to, src[r]);
+      }
+      src[r] += advance;
     }
-    const float2 v = *reinterpret_cast<const float2*>(in + 2 * D + 2 * cg);
-    const float beta = in[4 * n16], g = CH ? 1.0f : in[4 * n16 + 1];
-    float2 sk = make_float2(0.f, 0.f), sk2 = make_float2(0.f, 0.f);
-    if (CH) {                                                // the decay of every row, before anything reads the state
+    asked += REC_BATCH;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  pdl_wait();                                                // (so far: the step's sizes and this thread's places only)
+  pdl_launch_dependents();
+#pragma unroll
+  for (int s = 0; s < REC_STAGES - 1; ++s) issue(s);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 S_r[2][NI][2];                                      // [column][chunk][pair of entries]
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const float4 v = holds ? *reinterpret_cast<const float4*>(S_g + c * D + 64 * i + 4 * sub) : zero;
+      S_r[c][i][0] = make_float2(v.x, v.y);
+      S_r[c][i][1] = make_float2(v.z, v.w);
+    }
+  float2 o_pend = make_float2(0.f, 0.f);                     // my parts of the token before's Sᵀ q, of both columns
+  float* o_at = o_raw + (size_t)r0 * ldo + (size_t)h * Dv + col0 + (sub & 1);      // (lanes sub = 2, 3 write)
+  int stage = 0;
+  for (int i0 = 0; i0 < n; i0 += REC_BATCH) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(REC_STAGES - 2) : "memory");
+    __syncthreads();                                         // this batch is there; the one before is read out
+    issue(stage == 0 ? REC_STAGES - 1 : stage - 1);
+    const float* in = sm + stage * stage_floats;
+    stage = stage == REC_STAGES - 1 ? 0 : stage + 1;
+    const int here = min(REC_BATCH, n - i0);
+#pragma unroll
+    for (int u = 0; u < REC_BATCH; ++u, in += pitch) {
+      if (u >= here) break;
+      float4 kk[NI], qq[NI];
 #pragma unroll
       for (int c = 0; c < NI; ++c) {
-        const float4 gg = holds ? *reinterpret_cast<const float4*>(in + 2 * D + CB + 64 * c + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-        S_r[c][0].x *= gg.x; S_r[c][0].y *= gg.x;
-        S_r[c][1].x *= gg.y; S_r[c][1].y *= gg.y;
-        S_r[c][2].x *= gg.z; S_r[c][2].y *= gg.z;
-        S_r[c][3].x *= gg.w; S_r[c][3].y *= gg.w;
+        kk[c] = holds ? *reinterpret_cast<const float4*>(in + 64 * c + 4 * sub) : zero;
+        qq[c] = holds ? *reinterpret_cast<const float4*>(in + D + 64 * c + 4 * sub) : zero;
       }
-    }
+      const float2 v = *reinterpret_cast<const float2*>(in + 2 * D + 2 * cg);
+      const float beta = in[4 * n16], g = CH ? 1.0f : in[4 * n16 + 1];
+      if (CH) {                                              // the decay of every row, before anything reads the state
 #pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      sk.x = fmaf(S_r[c][0].x, kk[c].x, sk.x);
-      sk.y = fmaf(S_r[c][0].y, kk[c].x, sk.y);
-      sk2.x = fmaf(S_r[c][1].x, kk[c].y, sk2.x);
-      sk2.y = fmaf(S_r[c][1].y, kk[c].y, sk2.y);
-      sk.x = fmaf(S_r[c][2].x, kk[c].z, sk.x);
-      sk.y = fmaf(S_r[c][2].y, kk[c].z, sk.y);
-      sk2.x = fmaf(S_r[c][3].x, kk[c].w, sk2.x);
-      sk2.y = fmaf(S_r[c][3].y, kk[c].w, sk2.y);
-    }
-    sk.x += sk2.x;
-    sk.y += sk2.y;
+        for (int c = 0; c < NI; ++c) {
+          const float4 gg = holds ? *reinterpret_cast<const float4*>(in + 2 * D + CB + 64 * c + 4 * sub) : zero;
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      sk.x += __shfl_xor_sync(0xffffffffu, sk.x, o);
-      sk.y += __shfl_xor_sync(0xffffffffu, sk.y, o);
-    }
-    const float ux = beta * (v.x - (CH ? sk.x : g * sk.x)), uy = beta * (v.y - (CH ? sk.y : g * sk.y));
-    float2 o2 = make_float2(0.f, 0.f), o3 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      const float ke[4] = {kk[c].x, kk[c].y, kk[c].z, kk[c].w};
-      const float qe[4] = {qq[c].x, qq[c].y, qq[c].z, qq[c].w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float2 s = S_r[c][e];
-        s.x = fmaf(ke[e], ux, CH ? s.x : g * s.x);
-        s.y = fmaf(ke[e], uy, CH ? s.y : g * s.y);
-        S_r[c][e] = s;
-        if (e & 1) {
-          o3.x = fmaf(s.x, qe[e], o3.x);
-          o3.y = fmaf(s.y, qe[e], o3.y);
-        } else {
-          o2.x = fmaf(s.x, qe[e], o2.x);
-          o2.y = fmaf(s.y, qe[e], o2.y);
+          for (int col = 0; col < 2; ++col) {
+            S_r[col][c][0] = __fmul2_rn(S_r[col][c][0], make_float2(gg.x, gg.y));
+            S_r[col][c][1] = __fmul2_rn(S_r[col][c][1], make_float2(gg.z, gg.w));
+          }
         }
       }
-    }
-    o2.x += o3.x;
-    o2.y += o3.y;
+      float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      o2.x += __shfl_xor_sync(0xffffffffu, o2.x, o);
-      o2.y += __shfl_xor_sync(0xffffffffu, o2.y, o);
+      for (int c = 0; c < NI; ++c)
+#pragma unroll
+        for (int col = 0; col < 2; ++col) {
+          acc[col] = __ffma2_rn(S_r[col][c][0], make_float2(kk[c].x, kk[c].y), acc[col]);
+          acc[col] = __ffma2_rn(S_r[col][c][1], make_float2(kk[c].z, kk[c].w), acc[col]);
+        }
+      float skx = pair_sum(acc[0]), sky = pair_sum(acc[1]);
+      const float o_before = join_four(skx, sky, o_pend.x, o_pend.y, sub);
+      if (i0 + u > 0) {
+        if ((sub & ~1) == 2) *o_at = o_before;
+        o_at += ldo;
+      }
+      const float2 u2[2] = {pair_of(beta * (v.x - (CH ? skx : g * skx))), pair_of(beta * (v.y - (CH ? sky : g * sky)))};
+      const float2 g2 = pair_of(g);
+      float2 o2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int c = 0; c < NI; ++c) {
+        const float2 kp[2] = {make_float2(kk[c].x, kk[c].y), make_float2(kk[c].z, kk[c].w)};
+        const float2 qp[2] = {make_float2(qq[c].x, qq[c].y), make_float2(qq[c].z, qq[c].w)};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int col = 0; col < 2; ++col) {
+            const float2 kept = CH ? S_r[col][c][e] : __fmul2_rn(g2, S_r[col][c][e]);
+            S_r[col][c][e] = __ffma2_rn(kp[e], u2[col], kept);
+            o2[col] = __ffma2_rn(S_r[col][c][e], qp[e], o2[col]);
+          }
+      }
+      o_pend = make_float2(pair_sum(o2[0]), pair_sum(o2[1]));
     }
-    if (sub == 0) *reinterpret_cast<float2*>(o_raw + (size_t)(r0 + i) * ldo + (size_t)h * Dv + col0) = o2;
+  }
+  {
+    float none = 0.f, none2 = 0.f;
+    const float o_last = join_four(none, none2, o_pend.x, o_pend.y, sub);
+    if ((sub & ~1) == 2) *o_at = o_last;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (write_state && holds) {
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      *reinterpret_cast<float4*>(S_g + 64 * i + 4 * sub) = make_float4(S_r[i][0].x, S_r[i][1].x, S_r[i][2].x, S_r[i][3].x);
-      *reinterpret_cast<float4*>(S_g + D + 64 * i + 4 * sub) = make_float4(S_r[i][0].y, S_r[i][1].y, S_r[i][2].y, S_r[i][3].y);
-    }
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        *reinterpret_cast<float4*>(S_g + c * D + 64 * i + 4 * sub) =
+            make_float4(S_r[c][i][0].x, S_r[c][i][0].y, S_r[c][i][1].x, S_r[c][i][1].y);
   }
 }
 
@@ -501,7 +509,7 @@ int launch_delta_recurrence_quad(const float* prep, long ldp, DeltaDims m, float
                                  const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state,
                                  cudaStream_t stream) {
   const int CB = m.Dv % 32 == 0 ? 32 : 16;                   // columns per block
-  size_t smem = (size_t)DELTA_RING * ((CH ? 3 : 2) * D + CB + 4) * sizeof(float);
+  size_t smem = (size_t)REC_STAGES * REC_BATCH * ((CH ? 3 : 2) * D + CB + 4) * sizeof(float);
   // Few blocks, each a chain over the tokens: two on one SM slow each other down while other SMs stand idle, and that is
   // where they land when they are launched while the kernels before still fill the device (measured, 2,048 tokens, 16 heads
   // of 128: 1.72 ms instead of 1.03).  A block asks for so much shared memory that no more fit an SM than must.

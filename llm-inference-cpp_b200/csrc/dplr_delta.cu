@@ -16,6 +16,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "recurrence.cuh"
 
 namespace llmi {
 
@@ -135,29 +136,22 @@ dplr_recurrence_kernel(const float* __restrict__ proj, long ld, const float* __r
 }
 
 // The form for D = 32, 64, 128 and Dv a multiple of 16.  A thread holds TWO neighbouring columns of S and a sixteenth
-// of their entries (lane `sub` of sixteen: d = 64 i + 4 sub + 0..3, while d < D) in registers; partial sums over d are
-// joined by four shuffles.  The recurrence is a chain over the tokens, so the work of a token is spread thin (16
-// columns a warp), a head's columns are cut into slices of 32 (or 16), every slice a block of its own (blockIdx.z),
-// and what a token needs — w, p, m, k, r of the head, the slice's v — is copied into a ring of DPLR_RING entries
-// DPLR_RING - 1 tokens ahead (cp.async, 16 bytes a copy), so that no load's latency lies on the chain from token to
-// token; one barrier per token.  (Two tokens per round — the second one's sum over the state follows from the state
-// before the first, (p_B * w_A) . S + (p_B . m_A)(p_A . S) + (p_B . k_A) v_A, so one round of shuffles serves both — was
-// measured slower, 1.10 against 0.96 ms for 2,048 tokens: the time of a token is its instructions, not the shuffles.)
-constexpr int DPLR_RING = 8;
-
-__device__ __forceinline__ void dplr_cp16(void* dst, const void* src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
+// of their entries (lane `sub` of sixteen: d = 64 i + 4 sub + 0..3, while d < D) in registers, as pairs of entries; partial
+// sums over d are joined by join_four, a token's p . S beside the token before's S . r.  The recurrence is a chain over the
+// tokens, so the work of a token is spread thin (16 columns a warp), a head's columns are cut into slices of 32 (or 16),
+// every slice a block of its own (blockIdx.z), and what a token needs — w, p, m, k, r of the head, the slice's v — is
+// copied into a ring of REC_STAGES batches of REC_BATCH tokens (cp.async, 16 bytes a copy, each thread's places worked out
+// once), so that no load's latency lies on the chain from token to token; one barrier per batch.  (Two tokens per round of
+// shuffles — the second one's sum over the state follows from the state before the first, (p_B * w_A) . S + (p_B . m_A)(p_A .
+// S) + (p_B . k_A) v_A — was measured slower, 1.10 against 0.96 ms for 2,048 tokens: the time of a token is its
+// instructions.)
+// 1,300 tokens, two sequences, 32 heads of 64: 442 -> 251 ns a token; six of 400 1,094 -> 481 (same bits).
 template <int D>
 __global__ void __launch_bounds__(256)
 dplr_recurrence_quad_kernel(const float* __restrict__ proj, long ld, const float* __restrict__ prep, long ldp, int H, int Dv,
                             float* __restrict__ state, long state_stride, const int32_t* __restrict__ seq_q_start,
                             const int32_t* __restrict__ seq_slot, float* __restrict__ o_raw, long ldo, int write_state) {
   extern __shared__ __align__(16) float sm[];
-  pdl_wait();
-  pdl_launch_dependents();
   const int h = blockIdx.x, seq = blockIdx.y;
   const int slot = seq_slot[seq];
   if (slot < 0) return;
@@ -170,112 +164,119 @@ dplr_recurrence_quad_kernel(const float* __restrict__ proj, long ld, const float
   const bool holds = 4 * sub < D;
   const int HD = H * D;
   float* S_g = state + (size_t)slot * state_stride + (size_t)h * D * Dv + (size_t)col0 * D;     // [column][entry]
-  float2 S_r[NI][4];                                         // [chunk][entry of the chunk] . (x, y) = the two columns
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const float4 c0 = holds ? *reinterpret_cast<const float4*>(S_g + 64 * i + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 c1 = holds ? *reinterpret_cast<const float4*>(S_g + D + 64 * i + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
-    S_r[i][0] = make_float2(c0.x, c1.x);
-    S_r[i][1] = make_float2(c0.y, c1.y);
-    S_r[i][2] = make_float2(c0.z, c1.z);
-    S_r[i][3] = make_float2(c0.w, c1.w);
-  }
-  // ring entry: [w | p | m | k | r (D each) | v of the slice (CB)]; all parts are whole 16-byte pieces
+  // a token's place in the ring: [w | p | m | k | r (D each) | v of the slice (CB)]; all parts are whole 16-byte pieces
   constexpr int Q = D / 4;                                   // 16-byte pieces of one vector
-  const int n16 = 5 * Q + CB / 4, pitch = 5 * D + CB;
-  const float* w_src = prep + (size_t)h * D;
-  const float* x_src = proj + (size_t)h * D;
-  const float* v_src = proj + 2 * (size_t)HD + (size_t)h * Dv + blockIdx.z * CB;
-  auto issue = [&](int i) {
-    float* dst = sm + (size_t)(i % DPLR_RING) * pitch;
-    const size_t prow = (size_t)(r0 + i) * ldp, xrow = (size_t)(r0 + i) * ld;
-    for (int e = threadIdx.x; e < n16; e += blockDim.x) {
-      const int part = e / Q, off = 4 * (e - part * Q);
-      if (part < 3) dplr_cp16(dst + 4 * e, w_src + prow + (size_t)part * HD + off);            // w, p, m
-      else if (part == 3) dplr_cp16(dst + 4 * e, x_src + xrow + HD + off);                        // k
-      else if (part == 4) dplr_cp16(dst + 4 * e, x_src + xrow + off);                             // r
-      else dplr_cp16(dst + 4 * e, v_src + xrow + 4 * (e - 5 * Q));
-    }
-  };
+  const int pieces = 5 * Q + CB / 4, pitch = 5 * D + CB;
+  // My copies: piece (threadIdx.x + r blockDim.x) of a batch, counted over its tokens.  (CB = 16, D = 128: 4 x 164 pieces for
+  // 128 threads.)
+  constexpr int COPIES = 6;
+  const float* src[COPIES];
+  int dst[COPIES], of_token[COPIES];
 #pragma unroll
-  for (int s = 0; s < DPLR_RING - 1; ++s) {
-    if (s < n) issue(s);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int r = 0; r < COPIES; ++r) {
+    const int x = threadIdx.x + r * blockDim.x, u = x / pieces, e = x - u * pieces;
+    of_token[r] = u < REC_BATCH ? u : 0x7fffffff / 2;        // (behind every sequence's end: never copied)
+    const int tok = u < REC_BATCH ? u : 0, part = e / Q, off = 4 * (e - part * Q);
+    const float* prow = prep + (size_t)(r0 + tok) * ldp + (size_t)h * D;
+    const float* xrow = proj + (size_t)(r0 + tok) * ld;
+    dst[r] = tok * pitch + 4 * e;
+    if (part < 3) src[r] = prow + (size_t)part * HD + off;                                       // w, p, m
+    else if (part == 3) src[r] = xrow + (size_t)h * D + HD + off;                               // k
+    else if (part == 4) src[r] = xrow + (size_t)h * D + off;                                     // r
+    else src[r] = xrow + 2 * (size_t)HD + (size_t)h * Dv + blockIdx.z * CB + 4 * (e - 5 * Q);
+    if (part < 3) dst[r] |= 1 << 30;                         // from prep
   }
-  float2 o_pend = make_float2(0.f, 0.f);                       // my part of the token before's S . r
-  for (int i = 0; i < n; ++i) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(DPLR_RING - 2) : "memory");
-    __syncthreads();                                         // token i's entry is there; token i-1's entry is read out
-    if (i + DPLR_RING - 1 < n) issue(i + DPLR_RING - 1);
+  const int stage_floats = REC_BATCH * pitch;
+  const size_t advance_p = (size_t)REC_BATCH * ldp, advance_x = (size_t)REC_BATCH * ld;
+  int asked = 0;                                             // tokens asked for so far (whole batches)
+  auto issue = [&](int stage) {
+    float* base = sm + stage * stage_floats;
+#pragma unroll
+    for (int r = 0; r < COPIES; ++r) {
+      if (asked + of_token[r] < n) rec_copy16(base + (dst[r] & ~(1 << 30)), src[r]);
+      src[r] += (dst[r] >> 30) ? advance_p : advance_x;
+    }
+    asked += REC_BATCH;
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* in = sm + (size_t)(i % DPLR_RING) * pitch;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 pp[NI];
-    float2 dot = make_float2(0.f, 0.f), dot2 = make_float2(0.f, 0.f);
+  };
+  pdl_wait();                                                // (so far: the step's sizes and this thread's places only)
+  pdl_launch_dependents();
 #pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      pp[c] = holds ? *reinterpret_cast<const float4*>(in + D + 64 * c + 4 * sub) : zero;
-      dot.x = fmaf(S_r[c][0].x, pp[c].x, dot.x);
-      dot.y = fmaf(S_r[c][0].y, pp[c].x, dot.y);
-      dot2.x = fmaf(S_r[c][1].x, pp[c].y, dot2.x);
-      dot2.y = fmaf(S_r[c][1].y, pp[c].y, dot2.y);
-      dot.x = fmaf(S_r[c][2].x, pp[c].z, dot.x);
-      dot.y = fmaf(S_r[c][2].y, pp[c].z, dot.y);
-      dot2.x = fmaf(S_r[c][3].x, pp[c].w, dot2.x);
-      dot2.y = fmaf(S_r[c][3].y, pp[c].w, dot2.y);
+  for (int s = 0; s < REC_STAGES - 1; ++s) issue(s);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float2 S_r[2][NI][2];                                      // [column][chunk][pair of entries]
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const float4 v = holds ? *reinterpret_cast<const float4*>(S_g + c * D + 64 * i + 4 * sub) : zero;
+      S_r[c][i][0] = make_float2(v.x, v.y);
+      S_r[c][i][1] = make_float2(v.z, v.w);
     }
-    dot.x += dot2.x;
-    dot.y += dot2.y;
-    // the sums of this token's p . S and of the token BEFORE's S . r ride the same four rounds of shuffles: the latter
-    // are not on the chain from token to token, and a round of their own per token would be
+  float2 o_pend = make_float2(0.f, 0.f);                     // my parts of the token before's S . r, of both columns
+  float* o_at = o_raw + (size_t)r0 * ldo + (size_t)h * Dv + col0 + (sub & 1);      // (lanes sub = 2, 3 write)
+  int stage = 0;
+  for (int i0 = 0; i0 < n; i0 += REC_BATCH) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(REC_STAGES - 2) : "memory");
+    __syncthreads();                                         // this batch is there; the one before is read out
+    issue(stage == 0 ? REC_STAGES - 1 : stage - 1);
+    const float* in = sm + stage * stage_floats;
+    stage = stage == REC_STAGES - 1 ? 0 : stage + 1;
+    const int here = min(REC_BATCH, n - i0);
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-      dot.x += __shfl_xor_sync(0xffffffffu, dot.x, o);
-      dot.y += __shfl_xor_sync(0xffffffffu, dot.y, o);
-      o_pend.x += __shfl_xor_sync(0xffffffffu, o_pend.x, o);
-      o_pend.y += __shfl_xor_sync(0xffffffffu, o_pend.y, o);
-    }
-    if (i > 0 && sub == 0) *reinterpret_cast<float2*>(o_raw + (size_t)(r0 + i - 1) * ldo + (size_t)h * Dv + col0) = o_pend;
-    const float2 v = *reinterpret_cast<const float2*>(in + 5 * D + 2 * cg);
-    float2 o2 = make_float2(0.f, 0.f), o3 = make_float2(0.f, 0.f);
+    for (int u = 0; u < REC_BATCH; ++u, in += pitch) {
+      if (u >= here) break;
+      float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-    for (int c = 0; c < NI; ++c) {
-      const float4 ww = holds ? *reinterpret_cast<const float4*>(in + 64 * c + 4 * sub) : zero;
-      const float4 mm = holds ? *reinterpret_cast<const float4*>(in + 2 * D + 64 * c + 4 * sub) : zero;
-      const float4 kk = holds ? *reinterpret_cast<const float4*>(in + 3 * D + 64 * c + 4 * sub) : zero;
-      const float4 rr = holds ? *reinterpret_cast<const float4*>(in + 4 * D + 64 * c + 4 * sub) : zero;
-      const float we[4] = {ww.x, ww.y, ww.z, ww.w}, me[4] = {mm.x, mm.y, mm.z, mm.w};
-      const float ke[4] = {kk.x, kk.y, kk.z, kk.w}, re[4] = {rr.x, rr.y, rr.z, rr.w};
+      for (int c = 0; c < NI; ++c) {
+        const float4 pp = holds ? *reinterpret_cast<const float4*>(in + D + 64 * c + 4 * sub) : zero;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float2 s = S_r[c][e];
-        s.x = fmaf(ke[e], v.x, fmaf(me[e], dot.x, we[e] * s.x));
-        s.y = fmaf(ke[e], v.y, fmaf(me[e], dot.y, we[e] * s.y));
-        S_r[c][e] = s;
-        if (e & 1) {
-          o3.x = fmaf(s.x, re[e], o3.x);
-          o3.y = fmaf(s.y, re[e], o3.y);
-        } else {
-          o2.x = fmaf(s.x, re[e], o2.x);
-          o2.y = fmaf(s.y, re[e], o2.y);
+        for (int col = 0; col < 2; ++col) {
+          acc[col] = __ffma2_rn(S_r[col][c][0], make_float2(pp.x, pp.y), acc[col]);
+          acc[col] = __ffma2_rn(S_r[col][c][1], make_float2(pp.z, pp.w), acc[col]);
         }
       }
-    }
-    o_pend = make_float2(o2.x + o3.x, o2.y + o3.y);           // joined over the lanes in the next token's rounds
-  }
+      float dx = pair_sum(acc[0]), dy = pair_sum(acc[1]);
+      const float o_before = join_four(dx, dy, o_pend.x, o_pend.y, sub);
+      if (i0 + u > 0) {
+        if ((sub & ~1) == 2) *o_at = o_before;
+        o_at += ldo;
+      }
+      const float2 v = *reinterpret_cast<const float2*>(in + 5 * D + 2 * cg);
+      const float2 d2[2] = {pair_of(dx), pair_of(dy)}, v2[2] = {pair_of(v.x), pair_of(v.y)};
+      float2 o2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-  for (int o = 1; o < 16; o <<= 1) {                           // the last token's
-    o_pend.x += __shfl_xor_sync(0xffffffffu, o_pend.x, o);
-    o_pend.y += __shfl_xor_sync(0xffffffffu, o_pend.y, o);
+      for (int c = 0; c < NI; ++c) {
+        const float4 ww = holds ? *reinterpret_cast<const float4*>(in + 64 * c + 4 * sub) : zero;
+        const float4 mm = holds ? *reinterpret_cast<const float4*>(in + 2 * D + 64 * c + 4 * sub) : zero;
+        const float4 kk = holds ? *reinterpret_cast<const float4*>(in + 3 * D + 64 * c + 4 * sub) : zero;
+        const float4 rr = holds ? *reinterpret_cast<const float4*>(in + 4 * D + 64 * c + 4 * sub) : zero;
+        const float2 wp[2] = {make_float2(ww.x, ww.y), make_float2(ww.z, ww.w)}, mp[2] = {make_float2(mm.x, mm.y), make_float2(mm.z, mm.w)};
+        const float2 kp[2] = {make_float2(kk.x, kk.y), make_float2(kk.z, kk.w)}, rp[2] = {make_float2(rr.x, rr.y), make_float2(rr.z, rr.w)};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int col = 0; col < 2; ++col) {
+            S_r[col][c][e] = __ffma2_rn(kp[e], v2[col], __ffma2_rn(mp[e], d2[col], __fmul2_rn(wp[e], S_r[col][c][e])));
+            o2[col] = __ffma2_rn(S_r[col][c][e], rp[e], o2[col]);
+          }
+      }
+      o_pend = make_float2(pair_sum(o2[0]), pair_sum(o2[1]));       // joined over the lanes in the next token's rounds
+    }
   }
-  if (sub == 0) *reinterpret_cast<float2*>(o_raw + (size_t)(r0 + n - 1) * ldo + (size_t)h * Dv + col0) = o_pend;
+  {
+    float none = 0.f, none2 = 0.f;
+    const float o_last = join_four(none, none2, o_pend.x, o_pend.y, sub);
+    if ((sub & ~1) == 2) *o_at = o_last;
+  }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (write_state && holds) {
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      *reinterpret_cast<float4*>(S_g + 64 * i + 4 * sub) = make_float4(S_r[i][0].x, S_r[i][1].x, S_r[i][2].x, S_r[i][3].x);
-      *reinterpret_cast<float4*>(S_g + D + 64 * i + 4 * sub) = make_float4(S_r[i][0].y, S_r[i][1].y, S_r[i][2].y, S_r[i][3].y);
-    }
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        *reinterpret_cast<float4*>(S_g + c * D + 64 * i + 4 * sub) =
+            make_float4(S_r[c][i][0].x, S_r[c][i][0].y, S_r[c][i][1].x, S_r[c][i][1].y);
   }
 }
 
@@ -284,7 +285,7 @@ int launch_dplr_quad(const float* proj, long ld, const float* prep, long ldp, in
                      const int32_t* seq_q_start, const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state,
                      cudaStream_t stream) {
   const int CB = Dv % 32 == 0 ? 32 : 16;                     // columns per block
-  const size_t smem = (size_t)DPLR_RING * (5 * D + CB) * sizeof(float);
+  const size_t smem = (size_t)REC_STAGES * REC_BATCH * (5 * D + CB) * sizeof(float);       // (at most 32 KB)
   return launch_pdl(PDL_ATTENTION, dplr_recurrence_quad_kernel<D>, dim3(H, n_seqs, Dv / CB), dim3(8 * CB), smem, stream, proj, ld,
                     prep, ldp, H, Dv, state, state_stride, seq_q_start, seq_slot, o_raw, ldo, write_state);
 }
