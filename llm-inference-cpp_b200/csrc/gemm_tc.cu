@@ -317,22 +317,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 //
 //   full[s]      in the leader; 64 KB expected per stage (both SMs' A and B halves)
 //   empty[s]     in each SM; signalled by the leader's tcgen05.commit, multicast to the pair
-//   acc_full[b]  in each SM (multicast commit);  acc_empty[b] in the leader, 8 arrivals (4 warps x 2 SMs)
+//   acc_full[b]  in each SM (multicast commit);  acc_empty[b] in the leader, 16 arrivals (8 warps x 2 SMs)
+//
+// Two groups of four epilogue warps take a tile's chunks of 16 tokens in turn: with one group the way out of a tile was longer
+// than its products where k is short (k = 960, 256 tokens: 5.7 us of MMAs, 16 chunks of 0.4 us), and the last tile's is never
+// hidden.  The first stages' weights are asked for before the wait for the kernel ahead.  Tokens x rows x k, before -> after:
+// 4,860 x 4,096 x 512 45.9 -> 28.8 us, 7,931 x 5,120 x 960 gated 109 -> 65, 2,048 x 5,120 x 960 gated 29.5 -> 25.5, 4,860 x 1,600
+// x 960 21.8 -> 19.6; long k and the residual add unchanged (2,048 x 16,384 x 2,048 101.5 -> 101.2; 4,860 x 960 x 960 16.8 ->
+// 18.2, x 2,560 31.6 -> 32.0).
 constexpr int TP_BN = 256;              // widest token tile; an accumulator's columns in TMEM
 constexpr int TP_STAGES = 6;
 constexpr int TP_STAGE_BYTES = 2 * TC_BM * TC_BK * 2;   // A half-tile + B half-tile, 16 KB each
 constexpr int TP_OUT_BYTES = 16 * TC_BM * 4;             // residual-add epilogue: [16 tokens][128 rows] fp32 on its way out
-constexpr int TP_SMEM = TP_STAGES * TP_STAGE_BYTES + 2 * TP_OUT_BYTES + 1024 + 8 * (2 * TP_STAGES + 4) + 16;
+constexpr int TP_GROUPS = 2;                             // groups of four epilogue warps, which take the chunks of 16 tokens in turn
+constexpr int TP_THREADS = 64 + 128 * TP_GROUPS;
+constexpr int TP_SMEM = TP_STAGES * TP_STAGE_BYTES + 2 * TP_GROUPS * TP_OUT_BYTES + 1024 + 8 * (2 * TP_STAGES + 4) + 16;
 
-__global__ void __launch_bounds__(TC_THREADS)
+__global__ void __launch_bounds__(TP_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                     const __grid_constant__ CUtensorMap map_out, TcParams p, int m_tiles, int n_tiles, int bn,
                     int out_tma) {   // tiles of 256 weight rows x bn tokens (bn % 16 == 0, <= 256); out_tma: map_out describes the output
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t out_smem = base + TP_STAGES * TP_STAGE_BYTES;      // two buffers of TP_OUT_BYTES
+  const uint32_t out_smem = base + TP_STAGES * TP_STAGE_BYTES;      // two buffers of TP_OUT_BYTES per group of epilogue warps
   uint8_t* const out_ptr = smem_raw + (out_smem - smem_u32(smem_raw));   // the same place as a generic address
-  const uint32_t bars = out_smem + 2 * TP_OUT_BYTES;
+  const uint32_t bars = out_smem + 2 * TP_GROUPS * TP_OUT_BYTES;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (TP_STAGES + s); };
   auto acc_full = [&](int b) { return bars + 8u * (2 * TP_STAGES + b); };
@@ -354,7 +363,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full(b), 1);
-      mbar_init(acc_empty(b), 8);
+      mbar_init(acc_empty(b), 8 * TP_GROUPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -374,19 +383,30 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   if (warp == 0) {
     if (lane == 0) {
       // ---- TMA producer (both CTAs): own 128 weight rows and own half of the token tile ----
+      // The weights of the first stages are asked for before the wait: only x comes from the kernel before.
+      const int mine = pair < n_units ? (n_units - pair + n_pairs - 1) / n_pairs : 0;
+      const int total = mine * kblocks, ahead = total < TP_STAGES ? total : TP_STAGES;
+      auto load_w = [&](int it, int u, int i) {
+        const int s = it % TP_STAGES;
+        if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (TC_BM * TC_BK * 2 + (bn >> 1) * TC_BK * 2));
+        tma_load_2d_pair(base + s * TP_STAGE_BYTES, &map_w, i * TC_BK, (u % m_tiles) * 256 + (int)rank * TC_BM, map_to_rank(full_bar(s), 0));
+      };
+      auto load_x = [&](int it, int u, int i) {
+        const int s = it % TP_STAGES;
+        tma_load_2d_pair(base + s * TP_STAGE_BYTES + TC_BM * TC_BK * 2, &map_x, i * TC_BK, (u / m_tiles) * bn + (int)rank * (bn >> 1),
+                         map_to_rank(full_bar(s), 0));
+      };
+      for (int it = 0; it < ahead; ++it) load_w(it, pair + it / kblocks * n_pairs, it % kblocks);
       pdl_wait();
-      int it = 0;
-      bool ok = true;
-      for (int u = pair; u < n_units && ok; u += n_pairs) {
-        const int mt = u % m_tiles, nt = u / m_tiles;
-        for (int i = 0; i < kblocks; ++i, ++it) {
-          const int s = it % TP_STAGES;
-          if (it >= TP_STAGES && !mbar_wait(empty_bar(s), ((it / TP_STAGES) - 1) & 1, p.error_flag, 5)) { ok = false; break; }
-          const uint32_t leader_full = map_to_rank(full_bar(s), 0);
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (TC_BM * TC_BK * 2 + (bn >> 1) * TC_BK * 2));
-          const uint32_t dst = base + s * TP_STAGE_BYTES;
-          tma_load_2d_pair(dst, &map_w, i * TC_BK, mt * 256 + (int)rank * TC_BM, leader_full);
-          tma_load_2d_pair(dst + TC_BM * TC_BK * 2, &map_x, i * TC_BK, nt * bn + (int)rank * (bn >> 1), leader_full);
+      for (int it = 0; it < ahead; ++it) load_x(it, pair + it / kblocks * n_pairs, it % kblocks);
+      int u = pair + ahead / kblocks * n_pairs, i = ahead % kblocks;
+      for (int it = ahead; it < total; ++it) {
+        if (!mbar_wait(empty_bar(it % TP_STAGES), ((it / TP_STAGES) - 1) & 1, p.error_flag, 5)) break;
+        load_w(it, u, i);
+        load_x(it, u, i);
+        if (++i == kblocks) {
+          i = 0;
+          u += n_pairs;
         }
       }
     }
@@ -417,10 +437,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
     }
   } else {
-    // ---- epilogue warps (both CTAs): this CTA's 128 rows x 256 tokens ----
-    const int quad = warp & 3;
+    // ---- epilogue warps (both CTAs): this CTA's 128 rows x 256 tokens, 16 tokens at a time, the groups in turn ----
+    const int quad = warp & 3, group = (warp - 2) >> 2;
+    const bool sends = ((warp - 2) & 3) == 0 && lane == 0;      // the thread of a group that issues and waits for its copies
     pdl_wait();
-    int j = 0, n_out = 0;       // n_out: chunks this CTA has sent out through shared memory (residual-add epilogue)
+    int j = 0, n_out = 0;       // n_out: chunks this group has sent out through shared memory
     for (int u = pair; u < n_units; u += n_pairs, ++j) {
       const int mt = u % m_tiles, nt = u / m_tiles;
       const int b = j & 1;
@@ -431,6 +452,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       if (!mbar_wait(acc_full(b), (j >> 1) & 1, p.error_flag, 8)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int nch = (min(bn, p.n_tok - n0) + 15) / 16;
+      if (group >= nch && lane == 0) mbar_arrive_remote(leader_empty);      // (nothing for this group in a tile of so few tokens)
       if (out_tma) {
         // The tile goes out through shared memory, 16 tokens at a time ([16 tokens][128 rows] in the output's type,
         // gated: [16][64 features]; two buffers), and is stored by TMA — for the residual stream ADDED by TMA
@@ -441,21 +463,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // Rows and tokens past the ends of `out` are clipped by the copy.
         const float bias = (p.bias && m < p.m_out) ? p.bias[m] : 0.f, os = (p.oscale && m < p.m_out) ? p.oscale[m] : 1.f;
         const int row_in_cta = quad * 32 + lane;
-        for (int ci = 0; ci < nch; ++ci) {
+        for (int ci = group; ci < nch; ci += TP_GROUPS) {
           float v[16];
           tmem_ld16(t_base + ci * 16, v);
-          if (ci == nch - 1) {
+          if (ci + TP_GROUPS >= nch) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(leader_empty);
           }
-          const uint32_t buf_off = (uint32_t)((n_out & 1) * TP_OUT_BYTES);
+          const uint32_t buf_off = (uint32_t)((2 * group + (n_out & 1)) * TP_OUT_BYTES);
           const uint32_t buf = out_smem + buf_off;
           uint8_t* const bufp = out_ptr + buf_off;
           if (n_out >= 2) {
             // the copy that read this buffer two chunks ago has to be done with it
-            if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (sends) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
           }
           if (p.mode == OUT_SWIGLU) {
             // rows alternate gate and up (src/model/transformer.cpp:290; src/model/kernels.cpp:148): the even lane finishes
@@ -485,8 +507,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             for (int c = 0; c < 16; ++c) o[c * TC_BM] = (v[c] + bias) * os;
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (warp == 2 && lane == 0) {
+          asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
+          if (sends) {
             const int r0 = mt * 256 + (int)rank * TC_BM;
             const int c0 = p.mode == OUT_SWIGLU ? (r0 >> 1) : r0;
             if (p.mode == OUT_ADD_F32)
@@ -503,10 +525,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           ++n_out;
         }
       } else {
-        for (int ci = 0; ci < nch; ++ci) {
+        for (int ci = group; ci < nch; ci += TP_GROUPS) {
           float v[16];
           tmem_ld16(t_base + ci * 16, v);
-          if (ci == nch - 1) {
+          if (ci + TP_GROUPS >= nch) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(leader_empty);
@@ -516,7 +538,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
     }
     // the additions still on their way read this CTA's shared memory: they are done before anybody leaves
-    if (warp == 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    if (sends) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   // nobody leaves while its partner may still signal it or read its shared memory
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -570,7 +592,7 @@ static int launch_tc_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CU
   const long pairs = n_units < n_pairs ? n_units : n_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs));
-  cfg.blockDim = dim3(TC_THREADS);
+  cfg.blockDim = dim3(TP_THREADS);
   cfg.dynamicSmemBytes = TP_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
