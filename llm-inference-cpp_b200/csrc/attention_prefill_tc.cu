@@ -47,22 +47,25 @@ namespace llmi {
 
 constexpr int FT_BM = 128, FT_PAGE = 64;
 constexpr int FT_SUB = FT_PAGE * 64 * 2;              // 8 KB: 64 rows x 64 columns of bf16, one swizzled sub-tile
-constexpr int FT_TMEM_COLS = 256;                     // S_j (then P_j) at columns 64 * (j & 1); O of key half h at 128 + HD * h
+constexpr int FT_TMEM_COLS = 256;                     // S_j (then P_j) at columns 64 * (j & 1); O of key half h at 128 + DV * h
 constexpr float FT_LAZY = 8.0f;                       // the reference maximum follows the running one in steps of 2^8
 
-// Head size 64: two softmax threads per query row (HALVES = 2), each with 32 keys of a page and an O of 64 columns.
-// Head size 128: one thread per row with all 64 keys and an O of 128 columns.  Either way S0, S1 and O fill 256
-// TMEM columns and two blocks are resident per SM.
-template <int HD>
+// Values of size 64: two softmax threads per query row (HALVES = 2), each with 32 keys of a page and an O of 64 columns.
+// Of size 128: one thread per row with all 64 keys and an O of 128 columns.  Either way S0, S1 and O fill 256
+// TMEM columns and two blocks are resident per SM.  Keys of 64 with values of 128 are the two maps of a differential head.
+// (Several maps a head, values of their own size and factors per head came here from the mma.sync tiles of attention_maps_mma.cu:
+// two prompts of 701 and 1,900 tokens, 2 x 16 maps of 64 over values of 128 and 32 heads of 64 with factors took 468 and 263 us a
+// layer there; a whole request step of eight such layers' model 11.2 -> 9.9 ms.)
+template <int DK, int DV>
 struct FtCfg {
-  static constexpr int NSUB = HD / 64;                        // 64-column sub-tiles of a Q, K or V tile
-  static constexpr int HALVES = 128 / HD;
+  static constexpr int KSUB = DK / 64, VSUB = DV / 64;        // 64-column sub-tiles of a Q or K, and of a V tile
+  static constexpr int HALVES = 128 / DV;
   static constexpr int KEYS = FT_PAGE / HALVES;               // keys of a page per softmax thread
   static constexpr int THREADS = 64 + 128 * HALVES;           // producer warp, MMA warp, 4 * HALVES softmax warps
-  static constexpr int STAGES = HD == 64 ? 3 : 2;
-  static constexpr int TILE = NSUB * FT_SUB;                  // one K or V page
-  static constexpr int QBYTES = 2 * NSUB * FT_SUB;            // 128 query rows
-  static constexpr int SMEM = QBYTES + STAGES * 2 * TILE + 1024 + 128;
+  static constexpr int STAGES = DK == 64 ? 3 : 2;
+  static constexpr int K_TILE = KSUB * FT_SUB, STAGE = (KSUB + VSUB) * FT_SUB;      // a K page; K and V
+  static constexpr int QBYTES = 2 * KSUB * FT_SUB;            // 128 query rows
+  static constexpr int SMEM = QBYTES + STAGES * STAGE + 1024 + 128;
 };
 
 struct PrefillTcParams {
@@ -79,7 +82,7 @@ struct PrefillTcParams {
   int* error_flag;
   int n_tiles;              // blocks of 128 queries over all sequences
   int split_pages;          // 0: a query block's keys are one job; else jobs of at most this many pages
-  float* partials;          // [job (gridDim.y)][head][HD + 2][128]: per row m_ref, l, O[HD], when split
+  float* partials;          // [job (gridDim.y)][head][DV + 2][128]: per row m_ref, l, O[DV], when split
   int* tickets;             // [n_tiles * n_heads], zero before and after the launch
   // Pooled blocks ahead of the window (pool > 0, window > 0): block b of `pool` positions has ONE key and value row, row b
   // of the sequence's pooled pages (a cache and page table of their own); the query at position p sees the blocks with
@@ -92,6 +95,10 @@ struct PrefillTcParams {
   const float* r1;          // [n_heads] fp32 or null: the bias by distance (base 2: r1 * log2(1 + r2 * d))
   const float* r2;
   const float* sink;        // [n_heads] fp32 or null
+  // `maps` score maps per head over the same values: query row [head][map][DK], key heads [kv head][map], out [head][map][DV]
+  int maps;
+  int out_f32;              // the output is fp32
+  const float* head_scale;  // [n_heads] fp32 or null: the head's scores times it (of any sign)
 };
 
 __device__ __forceinline__ void ft_tma(uint32_t dst, const CUtensorMap* map, int col, int row, uint32_t bar) {
@@ -156,18 +163,18 @@ __device__ __forceinline__ void ft_st16u(uint32_t taddr, const uint32_t* v) {
       : "memory");
 }
 
-template <int HD, bool BIAS>
-__global__ void __launch_bounds__(FtCfg<HD>::THREADS, 2)
+template <int DK, int DV, bool BIAS>
+__global__ void __launch_bounds__(FtCfg<DK, DV>::THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_kp,
                             const __grid_constant__ CUtensorMap map_vp, PrefillTcParams p) {
-  using C = FtCfg<HD>;
-  constexpr int STAGES = C::STAGES, NSUB = C::NSUB, HALVES = C::HALVES, KEYS = C::KEYS;
+  using C = FtCfg<DK, DV>;
+  constexpr int STAGES = C::STAGES, KSUB = C::KSUB, VSUB = C::VSUB, HALVES = C::HALVES, KEYS = C::KEYS;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_smem = base;                                      // sub-tile u (dims 64u..): + u * 16 KB
-  const uint32_t kv_smem = base + C::QBYTES;                         // stage s: K at + s * 2 * TILE, V a TILE further
-  const uint32_t bars = kv_smem + STAGES * 2 * C::TILE;
+  const uint32_t kv_smem = base + C::QBYTES;                         // stage s: K at + s * STAGE, V K_TILE further
+  const uint32_t bars = kv_smem + STAGES * C::STAGE;
   // barriers: q_full, kv_full[stages], kv_empty[stages], s_full[2], p_ready[2], o_done, tmem slot
   const uint32_t q_full = bars;
   auto kv_full = [&](int s) { return bars + 8u * (1 + s); };
@@ -223,8 +230,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
   // page j of this part: pooled page v_first + j while that is below n_ppg, else token page pg_first + (v_first + j - n_ppg)
   const int32_t* ppages = p.pool > 0 ? p.pool_pages + (size_t)seq * p.pool_pages_stride : nullptr;
-  const int head = blockIdx.x;
-  const int kvh = head / (p.n_heads / p.n_kv_heads);
+  const int head = blockIdx.x;             // (of maps heads each: the head's map)
+  const int real_head = head / p.maps, v_head = real_head / (p.n_heads / p.n_kv_heads), k_head = v_head * p.maps + head % p.maps;
   const int32_t* pages = p.seq_pages + (size_t)seq * p.pages_stride;
   __shared__ int s_last;
   __shared__ float bias_s[BIAS ? 4 * HALVES * (31 + KEYS + 1) : 1];
@@ -271,21 +278,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       pdl_wait();   // q and the cache pages of this step come from the kernels before
       mbar_expect_tx(q_full, C::QBYTES);
 #pragma unroll
-      for (int u = 0; u < NSUB; ++u) ft_tma(q_smem + u * 2 * FT_SUB, &map_q, head * HD + 64 * u, q_start + m0, q_full);
+      for (int u = 0; u < KSUB; ++u) ft_tma(q_smem + u * 2 * FT_SUB, &map_q, head * DK + 64 * u, q_start + m0, q_full);
       for (int j = 0; j < n_pg; ++j) {
         const int s = j % STAGES;
         if (j >= STAGES && !mbar_wait(kv_empty(s), ((j / STAGES) - 1) & 1, p.error_flag, 41)) break;
         const int v = v_first + j;
         const bool pooled = v < n_ppg;
-        const int row = ((pooled ? ppages[v] : pages[pg_first + v - n_ppg]) * p.n_kv_heads + kvh) * FT_PAGE;
+        const int page = pooled ? ppages[v] : pages[pg_first + v - n_ppg];
+        const int k_row = (page * p.n_kv_heads * p.maps + k_head) * FT_PAGE, v_row = (page * p.n_kv_heads + v_head) * FT_PAGE;
         const CUtensorMap* mk = pooled ? &map_kp : &map_k;
         const CUtensorMap* mv = pooled ? &map_vp : &map_v;
-        mbar_expect_tx(kv_full(s), 2 * C::TILE);
+        mbar_expect_tx(kv_full(s), C::STAGE);
 #pragma unroll
-        for (int u = 0; u < NSUB; ++u) {
-          ft_tma(kv_smem + s * 2 * C::TILE + u * FT_SUB, mk, 64 * u, row, kv_full(s));
-          ft_tma(kv_smem + s * 2 * C::TILE + C::TILE + u * FT_SUB, mv, 64 * u, row, kv_full(s));
-        }
+        for (int u = 0; u < KSUB; ++u) ft_tma(kv_smem + s * C::STAGE + u * FT_SUB, mk, 64 * u, k_row, kv_full(s));
+#pragma unroll
+        for (int u = 0; u < VSUB; ++u) ft_tma(kv_smem + s * C::STAGE + C::K_TILE + u * FT_SUB, mv, 64 * u, v_row, kv_full(s));
       }
     }
   } else if (warp == 1) {
@@ -300,8 +307,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       auto issue_s = [&](int j) {
         const uint32_t d = tmem_s + (uint32_t)(64 * (j & 1));
 #pragma unroll
-        for (int k4 = 0; k4 < HD / 16; ++k4) {
-          const uint64_t a = ft_desc(q_smem + (k4 / 4) * 2 * FT_SUB), b = ft_desc(kv_smem + (j % STAGES) * 2 * C::TILE + (k4 / 4) * FT_SUB);
+        for (int k4 = 0; k4 < DK / 16; ++k4) {
+          const uint64_t a = ft_desc(q_smem + (k4 / 4) * 2 * FT_SUB), b = ft_desc(kv_smem + (j % STAGES) * C::STAGE + (k4 / 4) * FT_SUB);
           ft_mma(d, a + 2 * (k4 % 4), b + 2 * (k4 % 4), idesc_s, k4 > 0);
         }
         ft_commit(s_full(j & 1));
@@ -323,7 +330,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a = tmem_s + (uint32_t)(64 * (j & 1));
-        const uint32_t v_tile = kv_smem + (j % STAGES) * 2 * C::TILE + C::TILE;
+        const uint32_t v_tile = kv_smem + (j % STAGES) * C::STAGE + C::K_TILE;
         // the keys of half h accumulate into their own O (their softmax threads keep their own reference maximum):
         // P of half h lies at columns 32h.. of the S buffer; 16 keys further: 8 columns of P, 16 rows of 128 bytes of V
 #pragma unroll
@@ -331,8 +338,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
           for (int k4 = 0; k4 < KEYS / 16; ++k4)
 #pragma unroll
-            for (int u = 0; u < NSUB; ++u)
-              ft_mma_ts(tmem_o + (uint32_t)(HD * h + 64 * u), a + (uint32_t)(32 * h + 8 * k4),
+            for (int u = 0; u < VSUB; ++u)
+              ft_mma_ts(tmem_o + (uint32_t)(DV * h + 64 * u), a + (uint32_t)(32 * h + 8 * k4),
                         ft_desc(v_tile + u * FT_SUB) + (uint64_t)(((KEYS / 16) * h + k4) * ((16 * 128) >> 4)), idesc_o,
                         (j > 0 || k4 > 0) ? 1u : 0u);
         ft_commit(o_done);
@@ -350,10 +357,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const bool row_ok = qrow < q_len;
     const int qpos = pos0 + qrow;
     const uint32_t t_lane = (uint32_t)(quad * 32) << 16;
-    const uint32_t t_o = tmem_o + t_lane + (uint32_t)(HD * half);
+    const uint32_t t_o = tmem_o + t_lane + (uint32_t)(DV * half);
     float m_run = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // maxima in base 2, scaled
     float* bias_w = bias_s + (BIAS ? (warp - 2) * (31 + KEYS + 1) : 0);
     const float r1 = BIAS ? p.r1[head] : 0.f, r2 = BIAS ? p.r2[head] : 0.f;      // (weights: no kernel before writes them)
+    // A head's own factor: its size goes into the scale (never quite 0: 0 times a masked key's -inf is no number), its sign
+    // into the scores.
+    float scale_log2 = p.scale_log2;
+    bool flip = false;
+    if (!BIAS && p.head_scale) {
+      const float f = p.head_scale[real_head];
+      flip = f < 0.f;
+      scale_log2 = fmaxf(fabsf(f) * scale_log2, 1e-30f);
+    }
     bool ok = true;
     for (int j = 0; j < n_pg && ok; ++j) {
       ok = mbar_wait(s_full(j & 1), (j >> 1) & 1, p.error_flag, 48);
@@ -364,6 +380,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
       for (int c = 0; c < KEYS; c += 16) ft_ld16(t_s + (uint32_t)c, sc + c);
       ft_ld_wait();
+      if (flip) {
+#pragma unroll
+        for (int c = 0; c < KEYS; ++c) sc[c] = -sc[c];
+      }
       const int v = v_first + j;
       const bool pooled = v < n_ppg;
       // a pooled page: `page_key0` counts blocks; its rows from the first one that no query of this block sees are unused
@@ -395,7 +415,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
         for (int c = 0; c < KEYS; ++c) sc[c] = fmaf(sc[c], p.scale_log2, -bias_l[-c]);
       }
-      const float to_log2 = BIAS ? 1.0f : p.scale_log2;
+      const float to_log2 = BIAS ? 1.0f : scale_log2;
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains instead of one long one
 #pragma unroll
       for (int c = 0; c < KEYS; c += 8) {
@@ -440,7 +460,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           // this half's O is rescaled in place
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-          for (int c = 0; c < HD; c += 16) {
+          for (int c = 0; c < DV; c += 16) {
             float t[16];
             ft_ld16(t_o + (uint32_t)c, t);
             ft_ld_wait();
@@ -458,10 +478,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (page_key0 + FT_PAGE > rows_end) {
         // The sequence ends inside this page: value rows behind its end are cleared so that their zero
         // probabilities cannot meet a NaN.  (The page is in shared memory: S_j was computed from it.)
-        const uint32_t v_tile = kv_smem + (j % STAGES) * 2 * C::TILE + C::TILE;
+        const uint32_t v_tile = kv_smem + (j % STAGES) * C::STAGE + C::K_TILE;
         const int first_bad = rows_end - page_key0;
-        for (int idx = (warp - 2) * 32 + lane; idx < (FT_PAGE - first_bad) * 8 * NSUB; idx += 128 * HALVES) {
-          const int r = first_bad + (idx >> 3) / NSUB, u = (idx >> 3) % NSUB, ch = idx & 7;
+        for (int idx = (warp - 2) * 32 + lane; idx < (FT_PAGE - first_bad) * 8 * VSUB; idx += 128 * HALVES) {
+          const int r = first_bad + (idx >> 3) / VSUB, u = (idx >> 3) % VSUB, ch = idx & 7;
           asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(v_tile + (uint32_t)(u * FT_SUB + r * 128 + (ch << 4))), "r"(0u) : "memory");
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA's reads
@@ -477,7 +497,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // A row's halves meet: (reference maximum, sum) through shared memory, the O's straight from TMEM; each of the
       // row's threads finishes DH of the output dims, 32 at a time.
-      constexpr int DH = HD / HALVES;
+      constexpr int DH = DV / HALVES;
       float M = m_ref, L = l_run, w_a = 1.f, w_b = 0.f;
       if (HALVES == 2) {
         s_ml[half][row][0] = m_ref;
@@ -490,12 +510,13 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         L = s_ml[0][row][1] * w_a + s_ml[1][row][1] * w_b;
       }
       const uint32_t t_mine = tmem_o + t_lane + (uint32_t)(DH * half);          // this thread's dims in the first O
-      const size_t slot_floats = (size_t)(HD + 2) * FT_BM;
-      const size_t part_stride = (size_t)p.n_heads * slot_floats;
+      const size_t slot_floats = (size_t)(DV + 2) * FT_BM;
+      const int all_heads = p.n_heads * p.maps;
+      const size_t part_stride = (size_t)all_heads * slot_floats;
       bool write_out = fine, merge = false;
       if (n_parts > 1) {
         // this part's (maximum, sum, O) to the workspace; the part that comes last adds them all in key order
-        float* mine = p.partials + ((size_t)job * p.n_heads + head) * slot_floats + row;
+        float* mine = p.partials + ((size_t)job * all_heads + head) * slot_floats + row;
         if (half == 0) {
           mine[0] = M;
           mine[FT_BM] = L;
@@ -506,8 +527,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           ft_ld16(t_mine + (uint32_t)c0, oa);
           ft_ld16(t_mine + (uint32_t)(c0 + 16), oa + 16);
           if (HALVES == 2) {
-            ft_ld16(t_mine + (uint32_t)(HD + c0), ob);
-            ft_ld16(t_mine + (uint32_t)(HD + c0 + 16), ob + 16);
+            ft_ld16(t_mine + (uint32_t)(DV + c0), ob);
+            ft_ld16(t_mine + (uint32_t)(DV + c0 + 16), ob + 16);
           }
           ft_ld_wait();
 #pragma unroll
@@ -516,14 +537,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
         __threadfence();
         asm volatile("bar.sync 1, %0;" ::"n"(128 * HALVES) : "memory");
-        int* ticket = p.tickets + tile_id * p.n_heads + head;
+        int* ticket = p.tickets + tile_id * all_heads + head;
         if (threadIdx.x == 64) s_last = (atomicAdd(ticket, 1) == n_parts - 1);
         asm volatile("bar.sync 1, %0;" ::"n"(128 * HALVES) : "memory");
         merge = s_last != 0;
         write_out = fine && merge;
         if (merge) {
           __threadfence();
-          const float* first = p.partials + ((size_t)(job - part) * p.n_heads + head) * slot_floats + row;
+          const float* first = p.partials + ((size_t)(job - part) * all_heads + head) * slot_floats + row;
           M = -INFINITY;
           for (int z = 0; z < n_parts; ++z) M = fmaxf(M, __ldcg(first + z * part_stride));
           L = 0.f;
@@ -537,12 +558,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (write_out) {      // every lane takes part in the TMEM loads; only the rows that exist are stored
         float inv = 1.f / (p.sink ? L + fast_exp2(p.sink[head] * 1.4426950408889634f - M) : L);
         if (p.gate && row_ok) inv *= 1.0f / (1.0f + expf(-p.gate[(size_t)(q_start + qrow) * p.ldg + head]));
-        __nv_bfloat16* dst = p.out + (size_t)(q_start + qrow) * p.ldo + (size_t)head * HD + DH * half;
+        const size_t at = (size_t)(q_start + qrow) * p.ldo + (size_t)head * DV + DH * half;
+        __nv_bfloat16* dst = p.out + at;
+        float* dst_f = reinterpret_cast<float*>(p.out) + at;
 #pragma unroll 1
         for (int c0 = 0; c0 < DH; c0 += 32) {
           float o[32];
           if (merge) {
-            const float* first = p.partials + ((size_t)(job - part) * p.n_heads + head) * slot_floats + row;
+            const float* first = p.partials + ((size_t)(job - part) * all_heads + head) * slot_floats + row;
 #pragma unroll
             for (int c = 0; c < 32; ++c) o[c] = 0.f;
             for (int z = 0; z < n_parts; ++z) {
@@ -557,14 +580,20 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             ft_ld16(t_mine + (uint32_t)c0, o);
             ft_ld16(t_mine + (uint32_t)(c0 + 16), o + 16);
             if (HALVES == 2) {
-              ft_ld16(t_mine + (uint32_t)(HD + c0), ob);
-              ft_ld16(t_mine + (uint32_t)(HD + c0 + 16), ob + 16);
+              ft_ld16(t_mine + (uint32_t)(DV + c0), ob);
+              ft_ld16(t_mine + (uint32_t)(DV + c0 + 16), ob + 16);
             }
             ft_ld_wait();
             if (HALVES == 2) {
 #pragma unroll
               for (int c = 0; c < 32; ++c) o[c] = w_a * o[c] + w_b * ob[c];
             }
+          }
+          if (p.out_f32) {
+#pragma unroll
+            for (int c = 0; c < 32 && row_ok; c += 4)
+              *reinterpret_cast<float4*>(dst_f + c0 + c) = make_float4(o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv);
+            continue;
           }
 #pragma unroll
           for (int c = 0; c < 32 && row_ok; c += 8) {
@@ -617,28 +646,31 @@ static int ft_make_map(CUtensorMap* map, const void* ptr, long rows, long cols, 
 using namespace llmi;
 
 LLMI_EXPORT int llmi_attention_prefill_tc_supported(int head_dim) { return head_dim == 64 || head_dim == 128; }
+// Keys and values of different sizes, several maps a head: keys of 64 with values of 64 or 128, 128 with 128.
+LLMI_EXPORT int llmi_attention_prefill_tc_sizes(int dk, int dv) { return (dk == 64 && (dv == 64 || dv == 128)) || (dk == 128 && dv == 128); }
 
 namespace llmi {
-template <int HD, bool BIAS>
+template <int DK, int DV, bool BIAS>
 static int ft_launch_b(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkp,
                      const CUtensorMap& mvp, const PrefillTcParams& p, dim3 grid, cudaStream_t stream) {
-  using C = FtCfg<HD>;
+  using C = FtCfg<DK, DV>;
   static PerDevice<bool> configured_on;
   bool& configured = configured_on.here();
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<DK, DV, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
       return LLMI_ERR_LAUNCH;
     configured = true;
   }
   // a programmatic dependent: its blocks set themselves up (barriers, tensor memory, descriptors) while the kernel
   // before drains; the producer waits before its first copy, and nothing else reads or writes global memory earlier
-  return launch_pdl(PDL_ATTENTION, attention_prefill_tc_kernel<HD, BIAS>, grid, dim3(C::THREADS), C::SMEM, stream, mq, mk, mv, mkp, mvp, p);
+  return launch_pdl(PDL_ATTENTION, attention_prefill_tc_kernel<DK, DV, BIAS>, grid, dim3(C::THREADS), C::SMEM, stream, mq, mk, mv, mkp, mvp, p);
 }
-template <int HD>
+template <int DK, int DV>
 static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkp,
                      const CUtensorMap& mvp, const PrefillTcParams& p, dim3 grid, cudaStream_t stream) {
-  if (p.r1) return ft_launch_b<HD, true>(mq, mk, mv, mkp, mvp, p, grid, stream);
-  const int rc = ft_launch_b<HD, false>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  if constexpr (DK == DV)
+    if (p.r1) return ft_launch_b<DK, DV, true>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  const int rc = ft_launch_b<DK, DV, false>(mq, mk, mv, mkp, mvp, p, grid, stream);
   pairs_may_start_early = true;
   return rc;
 }
@@ -651,7 +683,11 @@ static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 // keys.  gate (optional): fp32 [n_tokens, ldg], head h's output is multiplied by logistic(gate[t, h]).  r1, r2 (optional, not
 // with pooled rows): fp32 [n_heads], a key d positions back loses r1 * ln(1 + r2 * d) of its score; sink (optional): fp32
 // [n_heads], exp(sink) joins the head's softmax sum.
-// With split_pages > 0: partials holds n_jobs * n_heads * (head_dim + 2) * 128 floats.
+// maps > 1: that many score maps per head over the same values (query row [head][map][head_dim], key heads [kv head][map],
+// out [head][map][v_dim]); v_dim: the values' size; out_f32: the output is fp32 (ldo in its elements); head_scale (or null,
+// not with r1): fp32 [n_heads], multiplies a head's scores.  None of them with pooled rows, and maps and v_dim != head_dim
+// neither with gate, r1 or sink.
+// With split_pages > 0: partials holds n_jobs * n_heads * maps * (v_dim + 2) * 128 floats.
 LLMI_EXPORT int llmi_attention_prefill_tc(const void* q, long ldq, long n_tokens, void* out, long ldo, const void* k_cache,
                                           const void* v_cache, long n_cache_pages, const int32_t* seq_pages,
                                           int pages_stride, const int32_t* seq_q_start, const int32_t* seq_kv_len,
@@ -660,23 +696,26 @@ LLMI_EXPORT int llmi_attention_prefill_tc(const void* q, long ldq, long n_tokens
                                           int* tickets, int n_tickets, int* error_flag, int pool, const void* k_pool,
                                           const void* v_pool, long n_pool_cache_pages, const int32_t* pool_pages,
                                           int pool_pages_stride, const float* gate, long ldg, const float* r1, const float* r2,
-                                          const float* sink, cudaStream_t stream) {
+                                          const float* sink, int maps, int v_dim, int out_f32, const float* head_scale,
+                                          cudaStream_t stream) {
   if (n_seqs <= 0 || n_blocks <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0 || n_tokens <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads) return LLMI_ERR_BAD_SIZE;
-  if (!llmi_attention_prefill_tc_supported(head_dim)) return LLMI_ERR_UNSUPPORTED;
+  if (!llmi_attention_prefill_tc_sizes(head_dim, v_dim) || maps < 1 || maps > 16 || n_heads > 0x7fff) return LLMI_ERR_UNSUPPORTED;
+  if ((maps > 1 || v_dim != head_dim) && (pool > 0 || gate || r1 || sink)) return LLMI_ERR_UNSUPPORTED;
+  if (head_scale && (r1 || pool > 0 || scale <= 0.f)) return LLMI_ERR_UNSUPPORTED;
   if ((r1 == nullptr) != (r2 == nullptr) || (r1 && scale <= 0.f)) return LLMI_ERR_BAD_SIZE;
   if (r1 && pool > 0) return LLMI_ERR_UNSUPPORTED;            // a pooled row has no distance
   if (((uintptr_t)q & 15) || (ldq & 7) || ((uintptr_t)out & 15) || (ldo & 7) || ((uintptr_t)k_cache & 15) ||
       ((uintptr_t)v_cache & 15))
     return LLMI_ERR_ALIGN;
   const long rows = n_cache_pages * n_kv_heads * FT_PAGE;
-  if (rows > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;
+  if (rows * maps > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;
   CUtensorMap mq, mk, mv;
-  int rc = ft_make_map(&mq, q, n_tokens, (long)n_heads * head_dim, ldq, FT_BM);
+  int rc = ft_make_map(&mq, q, n_tokens, (long)n_heads * maps * head_dim, ldq, FT_BM);
   if (rc != LLMI_OK) return rc;
-  rc = ft_make_map(&mk, k_cache, rows, head_dim, head_dim, FT_PAGE);
+  rc = ft_make_map(&mk, k_cache, rows * maps, head_dim, head_dim, FT_PAGE);
   if (rc != LLMI_OK) return rc;
-  rc = ft_make_map(&mv, v_cache, rows, head_dim, head_dim, FT_PAGE);
+  rc = ft_make_map(&mv, v_cache, rows, v_dim, v_dim, FT_PAGE);
   if (rc != LLMI_OK) return rc;
   CUtensorMap mkp = mk, mvp = mv;
   if (pool > 0) {
@@ -695,16 +734,17 @@ LLMI_EXPORT int llmi_attention_prefill_tc(const void* q, long ldq, long n_tokens
   // n_jobs: blocks along y — n_blocks without a split, else the sum over the query blocks of their parts (the caller
   // counts them with the same rule as the kernel); the workspace holds one slot per job and head
   if (split_pages > 0) {
-    if (n_jobs < n_blocks || !partials || !tickets || (long)n_jobs * n_heads * (head_dim + 2) * FT_BM > partials_floats ||
-        (long)n_blocks * n_heads > n_tickets)
+    if (n_jobs < n_blocks || !partials || !tickets || (long)n_jobs * n_heads * maps * (v_dim + 2) * FT_BM > partials_floats ||
+        (long)n_blocks * n_heads * maps > n_tickets)
       return LLMI_ERR_BAD_SIZE;
   } else {
     n_jobs = n_blocks;
   }
   PrefillTcParams p{(__nv_bfloat16*)out, ldo, seq_pages, seq_q_start, seq_kv_len, pages_stride, n_seqs, n_heads,
                     n_kv_heads, scale * 1.4426950408889634f, window, error_flag, n_blocks, split_pages, partials, tickets,
-                    pool, pool_pages, pool_pages_stride, gate, ldg, r1, r2, sink};
+                    pool, pool_pages, pool_pages_stride, gate, ldg, r1, r2, sink, maps, out_f32 ? 1 : 0, head_scale};
   if (n_jobs > 65535) return LLMI_ERR_BAD_SIZE;
-  dim3 grid(n_heads, n_jobs);
-  return head_dim == 64 ? ft_launch<64>(mq, mk, mv, mkp, mvp, p, grid, stream) : ft_launch<128>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  dim3 grid(n_heads * maps, n_jobs);
+  if (head_dim == 128) return ft_launch<128, 128>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  return v_dim == 64 ? ft_launch<64, 64>(mq, mk, mv, mkp, mvp, p, grid, stream) : ft_launch<64, 128>(mq, mk, mv, mkp, mvp, p, grid, stream);
 }

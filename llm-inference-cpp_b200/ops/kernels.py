@@ -155,7 +155,8 @@ def lib():
                      "llmi_attention_decode_fused", "llmi_attention_decode_mma", "llmi_attention_decode_mma_supported",
                      "llmi_attention_decode_mma_resident", "llmi_attention_decode_clusters_resident",
                      "llmi_attention_prefill", "llmi_attention_prefill_supported", "llmi_gemm_skinny",
-                     "llmi_gemm_skinny_max_tokens", "llmi_attention_prefill_tc", "llmi_attention_prefill_tc_supported", "llmi_attention_short",
+                     "llmi_gemm_skinny_max_tokens", "llmi_attention_prefill_tc", "llmi_attention_prefill_tc_supported",
+                     "llmi_attention_prefill_tc_sizes", "llmi_attention_short",
                      "llmi_attention_short_supported",
                      "llmi_sm_count", "llmi_dyt", "llmi_dyt_add", "llmi_stream_add", "llmi_linear_simt_batched",
                      "llmi_attention_expanded",
@@ -182,7 +183,7 @@ def lib():
         l.llmi_gemm_tc.argtypes = [P, L, P, L, P, P, L, I, I, I, I, P, L, P, I, P, P, F, F, P]
         l.llmi_rmsnorm.argtypes = [I, P, P, P, P, I, I, F, P]
         l.llmi_rope_store.argtypes = [I, P, L, P, I, P, P, P, I, I, P, P, I, I, I, I, I, P]
-        l.llmi_attention_prefill_tc.argtypes = [P, L, L, P, L, P, P, L, P, I, P, P, I, I, I, I, I, F, I, I, I, P, L, P, I, P, I, P, P, L, P, I, P, L, P, P, P, P]
+        l.llmi_attention_prefill_tc.argtypes = [P, L, L, P, L, P, P, L, P, I, P, P, I, I, I, I, I, F, I, I, I, P, L, P, I, P, I, P, P, L, P, I, P, L, P, P, P, I, I, I, P, P]
         _configured = True
     return l
 
@@ -860,8 +861,11 @@ def prefill_split_jobs(q_lens, kv_lens, window: int, split_pages: int, pool: int
 
 def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len,
                          n_blocks: int, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0,
-                         split=None, pooled=None, gate=None, bias=None, sink=None) -> None:
+                         split=None, pooled=None, gate=None, bias=None, sink=None, maps: int = 1, v_dim: int | None = None,
+                         head_scale=None) -> None:
     """The same prompt attention on the tcgen05 tensor cores (head size 64 or 128); arguments as ``attention_prefill``.
+    ``maps``, ``v_dim`` and an fp32 ``out``: that many score maps per head over the same values of their own size (the layouts
+    of :func:`attention_maps`; without pooled rows, gate, bias, sink); ``head_scale`` fp32 [n_heads]: a head's scores times it.
     ``pooled = (pool, k_pool, v_pool, pool_pages)``: beside its window a query sees one pooled row per block of ``pool``
     positions that lies wholly before the window (row b of the sequence's pooled pages is block b; caches shaped as the
     token caches).  ``gate``: fp32 [tokens, >= n_heads]; head h's output is multiplied by logistic(gate[t, h]).
@@ -871,7 +875,10 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, s
     n_jobs * n_heads * (head_dim + 2) * 128 floats)."""
     _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)
     S = seq_pages.shape[0]
-    assert q.dtype == out.dtype == k_cache.dtype == torch.bfloat16 and q.stride(1) == 1 and out.stride(1) == 1
+    v_dim = head_dim if v_dim is None else v_dim
+    assert q.dtype == k_cache.dtype == torch.bfloat16 and q.stride(1) == 1 and out.stride(1) == 1
+    assert out.dtype in (torch.bfloat16, torch.float32)
+    assert head_scale is None or (head_scale.is_cuda and head_scale.dtype == torch.float32 and head_scale.numel() == n_heads)
     assert k_cache.shape[-2] == 64 and k_cache.is_contiguous() and v_cache.is_contiguous()
     sc = tc_scratch(q.device)
     n_jobs, split_pages, ws = split if split is not None else (n_blocks, 0, None)
@@ -893,7 +900,8 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, s
         n_blocks, n_heads, n_kv_heads, head_dim, scale, window, n_jobs, split_pages, _addr(ws),
         ws.numel() if ws is not None else 0, sc.attn_tickets.data_ptr(), sc.N_ATTN_TICKETS, sc.error.data_ptr(), pool,
         _addr(k_pool), _addr(v_pool), k_pool.shape[0] if pool else 0, _addr(pool_pages), pool_pages.stride(0) if pool else 0,
-        _addr(gate), gate.stride(0) if gate is not None else 0, _addr(r1), _addr(r2), _addr(sink), _stream_int()))
+        _addr(gate), gate.stride(0) if gate is not None else 0, _addr(r1), _addr(r2), _addr(sink), maps, v_dim,
+        1 if out.dtype == torch.float32 else 0, _addr(head_scale), _stream_int()))
 
 
 # attention_short, by head size and rows of a tile: (us of a block alone, us a page of it, us a page and item when every SM is
@@ -1205,26 +1213,29 @@ def attention_maps(q, out, k_cache, v_cache, ctx, seq_pages, page_size: int, n_h
     tensor-core kernel takes go there — prompts as blocks of 128 query rows, steps of single tokens cut over the
     positions (``rt`` lends the workspace of the cuts) —, everything else, and the 32-bit path, to the generic kernel."""
     gate_per = _gate_per(gate, n_heads, maps, dv)
-    if (not ctx.decode and maps == 1 and chunk == 0 and head_scale is None and dk == dv and softcap == 0.0 and gate_per == 1 and page_size == 64 and scale > 0
-            and q.dtype == out.dtype == k_cache.dtype == torch.bfloat16 and rt is not None and _MAPS_ATTENTION == "mma"
-            and _PREFILL_ATTENTION == "tc" and not _FORCE_GENERIC_ATTENTION and attention_prefill_tc_supported(dk)
+    plain = maps == 1 and dk == dv                  # more maps, or values of their own size: nothing else beside them
+    if (not ctx.decode and (chunk == 0 or seq_pages.shape[1] * 64 <= chunk) and softcap == 0.0 and gate_per == 1 and page_size == 64 and scale > 0
+            and q.dtype == k_cache.dtype == torch.bfloat16 and rt is not None and _MAPS_ATTENTION == "mma"
+            and _PREFILL_ATTENTION == "tc" and not _FORCE_GENERIC_ATTENTION and lib().llmi_attention_prefill_tc_sizes(c_int(dk), c_int(dv))
             and q.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-            and (pooled is None or not pooled[0] or window > 0)):
-        # one map, equal head sizes, no mask of chunks: the prompt kernel of the tcgen05 tensor cores (its window, the
-        # pooled rows ahead of it, the gate per head); key ranges are cut when the step has fewer jobs than the device SMs
+            and (pooled is None or not pooled[0] or (window > 0 and plain and head_scale is None))
+            and (plain or (gate is None and bias is None and sink is None)) and (head_scale is None or bias is None)):
+        # No mask of chunks (or no sequence reaches a second one: the page tables end before it): the prompt kernel of the
+        # tcgen05 tensor cores (its window, the pooled rows ahead of it, the gate per head); key ranges are cut when the step has
+        # fewer jobs than the device SMs.
         pool = pooled[0] if pooled is not None else 0
         split = None
         q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)
         n_q_blocks = getattr(ctx, "n_q_blocks", None)
         if not n_q_blocks:      # exact where the lengths are known (a cut key range counts its jobs from them), else an upper bound
             n_q_blocks = sum((n + 127) // 128 for n in q_lens) if q_lens is not None else q.shape[0] // 128 + seq_pages.shape[0]
-        if _PREFILL_SPLIT and q_lens is not None and n_q_blocks * n_heads < sm_count():
+        if _PREFILL_SPLIT and q_lens is not None and n_q_blocks * n_heads * maps < sm_count():
             jobs = prefill_split_jobs(q_lens, kv_lens, window, PREFILL_SPLIT_PAGES, pool)
             if jobs > n_q_blocks:
-                ws = rt.scratch("attn_prefill_partials", (jobs * n_heads * (dk + 2) * 128,), torch.float32)
+                ws = rt.scratch("attn_prefill_partials", (jobs * n_heads * maps * (dv + 2) * 128,), torch.float32)
                 split = (jobs, PREFILL_SPLIT_PAGES, ws)
         attention_prefill_tc(q, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, n_q_blocks, n_heads,
-                             n_kv_heads, dk, scale, window, split, pooled if pool else None, gate, bias, sink)
+                             n_kv_heads, dk, scale, window, split, pooled if pool else None, gate, bias, sink, maps, dv, head_scale)
         return
     if (q.dtype == torch.bfloat16 and rt is not None and _MAPS_ATTENTION == "mma" and not _FORCE_GENERIC_ATTENTION
             and lib().llmi_attention_maps_mma_supported(c_int(dk), c_int(dv), c_int(n_heads // n_kv_heads), c_int(page_size))
