@@ -13,6 +13,16 @@
 //   * a cluster of 1, 2, 4 or 8 blocks shares a (sequence, kv head, row tile): every block takes a run of its pages and
 //     leaves (values, maximum, sum) in its shared memory; the cluster's warps then add them, a row a warp, in key order.  No workspace, no tickets.
 //
+// The weights (probabilities) meet V as bf16, as in the other tensor-core kernels — but for the decode steps of ungrouped heads
+// (WIDE), whose weights are 32 bits wide in the kernel that has the rest of them (attention_decode.cu).  There a tile has ONE
+// row, and the other fifteen are free: all of them hold its query, so that every thread group has its weights, and a weight goes
+// in as three bf16 numbers that add up to it exactly, in three rows: no more matrix instructions than with one.  Every product is
+// exact; the products of a page are summed by the matrix instruction and join the running sums by a rounded addition (running
+// sums inside the instruction are cut off, not rounded).  Against 64 bits the same error as attention_decode.cu's, also where the
+values' weighted sum all but cancels (there, 64 sequences of 2,200: 1.681e-3 both, of which the output's rounding is all; bf16
+weights 0.7).  What it costs (with bf16 weights -> with these): 16 x 1 x 128, 64 sequences of 2,200 172 -> 180 us, 1 of 4,000 12.5
+-> 13.6; 32 x 1 x 64, 64 of 2,200 173 -> 180.
+//
 // Measured against the tiles of 128 queries (kv heads x group x head size, positions, tokens; with about 8 us of launch):
 // 64 sequences, 32 x 1 x 64, 1,500, 8: 239 -> 140 us (the read of the cache alone: 120 us); 24, 8 x 4 x 128, 2,200, 9:
 // 191 -> 82 (33); 8, 32 x 1 x 64, 3,900, 16: 76 -> 61 (39); 1, 32 x 1 x 64, 4,000, 21: 27.5 -> 19.4 (5); 8, 5 x 3 x 64,
@@ -80,9 +90,17 @@ __device__ __forceinline__ void sh_tma(uint32_t dst, const CUtensorMap* map, int
       : "memory");
 }
 
+// v as the sum of three bf16 numbers (8 + 8 + 8 bits; exact for |v| > 2^-110, where the last of them is no denormal number)
+__device__ __forceinline__ void sh_split(float v, float& hi, float& mid, float& lo) {
+  hi = __bfloat162float(__float2bfloat16_rn(v));
+  const float rest = __fsub_rn(v, hi);
+  mid = __bfloat162float(__float2bfloat16_rn(rest));
+  lo = __fsub_rn(rest, mid);
+}
+
 // FUSE: one token a sequence; its q is rotated as it is read, its k (rotated) and v are appended to the cache by the block that
 // has the newest page, before it asks for that page (rope_store.cu's arithmetic: the same bits).
-template <int HD, int ROWS, bool FUSE>
+template <int HD, int ROWS, bool FUSE, bool WIDE>
 __global__ void __launch_bounds__(SH_THREADS, HD == 64 ? 3 : 2)
 attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, ShortParams p) {
   using C = ShCfg<HD>;
@@ -195,7 +213,7 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int r = wr * 16 + gq + 8 * h;
-        live[h] = r < rows;
+        live[h] = WIDE || r < rows;
         const int x = row0 + min(r, rows - 1), i = x / G;
         qpos[h] = pos0 + i;
         src[h] = p.q + (size_t)(q_start + i) * p.ldq + (size_t)(kvh * G + x - i * G) * HD;
@@ -305,8 +323,16 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           const float p2 = fast_exp2(fmaf(x[2], p.scale_log2, neg[1])), p3 = fast_exp2(fmaf(x[3], p.scale_log2, neg[1]));
           lrow[0] += p0 + p1;
           lrow[1] += p2 + p3;
-          pa[n * 2 + 0] = sh_pack(p0, p1);
-          pa[n * 2 + 1] = sh_pack(p2, p3);
+          if (WIDE) {                                        // rows 0 (thread group 0), 1 (group 1) and 8 (group 0): the three parts
+            float hi[2], mid[2], lo[2];
+            sh_split(p0, hi[0], mid[0], lo[0]);
+            sh_split(p1, hi[1], mid[1], lo[1]);
+            pa[n * 2 + 0] = gq == 0 ? sh_pack(hi[0], hi[1]) : gq == 1 ? sh_pack(lo[0], lo[1]) : 0u;
+            pa[n * 2 + 1] = gq == 0 ? sh_pack(mid[0], mid[1]) : 0u;
+          } else {
+            pa[n * 2 + 0] = sh_pack(p0, p1);
+            pa[n * 2 + 1] = sh_pack(p2, p3);
+          }
         }
 #pragma unroll
         for (int dc = 0; dc < HD / 8; dc += 2) {
@@ -316,8 +342,19 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                        : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                        : "r"(v_tile + (dchunk / 8) * C::SUB_BYTES + (uint32_t)(key * 128 + (((dchunk & 7) ^ (key & 7)) << 4))));
-          mma_bf16(o[dc], pa, r0, r1);
-          mma_bf16(o[dc + 1], pa, r2, r3);
+          if (WIDE) {
+            float f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_bf16(f0, pa, r0, r1);
+            mma_bf16(f1, pa, r2, r3);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              o[dc][e] = __fadd_rn(o[dc][e], f0[e]);
+              o[dc + 1][e] = __fadd_rn(o[dc + 1][e], f1[e]);
+            }
+          } else {
+            mma_bf16(o[dc], pa, r0, r1);
+            mma_bf16(o[dc + 1], pa, r2, r3);
+          }
         }
       }
       fence_reads_before_async_writes();
@@ -328,6 +365,15 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int h = 0; h < 2; ++h) {
       lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 1);
       lrow[h] += __shfl_xor_sync(0xffffffffu, lrow[h], 2);
+    }
+    if (WIDE) {                                              // the row's three parts meet in the threads of row 0
+#pragma unroll
+      for (int dc = 0; dc < HD / 8; ++dc)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float lo = __shfl_down_sync(0xffffffffu, o[dc][e], 4);
+          o[dc][e] = __fadd_rn(o[dc][e], __fadd_rn(o[dc][e + 2], lo));
+        }
     }
     if (WK == 1 && parts == 1) {                            // a row's only piece: straight out
 #pragma unroll
@@ -440,13 +486,13 @@ static int sh_cache_map(CUtensorMap* map, const void* ptr, long rows, int head_d
              : LLMI_ERR_DRIVER;
 }
 
-template <int HD, int ROWS, bool FUSE>
+template <int HD, int ROWS, bool FUSE, bool WIDE>
 static int sh_launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShortParams& p, int n_items, int parts, cudaStream_t stream) {
   using C = ShCfg<HD>;
   static PerDevice<bool> configured_on;
   bool& configured = configured_on.here();
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_short_kernel<HD, ROWS, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_short_kernel<HD, ROWS, FUSE, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
       return LLMI_ERR_LAUNCH;
     configured = true;
   }
@@ -464,16 +510,18 @@ static int sh_launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShortPa
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   pairs_may_start_early = false;
-  return cudaLaunchKernelEx(&cfg, attention_short_kernel<HD, ROWS, FUSE>, mk, mv, p) == cudaSuccess ? LLMI_OK : LLMI_ERR_LAUNCH;
+  return cudaLaunchKernelEx(&cfg, attention_short_kernel<HD, ROWS, FUSE, WIDE>, mk, mv, p) == cudaSuccess ? LLMI_OK : LLMI_ERR_LAUNCH;
 }
 
 template <int HD>
 static int sh_launch_rows(const CUtensorMap& mk, const CUtensorMap& mv, const ShortParams& p, int n_items, int rows, int parts,
-                          cudaStream_t stream) {
-  if (p.k_cache_w) return sh_launch<HD, 16, true>(mk, mv, p, n_items, parts, stream);
-  if (rows <= 16) return sh_launch<HD, 16, false>(mk, mv, p, n_items, parts, stream);
-  if (rows <= 32) return sh_launch<HD, 32, false>(mk, mv, p, n_items, parts, stream);
-  return sh_launch<HD, 64, false>(mk, mv, p, n_items, parts, stream);
+                          bool wide, cudaStream_t stream) {
+  if (p.k_cache_w)
+    return wide ? sh_launch<HD, 16, true, true>(mk, mv, p, n_items, parts, stream) : sh_launch<HD, 16, true, false>(mk, mv, p, n_items, parts, stream);
+  if (wide) return sh_launch<HD, 16, false, true>(mk, mv, p, n_items, parts, stream);
+  if (rows <= 16) return sh_launch<HD, 16, false, false>(mk, mv, p, n_items, parts, stream);
+  if (rows <= 32) return sh_launch<HD, 32, false, false>(mk, mv, p, n_items, parts, stream);
+  return sh_launch<HD, 64, false, false>(mk, mv, p, n_items, parts, stream);
 }
 
 }  // namespace llmi
@@ -486,17 +534,19 @@ LLMI_EXPORT int llmi_attention_short_supported(int head_dim) { return head_dim =
 // tokens a sequence brings; parts: blocks that share a (sequence, kv head, row tile): 1, 2, 4 or 8.
 // fuse = 1 (max_q 1, groups up to 16): a decode step as for llmi_attention_decode_fused — `q` is the step's un-rotated
 // [q | k | v] rows, rotary_dim is head_dim or 0, the new k (rotated) and v are appended with write_kv.
+// wide = 1 (max_q 1, ungrouped heads): 32-bit weights.
 LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ldo, void* k_cache, void* v_cache,
                                      long n_cache_pages, const int32_t* seq_pages, int pages_stride, const int32_t* seq_q_start,
                                      const int32_t* seq_kv_len, int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim,
                                      float scale, int window, int parts, int fuse, const float* inv_freq, int rotary_dim,
-                                     int write_kv, int* error_flag, cudaStream_t stream) {
+                                     int write_kv, int wide, int* error_flag, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return LLMI_ERR_BAD_SIZE;
   if (!llmi_attention_short_supported(head_dim)) return LLMI_ERR_UNSUPPORTED;
   if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)out & 3) || (ldo & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
   const int group = n_heads / n_kv_heads;
   if (fuse && (max_q != 1 || group > 16 || (rotary_dim != 0 && (rotary_dim != head_dim || !inv_freq)))) return LLMI_ERR_UNSUPPORTED;
+  if (wide && (max_q != 1 || group != 1)) return LLMI_ERR_UNSUPPORTED;
   const long rows = n_cache_pages * n_kv_heads * SH_PAGE, tile_rows = (long)max_q * group;
   const long tiles = (tile_rows + SH_MAX_ROWS - 1) / SH_MAX_ROWS, items = (long)n_seqs * n_kv_heads * tiles;
   if (rows > 0x7fffffffL || items * parts > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;
@@ -509,6 +559,6 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
                 group, (int)tiles, scale * 1.4426950408889634f, window, error_flag, inv_freq, fuse ? rotary_dim : 0, n_heads,
                 write_kv ? 1 : 0, fuse ? (__nv_bfloat16*)k_cache : nullptr, fuse ? (__nv_bfloat16*)v_cache : nullptr};
   const int per_tile = (int)(tile_rows < SH_MAX_ROWS ? tile_rows : SH_MAX_ROWS);
-  return head_dim == 64 ? sh_launch_rows<64>(mk, mv, p, (int)items, per_tile, parts, stream)
-                        : sh_launch_rows<128>(mk, mv, p, (int)items, per_tile, parts, stream);
+  return head_dim == 64 ? sh_launch_rows<64>(mk, mv, p, (int)items, per_tile, parts, wide != 0, stream)
+                        : sh_launch_rows<128>(mk, mv, p, (int)items, per_tile, parts, wide != 0, stream);
 }

@@ -723,8 +723,8 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
     many pages, which the persistent kernels cut finer, stay with them, as do ungrouped heads of 64 up to that point, and
     items that need a second, nearly empty wave.  Measured, persistent -> this (us, with the position encoding; kv heads x
     group x size, sequences, positions): 3 x 3 x 64, 1, 1,000 8.0 -> 5.1, 8, 4,000 11.2 -> 10.0, 1, 8,000 10.4 -> 10.6; 8 x 4 x
-    128, 1, 1,000 9.8 -> 6.1, 24, 2,200 39.5 -> 38.5; 16 x 128, 4, 4,000 31.9 -> 24.3, 64, 2,200 228 -> 172; 32 x 64, 64, 2,200 191
-    -> 171, 16, 2,200 51 -> 58, 4, 2,200 16.4 -> 15.9."""
+    128, 1, 1,000 9.8 -> 6.1, 24, 2,200 39.5 -> 38.5; 16 x 128, 4, 4,000 33.8 -> 26.4, 64, 2,200 229 -> 180; 32 x 64, 64, 2,200 188
+    -> 180, 24, 2,200 74.9 -> 71.9; with bf16 weights, 16, 2,200 51 -> 58, 4, 2,200 16.4 -> 15.9."""
     if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma":
         return 0
     resident, items = (3 if head_dim == 64 else 2) * sm_count(), n_live * n_kv_heads
@@ -949,10 +949,12 @@ def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, 
 
 
 def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
-                    n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1, rope=None) -> None:
+                    n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1, rope=None,
+                    wide: bool = False) -> None:
     """Causal attention of at most ``max_q`` tokens a sequence over its cache pages (bf16, head size 64 or 128, page 64):
     arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head.  ``rope``
-    (``max_q`` 1): see :func:`attention_decode_mma`."""
+    (``max_q`` 1): see :func:`attention_decode_mma`.  ``wide`` (``max_q`` 1, ungrouped heads): the
+    weights meet the values as 32-bit numbers."""
     inv_freq, rotary_dim, write_kv = rope if rope is not None else (None, 0, False)
     assert rotary_dim == 0 or (inv_freq is not None and inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2)
     _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)
@@ -963,7 +965,7 @@ def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pa
         _ptr(seq_pages), c_int(seq_pages.stride(0)), _ptr(seq_q_start), _ptr(seq_kv_len), c_int(seq_pages.shape[0]), c_int(max_q),
         c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), c_int(parts),
         c_int(0 if rope is None else 1), _ptr(inv_freq) if rotary_dim else None, c_int(rotary_dim), c_int(1 if write_kv else 0),
-        _ptr(tc_scratch(q.device).error), _stream()))
+        c_int(1 if wide else 0), _ptr(tc_scratch(q.device).error), _stream()))
 
 
 # Which prompt-attention kernel runs: "tc" (tcgen05: about 43 us for a 2,048-token prompt of 32 heads of 64) or
@@ -1024,8 +1026,9 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
         pps, n_live, cluster = decode_plan(ctx, S, P, page_size, n_kv_heads, head_dim, n_heads // n_kv_heads)
         parts = decode_short_parts(n_live, n_kv_heads, P, head_dim, n_heads // n_kv_heads)
         if parts:
+            # (the kernels it stands in for: ungrouped heads have 32-bit weights, grouped ones bf16)
             attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, 1, n_heads, n_kv_heads, head_dim,
-                            scale, window, parts, rope)
+                            scale, window, parts, rope, wide=n_heads == n_kv_heads)
             return
         partials = rt.scratch("attn_partials", (attention_decode_workspace(S, n_heads, head_dim, P, pps),), torch.float32)
         if decode_uses_mma(head_dim, n_heads // n_kv_heads):

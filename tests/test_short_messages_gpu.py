@@ -97,3 +97,58 @@ def test_attention_short_decode_same_bits(hd, group, window, rot, write):
         for a, b in ((kr, k1), (vr, v1)):
             assert torch.equal(torch.nan_to_num(a.float(), nan=-7.0), torch.nan_to_num(b.float(), nan=-7.0))
     k.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("nkv,hd,S,pages,parts", [(32, 64, 24, 12, 1), (16, 128, 24, 3, 1), (16, 128, 4, 16, 4), (8, 128, 2, 40, 8)])
+@pytest.mark.parametrize("fused", [True, False])
+def test_ungrouped_decode_has_32_bit_weights(nkv, hd, S, pages, parts, fused):
+    """A decode step of ungrouped heads, by the kernel that ``attention`` sends it to and by the one that has the other sizes:
+    values whose weighted sum all but cancels, so that weights rounded to bf16 would be as wrong as the result is large.  With
+    32-bit ones: the output's rounding (at most 2^-8; spread evenly over that, 1 / sqrt(3) of it in norm) and, of the terms' norm
+    (at most 2^9.3 times the result's), the scores' and exponentials' 2^-21 in all."""
+    import types
+    from llmi_b200.engine.runtime import Runtime
+    k = K()
+    dev = "cuda"
+    torch.manual_seed(nkv + S)
+    lens = [64 * pages - 17 * (s % 3) for s in range(S)]
+    i32 = lambda x: torch.as_tensor(x).to(torch.int32).to(dev)      # noqa: E731
+    table = i32(torch.randperm(S * pages).view(S, pages))
+    kc = torch.randn(S * pages, nkv, 64, hd, device=dev).bfloat16()
+    vc = torch.full_like(kc, float("nan"))
+    qkv = torch.randn(S, 3 * nkv * hd, device=dev).bfloat16()
+    scale, ref, terms = hd ** -0.5, [], 0.0
+    for s, n in enumerate(lens):
+        at = table[s].long()
+        keys = kc[at].transpose(1, 2).reshape(-1, nkv, hd)[:n].double()
+        if fused:                                              # (nothing turns: the new key is the row's own)
+            keys[-1] = qkv[s, nkv * hd:2 * nkv * hd].view(nkv, hd).double()
+        p = (torch.einsum("hd,khd->hk", qkv[s, :nkv * hd].view(nkv, hd).double(), keys) * scale).softmax(-1)
+        r = torch.randn(n, nkv, hd, device=dev, dtype=torch.float64)
+        vals = (r - torch.einsum("hk,khd->hd", p, r)).bfloat16()
+        if fused:
+            qkv[s, 2 * nkv * hd:] = vals[-1].reshape(-1)
+        full = torch.full((64 * pages, nkv, hd), float("nan"), device=dev, dtype=torch.bfloat16)
+        full[:n] = vals
+        vc[at] = full.view(pages, 64, nkv, hd).transpose(1, 2)
+        ref.append(torch.einsum("hk,khd->hd", p, vals.double()).reshape(-1))
+        terms = max(terms, float(torch.einsum("hk,khd->hd", p ** 2, vals.double() ** 2).sqrt().norm() / ref[-1].norm()))
+    ref = torch.stack(ref)
+    assert terms < 2 ** 9.3
+    ctx = types.SimpleNamespace(decode=True, seq_q_start=i32(range(S + 1)), seq_kv_len=i32(lens), tok_seq=i32(range(S)),
+                                tok_pos=i32([n - 1 for n in lens]), n_real_seqs=S, host_q_lens=None, host_kv_lens=None)
+    assert k.decode_short_parts(S, nkv, pages, hd, 1) == parts
+    rt, rope = Runtime(torch.bfloat16, dev), (None, 0, True) if fused else None
+    errors = []
+    rule = k.decode_short_parts
+    try:
+        for other in (False, True):
+            if other:
+                k.decode_short_parts = lambda *a: 0
+            out = torch.full((S, nkv * hd), 7.0, device=dev, dtype=torch.bfloat16)
+            k.attention(qkv, out, kc.clone(), vc.clone(), ctx, table, 64, nkv, nkv, hd, scale, rt=rt, rope=rope)
+            errors.append(float((out.double() - ref).norm() / ref.norm()))
+    finally:
+        k.decode_short_parts = rule
+    assert max(errors) < 2 ** -8 / 3 ** 0.5 + 2 ** (9.3 - 21), errors
+    k.check_device_errors("cuda:0")
