@@ -19,9 +19,9 @@
 // in as three bf16 numbers that add up to it exactly, in three rows: no more matrix instructions than with one.  Every product is
 // exact; the products of a page are summed by the matrix instruction and join the running sums by a rounded addition (running
 // sums inside the instruction are cut off, not rounded).  Against 64 bits the same error as attention_decode.cu's, also where the
-values' weighted sum all but cancels (there, 64 sequences of 2,200: 1.681e-3 both, of which the output's rounding is all; bf16
-weights 0.7).  What it costs (with bf16 weights -> with these): 16 x 1 x 128, 64 sequences of 2,200 172 -> 180 us, 1 of 4,000 12.5
--> 13.6; 32 x 1 x 64, 64 of 2,200 173 -> 180.
+// values' weighted sum all but cancels (there, 64 sequences of 2,200: 1.681e-3 both, of which the output's rounding is all; bf16
+// weights 0.7).  What it costs (with bf16 weights -> with these): 16 x 1 x 128, 64 sequences of 2,200 172 -> 180 us, 1 of 4,000 12.5
+// -> 13.6; 32 x 1 x 64, 64 of 2,200 173 -> 180.
 //
 // Measured against the tiles of 128 queries (kv heads x group x head size, positions, tokens; with about 8 us of launch):
 // 64 sequences, 32 x 1 x 64, 1,500, 8: 239 -> 140 us (the read of the cache alone: 120 us); 24, 8 x 4 x 128, 2,200, 9:
