@@ -1561,12 +1561,12 @@ EXPANDED_MIN_PER_SEQUENCE = 48      # queries that share a sequence's expansion;
 EXPANDED_MAX_BYTES = 512 << 20      # of keys and values
 
 
-def latent_expanded_pages(ctx, n_tokens: int, seq_pages, H: int, D: int) -> int:
+def latent_expanded_pages(ctx, n_tokens: int, seq_pages, H: int, D: int, page_size: int = 64) -> int:
     """How many pages of rows a step's latent attention multiplies out into keys and values, or 0 where it works on the
-    latent rows themselves.  Depends on the step's padded shape only where the step has no lengths on the host, so a
+    latent rows themselves (always where the cache's pages are not of 64 rows).  Depends on the step's padded shape only where the step has no lengths on the host, so a
     recorded step can be replayed."""
     S, P = seq_pages.shape
-    if ctx.decode or n_tokens < EXPANDED_MIN_TOKENS or n_tokens < EXPANDED_MIN_PER_SEQUENCE * S:
+    if page_size != 64 or ctx.decode or n_tokens < EXPANDED_MIN_TOKENS or n_tokens < EXPANDED_MIN_PER_SEQUENCE * S:
         return 0
     q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)
     pages = S * P if q_lens is None else sum((kv + 63) // 64 for q, kv in zip(q_lens, kv_lens) if q)

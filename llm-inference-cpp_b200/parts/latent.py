@@ -118,7 +118,7 @@ class LatentAttention:
                                    g.page_size, cache, cq, write_kv=binding.writes, pairing=self.pairing, amplitude=self.amplitude)
             q = rt.scratch("latent_q", (T, H * (D + R)))
             kernels.linear(cq, self.w_uq, q)
-            n_pages = kernels.latent_expanded_pages(ctx, T, pages, H, D) if self.w_kv is not None else 0
+            n_pages = kernels.latent_expanded_pages(ctx, T, pages, H, D, g.page_size) if self.w_kv is not None else 0
             if n_pages:
                 rows = 64 * n_pages
                 xc, xr, qr = rt.scratch("latent_xc", (rows, C)), rt.scratch("latent_xr", (rows, 64)), rt.scratch("latent_qr", (T, H * 64))

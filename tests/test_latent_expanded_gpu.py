@@ -74,3 +74,39 @@ def test_attention_expanded(H, D, R, C, rot_dims, pairing, spare):
     assert float((out[:n].double() - ref).norm() / ref.norm()) < 1.2 * 2 ** -9 * 5 ** 0.5
     assert bool((out[n:] == 7.0).all())
     K.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("page_size", [16, 32, 64, 128])
+def test_latent_part_on_pages_of_any_size(page_size):
+    """A prompt of as many tokens as the expanded form takes, and a second one on top of it, through the mixer: what the cache's
+    page size is does not matter (the expanded form is for pages of 64; the others keep the form on the latent rows)."""
+    from llmi_b200.cache.storage import CacheBinding, SequenceCache
+    from llmi_b200.engine.batch import SequenceStep, StepBuffers, plan_step
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels as K
+    from llmi_b200.parts import PartSpec, get_part
+    W, H, D, R, C, Q = 128, 2, 64, 32, 64, 64
+    params = {"width": W, "heads": H, "dim": D, "rot_dim": R, "vdim": D, "kv_rank": C, "q_rank": Q, "scale": (D + R) ** -0.5, "rot_base": 1e4,
+              "eps": 1e-6}
+    make = get_part("mixer", "latent_attention")
+    torch.manual_seed(5)
+    tensors = {n: (torch.ones(d.shape) if n.endswith("norm") else torch.randn(d.shape) * d.shape[1] ** -0.5)
+               for n, d in make.declare(PartSpec("latent_attention", params, "")).items()}
+    h = torch.randn(300, W, device="cuda")
+    outs = {}
+    for dtype, size in ((torch.float32, 64), (torch.bfloat16, page_size)):
+        rt = Runtime(dtype, "cuda:0")
+        part = make(PartSpec("latent_attention", params, ""), {n: t.to(dtype).float() for n, t in tensors.items()}, rt)
+        cache = SequenceCache([(part.cache_request(), 1)], [], 512, 512, dtype, "cuda:0", page_size=size)
+        buffers, slot, rows = StepBuffers("cuda:0"), cache.alloc_slot(), []
+        for a, b in ((0, 160), (160, 300)):
+            ctx = plan_step(cache, [SequenceStep(slot, list(range(b - a)), [])], 1000, buffers)
+            x = torch.zeros(b - a, W, device="cuda")
+            part.forward(h[a:b].to(dtype), x, ctx, CacheBinding(cache.kv_groups[0], 0))
+            rows.append(x)
+        outs[dtype] = torch.cat(rows).double()
+    ref = outs[torch.float32]
+    # rounded to bf16 (2^-8 at most, 1 / sqrt(3) of that in norm), one after another: weights (five products deep), input, latents, rows,
+    # queries, keys or folded queries, weights of the sum, values or sums, heads: at most 16 in all
+    assert float((outs[torch.bfloat16] - ref).norm() / ref.norm()) < 4 * 2 ** -8 / 3 ** 0.5
+    K.check_device_errors("cuda:0")
