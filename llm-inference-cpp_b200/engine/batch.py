@@ -22,8 +22,7 @@ import torch
 from ..cache.pages import CacheError, pages_for
 
 
-# Most tokens that a sequence of a prompt step brings, as the launches of the attention of short messages know it: what a
-# recorded prompt step's launches may depend on beside its padded shape
+# Most tokens that a sequence of a prompt step brings, as the launches of the attention of short messages know it
 SHORT_MESSAGES = (4, 8, 16, 32, 48, 64)
 
 
@@ -94,6 +93,7 @@ class StepContext:
         self.seq_q_start = self.seq_kv_len = self.seq_slot = None
         self._pages = {}
         self.h2d_bytes = 0
+        self.asked = {}          # what the step's launches asked beside its padded shape: (rule, sizes) (see kernels.decide)
 
     def pages_of(self, group) -> torch.Tensor:
         """[n_seqs, pages] int32 page table of this step's sequences in a cache group."""

@@ -25,7 +25,9 @@ Prompt steps (:class:`PromptGraphs`).  A prompt of a few hundred tokens is bound
 hundred launches of 6 to 15 us each, 2.9 ms whether the prompt has 16 or 256 tokens, where the device needs a
 third of that.  Such steps are padded to a shape — token rows to 16, 32 or a multiple of 64 (128 from 512 on), sequences and
 wanted rows to a power of two, page tables as for decode steps; the padding rows belong to no sequence — and a
-shape that comes a second time is recorded and replayed from then on.  Prompts beyond 1,024 tokens keep the device
+shape that comes a second time is recorded and replayed from then on.  What a launch follows beside the shape (how the
+attention of short messages shares its work) it asks through ``kernels.decide``: the first run of a shape tells what is
+asked, and recordings with other answers are told apart.  Prompts beyond 1,024 tokens keep the device
 busy for longer than their launches take and run launch by launch, unpadded.
 """
 from __future__ import annotations
@@ -190,18 +192,21 @@ class PromptGraphs:
         self.model = model
         self.graphs = {}         # key -> (graph, logits, kernels launched)
         self.seen = {}           # key -> times the shape has come without a graph
+        self.asked = {}          # padded shape -> what its launches ask (kernels.decide)
         self.replays = 0
         self._watched = set()
 
     def _drop_cache(self, serial: int) -> None:
-        for table in (self.graphs, self.seen):
+        for table in (self.graphs, self.seen, self.asked):
             for key in [k for k in table if k[4] == serial]:
                 del table[key]
         self._watched.discard(serial)
 
-    def _key(self, T, S, W, P, cache):
+    def _key(self, shape, ctx):
+        """A recording's key, or None for a shape that has not run yet."""
         m = self.model
-        return (T, S, W, P, cache.serial, m.rt.generation, m.buffers.dev.data_ptr())
+        asked = self.asked.get(shape)
+        return None if asked is None else (*shape, m.rt.generation, m.buffers.dev.data_ptr(), tuple(rule(ctx, *sizes) for rule, sizes in asked))
 
     def step(self, cache, seqs):
         """fp32 logits [wanted, vocab] of a prompt step (scratch: valid until the next step), or None if the step
@@ -224,8 +229,8 @@ class PromptGraphs:
         P = max(need_pages, min(bucket(need_pages), cache.max_pages_per_seq))
         ctx = plan_step(cache, seqs, m.spec.vocab_size, m.buffers, pad_seqs_to=S, pad_pages_to=P, pad_tokens_to=T, pad_want_to=W)
         m._last_h2d = ctx.h2d_bytes
-        P = (P, ctx.short_message)                  # (the attention's launches follow both)
-        key = self._key(T, S, W, P, cache)
+        shape = (T, S, W, P, cache.serial)
+        key = self._key(shape, ctx)
         entry = self.graphs.get(key)
         if entry is not None:
             g, rec_logits, n_kernels = entry
@@ -234,11 +239,12 @@ class PromptGraphs:
             kernels.launch_count(n_kernels)
             return rec_logits[:n_want_real]
         logits = m.run(ctx, cache)
-        key = self._key(T, S, W, P, cache)          # the plain run may have grown a scratch buffer
+        self.asked[shape] = tuple({**dict.fromkeys(self.asked.get(shape, ())), **ctx.asked})
+        key = self._key(shape, ctx)                  # (the plain run may have grown a scratch buffer)
         self.seen[key] = self.seen.get(key, 0) + 1
         if RECORD and self.seen[key] >= 2:
             for table in (self.graphs, self.seen):   # shapes recorded or counted before a buffer moved never come again
-                for stale in [k for k in table if k[4] == cache.serial and k[5:] != key[5:]]:
+                for stale in [k for k in table if k[4] == cache.serial and k[5:7] != key[5:7]]:
                     del table[stale]
             while len(self.graphs) >= self.MAX_GRAPHS:
                 del self.graphs[next(iter(self.graphs))]

@@ -948,6 +948,24 @@ def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, 
     return best
 
 
+def decide(ctx, rule, *sizes):
+    """``rule(ctx, *sizes)``: what a prompt step's launches follow beside its padded shape.  The context notes the question, so
+    that a recorded step is replayed only for a step whose answers are the same (``PromptGraphs``)."""
+    asked = getattr(ctx, "asked", None)
+    if asked is not None:
+        asked[(rule, sizes)] = True
+    return rule(ctx, *sizes)
+
+
+def short_message_plan(ctx, n_seqs: int, n_pages: int, n_kv_heads: int, group: int, head_dim: int) -> tuple:
+    """How attention_short takes a prompt step: (blocks of a cluster, rows of a sequence and kv head in whole tiles), or () where it
+    goes elsewhere.  (The rows, not the message's length: more tokens than a recording was made with need more tiles.)"""
+    max_q = getattr(ctx, "short_message", 0)
+    parts = attention_short_parts(n_seqs, n_kv_heads, max_q, group, n_pages, head_dim) if max_q else 0
+    rows = max_q * group
+    return (parts, 16 if rows <= 16 else 32 if rows <= 32 else -(-rows // 64) * 64) if parts else ()
+
+
 def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
                     n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1, rope=None,
                     wide: bool = False) -> None:
@@ -1052,12 +1070,10 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             # longest job: then the key ranges are cut (see the kernel's head).  Measured: 2,048 tokens x 8 heads 28.0 ->
             # 22.2 us, x 4 heads 27.5 -> 21.0 us; with 256 jobs and more the cut gains nothing or costs (4,096 x 8:
             # 49.3 -> 50.5 us; 2,048 x 32: 42.1 -> 49.6 us).
-            max_q = getattr(ctx, "short_message", 0)
-            parts = attention_short_parts(seq_pages.shape[0], n_kv_heads, max_q, n_heads // n_kv_heads,
-                                          seq_pages.shape[1], head_dim) if max_q else 0
-            if parts:
-                attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, max_q, n_heads, n_kv_heads,
-                                head_dim, scale, window, parts)
+            short = decide(ctx, short_message_plan, seq_pages.shape[0], seq_pages.shape[1], n_kv_heads, n_heads // n_kv_heads, head_dim)
+            if short:
+                attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, ctx.short_message, n_heads,
+                                n_kv_heads, head_dim, scale, window, short[0])
                 return
             split = None
             q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)

@@ -152,3 +152,50 @@ def test_ungrouped_decode_has_32_bit_weights(nkv, hd, S, pages, parts, fused):
         k.decode_short_parts = rule
     assert max(errors) < 2 ** -8 / 3 ** 0.5 + 2 ** (9.3 - 21), errors
     k.check_device_errors("cuda:0")
+
+
+def _small_llama(tmp_path, heads, kv_heads, head_dim):
+    import llmi_b200 as L
+    d = str(tmp_path / f"m{heads}_{kv_heads}_{head_dim}")
+    L.write_random_model(d, {"architectures": ["LlamaForCausalLM"], "num_hidden_layers": 2, "hidden_size": 256, "num_attention_heads": heads,
+                             "num_key_value_heads": kv_heads, "head_dim": head_dim, "intermediate_size": 512, "vocab_size": 300,
+                             "rope_theta": 10000.0, "rms_norm_eps": 1e-5, "tie_word_embeddings": True, "max_position_embeddings": 1024,
+                             "hidden_act": "silu"}, 3, torch.bfloat16)
+    return L.load(d, "bfloat16")
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(6, 2, 64), (4, 4, 64), (8, 2, 128), (4, 2, 32)])
+def test_recorded_messages_of_one_padded_shape(tmp_path, heads, kv_heads, head_dim):
+    """Messages of one padded shape (as many tokens in all, page tables as wide) but of other lengths, one step after another, so
+    that recordings made for some meet others: the logits of steps that are neither padded nor recorded.  A recording is told
+    apart by what its launches follow, so heads that attention_short does not take share one."""
+    import llmi_b200 as L
+    from llmi_b200.engine import graphs
+    from llmi_b200.ops import kernels
+    if not graphs.RECORD:
+        pytest.skip("recording is switched off")
+    model = _small_llama(tmp_path, heads, kv_heads, head_dim)
+    rng = np.random.default_rng(1)
+    held, messages = [260, 300, 280, 310], [[4, 4, 4, 4], [13, 1, 1, 1], [1, 1, 2, 12], [4, 3, 4, 4], [2, 12, 1, 1], [3, 4, 4, 4], [1, 2, 10, 2], [4, 4, 4, 4]]
+    caches = [model.new_cache(4 * 1024) for _ in range(2)]
+    slots = [[c.alloc_slot() for _ in held] for c in caches]
+    toks = [rng.integers(0, 300, n).tolist() for n in held]
+    for c, s in zip(caches, slots):
+        for slot, t in zip(s, toks):
+            model.step(c, [L.SequenceStep(slot, t, [])])
+    g = model._prompt_graphs
+    before, had = g.replays, set(g.graphs)
+    plans = set()
+    for lens in messages:
+        new = [rng.integers(0, 300, n).tolist() for n in lens]
+        got, want = (model.step(c, [L.SequenceStep(slot, t, list(range(len(t)))) for slot, t in zip(s, new)], **kw).clone()
+                     for c, s, kw in ((caches[0], slots[0], {}), (caches[1], slots[1], {"pad_pages_to": 1})))
+        # every row: bf16 roundings of another batch's products, two layers deep; a row that no launch wrote would be of another size
+        assert bool(((got - want).norm(dim=1) < 2e-2 * want.norm(dim=1)).all()), lens
+        short = 4 if max(lens) <= 4 else 16
+        parts = kernels.attention_short_parts(4, kv_heads, short, heads // kv_heads, 8, head_dim) if head_dim != 32 else 0
+        rows = short * heads // kv_heads
+        plans.add((parts, 16 if rows <= 16 else 32 if rows <= 32 else -(-rows // 64) * 64) if parts else ())
+    assert len(set(g.graphs) - had) == len(plans) and g.replays - before == len(messages) - 2 * len(plans)
+    assert len(plans) == (1 if head_dim == 32 or heads == kv_heads else 2)
+    kernels.check_device_errors("cuda:0")
