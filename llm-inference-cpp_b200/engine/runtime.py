@@ -22,14 +22,15 @@ class Runtime:
         self._buffers: dict[str, torch.Tensor] = {}
         self.generation = 0
 
-    def scratch(self, name: str, shape, dtype=None) -> torch.Tensor:
+    def scratch(self, name: str, shape, dtype=None, most: int = 0) -> torch.Tensor:
+        """A buffer of that shape; a growing one doubles, but to no more than ``most`` elements (0: no bound)."""
         dtype = dtype or self.dtype
         n = 1
         for s in shape:
             n *= int(s)
         buf = self._buffers.get(name)
         if buf is None or buf.dtype != dtype or buf.numel() < n:
-            grow = n if buf is None or buf.dtype != dtype else max(n, 2 * buf.numel())
+            grow = n if buf is None or buf.dtype != dtype else max(n, min(2 * buf.numel(), most) if most else 2 * buf.numel())
             buf = torch.empty(grow, dtype=dtype, device=self.device)
             self._buffers[name] = buf
             self.generation += 1

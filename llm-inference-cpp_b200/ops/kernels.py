@@ -1571,10 +1571,12 @@ def attention_expanded_supported(rt, D: int, Dv: int, R: int, C: int, scale: flo
 
 # From here on the expanded form is the faster one: a prompt step of eight layers, four of them latent attention (2,048 wide, 16
 # heads of 128, rank 512), absorbed / expanded: 100 tokens 1.17 / 1.15 ms, 200 1.30 / 1.23, 500 2.01 / 1.76, 2,600 9.81 / 5.90;
-# six prompts of about 60 tokens 1.19 / 1.19, of 150 1.98 / 1.81.
+# six prompts of about 60 tokens 1.19 / 1.19, of 150 1.98 / 1.81.  The lines are on the expanded form's safe side, however unequal
+# the sequences: the mixer alone (us), 500 tokens beside seven single tokens on 8,000 positions 1,245 / 464, 8 messages of 20 on
+# 2,000 200 / 176; a step padded to a shape, whose whole page tables are multiplied out: 8 of 48, one of them on 8,000, 632 / 464.
 EXPANDED_MIN_TOKENS = 128
-EXPANDED_MIN_PER_SEQUENCE = 48      # queries that share a sequence's expansion; it costs as much as 12 to 16 of them save
-EXPANDED_MAX_BYTES = 512 << 20      # of keys and values
+EXPANDED_MIN_PER_SEQUENCE = 48      # queries that share a sequence's expansion
+EXPANDED_MAX_BYTES = 512 << 20      # of keys and values: the most that the form's scratch buffers grow to
 
 
 def latent_expanded_pages(ctx, n_tokens: int, seq_pages, H: int, D: int, page_size: int = 64) -> int:
@@ -1586,7 +1588,12 @@ def latent_expanded_pages(ctx, n_tokens: int, seq_pages, H: int, D: int, page_si
         return 0
     q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)
     pages = S * P if q_lens is None else sum((kv + 63) // 64 for q, kv in zip(q_lens, kv_lens) if q)
-    return pages if pages * 64 * H * 2 * D * 2 <= EXPANDED_MAX_BYTES else 0
+    return pages if 64 * pages <= expanded_max_rows(H, D) else 0
+
+
+def expanded_max_rows(H: int, D: int) -> int:
+    """The most rows whose keys and values the expanded form keeps in scratch."""
+    return EXPANDED_MAX_BYTES // (H * 2 * D * 2) // 64 * 64
 
 
 def latent_expand_prepare(cache: torch.Tensor, ctx, seq_pages, xc: torch.Tensor, xr: torch.Tensor, q: torch.Tensor, qr: torch.Tensor,

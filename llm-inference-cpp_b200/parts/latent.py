@@ -120,11 +120,12 @@ class LatentAttention:
             kernels.linear(cq, self.w_uq, q)
             n_pages = kernels.latent_expanded_pages(ctx, T, pages, H, D, g.page_size) if self.w_kv is not None else 0
             if n_pages:
-                rows = 64 * n_pages
-                xc, xr, qr = rt.scratch("latent_xc", (rows, C)), rt.scratch("latent_xr", (rows, 64)), rt.scratch("latent_qr", (T, H * 64))
+                rows, most = 64 * n_pages, kernels.expanded_max_rows(H, D)
+                xc, xr = rt.scratch("latent_xc", (rows, C), most=most * C), rt.scratch("latent_xr", (rows, 64), most=most * 64)
+                qr = rt.scratch("latent_qr", (T, H * 64))
                 kernels.latent_expand_prepare(cache, ctx, pages, xc, xr, q, qr, H, D, R, self.inv_freq, self.rot_dims, self.pairing,
                                               self.amplitude)
-                kv = rt.scratch("latent_kv", (rows, H * 2 * D))
+                kv = rt.scratch("latent_kv", (rows, H * 2 * D), most=most * H * 2 * D)
                 kernels.linear(xc, self.w_kv, kv)
                 heads = rt.scratch("attn_out", (T, H * Dv))
                 kernels.attention_expanded(q, qr, kv, xr, heads, ctx, H, D, R, self.scale)

@@ -110,3 +110,30 @@ def test_latent_part_on_pages_of_any_size(page_size):
     # queries, keys or folded queries, weights of the sum, values or sums, heads: at most 16 in all
     assert float((outs[torch.bfloat16] - ref).norm() / ref.norm()) < 4 * 2 ** -8 / 3 ** 0.5
     K.check_device_errors("cuda:0")
+
+
+def test_expanded_form_keeps_no_more_than_its_bound(monkeypatch):
+    """A prompt that grows portion by portion: the buffers of keys and values, which double as they grow, stop at the bound; beyond
+    it the step works on the latent rows."""
+    from llmi_b200.cache.storage import CacheBinding, SequenceCache
+    from llmi_b200.engine.batch import SequenceStep, StepBuffers, plan_step
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels as K
+    from llmi_b200.parts import PartSpec, get_part
+    W, H, D, R, C = 128, 2, 64, 32, 64
+    params = {"width": W, "heads": H, "dim": D, "rot_dim": R, "vdim": D, "kv_rank": C, "q_rank": 64, "scale": (D + R) ** -0.5, "rot_base": 1e4,
+              "eps": 1e-6}
+    make, spec = get_part("mixer", "latent_attention"), PartSpec("latent_attention", params, "")
+    bound = 700 * H * 2 * D * 2                                   # 700 rows: ten pages of 64
+    monkeypatch.setattr(K, "EXPANDED_MAX_BYTES", bound)
+    rt = Runtime(torch.bfloat16, "cuda:0")
+    part = make(spec, {n: (torch.ones(d.shape) if n.endswith("norm") else torch.randn(d.shape) * 0.1) for n, d in make.declare(spec).items()}, rt)
+    cache = SequenceCache([(part.cache_request(), 1)], [], 1024, 1024, torch.bfloat16, "cuda:0")
+    buffers, slot = StepBuffers("cuda:0"), cache.alloc_slot()
+    for n in range(6):                                            # 2, 4, .. pages; 10 are the most, 12 are too many
+        ctx = plan_step(cache, [SequenceStep(slot, [1] * 128, [])], 1000, buffers)
+        part.forward(torch.randn(128, W, device="cuda").bfloat16(), torch.zeros(128, W, device="cuda"), ctx, CacheBinding(cache.kv_groups[0], 0))
+        used = rt._buffers["latent_kv"].numel()
+        assert min(128 * (n + 1), 640) * H * 2 * D <= used <= 640 * H * 2 * D and 2 * used <= bound
+        assert rt._buffers["latent_xc"].numel() <= 640 * C and rt._buffers["latent_xr"].numel() <= 640 * 64
+    K.check_device_errors("cuda:0")
