@@ -361,14 +361,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float m_run = -INFINITY, m_ref = -INFINITY, l_run = 0.f;   // maxima in base 2, scaled
     float* bias_w = bias_s + (BIAS ? (warp - 2) * (31 + KEYS + 1) : 0);
     const float r1 = BIAS ? p.r1[head] : 0.f, r2 = BIAS ? p.r2[head] : 0.f;      // (weights: no kernel before writes them)
-    // A head's own factor: its size goes into the scale (never quite 0: 0 times a masked key's -inf is no number), its sign
-    // into the scores.
+    // A head's own factor: its size goes into the scale (never quite 0: 0 times a masked key's -inf is no number; a factor that
+    // is no number stays one), its sign into the scores.
     float scale_log2 = p.scale_log2;
     bool flip = false;
     if (!BIAS && p.head_scale) {
       const float f = p.head_scale[real_head];
       flip = f < 0.f;
-      scale_log2 = fmaxf(fabsf(f) * scale_log2, 1e-30f);
+      scale_log2 *= fabsf(f);
+      if (scale_log2 < 1e-30f) scale_log2 = 1e-30f;
     }
     bool ok = true;
     for (int j = 0; j < n_pg && ok; ++j) {

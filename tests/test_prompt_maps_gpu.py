@@ -69,3 +69,30 @@ def test_attention_maps_prompt_on_tcgen05(H, G, maps, dk, dv, f32, scaled, windo
         K.attention_prefill_tc = tc
     assert len(seen) == 2
     K.check_device_errors("cuda:0")
+
+
+def test_a_factor_that_is_no_number_stays_one():
+    """A head whose factor is NaN gives NaN, as in the general kernel; the heads beside it, one with a factor of 0 among them, do
+    not."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels as K
+    dev, H, d, n = "cuda", 4, 64, 150
+    torch.manual_seed(2)
+    i32 = lambda x: torch.as_tensor(x).to(torch.int32).to(dev)      # noqa: E731
+    q, kc, vc = (torch.randn(s, device=dev).bfloat16() for s in ((n, H * d), (3, H, 64, d), (3, H, 64, d)))
+    factor = torch.tensor([1.5, float("nan"), 0.0, -2.0], device=dev)
+    ctx = types.SimpleNamespace(decode=False, seq_q_start=i32([0, n]), seq_kv_len=i32([n]), n_q_blocks=2, tok_seq=i32([0] * n), tok_pos=i32(range(n)),
+                                host_q_lens=[n], host_kv_lens=[n])
+    out, plain = (torch.full((n, H * d), 7.0, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    seen, tc = [], K.attention_prefill_tc
+    K.attention_prefill_tc = lambda *a, **kw: (seen.append(1), tc(*a, **kw))
+    try:
+        K.attention_maps(q, out, kc, vc, ctx, i32([[0, 1, 2]]), 64, H, H, 1, d, d, d ** -0.5, factor, rt=Runtime(torch.bfloat16, dev))
+    finally:
+        K.attention_prefill_tc = tc
+    K.attention_flex(q, plain, kc, vc, ctx, i32([[0, 1, 2]]), 64, H, H, 1, d, d, d ** -0.5, factor)
+    assert seen and torch.equal(out.isnan(), plain.isnan()) and bool(out.view(n, H, d)[:, 1].isnan().all())
+    rest = [0, 2, 3]
+    a, b = out.view(n, H, d)[:, rest].double(), plain.view(n, H, d)[:, rest].double()
+    assert float((a - b).norm() / b.norm()) < 1.2 * 2 ** -9 * 2 ** 0.5
+    K.check_device_errors("cuda:0")
