@@ -163,7 +163,10 @@ __device__ __forceinline__ void ft_st16u(uint32_t taddr, const uint32_t* v) {
       : "memory");
 }
 
-template <int DK, int DV, bool BIAS>
+// FORMS: several maps a head, values of their own size, factors per head, an fp32 output; an instantiation of its own, since the
+// plain one is 1 to 7 % slower with them inside (32 x 1 x 64: 7,931 tokens 412 -> 401 us, 2,048 42.6 -> 41.4; 32 sequences of 48
+// tokens on 4,000 positions, window 2,048, 216 -> 200).
+template <int DK, int DV, bool BIAS, bool FORMS>
 __global__ void __launch_bounds__(FtCfg<DK, DV>::THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_kp,
@@ -231,7 +234,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   // page j of this part: pooled page v_first + j while that is below n_ppg, else token page pg_first + (v_first + j - n_ppg)
   const int32_t* ppages = p.pool > 0 ? p.pool_pages + (size_t)seq * p.pool_pages_stride : nullptr;
   const int head = blockIdx.x;             // (of maps heads each: the head's map)
-  const int real_head = head / p.maps, v_head = real_head / (p.n_heads / p.n_kv_heads), k_head = v_head * p.maps + head % p.maps;
+  const int maps = FORMS ? p.maps : 1;
+  const int real_head = head / maps, v_head = real_head / (p.n_heads / p.n_kv_heads), k_head = v_head * maps + head % maps;
   const int32_t* pages = p.seq_pages + (size_t)seq * p.pages_stride;
   __shared__ int s_last;
   __shared__ float bias_s[BIAS ? 4 * HALVES * (31 + KEYS + 1) : 1];
@@ -285,14 +289,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int v = v_first + j;
         const bool pooled = v < n_ppg;
         const int page = pooled ? ppages[v] : pages[pg_first + v - n_ppg];
-        const int k_row = (page * p.n_kv_heads * p.maps + k_head) * FT_PAGE, v_row = (page * p.n_kv_heads + v_head) * FT_PAGE;
+        const int k_row = (page * p.n_kv_heads * maps + k_head) * FT_PAGE, v_row = (page * p.n_kv_heads + v_head) * FT_PAGE;
         const CUtensorMap* mk = pooled ? &map_kp : &map_k;
         const CUtensorMap* mv = pooled ? &map_vp : &map_v;
         mbar_expect_tx(kv_full(s), C::STAGE);
 #pragma unroll
-        for (int u = 0; u < KSUB; ++u) ft_tma(kv_smem + s * C::STAGE + u * FT_SUB, mk, 64 * u, k_row, kv_full(s));
-#pragma unroll
-        for (int u = 0; u < VSUB; ++u) ft_tma(kv_smem + s * C::STAGE + C::K_TILE + u * FT_SUB, mv, 64 * u, v_row, kv_full(s));
+        for (int u = 0; u < (KSUB > VSUB ? KSUB : VSUB); ++u) {
+          if (u < KSUB) ft_tma(kv_smem + s * C::STAGE + u * FT_SUB, mk, 64 * u, k_row, kv_full(s));
+          if (u < VSUB) ft_tma(kv_smem + s * C::STAGE + C::K_TILE + u * FT_SUB, mv, 64 * u, v_row, kv_full(s));
+        }
       }
     }
   } else if (warp == 1) {
@@ -365,7 +370,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // is no number stays one), its sign into the scores.
     float scale_log2 = p.scale_log2;
     bool flip = false;
-    if (!BIAS && p.head_scale) {
+    if (FORMS && !BIAS && p.head_scale) {
       const float f = p.head_scale[real_head];
       flip = f < 0.f;
       scale_log2 *= fabsf(f);
@@ -381,7 +386,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
       for (int c = 0; c < KEYS; c += 16) ft_ld16(t_s + (uint32_t)c, sc + c);
       ft_ld_wait();
-      if (flip) {
+      if (FORMS && flip) {
 #pragma unroll
         for (int c = 0; c < KEYS; ++c) sc[c] = -sc[c];
       }
@@ -416,7 +421,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 #pragma unroll
         for (int c = 0; c < KEYS; ++c) sc[c] = fmaf(sc[c], p.scale_log2, -bias_l[-c]);
       }
-      const float to_log2 = BIAS ? 1.0f : scale_log2;
+      const float to_log2 = BIAS ? 1.0f : FORMS ? scale_log2 : p.scale_log2;
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains instead of one long one
 #pragma unroll
       for (int c = 0; c < KEYS; c += 8) {
@@ -512,7 +517,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       const uint32_t t_mine = tmem_o + t_lane + (uint32_t)(DH * half);          // this thread's dims in the first O
       const size_t slot_floats = (size_t)(DV + 2) * FT_BM;
-      const int all_heads = p.n_heads * p.maps;
+      const int all_heads = p.n_heads * maps;
       const size_t part_stride = (size_t)all_heads * slot_floats;
       bool write_out = fine, merge = false;
       if (n_parts > 1) {
@@ -590,7 +595,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
               for (int c = 0; c < 32; ++c) o[c] = w_a * o[c] + w_b * ob[c];
             }
           }
-          if (p.out_f32) {
+          if (FORMS && p.out_f32) {
 #pragma unroll
             for (int c = 0; c < 32 && row_ok; c += 4)
               *reinterpret_cast<float4*>(dst_f + c0 + c) = make_float4(o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv);
@@ -651,27 +656,35 @@ LLMI_EXPORT int llmi_attention_prefill_tc_supported(int head_dim) { return head_
 LLMI_EXPORT int llmi_attention_prefill_tc_sizes(int dk, int dv) { return (dk == 64 && (dv == 64 || dv == 128)) || (dk == 128 && dv == 128); }
 
 namespace llmi {
-template <int DK, int DV, bool BIAS>
+template <int DK, int DV, bool BIAS, bool FORMS>
 static int ft_launch_b(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkp,
                      const CUtensorMap& mvp, const PrefillTcParams& p, dim3 grid, cudaStream_t stream) {
   using C = FtCfg<DK, DV>;
   static PerDevice<bool> configured_on;
   bool& configured = configured_on.here();
   if (!configured) {
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<DK, DV, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<DK, DV, BIAS, FORMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
       return LLMI_ERR_LAUNCH;
     configured = true;
   }
   // a programmatic dependent: its blocks set themselves up (barriers, tensor memory, descriptors) while the kernel
   // before drains; the producer waits before its first copy, and nothing else reads or writes global memory earlier
-  return launch_pdl(PDL_ATTENTION, attention_prefill_tc_kernel<DK, DV, BIAS>, grid, dim3(C::THREADS), C::SMEM, stream, mq, mk, mv, mkp, mvp, p);
+  return launch_pdl(PDL_ATTENTION, attention_prefill_tc_kernel<DK, DV, BIAS, FORMS>, grid, dim3(C::THREADS), C::SMEM, stream, mq, mk, mv, mkp, mvp, p);
 }
 template <int DK, int DV>
 static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mkp,
                      const CUtensorMap& mvp, const PrefillTcParams& p, dim3 grid, cudaStream_t stream) {
+  const bool forms = DK != DV || p.maps > 1 || p.out_f32 || p.head_scale;
   if constexpr (DK == DV)
-    if (p.r1) return ft_launch_b<DK, DV, true>(mq, mk, mv, mkp, mvp, p, grid, stream);
-  const int rc = ft_launch_b<DK, DV, false>(mq, mk, mv, mkp, mvp, p, grid, stream);
+    if (p.r1)
+      return forms ? ft_launch_b<DK, DV, true, true>(mq, mk, mv, mkp, mvp, p, grid, stream)
+                   : ft_launch_b<DK, DV, true, false>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  int rc;
+  if constexpr (DK == DV)
+    rc = forms ? ft_launch_b<DK, DV, false, true>(mq, mk, mv, mkp, mvp, p, grid, stream)
+               : ft_launch_b<DK, DV, false, false>(mq, mk, mv, mkp, mvp, p, grid, stream);
+  else
+    rc = ft_launch_b<DK, DV, false, true>(mq, mk, mv, mkp, mvp, p, grid, stream);
   pairs_may_start_early = true;
   return rc;
 }
