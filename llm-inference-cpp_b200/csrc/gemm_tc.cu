@@ -321,10 +321,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 //
 // Two groups of four epilogue warps take a tile's chunks of 16 tokens in turn: with one group the way out of a tile was longer
 // than its products where k is short (k = 960, 256 tokens: 5.7 us of MMAs, 16 chunks of 0.4 us), and the last tile's is never
-// hidden.  The first stages' weights are asked for before the wait for the kernel ahead.  Tokens x rows x k, before -> after:
-// 4,860 x 4,096 x 512 45.9 -> 28.8 us, 7,931 x 5,120 x 960 gated 109 -> 65, 2,048 x 5,120 x 960 gated 29.5 -> 25.5, 4,860 x 1,600
-// x 960 21.8 -> 19.6; long k and the residual add unchanged (2,048 x 16,384 x 2,048 101.5 -> 101.2; 4,860 x 960 x 960 16.8 ->
-// 18.2, x 2,560 31.6 -> 32.0).
+// hidden.  Tokens x rows x k, one group -> two (one after another, their operands cold): 4,860 x 4,096 x 512 38.7 -> 31.4 us,
+// 4,860 x 5,120 x 960 gated 56.6 -> 45.0, 4,860 x 1,600 x 960 23.2 -> 19.4; residual add: 2,048 x 2,048 x 2,048 20.7 -> 19.4, 4,860 x
+// 576 x 1,536 17.7 -> 16.4, 4,860 x 960 x 960 18.3 -> 18.2, 7,931 x 2,048 x 2,048 55.4 -> 56.2, x 8,192 191.5 -> 191.8.
+// (The weights of the first stages asked for before the wait for the kernel ahead, as the kernels for few tokens do it, cost 1 to
+// 5 %: a pair reads them while the product before still waits for its last tiles: 4,860 x 960 x 2,560 31.1 -> 32.6, 7,931 x 2,048 x
+// 8,192 191.8 -> 196.6, 2,601 likewise 80.9 -> 85.1.)
 constexpr int TP_BN = 256;              // widest token tile; an accumulator's columns in TMEM
 constexpr int TP_STAGES = 6;
 constexpr int TP_STAGE_BYTES = 2 * TC_BM * TC_BK * 2;   // A half-tile + B half-tile, 16 KB each
@@ -383,30 +385,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   if (warp == 0) {
     if (lane == 0) {
       // ---- TMA producer (both CTAs): own 128 weight rows and own half of the token tile ----
-      // The weights of the first stages are asked for before the wait: only x comes from the kernel before.
-      const int mine = pair < n_units ? (n_units - pair + n_pairs - 1) / n_pairs : 0;
-      const int total = mine * kblocks, ahead = total < TP_STAGES ? total : TP_STAGES;
-      auto load_w = [&](int it, int u, int i) {
-        const int s = it % TP_STAGES;
-        if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (TC_BM * TC_BK * 2 + (bn >> 1) * TC_BK * 2));
-        tma_load_2d_pair(base + s * TP_STAGE_BYTES, &map_w, i * TC_BK, (u % m_tiles) * 256 + (int)rank * TC_BM, map_to_rank(full_bar(s), 0));
-      };
-      auto load_x = [&](int it, int u, int i) {
-        const int s = it % TP_STAGES;
-        tma_load_2d_pair(base + s * TP_STAGE_BYTES + TC_BM * TC_BK * 2, &map_x, i * TC_BK, (u / m_tiles) * bn + (int)rank * (bn >> 1),
-                         map_to_rank(full_bar(s), 0));
-      };
-      for (int it = 0; it < ahead; ++it) load_w(it, pair + it / kblocks * n_pairs, it % kblocks);
       pdl_wait();
-      for (int it = 0; it < ahead; ++it) load_x(it, pair + it / kblocks * n_pairs, it % kblocks);
-      int u = pair + ahead / kblocks * n_pairs, i = ahead % kblocks;
-      for (int it = ahead; it < total; ++it) {
-        if (!mbar_wait(empty_bar(it % TP_STAGES), ((it / TP_STAGES) - 1) & 1, p.error_flag, 5)) break;
-        load_w(it, u, i);
-        load_x(it, u, i);
-        if (++i == kblocks) {
-          i = 0;
-          u += n_pairs;
+      int it = 0;
+      bool ok = true;
+      for (int u = pair; u < n_units && ok; u += n_pairs) {
+        const int mt = u % m_tiles, nt = u / m_tiles;
+        for (int i = 0; i < kblocks; ++i, ++it) {
+          const int s = it % TP_STAGES;
+          if (it >= TP_STAGES && !mbar_wait(empty_bar(s), ((it / TP_STAGES) - 1) & 1, p.error_flag, 5)) { ok = false; break; }
+          const uint32_t leader_full = map_to_rank(full_bar(s), 0);
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (TC_BM * TC_BK * 2 + (bn >> 1) * TC_BK * 2));
+          const uint32_t dst = base + s * TP_STAGE_BYTES;
+          tma_load_2d_pair(dst, &map_w, i * TC_BK, mt * 256 + (int)rank * TC_BM, leader_full);
+          tma_load_2d_pair(dst + TC_BM * TC_BK * 2, &map_x, i * TC_BK, nt * bn + (int)rank * (bn >> 1), leader_full);
         }
       }
     }
