@@ -237,8 +237,8 @@ linear_f32_tile_kernel(const float* __restrict__ x, long ldx, const float* __res
 // ---------------------------------------------------------------------------------------------------------------------
 // Few tokens.  Bound by reading w once, and by latency: a decode step of a small model is a chain of such products.  A block
 // takes ROWS rows of w; rows and tokens go to shared memory in segments of 256 places (places 260 floats apart: a quarter
-// warp's 16-byte loads of its four rows touch different banks), w before the kernel before has ended (it does not depend on
-// it).  A thread makes the sums of one segment for two rows and two (or four) tokens: 4 (6) shared loads of 16 bytes per 16
+// warp's 16-byte loads of its four rows touch different banks), w, where the caller says that the kernel before does not write
+// it (`early`: a model's weights), before that kernel has ended (a request step of the 360M shape 39.9 -> 38.9 ms).  A thread makes the sums of one segment for two rows and two (or four) tokens: 4 (6) shared loads of 16 bytes per 16
 // (32) FMAs, which is what a block spends its time on: with one row a thread it is 1.5 (1.7) times as many.  A chain of 256
 // FMAs is 1,024 clocks, half a microsecond, whatever K is, where one chain over K = 2,560 is 5 us.
 // Four tokens, as they follow one another in a step (rows of w x K): 960 x 960 22.3 -> 6.0 us, 5,120 x 960 23.4 -> 11.3, 960 x
@@ -253,7 +253,7 @@ template <int MODE, int TOKENS>
 __global__ void __launch_bounds__(512)
 linear_f32_rows_kernel(const float* __restrict__ x, long ldx, const float* __restrict__ w, long ldw, const float* __restrict__ bias,
                        const float* __restrict__ oscale, float* __restrict__ y, long ldy, int M, int N, int K, int staged, int pass,
-                       long bx, long bw, long by) {
+                       int early, long bx, long bw, long by) {
   extern __shared__ __align__(16) float rows_smem[];
   x += (long)blockIdx.z * bx;
   w += (long)blockIdx.z * bw;
@@ -269,7 +269,8 @@ linear_f32_rows_kernel(const float* __restrict__ x, long ldx, const float* __res
   const int row = tid & 3, tg = (tid >> 2) % groups, seg_lane = (tid >> 2) / groups;      // rows `row` and `row` + 4
   const int seg_lanes = (n_threads >> 2) / groups;
   pdl_launch_dependents();
-  bool waited = false;
+  bool waited = !early;
+  if (!early) pdl_wait();
   float total[ROWS_MAX_TOKENS / ROWS_PASS] = {};                      // this thread's output of every pass, over the rounds
 
   for (int s0 = 0; s0 < n_seg; s0 += staged) {
@@ -337,7 +338,7 @@ linear_f32_rows_kernel(const float* __restrict__ x, long ldx, const float* __res
 
 template <int MODE, int TOKENS>
 int launch_linear_f32_rows(const float* x, long ldx, const float* w, long ldw, const float* bias, const float* oscale, float* y, long ldy,
-                           int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by) {
+                           int M, int N, int K, int early, cudaStream_t stream, int batch, long bx, long bw, long by) {
   static PerDevice<bool> configured;
   if (!configured.here()) {
     if (cudaFuncSetAttribute(linear_f32_rows_kernel<MODE, TOKENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
@@ -354,7 +355,7 @@ int launch_linear_f32_rows(const float* x, long ldx, const float* w, long ldw, c
   int threads = 4 * (pass / TOKENS) * staged;
   threads = threads < ROWS_THREADS ? ROWS_THREADS : (threads > 512 ? 512 : (threads + 31) / 32 * 32);
   return launch_pdl(PDL_GEMM, linear_f32_rows_kernel<MODE, TOKENS>, dim3(blocks, 1, batch), dim3(threads), (size_t)staged * seg_bytes, stream,
-                    x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, staged, pass, bx, bw, by);
+                    x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, staged, pass, early, bx, bw, by);
 }
 
 // Which kernel: fp32 rows that 16-byte copies can take go to the two fast ones.  Up to 8 tokens the rows kernel; up to 64 while
@@ -363,10 +364,10 @@ int launch_linear_f32_rows(const float* x, long ldx, const float* w, long ldw, c
 constexpr long ROWS_MAX_OUTPUTS = 104 * 1024;
 template <int MODE>
 int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const float* bias, const float* oscale, float* y, long ldy,
-                      int M, int N, int K, cudaStream_t stream, int batch, long bx, long bw, long by) {
+                      int M, int N, int K, int early, cudaStream_t stream, int batch, long bx, long bw, long by) {
   if (M <= 8 || (M <= ROWS_MAX_TOKENS && (long)M * N * batch <= ROWS_MAX_OUTPUTS)) {
-    if (M <= 8) return launch_linear_f32_rows<MODE, 2>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, stream, batch, bx, bw, by);
-    return launch_linear_f32_rows<MODE, 4>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, stream, batch, bx, bw, by);
+    if (M <= 8) return launch_linear_f32_rows<MODE, 2>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, early, stream, batch, bx, bw, by);
+    return launch_linear_f32_rows<MODE, 4>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, early, stream, batch, bx, bw, by);
   }
   static PerDevice<bool> configured;
   if (!configured.here()) {
@@ -381,15 +382,15 @@ int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const 
 
 template <typename T>
 int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale, void* y, long ldy, int M,
-                       int N, int K, int mode, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
+                       int N, int K, int mode, int early, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
   if (grid.y > 65535 || batch < 1 || batch > 65535) return LLMI_ERR_BAD_SIZE;
   pairs_may_start_early = false;
   const bool rows_of_16 = (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && ((ldx | ldw | bx | bw | (long)K) & 3) == 0;
 #define LLMI_LAUNCH(MODE)                                                                                                     \
   if (sizeof(T) == 4 && rows_of_16)                                                                                           \
-    return launch_linear_f32<MODE>((const float*)x, ldx, (const float*)w, ldw, bias, oscale, (float*)y, ldy, M, N, K, stream, \
-                                   batch, bx, bw, by);                                                                        \
+    return launch_linear_f32<MODE>((const float*)x, ldx, (const float*)w, ldw, bias, oscale, (float*)y, ldy, M, N, K, early,  \
+                                   stream, batch, bx, bw, by);                                                                        \
   linear_simt_kernel<T, MODE><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by)
   switch (mode) {
     case OUT_STORE: LLMI_LAUNCH(OUT_STORE); break;
@@ -406,13 +407,14 @@ int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const f
 using namespace llmi;
 
 // x [M, K] (row pitch ldx), w [N, K] (row pitch ldw), y [M, N] (row pitch ldy), pitches in elements; y takes
-// (x · wᵀ + bias) * oscale, both [N] or null.
+// (x · wᵀ + bias) * oscale, both [N] or null.  early 1: the launch ahead does not write w (a model's weights), so that it may be
+// read before that launch has ended.
 LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale,
-                                 void* y, long ldy, int M, int N, int K, int mode, cudaStream_t stream) {
+                                 void* y, long ldy, int M, int N, int K, int mode, int early, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
-  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
+  if (dtype == LLMI_DTYPE_F32) return launch_linear_simt<float>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, early, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, stream);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, bias, oscale, y, ldy, M, N, K, mode, early, stream);
   return LLMI_ERR_BAD_DTYPE;
 }
 
@@ -420,12 +422,12 @@ LLMI_EXPORT int llmi_linear_simt(int dtype, const void* x, long ldx, const void*
 // elements; rows may be strided, so the operands of a batch may interleave: the heads of one activation row).
 // Arithmetic and order of additions are those of llmi_linear_simt.
 LLMI_EXPORT int llmi_linear_simt_batched(int dtype, const void* x, long ldx, long bx, const void* w, long ldw, long bw,
-                                         void* y, long ldy, long by, int batch, int M, int N, int K, int mode,
+                                         void* y, long ldy, long by, int batch, int M, int N, int K, int mode, int early,
                                          cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return LLMI_ERR_BAD_SIZE;
   if (dtype == LLMI_DTYPE_F32)
-    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
+    return launch_linear_simt<float>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, early, stream, batch, bx, bw, by);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, stream, batch, bx, bw, by);
+    return launch_linear_simt<__nv_bfloat16>(x, ldx, w, ldw, nullptr, nullptr, y, ldy, M, N, K, mode, early, stream, batch, bx, bw, by);
   return LLMI_ERR_BAD_DTYPE;
 }

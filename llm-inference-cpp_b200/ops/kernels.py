@@ -286,9 +286,10 @@ def _check_oscale(oscale, n: int, mode: int) -> None:
 
 
 def linear_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None,
-                mode: int = OUT_STORE, oscale: torch.Tensor | None = None) -> None:
+                mode: int = OUT_STORE, oscale: torch.Tensor | None = None, early: bool = False) -> None:
     """out (mode) (x·wᵀ + bias) * oscale with fp32 FMA arithmetic; x [M,K], w [N,K], rows may be strided; bias and oscale
-    fp32 [N], optional."""
+    fp32 [N], optional.  ``early``: the launch ahead does not write w (a model's weights), so it may be read before that
+    launch has ended."""
     _need_cuda(x, w, out, bias)
     _check_oscale(oscale, w.shape[0], mode)
     M, K = x.shape
@@ -303,7 +304,7 @@ def linear_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch
         assert bias.dtype == torch.float32 and bias.numel() == N
     _check("linear_simt", lib().llmi_linear_simt(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), _ptr(w), c_long(w.stride(0)), _ptr(bias), _ptr(oscale), _ptr(out),
-        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
+        c_long(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(mode), c_int(1 if early else 0), _stream()))
 
 
 class _TcScratch:
@@ -491,7 +492,8 @@ def linear(x, w, out, bias=None, mode: int = OUT_STORE, then_norm: DeferredNorm 
     """The matrix product of the step: the tensor-core kernels for bf16 operands they can take (16-byte
     aligned rows), the fp32 FMA kernel for the 32-bit path and for everything else.  ``x`` may be a filled
     :class:`DeferredNorm`; returns whether ``then_norm`` was filled (False: run that norm the plain way).  ``oscale`` (fp32,
-    one number per row of w): the product with its bias is multiplied by it before it is stored or added."""
+    one number per row of w): the product with its bias is multiplied by it before it is stored or added.  ``w`` is a
+    weight: the kernels for few tokens read it while the launch ahead still runs, so that launch must not write it."""
     xin = x.h if isinstance(x, DeferredNorm) else x
     if not _FORCE_SIMT and gemm_tc_eligible(xin, w):
         return gemm_bf16(x, w, out, bias, mode, then_norm, oscale)
@@ -500,10 +502,10 @@ def linear(x, w, out, bias=None, mode: int = OUT_STORE, then_norm: DeferredNorm 
             raise KernelError("a deferred norm that no product has filled")
         rmsnorm(x.source, x.weight, x.h, x.eps)
     if mode in _STORE_ACTIVATIONS:       # the fp32 FMA product has no activation in its epilogue: two steps
-        linear_simt(xin, w, out, bias, OUT_STORE, oscale)
+        linear_simt(xin, w, out, bias, OUT_STORE, oscale, early=True)
         activate(out, out, _STORE_ACTIVATIONS[mode])
         return False
-    linear_simt(xin, w, out, bias, mode, oscale)
+    linear_simt(xin, w, out, bias, mode, oscale, early=True)
     return False
 
 
@@ -1437,10 +1439,12 @@ def stream_add(x: torch.Tensor, add: torch.Tensor | None, vec: torch.Tensor | No
 HEADS_MMA_MIN_TOKENS = int(os.environ.get("LLMI_HEADS_MMA_MIN", "1"))      # from here on the per-head products of a step run on the tensor cores (bf16)
 
 
-def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor, by: int, K: int, mode: int = OUT_STORE) -> None:
+def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor, by: int, K: int, mode: int = OUT_STORE,
+                   early: bool = False) -> None:
     """``w.shape[0]`` products in one launch (one per head): out_b (mode) x_b . w[b]^T with x_b = x[:, b*bx : b*bx + K] and
     out_b = out[:, b*by : b*by + N]; w [batch, N, K] contiguous.  fp32 FMA arithmetic for the 32-bit path and for a
-    handful of rows; bf16 products of more rows run as tensor-core tiles (bf16 in, fp32 accumulation)."""
+    handful of rows; bf16 products of more rows run as tensor-core tiles (bf16 in, fp32 accumulation).  ``early``: see
+    :func:`linear_simt`."""
     _need_cuda(x, w, out)
     B, N, Kw = w.shape
     M = x.shape[0]
@@ -1456,7 +1460,8 @@ def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor,
         return
     _check("linear_batched", lib().llmi_linear_simt_batched(
         c_int(_dtype_code(x)), _ptr(x), c_long(x.stride(0)), c_long(bx), _ptr(w), c_long(K), c_long(N * K), _ptr(out),
-        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode), _stream()))
+        c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N), c_int(K), c_int(mode),
+        c_int(1 if early else 0), _stream()))
 
 
 # ---------------------------------------------------------------------------------------------

@@ -132,17 +132,17 @@ class LatentAttention:
                 return kernels.linear(heads, self.w_o, x, None, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,
                                       None if store else then_norm, out_scale)
             qa = rt.scratch("latent_qa", (T, H * (C + R)))
-            kernels.linear_batched(q, D + R, self.w_uk_t, qa, C + R, D)
+            kernels.linear_batched(q, D + R, self.w_uk_t, qa, C + R, D, early=True)
             kernels.latent_q_rotate(q, D, qa, C, R, H, self.inv_freq, self.rot_dims, ctx, self.pairing, self.amplitude)
         else:
             qa = rt.scratch("latent_qa", (T, H * (C + R)))
             qn = rt.scratch("latent_q", (T, H * D))
             kernels.latent_prepare_direct(down, H, D, C, R, self.w_cnorm, self.eps, self.inv_freq, self.rot_dims, self.pairing, ctx,
                                           pages, g.page_size, cache, qn, qa, write_kv=binding.writes, amplitude=self.amplitude)
-            kernels.linear_batched(qn, D, self.w_uk_t, qa, C + R, D)
+            kernels.linear_batched(qn, D, self.w_uk_t, qa, C + R, D, early=True)
         lat = rt.scratch("latent_ctx", (T, H * C))
         kernels.attention_latent(qa, lat, cache, ctx, pages, g.page_size, H, C, R, self.scale, rt=rt, window=self.window)
         heads = rt.scratch("attn_out", (T, H * Dv))
-        kernels.linear_batched(lat, C, self.w_uv, heads, Dv, C)
+        kernels.linear_batched(lat, C, self.w_uv, heads, Dv, C, early=True)
         return kernels.linear(heads, self.w_o, x, None, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,
                               None if store else then_norm, out_scale)

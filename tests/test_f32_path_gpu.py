@@ -122,3 +122,28 @@ def test_attention_f32_prompt_and_decode(nh, nkv, hd, window):
         k.attention(qd, got, kc, vc, one, pages[who].contiguous(), 64, nh, nkv, hd, scale, window)
         assert torch.equal(got[:-1], out[rows]) and bool((got[-1] == 0).all())
     k.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("M", [1, 8, 24])
+def test_a_matrix_that_the_launch_ahead_writes(M):
+    """Without ``early`` the second matrix may come out of the product just ahead, which lets the next launch start before it has
+    ended."""
+    k = K()
+    torch.manual_seed(M)
+    N, K_ = 24, 4096
+    base, x = torch.randn(N, 512, device="cuda"), torch.randn(M, K_, device="cuda")
+    w, y = torch.zeros(N, K_, device="cuda"), torch.empty(M, N, device="cuda")
+    for _ in range(50):
+        a = torch.randn(K_, 512, device="cuda") / 512 ** 0.5
+        w.zero_()
+        k.linear_simt(base, a, w)                    # w [N, 4096]: the launch ahead
+        k.linear_simt(x, w, y)
+        ref = x.double() @ (base.double() @ a.double().T).T
+        assert float((y.double() - ref).norm() / ref.norm()) < 2e-6
+        b = w.view(2, N // 2, K_)
+        out = torch.empty(M, N, device="cuda")
+        w.zero_()
+        k.linear_simt(base, a, w)
+        k.linear_batched(x, 0, b, out, N // 2, K_)
+        assert torch.equal(out, y)
+    k.check_device_errors("cuda:0")
