@@ -13,7 +13,8 @@
 //
 //  * with a top_k of at most 512 (what chats are sampled with): each block finds the top_k-th largest of its threads' own
 //    maxima, a bound that at least top_k values reach; the largest bound of the eight lets few more than top_k values
-//    through.  Those (up to 1,024) go to the first block, which ranks them by (value descending, id ascending), cuts the
+//    through (where a peaked row has fewer probabilities above 0, the bound is the smallest number above 0: what is 0 is
+//    never drawn and adds nothing to a mass).  Those (up to 1,024) go to the first block, which ranks them by (value descending, id ascending), cuts the
 //    ranks after top_k and top_p, and draws from the kept ones in id order: no pass over the row per bit.
 //  * otherwise: the kept set is { p > thr } plus the first n_eq ids with p == thr, and (thr, n_eq) is found by building
 //    thr's bit pattern from the top bit down with counting (top-k) or mass (top-p) passes: probabilities are non-negative
@@ -23,8 +24,8 @@
 // rows are in the launch.
 //
 // What bounds it: one block per row, its 31 bits' passes for top_k and 31 more for top_p each over the whole row, took
-// 304 us for a row of 49,152 with top_k 50 and top_p 0.95, a fifth of a decode step at batch 1.This way 20 us (8 rows
-// the same, 64 rows 43 us); the general way 56 us with top_k 0 and top_p 0.95.
+// 304 us for a row of 49,152 with top_k 50 and top_p 0.95, a fifth of a decode step at batch 1.  This way 20 us (8 rows
+// the same, 64 rows 43 us; peaked rows 20 and 37 us); the general way 56 us with top_k 0 and top_p 0.95.
 //
 // `probs` is caller-provided scratch of n_rows * vocab floats (used when an eighth of a row exceeds shared memory).
 #include <cooperative_groups.h>
@@ -180,7 +181,8 @@ struct RowReduce {
   }
 };
 
-__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_ROW_THREADS)
+// (three blocks an SM: with the 52 registers that are taken otherwise two, 64 rows 51 -> 59 us)
+__global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_ROW_THREADS, 3)
 sample_kernel(const float* __restrict__ logits, long ld, int vocab, float temperature, int top_k, float top_p,
               const double* __restrict__ uniforms, float* __restrict__ probs, int32_t* __restrict__ out, int chunk,
               int probs_in_smem) {
@@ -234,8 +236,8 @@ sample_kernel(const float* __restrict__ logits, long ld, int vocab, float temper
 
   if (k <= NT) {
     // ---- few candidates ----
-    // the k-th largest of the threads' maxima (0 when fewer ids than that are here), bit by bit; at least k values of
-    // this block, so of the row, reach it
+    // the k-th largest of the threads' maxima (0 when fewer than that are above 0), bit by bit; at least k values of this
+    // block, so of the row, reach it
     uint32_t bound = 0;
     for (int bit = 30; bit >= 0; --bit) {
       const uint32_t cand = bound | (1u << bit);
@@ -244,6 +246,7 @@ sample_kernel(const float* __restrict__ logits, long ld, int vocab, float temper
     const double* all = red.exchange((double)bound);
 #pragma unroll
     for (int r = 0; r < SAMPLE_CLUSTER; ++r) bound = max(bound, (uint32_t)all[r]);
+    bound = max(bound, 1u);                   // (the other ids of the k have probability 0)
     int* counter = cluster.map_shared_rank(&n_list, 0);
     uint2* dst = cluster.map_shared_rank(list, 0);
     if (own >= bound)
@@ -268,16 +271,17 @@ sample_kernel(const float* __restrict__ logits, long ld, int vocab, float temper
         if (before < k) kept_list[before] = me;
       }
       __syncthreads();
-      const bool in_k = tid < k;              // (m >= k values passed the bound)
+      const int found = (int)min(k, (long long)m);      // (fewer than k only where the others are 0)
+      const bool in_k = tid < found;
       const uint2 me = in_k ? kept_list[tid] : make_uint2(0u, 0u);
       const double mine = in_k ? (double)__uint_as_float(me.x) : 0.0;
-      int n_kept = (int)k;
+      int n_kept = found;
       if (top_p < 1.0f) {
         // the shortest prefix whose running sum reaches top_p (all of them when none does), at least one
         double total;
         const double upto = red.block_scan(mine, &total) + mine;
         const int below = __syncthreads_count(in_k && !(upto >= (double)top_p));
-        n_kept = min((int)k, below + 1);
+        n_kept = min(found, below + 1);
       }
       // the kept ones in id order
       const bool in = tid < n_kept;

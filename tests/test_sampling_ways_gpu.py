@@ -37,3 +37,51 @@ def test_sample_both_ways(V, top_k, top_p):
         # the draw's own interval holds the number, up to the rounding of the 32-bit probabilities
         slack = 1e-6 + 2e-7 * V ** 0.5
         assert cum[got] - prob[got] - slack <= float(u[i]) <= cum[got] + slack, (i, got)
+
+
+@pytest.mark.parametrize("above", [1, 2, 10, 49, 50, 51, 400, 3000])
+@pytest.mark.parametrize("top_p", [0.9, 1.0])
+def test_sample_peaked_rows(above, top_p):
+    """Rows with so many probabilities above 0, fewer and more than top_k, spread over the vocabulary or side by side: the plain
+    sampler's id."""
+    k = K()
+    V, top_k = 49152, 50
+    torch.manual_seed(above)
+    logits = torch.full((4, V), -1e4, device="cuda")
+    logits[0, torch.randperm(V)[:above].cuda()] = torch.randn(above, device="cuda")
+    logits[1, :above] = torch.randn(above, device="cuda")
+    logits[2, V - above:] = torch.randn(above, device="cuda")
+    logits[3, torch.randperm(V)[:above].cuda()] = 1.0
+    u = torch.tensor([0.3, 0.9999, 0.0001, 0.7], dtype=torch.float64, device="cuda")
+    out = torch.empty(4, dtype=torch.int32, device="cuda")
+    k.sample(logits, 1.0, top_k, top_p, u, torch.empty(4, V, device="cuda"), out)
+    for i in range(4):
+        prob = P.sampling_probabilities(logits[i].cpu().numpy(), 1.0, top_k, top_p)
+        cum = np.cumsum(prob.astype(np.float64))
+        got = int(out[i])
+        assert prob[got] > 0
+        assert cum[got] - prob[got] - 1e-6 <= float(u[i]) <= cum[got] + 1e-6, (i, got)      # (see test_sample_both_ways)
+
+
+def test_sample_peaked_rows_are_no_slower():
+    """A low temperature leaves a few dozen probabilities above 0: such rows take the way of ordinary ones, in about its time (the
+    way past a full list took five times as long)."""
+    k = K()
+    n, V = 64, 49152
+    torch.manual_seed(0)
+    logits, u = torch.randn(n, V, device="cuda") * 2.5, torch.rand(n, dtype=torch.float64, device="cuda")
+    probs, out = torch.empty(n, V, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+
+    def us(temperature):
+        times = []
+        for _ in range(15):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(10):
+                k.sample(logits, temperature, 50, 0.95, u, probs, out)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b) * 100)
+        return sorted(times)[3]
+    us(0.8)
+    assert us(0.01) < 2 * us(0.8)
