@@ -715,7 +715,12 @@ def decode_cluster(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int, gr
     return 0
 
 
-def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int, group: int) -> int:
+def visible_pages(n_pages: int, window: int, max_q: int = 1) -> int:
+    """Most pages that the newest ``max_q`` positions of a sequence see of page tables of ``n_pages``."""
+    return min(n_pages, -(-(window + max_q - 1) // 64) + 1) if window > 0 else n_pages
+
+
+def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int, group: int, window: int = 0) -> int:
     """Blocks of a cluster that share a (sequence, kv head) in attention_short for a decode step, or 0 where one of the
     persistent kernels (attention_decode_mma, attention_decode) is as fast or faster.
 
@@ -723,12 +728,14 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
     the last split's loads of all parts — and, ungrouped with heads of 128, by their arithmetic; here the parts meet in shared
     memory.  A cluster of up to eight blocks takes an item while all of them are resident at once; so a few sequences of very
     many pages, which the persistent kernels cut finer, stay with them, as do ungrouped heads of 64 up to that point, and
-    items that need a second, nearly empty wave.  Measured, persistent -> this (us, with the position encoding; kv heads x
+    items that need a second, nearly empty wave.  Under a window the pages are those that it spans (planned by the whole
+    history, 32 sequences of 4,000 under a window of 128, 3 x 3 x 64, took 7.7 us, the persistent kernel 6.6; by the window 5.5).  Measured, persistent -> this (us, with the position encoding; kv heads x
     group x size, sequences, positions): 3 x 3 x 64, 1, 1,000 8.0 -> 5.1, 8, 4,000 11.2 -> 10.0, 1, 8,000 10.4 -> 10.6; 8 x 4 x
     128, 1, 1,000 9.8 -> 6.1, 24, 2,200 39.5 -> 38.5; 16 x 128, 4, 4,000 33.8 -> 26.4, 64, 2,200 229 -> 180; 32 x 64, 64, 2,200 188
     -> 180, 24, 2,200 74.9 -> 71.9; with bf16 weights, 16, 2,200 51 -> 58, 4, 2,200 16.4 -> 15.9."""
     if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma":
         return 0
+    n_pages = visible_pages(n_pages, window)
     resident, items = (3 if head_dim == 64 else 2) * sm_count(), n_live * n_kv_heads
     if items > resident:
         if head_dim == 64:
@@ -744,10 +751,10 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
     return parts
 
 
-def decode_plan_token(ctx, n_seqs: int, n_pages: int, page_size: int, n_kv_heads: int, head_dim: int, group: int):
+def decode_plan_token(ctx, n_seqs: int, n_pages: int, page_size: int, n_kv_heads: int, head_dim: int, group: int, window: int = 0):
     """What tells two recorded decode steps of the same padded shape apart: the split and the kernel's variant."""
     pps, n_live, cluster = decode_plan(ctx, n_seqs, n_pages, page_size, n_kv_heads, head_dim, group)
-    parts = decode_short_parts(n_live, n_kv_heads, n_pages, head_dim, group)
+    parts = decode_short_parts(n_live, n_kv_heads, n_pages, head_dim, group, window)
     if parts:
         return ("short", parts)
     if decode_uses_mma(head_dim, group):
@@ -917,7 +924,7 @@ _PREFILL_US = {64: (3.3, 0.7, 0.048, 0.0025), 128: (3.4, 1.15, 0.048, 0.0047)}
 _short_plans: dict = {}
 
 
-def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int, head_dim: int) -> int:
+def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int, head_dim: int, window: int = 0) -> int:
     """Blocks of a cluster that share the pages of a (sequence, kv head, row tile) in attention_short, or 0 where the prompt
     kernel of 128-query tiles (attention_prefill_tc) is the faster one.
 
@@ -927,6 +934,7 @@ def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, 
     1 / 2 / 4 / 8 blocks against the prompt kernel (us): 3 x 3 x 64, 4 sequences of 1,500, 16 tokens 24.4 / 16.2 / 11.0 / 8.8
     against 22.0; 64 of 150 8.0 / 9.0 against 35.9; 16 of 250, 48 tokens 10.4 / 11.0 against 7.6; 32 x 64, 64 of 500, 16 tokens
     55 / 85 / 157 / 346 against 138; 4 of 1,500, 48 tokens 34.6 / 25.4 / 27.3 / 31.9 against 25.6."""
+    n_pages = visible_pages(n_pages, window, max_q)
     key = (n_seqs, n_kv_heads, max_q, group, n_pages, head_dim)
     best = _short_plans.get(key)
     if best is None:
@@ -959,11 +967,11 @@ def decide(ctx, rule, *sizes):
     return rule(ctx, *sizes)
 
 
-def short_message_plan(ctx, n_seqs: int, n_pages: int, n_kv_heads: int, group: int, head_dim: int) -> tuple:
+def short_message_plan(ctx, n_seqs: int, n_pages: int, n_kv_heads: int, group: int, head_dim: int, window: int) -> tuple:
     """How attention_short takes a prompt step: (blocks of a cluster, rows of a sequence and kv head in whole tiles), or () where it
     goes elsewhere.  (The rows, not the message's length: more tokens than a recording was made with need more tiles.)"""
     max_q = getattr(ctx, "short_message", 0)
-    parts = attention_short_parts(n_seqs, n_kv_heads, max_q, group, n_pages, head_dim) if max_q else 0
+    parts = attention_short_parts(n_seqs, n_kv_heads, max_q, group, n_pages, head_dim, window) if max_q else 0
     rows = max_q * group
     return (parts, 16 if rows <= 16 else 32 if rows <= 32 else -(-rows // 64) * 64) if parts else ()
 
@@ -1044,7 +1052,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
     if _decode_kernel_applies(qkv, ctx, seq_pages, page_size, n_heads, n_kv_heads, head_dim, rt):
         S, P = seq_pages.shape
         pps, n_live, cluster = decode_plan(ctx, S, P, page_size, n_kv_heads, head_dim, n_heads // n_kv_heads)
-        parts = decode_short_parts(n_live, n_kv_heads, P, head_dim, n_heads // n_kv_heads)
+        parts = decode_short_parts(n_live, n_kv_heads, P, head_dim, n_heads // n_kv_heads, window)
         if parts:
             # (the kernels it stands in for: ungrouped heads have 32-bit weights, grouped ones bf16)
             attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, 1, n_heads, n_kv_heads, head_dim,
@@ -1072,7 +1080,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             # longest job: then the key ranges are cut (see the kernel's head).  Measured: 2,048 tokens x 8 heads 28.0 ->
             # 22.2 us, x 4 heads 27.5 -> 21.0 us; with 256 jobs and more the cut gains nothing or costs (4,096 x 8:
             # 49.3 -> 50.5 us; 2,048 x 32: 42.1 -> 49.6 us).
-            short = decide(ctx, short_message_plan, seq_pages.shape[0], seq_pages.shape[1], n_kv_heads, n_heads // n_kv_heads, head_dim)
+            short = decide(ctx, short_message_plan, seq_pages.shape[0], seq_pages.shape[1], n_kv_heads, n_heads // n_kv_heads, head_dim, window)
             if short:
                 attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, ctx.short_message, n_heads,
                                 n_kv_heads, head_dim, scale, window, short[0])

@@ -76,7 +76,7 @@ class GQAttention:
         nh, nkv, hd = self.n_heads, self.n_kv_heads, self.head_dim
         if g.page_size != 64 or not kernels.attention_decode_supported(hd, nh // nkv):
             return None
-        return kernels.decode_plan_token(ctx, S, P, g.page_size, nkv, hd, nh // nkv)
+        return kernels.decode_plan_token(ctx, S, P, g.page_size, nkv, hd, nh // nkv, self.window)
 
     def forward(self, h, x, ctx, binding, then_norm=None) -> bool:
         T = h.shape[0]
