@@ -14,14 +14,14 @@
 //     leaves (values, maximum, sum) in its shared memory; the cluster's warps then add them, a row a warp, in key order.  No workspace, no tickets.
 //
 // The weights (probabilities) meet V as bf16, as in the other tensor-core kernels — but for the decode steps of ungrouped heads
-// (WIDE), whose weights are 32 bits wide in the kernel that has the rest of them (attention_decode.cu).  There a tile has ONE
+// of 128 (WIDE), whose weights are 32 bits wide in the kernel that has the rest of them (attention_decode.cu).  There a tile has ONE
 // row, and the other fifteen are free: all of them hold its query, so that every thread group has its weights, and a weight goes
 // in as three bf16 numbers that add up to it exactly, in three rows: no more matrix instructions than with one.  Every product is
 // exact; the products of a page are summed by the matrix instruction and join the running sums by a rounded addition (running
 // sums inside the instruction are cut off, not rounded).  Against 64 bits the same error as attention_decode.cu's, also where the
-// values' weighted sum all but cancels (there, 64 sequences of 2,200: 1.681e-3 both, of which the output's rounding is all; bf16
+// values' weighted sum all but cancels (there, 64 sequences of 2,200: 1.671e-3 both, of which the output's rounding is all; bf16
 // weights 0.7).  What it costs (with bf16 weights -> with these): 16 x 1 x 128, 64 sequences of 2,200 172 -> 180 us, 1 of 4,000 12.5
-// -> 13.6; 32 x 1 x 64, 64 of 2,200 173 -> 180.
+// -> 13.6.
 //
 // Measured against the tiles of 128 queries (kv heads x group x head size, positions, tokens; with about 8 us of launch):
 // 64 sequences, 32 x 1 x 64, 1,500, 8: 239 -> 140 us (the read of the cache alone: 120 us); 24, 8 x 4 x 128, 2,200, 9:
@@ -516,9 +516,11 @@ static int sh_launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShortPa
 template <int HD>
 static int sh_launch_rows(const CUtensorMap& mk, const CUtensorMap& mv, const ShortParams& p, int n_items, int rows, int parts,
                           bool wide, cudaStream_t stream) {
-  if (p.k_cache_w)
-    return wide ? sh_launch<HD, 16, true, true>(mk, mv, p, n_items, parts, stream) : sh_launch<HD, 16, true, false>(mk, mv, p, n_items, parts, stream);
-  if (wide) return sh_launch<HD, 16, false, true>(mk, mv, p, n_items, parts, stream);
+  if constexpr (HD == 128)
+    if (wide)
+      return p.k_cache_w ? sh_launch<HD, 16, true, true>(mk, mv, p, n_items, parts, stream)
+                         : sh_launch<HD, 16, false, true>(mk, mv, p, n_items, parts, stream);
+  if (p.k_cache_w) return sh_launch<HD, 16, true, false>(mk, mv, p, n_items, parts, stream);
   if (rows <= 16) return sh_launch<HD, 16, false, false>(mk, mv, p, n_items, parts, stream);
   if (rows <= 32) return sh_launch<HD, 32, false, false>(mk, mv, p, n_items, parts, stream);
   return sh_launch<HD, 64, false, false>(mk, mv, p, n_items, parts, stream);
@@ -534,7 +536,7 @@ LLMI_EXPORT int llmi_attention_short_supported(int head_dim) { return head_dim =
 // tokens a sequence brings; parts: blocks that share a (sequence, kv head, row tile): 1, 2, 4 or 8.
 // fuse = 1 (max_q 1, groups up to 16): a decode step as for llmi_attention_decode_fused — `q` is the step's un-rotated
 // [q | k | v] rows, rotary_dim is head_dim or 0, the new k (rotated) and v are appended with write_kv.
-// wide = 1 (max_q 1, ungrouped heads): 32-bit weights.
+// wide = 1 (max_q 1, ungrouped heads of 128): 32-bit weights.
 LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ldo, void* k_cache, void* v_cache,
                                      long n_cache_pages, const int32_t* seq_pages, int pages_stride, const int32_t* seq_q_start,
                                      const int32_t* seq_kv_len, int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim,
@@ -546,7 +548,7 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
   if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)out & 3) || (ldo & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
   const int group = n_heads / n_kv_heads;
   if (fuse && (max_q != 1 || group > 16 || (rotary_dim != 0 && (rotary_dim != head_dim || !inv_freq)))) return LLMI_ERR_UNSUPPORTED;
-  if (wide && (max_q != 1 || group != 1)) return LLMI_ERR_UNSUPPORTED;
+  if (wide && (max_q != 1 || group != 1 || head_dim != 128)) return LLMI_ERR_UNSUPPORTED;
   const long rows = n_cache_pages * n_kv_heads * SH_PAGE, tile_rows = (long)max_q * group;
   const long tiles = (tile_rows + SH_MAX_ROWS - 1) / SH_MAX_ROWS, items = (long)n_seqs * n_kv_heads * tiles;
   if (rows > 0x7fffffffL || items * parts > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;

@@ -727,13 +727,15 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
     Those are bound by the chain behind an item's last page — the four warps' results merged, to memory, a fence, a ticket,
     the last split's loads of all parts — and, ungrouped with heads of 128, by their arithmetic; here the parts meet in shared
     memory.  A cluster of up to eight blocks takes an item while all of them are resident at once; so a few sequences of very
-    many pages, which the persistent kernels cut finer, stay with them, as do ungrouped heads of 64 up to that point, and
-    items that need a second, nearly empty wave.  Under a window the pages are those that it spans (planned by the whole
+    many pages, which the persistent kernels cut finer, stay with them, as do items that need a second, nearly empty wave.  So
+    do ungrouped heads of 64, whose kernel gives its softmax 32-bit weights as this one does for heads of 128: with them
+    this one is between 5 % faster and 30 % slower (32 heads, sequences of 2,200: 20 65.4 -> 70.3, 28 88.8 -> 102, 32 95.5 -> 106, 64 190 ->
+    181, 96 273 -> 278).  Under a window the pages are those that it spans (planned by the whole
     history, 32 sequences of 4,000 under a window of 128, 3 x 3 x 64, took 7.7 us, the persistent kernel 6.6; by the window 5.5).  Measured, persistent -> this (us, with the position encoding; kv heads x
     group x size, sequences, positions): 3 x 3 x 64, 1, 1,000 8.0 -> 5.1, 8, 4,000 11.2 -> 10.0, 1, 8,000 10.4 -> 10.6; 8 x 4 x
-    128, 1, 1,000 9.8 -> 6.1, 24, 2,200 39.5 -> 38.5; 16 x 128, 4, 4,000 33.8 -> 26.4, 64, 2,200 229 -> 180; 32 x 64, 64, 2,200 188
-    -> 180, 24, 2,200 74.9 -> 71.9; with bf16 weights, 16, 2,200 51 -> 58, 4, 2,200 16.4 -> 15.9."""
-    if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma":
+    128, 1, 1,000 9.8 -> 6.1, 1, 200 in one part 5.6 -> 5.0, in two 5.8, 24, 2,200 39.5 -> 38.5; 16 x 128, 1, 2,000 9.7 -> 10.2, 1, 4,000 15.1
+    -> 13.8, 4, 4,000 33.8 -> 26.4, 64, 2,200 229 -> 180."""
+    if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma" or (group == 1 and head_dim == 64):
         return 0
     n_pages = visible_pages(n_pages, window)
     resident, items = (3 if head_dim == 64 else 2) * sm_count(), n_live * n_kv_heads
@@ -741,10 +743,10 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
         if head_dim == 64:
             return 1 if n_pages >= 12 and 10 * items >= 17 * resident else 0
         return 1 if group == 1 or n_pages >= 4 else 0
-    if group == 1 and (head_dim == 64 or (n_pages < 12 and 5 * items < 4 * resident)):
+    if group == 1 and ((n_pages < 12 and 5 * items < 4 * resident) or (16 < n_pages < 48 and 8 * items <= sm_count())):
         return 0
     parts = 1
-    while parts < 8 and 2 * items * parts <= resident and n_pages >= (4 if parts == 1 and head_dim == 128 else 8 * parts):
+    while parts < 8 and 2 * items * parts <= resident and n_pages >= (5 if parts == 1 and head_dim == 128 else 8 * parts):
         parts *= 2
     if parts == 8 and 2 * 8 * items <= resident and n_pages > (100 if head_dim == 64 else 256):
         return 0
@@ -981,8 +983,8 @@ def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pa
                     wide: bool = False) -> None:
     """Causal attention of at most ``max_q`` tokens a sequence over its cache pages (bf16, head size 64 or 128, page 64):
     arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head.  ``rope``
-    (``max_q`` 1): see :func:`attention_decode_mma`.  ``wide`` (``max_q`` 1, ungrouped heads): the
-    weights meet the values as 32-bit numbers."""
+    (``max_q`` 1): see :func:`attention_decode_mma`.  ``wide`` (``max_q`` 1, ungrouped heads of 128):
+    the weights meet the values as 32-bit numbers."""
     inv_freq, rotary_dim, write_kv = rope if rope is not None else (None, 0, False)
     assert rotary_dim == 0 or (inv_freq is not None and inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2)
     _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)

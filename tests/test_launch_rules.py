@@ -31,3 +31,11 @@ def test_a_window_is_planned_by_what_it_spans(kv, group, hd, window):
             seen = -(-(window + max_q - 1) // 64) + 1
             assert K.attention_short_parts(n_seqs, kv, max_q, group, 500, hd, window) == K.attention_short_parts(n_seqs, kv, max_q, group, seen, hd)
     K._plan_cache.clear()
+
+
+def test_ungrouped_decode_steps():
+    """Heads of 64 stay with the kernel that has 32-bit weights and is the faster one; of 128 the clusters begin where they win."""
+    assert not any(K.decode_short_parts(s, h, p, 64, 1) for s in (1, 8, 24, 28, 64, 96) for h in (3, 12, 32) for p in (1, 4, 12, 35, 125))
+    assert [K.decode_short_parts(1, 16, p, 128, 1) for p in (4, 8, 16, 17, 32, 47, 48, 63)] == [0, 0, 4, 0, 0, 0, 8, 8]
+    assert [K.decode_short_parts(1, 32, p, 128, 1) for p in (16, 32, 63)] == [4, 8, 8]
+    assert [K.decode_short_parts(1, 8, p, 128, 4) for p in (1, 4, 5, 8, 16)] == [1, 1, 2, 2, 4]

@@ -99,7 +99,7 @@ def test_attention_short_decode_same_bits(hd, group, window, rot, write):
     k.check_device_errors("cuda:0")
 
 
-@pytest.mark.parametrize("nkv,hd,S,pages,parts", [(32, 64, 24, 12, 1), (16, 128, 24, 3, 1), (16, 128, 4, 16, 4), (8, 128, 2, 40, 8)])
+@pytest.mark.parametrize("nkv,hd,S,pages,parts", [(32, 64, 24, 12, 0), (16, 128, 24, 3, 1), (16, 128, 4, 16, 4), (8, 128, 2, 52, 8)])
 @pytest.mark.parametrize("fused", [True, False])
 def test_ungrouped_decode_has_32_bit_weights(nkv, hd, S, pages, parts, fused):
     """A decode step of ungrouped heads, by the kernel that ``attention`` sends it to and by the one that has the other sizes:
