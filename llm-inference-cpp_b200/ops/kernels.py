@@ -915,43 +915,69 @@ def attention_prefill_tc(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, s
         1 if out.dtype == torch.float32 else 0, _addr(head_scale), _stream_int()))
 
 
-# attention_short, by head size and rows of a tile: (us of a block alone, us a page of it, us a page and item when every SM is
-# busy); a tile's share of that when it is one block, and one of several; the prompt kernel of 128-query tiles likewise (us of a
-# block alone, a page of it, a block, a page and block when every SM is busy).  Fitted to 1 to 64 sequences of 20 to 1,500 positions,
-# messages of 8 to 48 tokens, 32 x 64, 3 x 3 x 64 and 8 x 4 x 128 (kv heads x group x head size).
-_SHORT_US = {64: {16: (2.4, 0.42, 0.0021), 32: (2.9, 0.55, 0.0022), 64: (2.5, 0.93, 0.0034)},
-             128: {16: (3.5, 0.6, 0.004), 32: (4.1, 0.95, 0.0048), 64: (3.2, 1.42, 0.0072)}}
-_SHORT_BLOCK_US = {64: (0.009, 0.02), 128: (0.02, 0.04)}
-_PREFILL_US = {64: (3.3, 0.7, 0.048, 0.0025), 128: (3.4, 1.15, 0.048, 0.0047)}
+# Times in us of attention_short, by head size and rows of a tile, and of the prompt kernel of 128-query tiles, by head size:
+# (a block, a page of it; what both are longer where every place of the device is taken; [a cluster's join, per block of it;] a
+# further wave of blocks, a page of it [, its join]).  Fitted to 14 layouts (1 to 32 kv heads, groups of 1 to 16), 1 to 64 sequences
+# of 60 to 4,000 positions, messages of 2 to 64 tokens, windows of 128 to 2,048: of 1,392 such steps 4 take longer by this choice
+# than on the prompt kernel by more than 3 % (at most 6), and all of them 2 % longer than by the best choice; of 184 drawn ones
+# (other layouts, unequal lengths, padded tables) 5 (at most 6 %).
+_SHORT_US = {64: {16: (2.6, 0.39, 1.9, 0.57, 0.33, 0.19, 2.6, 0.79, 2.6), 32: (3.7, 0.49, 3.7, 0.65, 0.08, 0.1, 4.5, 0.82, 1.8),
+                  64: (2.7, 0.89, 3.5, 0.9, 2.3, 0.0, 1.9, 1.2, 5.1)},
+             128: {16: (3.0, 0.49, 1.6, 0.84, 0.31, 0.31, 2.9, 1.06, 2.6), 32: (4.3, 0.87, 3.7, 0.54, 0.0, 0.2, 6.1, 1.13, 2.0),
+                   64: (3.5, 1.4, 3.4, 0.78, 2.0, 0.14, 3.7, 1.7, 4.7)}}
+_PREFILL_US = {64: (3.1, 0.7, 2.6, 0.52, 13.9, 0.66), 128: (2.8, 1.26, 3.0, 0.66, 10.7, 1.43)}
+
+
+def _waves(blocks: int, resident: int) -> float:
+    """How often the device is filled (many blocks end at different times)."""
+    return float(-(-blocks // resident)) if blocks <= 4 * resident else blocks / resident + 0.5
+
+
+def _prefill_us(n_blocks: int, n_pages: int, head_dim: int) -> float:
+    block, page, full, full_page, wave, wave_page = _PREFILL_US[head_dim]
+    resident = 2 * sm_count()
+    c = min(n_blocks / resident, 1.0)
+    return block + page * n_pages + c * (full + full_page * n_pages) + (_waves(n_blocks, resident) - 1) * (wave + wave_page * n_pages)
+
+
+def _short_us(items: int, parts: int, n_pages: int, head_dim: int, tile: int) -> float:
+    block, page, full, full_page, join, join_block, wave, wave_page, wave_join = _SHORT_US[head_dim][tile]
+    resident, per = (3 if head_dim == 64 else 2) * sm_count(), -(-n_pages // parts)
+    c = min(items * parts / resident, 1.0)
+    us = block + page * per + c * (full + full_page * per) + (join + join_block * parts if parts > 1 else 0.0)
+    return us + (_waves(items * parts, resident) - 1) * (wave + wave_page * per + (wave_join if parts > 1 else 0.0))
+
+
 _short_plans: dict = {}
 
 
-def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int, head_dim: int, window: int = 0) -> int:
+def attention_short_parts(n_seqs: int, n_kv_heads: int, max_q: int, group: int, n_pages: int, head_dim: int, window: int = 0,
+                          cut: bool = False) -> int:
     """Blocks of a cluster that share the pages of a (sequence, kv head, row tile) in attention_short, or 0 where the prompt
-    kernel of 128-query tiles (attention_prefill_tc) is the faster one.
+    kernel of 128-query tiles (attention_prefill_tc) is the faster one.  ``cut``: that kernel would cut the key ranges of a step
+    of few blocks into jobs of 16 pages.
 
     A tile of 64 rows is slower a page than one of 128 queries, but covers all heads of a group, and up to 32 rows it is the
-    faster one; a block of the prompt kernel costs 48 ns however short its sequence (tensor memory, barriers), one of this
-    kernel 9.  A cluster is worth its barriers and its reads from other SMs only while SMs are idle.  Measured, this kernel in
-    1 / 2 / 4 / 8 blocks against the prompt kernel (us): 3 x 3 x 64, 4 sequences of 1,500, 16 tokens 24.4 / 16.2 / 11.0 / 8.8
-    against 22.0; 64 of 150 8.0 / 9.0 against 35.9; 16 of 250, 48 tokens 10.4 / 11.0 against 7.6; 32 x 64, 64 of 500, 16 tokens
-    55 / 85 / 157 / 346 against 138; 4 of 1,500, 48 tokens 34.6 / 25.4 / 27.3 / 31.9 against 25.6."""
+    faster one; a further wave of the prompt kernel's blocks costs 11 to 14 us however short their sequences (tensor memory, barriers),
+    one of this kernel's 2 to 6.  A cluster is worth its barriers and its reads from other SMs only while SMs are idle.  Measured,
+    this kernel in 1 / 2 / 4 / 8 blocks against the prompt kernel (us): 3 x 3 x 64, 4 sequences of 1,500, 16 tokens 25.2 / 16.4 / 10.9 /
+    8.9 against 21.4; 64 of 150 8.6 / 10.3 against 36.3; 16 of 250, 48 tokens 9.7 / 11.4 / 17.4 against 7.9; 32 x 64, 64 of 150, 16 tokens
+    34.2 / 63.3 against 112.9; 4 of 1,500, 48 tokens 30.7 / 28.0 / 30.6 / 38.2 against 27.7."""
     n_pages = visible_pages(n_pages, window, max_q)
-    key = (n_seqs, n_kv_heads, max_q, group, n_pages, head_dim)
+    key = (n_seqs, n_kv_heads, max_q, group, n_pages, head_dim, cut)
     best = _short_plans.get(key)
     if best is None:
         rows = max_q * group
         tiles, tile = -(-rows // 64), 16 if rows <= 16 else (32 if rows <= 32 else 64)
-        items, (fixed, page, busy) = n_seqs * n_kv_heads * tiles, _SHORT_US[head_dim][tile]
-        alone, a_page, block, busy_page = _PREFILL_US[head_dim]
-        cost = max(alone + a_page * n_pages, n_seqs * n_kv_heads * group * (block + busy_page * n_pages))
-        best, cost = 0, 0.92 * cost             # (near the line the prompt kernel: the fit is good to a tenth)
+        items, blocks = n_seqs * n_kv_heads * tiles, n_seqs * n_kv_heads * group
+        cost = _prefill_us(blocks, n_pages, head_dim)
+        if cut and n_pages > PREFILL_SPLIT_PAGES and blocks < sm_count():
+            cost = min(cost, _prefill_us(blocks * -(-n_pages // PREFILL_SPLIT_PAGES), PREFILL_SPLIT_PAGES, head_dim) + 1.5)     # (their merge)
+        best, cost = 0, 0.93 * cost             # (near the line the prompt kernel: the fit is good to a tenth)
         for parts in (1, 2, 4, 8):
             if parts > max(1, n_pages // 2):
                 break
-            of_block = _SHORT_BLOCK_US[head_dim][parts > 1]
-            c = max(fixed + (1.2 + 0.15 * parts if parts > 1 else 0.0) + page * -(-n_pages // parts),
-                    items * (parts * of_block + n_pages * busy))
+            c = _short_us(items, parts, n_pages, head_dim, tile)
             if c < cost:
                 best, cost = parts, c
         if len(_short_plans) >= 4096:
@@ -973,7 +999,8 @@ def short_message_plan(ctx, n_seqs: int, n_pages: int, n_kv_heads: int, group: i
     """How attention_short takes a prompt step: (blocks of a cluster, rows of a sequence and kv head in whole tiles), or () where it
     goes elsewhere.  (The rows, not the message's length: more tokens than a recording was made with need more tiles.)"""
     max_q = getattr(ctx, "short_message", 0)
-    parts = attention_short_parts(n_seqs, n_kv_heads, max_q, group, n_pages, head_dim, window) if max_q else 0
+    cut = _PREFILL_SPLIT and getattr(ctx, "host_q_lens", None) is not None
+    parts = attention_short_parts(n_seqs, n_kv_heads, max_q, group, n_pages, head_dim, window, cut) if max_q else 0
     rows = max_q * group
     return (parts, 16 if rows <= 16 else 32 if rows <= 32 else -(-rows // 64) * 64) if parts else ()
 
