@@ -714,7 +714,8 @@ LLMI_EXPORT int llmi_attention_prefill_tc(const void* q, long ldq, long n_tokens
                                           cudaStream_t stream) {
   if (n_seqs <= 0 || n_blocks <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0 || n_tokens <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads) return LLMI_ERR_BAD_SIZE;
-  if (!llmi_attention_prefill_tc_sizes(head_dim, v_dim) || maps < 1 || maps > 16 || n_heads > 0x7fff) return LLMI_ERR_UNSUPPORTED;
+  if (!llmi_attention_prefill_tc_sizes(head_dim, v_dim)) return LLMI_ERR_UNSUPPORTED;
+  if (maps < 1 || (long)n_heads * maps * v_dim > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;
   if ((maps > 1 || v_dim != head_dim) && (pool > 0 || gate || r1 || sink)) return LLMI_ERR_UNSUPPORTED;
   if (head_scale && (r1 || pool > 0 || scale <= 0.f)) return LLMI_ERR_UNSUPPORTED;
   if ((r1 == nullptr) != (r2 == nullptr) || (r1 && scale <= 0.f)) return LLMI_ERR_BAD_SIZE;

@@ -96,3 +96,21 @@ def test_a_factor_that_is_no_number_stays_one():
     a, b = out.view(n, H, d)[:, rest].double(), plain.view(n, H, d)[:, rest].double()
     assert float((a - b).norm() / b.norm()) < 1.2 * 2 ** -9 * 2 ** 0.5
     K.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("maps", [16, 17, 40])
+def test_any_number_of_maps(maps):
+    """More maps a head than anybody has: the general kernel's result."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels as K
+    dev, H, dk, dv, n = "cuda", 2, 64, 128, 100
+    torch.manual_seed(maps)
+    i32 = lambda x: torch.as_tensor(x).to(torch.int32).to(dev)      # noqa: E731
+    q, kc, vc = (torch.randn(s, device=dev).bfloat16() for s in ((n, H * maps * dk), (2, maps, 64, dk), (2, 1, 64, dv)))
+    ctx = types.SimpleNamespace(decode=False, seq_q_start=i32([0, n]), seq_kv_len=i32([n]), n_q_blocks=1, tok_seq=i32([0] * n), tok_pos=i32(range(n)),
+                                host_q_lens=[n], host_kv_lens=[n])
+    out, plain = (torch.empty(n, H * maps * dv, device=dev) for _ in range(2))
+    K.attention_maps(q, out, kc, vc, ctx, i32([[0, 1]]), 64, H, 1, maps, dk, dv, dk ** -0.5, rt=Runtime(torch.bfloat16, dev))
+    K.attention_flex(q, plain, kc, vc, ctx, i32([[0, 1]]), 64, H, 1, maps, dk, dv, dk ** -0.5)
+    assert float((out - plain).norm() / plain.norm()) < 1.2 * 2 ** -9 * 2 ** 0.5
+    K.check_device_errors("cuda:0")
