@@ -13,7 +13,7 @@
 // segments is the nearer one.)
 //
 // Three kernels:
-//  * linear_simt_kernel: any type, pitch and alignment (a tile of 64 x 64 outputs, scalar loads);
+//  * linear_simt_kernel: any type, pitch and alignment (a tile of 64 x 64 outputs, scalar loads), and fp32 rows of short k;
 //  * linear_f32_tile_kernel: fp32, 16-byte rows, many tokens: four segments of a 64 x 64 tile at a time;
 //  * linear_f32_rows_kernel: fp32, 16-byte rows, few tokens: bound by reading w once.
 #include "common.cuh"
@@ -380,6 +380,16 @@ int launch_linear_f32(const float* x, long ldx, const float* w, long ldw, const 
   return launch_status();
 }
 
+// fp32 rows of 16 bytes that linear_simt_kernel is the faster one for.  The tile kernel's four groups of threads take a segment each:
+// with k up to one segment three of them wait.  (us, tile / plain: 1,000 tokens x 4,096 rows of k = 64 53 / 27, 256 126 / 81, 320 131 /
+// 102, 512 about equal; x 320 rows of 64 9.3 / 6.7, of 256 19.7 / 16.5, of 320 equal; the rows kernel: 24 x 4,096 of 64 14.5 / 6.0, 40 x 1,024
+// of 128 11.2 / 9.2, 24 x 320 of 128 equal.)
+inline bool plain_is_faster(int M, int N, int K, int batch) {
+  if (M <= 8) return false;
+  if (K <= SEG) return !(M <= 24 && K >= 64 && (long)M * N * batch <= 16384);
+  return K <= 3 * SEG / 2 && M > ROWS_MAX_TOKENS && (long)((N + BN - 1) / BN) * ((M + BM - 1) / BM) * batch > sm_count();
+}
+
 template <typename T>
 int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const float* bias, const float* oscale, void* y, long ldy, int M,
                        int N, int K, int mode, int early, cudaStream_t stream, int batch = 1, long bx = 0, long bw = 0, long by = 0) {
@@ -387,8 +397,9 @@ int launch_linear_simt(const void* x, long ldx, const void* w, long ldw, const f
   if (grid.y > 65535 || batch < 1 || batch > 65535) return LLMI_ERR_BAD_SIZE;
   pairs_may_start_early = false;
   const bool rows_of_16 = (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && ((ldx | ldw | bx | bw | (long)K) & 3) == 0;
+  const bool plain = plain_is_faster(M, N, K, batch);
 #define LLMI_LAUNCH(MODE)                                                                                                     \
-  if (sizeof(T) == 4 && rows_of_16)                                                                                           \
+  if (sizeof(T) == 4 && rows_of_16 && !plain)                                                                                        \
     return launch_linear_f32<MODE>((const float*)x, ldx, (const float*)w, ldw, bias, oscale, (float*)y, ldy, M, N, K, early,  \
                                    stream, batch, bx, bw, by);                                                                        \
   linear_simt_kernel<T, MODE><<<grid, 256, 0, stream>>>((const T*)x, ldx, (const T*)w, ldw, bias, oscale, y, ldy, M, N, K, bx, bw, by)

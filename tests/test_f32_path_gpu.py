@@ -147,3 +147,29 @@ def test_a_matrix_that_the_launch_ahead_writes(M):
         k.linear_batched(x, 0, b, out, N // 2, K_)
         assert torch.equal(out, y)
     k.check_device_errors("cuda:0")
+
+
+def _us(f, reps=9, calls=20):
+    f()
+    times = []
+    for _ in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(calls):
+            f()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) * 1e3 / calls)
+    return min(times)
+
+
+@pytest.mark.parametrize("M,N,K_", [(1000, 4096, 64), (1000, 4096, 256), (3000, 1024, 128), (1000, 4096, 320), (24, 65536, 64)])
+def test_products_of_short_k_are_no_slower_than_the_kernel_for_any_rows(M, N, K_):
+    """fp32 rows of 16 bytes against rows that lie anywhere, which one kernel of the file takes (it took 0.4 to 0.8 times as long)."""
+    k = K()
+    y = torch.empty(M, N, device="cuda")
+
+    def call(odd):
+        x, w = (torch.randn(n * K_ + odd, device="cuda")[odd:].view(n, K_) for n in (M, N))
+        return _us(lambda: k.linear_simt(x, w, y))
+    assert call(0) < 1.15 * call(1)
