@@ -12,7 +12,8 @@
 // (attention_generic's one warp per query walks them one after another: 290 us a layer for four sequences of 30 to 400 positions
 // and 15 heads of 64, prompt and decode steps together; these kernels 91 us for the prompts and 21 us a decode step).
 //
-//  * attention_f32_decode_kernel: a block per (sequence, kv head), a warp per page, lanes over keys, then over entries;
+//  * attention_f32_decode_kernel: a block per (token, kv head, up to four of its heads), a warp per page, lanes over keys, then
+//    over entries;
 //  * attention_f32_prompt_kernel: a block per 32 queries and head, a page's 32 x 64 scores and its sums as register tiles.
 #include <math.h>
 
@@ -23,7 +24,7 @@
 namespace llmi {
 
 constexpr int F32_PAGE = 64;
-constexpr int F32_HEADS = 4;        // heads a warp of the decode kernel takes at a time
+constexpr int F32_HEADS = 4;        // most heads of a block of the decode kernel
 constexpr int F32_QUERIES = 32;     // queries of a block of the prompt kernel
 constexpr int F32_SMEM_LIMIT = 220 * 1024;
 
@@ -44,31 +45,34 @@ __device__ __forceinline__ float joined_sum(float state, float of_state, float p
   return __fmaf_rn(state, of_state, __fmul_rn(page, of_page));
 }
 
-__host__ __device__ constexpr int f32_decode_warps(int hd) { return hd <= 64 ? 8 : 4; }
-__host__ __device__ constexpr long f32_decode_floats(int hd, int group) {
-  const int warps = f32_decode_warps(hd);
-  return (long)group * hd                                  // q
+__host__ __device__ constexpr int f32_decode_warps(int hd) { return hd <= 64 ? 8 : 4; }      // at most
+__host__ __device__ constexpr long f32_decode_floats(int hd, int heads, int warps) {
+  return (long)heads * hd                                  // q
          + (long)warps * F32_PAGE * (hd + 4)               // keys of the warps' pages
-         + (long)warps * F32_HEADS * F32_PAGE              // p
-         + (long)warps * group * (hd + 2)                  // the pages' a, m, l
-         + (long)group * hd + 2 * group                    // A, M, L
-         + 2L * warps * group;                             // join factors
+         + (long)warps * heads * F32_PAGE                  // p
+         + (long)warps * heads * (hd + 2)                  // the pages' a, m, l
+         + (long)heads * hd + 2 * heads                    // A, M, L
+         + 2L * warps * heads;                             // join factors
 }
 
-// NJ: entries of a head per lane (ceil(head_dim / 32)).
-template <int NJ>
+// NJ: entries of a head per lane (ceil(head_dim / 32)).  HEADS: heads of a block (the last block of a kv head may have fewer): four
+// share the reads of a page's values; one or two where the device has SMs to spare, so that a warp's work on a page, which is all
+// that a short sequence has, is as long as that of so many heads.  As many warps as a sequence has pages: a block's shared
+// memory is theirs, so that several blocks of short sequences fit an SM.
+template <int NJ, int HEADS>
 __global__ void __launch_bounds__(256)
 attention_f32_decode_kernel(const float* __restrict__ q, long ldq, float* __restrict__ out, long ldo, const float* __restrict__ k_cache,
                             const float* __restrict__ v_cache, const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos,
-                            PagedKV kv, int group, float scale, int window) {
+                            PagedKV kv, int all_heads, float scale, int window) {
   extern __shared__ __align__(16) float f32_smem[];
   const int hd = kv.head_dim, pitch = hd + 4, n_warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x, t = blockIdx.y;
+  const int first = blockIdx.z * HEADS, group = min(HEADS, all_heads - first);      // this block's heads of the kv head's
   float* k_s = f32_smem + warp * F32_PAGE * pitch;
   float* q_s = f32_smem + n_warps * F32_PAGE * pitch;
-  float* p_s = q_s + group * hd + warp * F32_HEADS * F32_PAGE;
-  float* page_a = q_s + group * hd + n_warps * F32_HEADS * F32_PAGE;      // [warp][group][hd]
+  float* p_s = q_s + group * hd + warp * HEADS * F32_PAGE;
+  float* page_a = q_s + group * hd + n_warps * HEADS * F32_PAGE;          // [warp][group][hd]
   float* page_m = page_a + n_warps * group * hd;                          // [warp][group]
   float* page_l = page_m + n_warps * group;
   float* A = page_l + n_warps * group;                                    // [group][hd]
@@ -80,7 +84,7 @@ attention_f32_decode_kernel(const float* __restrict__ q, long ldq, float* __rest
   pdl_wait();
 
   const int seq = tok_seq[t];
-  float* o = out + (size_t)t * ldo + (size_t)kvh * group * hd;
+  float* o = out + (size_t)t * ldo + ((size_t)kvh * all_heads + first) * hd;
   if (seq < 0) {
     for (int i = threadIdx.x; i < group * hd; i += blockDim.x) o[i] = 0.f;
     return;
@@ -88,7 +92,7 @@ attention_f32_decode_kernel(const float* __restrict__ q, long ldq, float* __rest
   const int pos = tok_pos[t];
   const int lo = first_visible(pos, window, 0);
   const int first_page = lo / F32_PAGE, last_page = pos / F32_PAGE;
-  const float* qp = q + (size_t)t * ldq + (size_t)kvh * group * hd;
+  const float* qp = q + (size_t)t * ldq + ((size_t)kvh * all_heads + first) * hd;
   for (int i = threadIdx.x; i < group * hd; i += blockDim.x) {
     q_s[i] = qp[i];
     A[i] = 0.f;
@@ -114,66 +118,63 @@ attention_f32_decode_kernel(const float* __restrict__ q, long ldq, float* __rest
       asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
       __syncwarp();
       const bool in0 = lane >= k_lo && lane <= k_hi, in1 = lane + 32 >= k_lo && lane + 32 <= k_hi;
-      for (int h0 = 0; h0 < group; h0 += F32_HEADS) {
-        const int nh = min(F32_HEADS, group - h0);
-        for (int j = 0; j < nh; ++j) {
-          const float* qh = q_s + (h0 + j) * hd;
-          const float* k0 = k_s + lane * pitch;
-          const float* k1 = k0 + 32 * pitch;
-          float s0 = 0.f, s1 = 0.f;
+      for (int j = 0; j < group; ++j) {
+        const float* qh = q_s + j * hd;
+        const float* k0 = k_s + lane * pitch;
+        const float* k1 = k0 + 32 * pitch;
+        float s0 = 0.f, s1 = 0.f;
 #pragma unroll 4
-          for (int d = 0; d < hd; d += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(qh + d);
-            const float4 x = *reinterpret_cast<const float4*>(k0 + d);
-            const float4 y = *reinterpret_cast<const float4*>(k1 + d);
-            s0 = fmaf(a.x, x.x, s0);
-            s1 = fmaf(a.x, y.x, s1);
-            s0 = fmaf(a.y, x.y, s0);
-            s1 = fmaf(a.y, y.y, s1);
-            s0 = fmaf(a.z, x.z, s0);
-            s1 = fmaf(a.z, y.z, s1);
-            s0 = fmaf(a.w, x.w, s0);
-            s1 = fmaf(a.w, y.w, s1);
-          }
-          s0 = in0 ? __fmul_rn(s0, scale) : -INFINITY;      // (rows of the tile that no key is in are never used)
-          s1 = in1 ? __fmul_rn(s1, scale) : -INFINITY;
-          const float m = warp_max(fmaxf(s0, s1)), mb = page_base(m);
-          p_s[j * F32_PAGE + lane] = in0 ? expf(__fsub_rn(s0, mb)) : 0.f;
-          p_s[j * F32_PAGE + lane + 32] = in1 ? expf(__fsub_rn(s1, mb)) : 0.f;
-          if (lane == 0) page_m[warp * group + h0 + j] = m;
+        for (int d = 0; d < hd; d += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(qh + d);
+          const float4 x = *reinterpret_cast<const float4*>(k0 + d);
+          const float4 y = *reinterpret_cast<const float4*>(k1 + d);
+          s0 = fmaf(a.x, x.x, s0);
+          s1 = fmaf(a.x, y.x, s1);
+          s0 = fmaf(a.y, x.y, s0);
+          s1 = fmaf(a.y, y.y, s1);
+          s0 = fmaf(a.z, x.z, s0);
+          s1 = fmaf(a.z, y.z, s1);
+          s0 = fmaf(a.w, x.w, s0);
+          s1 = fmaf(a.w, y.w, s1);
         }
-        __syncwarp();
-        float acc[F32_HEADS][NJ], l[F32_HEADS];
-#pragma unroll
-        for (int j = 0; j < F32_HEADS; ++j) {
-          l[j] = 0.f;
-#pragma unroll
-          for (int e = 0; e < NJ; ++e) acc[j][e] = 0.f;
-        }
-        const int n_keys = k_hi + 1;
-#pragma unroll 8
-        for (int kk = k_lo; kk < n_keys; ++kk) {
-          float v[NJ];
-#pragma unroll
-          for (int e = 0; e < NJ; ++e) v[e] = lane + 32 * e < hd ? vp[kk * hd + lane + 32 * e] : 0.f;
-#pragma unroll
-          for (int j = 0; j < F32_HEADS; ++j) {
-            const float p = p_s[j * F32_PAGE + kk];           // (heads beyond the group: stale numbers that nobody reads on)
-            l[j] = __fadd_rn(l[j], p);
-#pragma unroll
-            for (int e = 0; e < NJ; ++e) acc[j][e] = fmaf(p, v[e], acc[j][e]);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < F32_HEADS; ++j) {
-          if (j >= nh) continue;
-          if (lane == 0) page_l[warp * group + h0 + j] = l[j];
-#pragma unroll
-          for (int e = 0; e < NJ; ++e)
-            if (lane + 32 * e < hd) page_a[(warp * group + h0 + j) * hd + lane + 32 * e] = acc[j][e];
-        }
-        __syncwarp();
+        s0 = in0 ? __fmul_rn(s0, scale) : -INFINITY;      // (rows of the tile that no key is in are never used)
+        s1 = in1 ? __fmul_rn(s1, scale) : -INFINITY;
+        const float m = warp_max(fmaxf(s0, s1)), mb = page_base(m);
+        p_s[j * F32_PAGE + lane] = in0 ? expf(__fsub_rn(s0, mb)) : 0.f;
+        p_s[j * F32_PAGE + lane + 32] = in1 ? expf(__fsub_rn(s1, mb)) : 0.f;
+        if (lane == 0) page_m[warp * group + j] = m;
       }
+      __syncwarp();
+      float acc[HEADS][NJ], l[HEADS];
+#pragma unroll
+      for (int j = 0; j < HEADS; ++j) {
+        l[j] = 0.f;
+#pragma unroll
+        for (int e = 0; e < NJ; ++e) acc[j][e] = 0.f;
+      }
+      const int n_keys = k_hi + 1;
+#pragma unroll 8
+      for (int kk = k_lo; kk < n_keys; ++kk) {
+        float v[NJ];
+#pragma unroll
+        for (int e = 0; e < NJ; ++e) v[e] = lane + 32 * e < hd ? vp[kk * hd + lane + 32 * e] : 0.f;
+#pragma unroll
+        for (int j = 0; j < HEADS; ++j) {
+          const float p = p_s[j * F32_PAGE + kk];           // (heads beyond the group: stale numbers that nobody reads on)
+          l[j] = __fadd_rn(l[j], p);
+#pragma unroll
+          for (int e = 0; e < NJ; ++e) acc[j][e] = fmaf(p, v[e], acc[j][e]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < HEADS; ++j) {
+        if (j >= group) continue;
+        if (lane == 0) page_l[warp * group + j] = l[j];
+#pragma unroll
+        for (int e = 0; e < NJ; ++e)
+          if (lane + 32 * e < hd) page_a[(warp * group + j) * hd + lane + 32 * e] = acc[j][e];
+      }
+      __syncwarp();
     }
     __syncthreads();
     const int here = min(n_warps, last_page - base + 1);
@@ -390,14 +391,20 @@ attention_f32_prompt_kernel(const float* __restrict__ q, long ldq, float* __rest
   }
 }
 
-// Head sizes in whole 16-byte pieces up to 128 and groups whose state fits shared memory; the generic kernel has the rest.
-inline bool attention_f32_takes(int hd, int group) {
-  return hd > 0 && hd <= 128 && hd % 4 == 0 && group > 0 && f32_decode_floats(hd, group) * 4 <= F32_SMEM_LIMIT;
-}
+// Head sizes in whole 16-byte pieces up to 128; the generic kernel has the rest.
+inline bool attention_f32_takes(int hd, int group) { return hd > 0 && hd <= 128 && hd % 4 == 0 && group > 0; }
+static_assert(f32_decode_floats(64, F32_HEADS, f32_decode_warps(64)) * 4 <= F32_SMEM_LIMIT && f32_decode_floats(128, F32_HEADS, f32_decode_warps(128)) * 4 <= F32_SMEM_LIMIT);
 
 template <typename K>
 int f32_configure(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32_SMEM_LIMIT) == cudaSuccess ? LLMI_OK : LLMI_ERR_LAUNCH;
+}
+
+template <int NJ>
+int f32_configure_decode() {
+  int rc = f32_configure(attention_f32_decode_kernel<NJ, 1>);
+  if (rc == LLMI_OK) rc = f32_configure(attention_f32_decode_kernel<NJ, 2>);
+  return rc == LLMI_OK ? f32_configure(attention_f32_decode_kernel<NJ, F32_HEADS>) : rc;
 }
 
 }  // namespace llmi
@@ -406,12 +413,13 @@ using namespace llmi;
 
 LLMI_EXPORT int llmi_attention_f32_supported(int head_dim, int group) { return attention_f32_takes(head_dim, group) ? 1 : 0; }
 
-// fp32 q [n_tokens, >= n_heads * head_dim] (row pitch ldq), out (row pitch ldo), caches of pages of 64.  `decode` 1: one token a
-// sequence (tok_seq -1: a row of zeros); 0: the tokens of the sequences one after another as seq_q_start says, no padding rows.
+// fp32 q [n_tokens, >= n_heads * head_dim] (row pitch ldq), out (row pitch ldo), caches of pages of 64.  `decode` 1: token by token
+// (tok_seq -1: a row of zeros), max_pages: most pages that a token sees (0: not known); 0: the tokens of the sequences one after
+// another as seq_q_start says, no padding rows.  Both may take a prompt.
 LLMI_EXPORT int llmi_attention_f32(const float* q, long ldq, float* out, long ldo, const float* k_cache, const float* v_cache,
                                    const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* seq_pages, int pages_stride, int page_size,
-                                   const int32_t* seq_q_start, int n_seqs, int n_tokens, int decode, int n_heads, int n_kv_heads,
-                                   int head_dim, float scale, int window, cudaStream_t stream) {
+                                   const int32_t* seq_q_start, int n_seqs, int n_tokens, int decode, int max_pages, int n_heads,
+                                   int n_kv_heads, int head_dim, float scale, int window, cudaStream_t stream) {
   if (n_tokens <= 0 || n_seqs <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return LLMI_ERR_BAD_SIZE;
   const int group = n_heads / n_kv_heads;
   if (page_size != F32_PAGE || !attention_f32_takes(head_dim, group)) return LLMI_ERR_UNSUPPORTED;
@@ -419,9 +427,9 @@ LLMI_EXPORT int llmi_attention_f32(const float* q, long ldq, float* out, long ld
   PagedKV kv{seq_pages, pages_stride, page_size, n_kv_heads, head_dim};
   static PerDevice<bool> configured;
   if (!configured.here()) {
-    int rc = f32_configure(attention_f32_decode_kernel<1>);
-    if (rc == LLMI_OK) rc = f32_configure(attention_f32_decode_kernel<2>);
-    if (rc == LLMI_OK) rc = f32_configure(attention_f32_decode_kernel<4>);
+    int rc = f32_configure_decode<1>();
+    if (rc == LLMI_OK) rc = f32_configure_decode<2>();
+    if (rc == LLMI_OK) rc = f32_configure_decode<4>();
     if (rc == LLMI_OK) rc = f32_configure(attention_f32_prompt_kernel<1>);
     if (rc == LLMI_OK) rc = f32_configure(attention_f32_prompt_kernel<2>);
     if (rc != LLMI_OK) return rc;
@@ -429,15 +437,22 @@ LLMI_EXPORT int llmi_attention_f32(const float* q, long ldq, float* out, long ld
   }
   if (decode) {
     if (n_tokens > 65535) return LLMI_ERR_BAD_SIZE;
-    const dim3 grid(n_kv_heads, n_tokens), block(32 * f32_decode_warps(head_dim));
-    const size_t smem = f32_decode_floats(head_dim, group) * sizeof(float);
-#define LLMI_LAUNCH(NJ)                                                                                                          \
-  launch_pdl(PDL_SMALL, attention_f32_decode_kernel<NJ>, grid, block, smem, stream, q, ldq, out, ldo, k_cache, v_cache, tok_seq, \
+    int heads = 1;
+    while (heads < F32_HEADS && heads < group && (long)n_tokens * n_kv_heads * ((group + heads - 1) / heads) > sm_count()) heads *= 2;
+    const int splits = (group + heads - 1) / heads, most = f32_decode_warps(head_dim);
+    if (splits > 65535) return LLMI_ERR_BAD_SIZE;
+    const int warps = max_pages > 0 && max_pages < most ? max_pages : most;
+    const dim3 grid(n_kv_heads, n_tokens, splits), block(32 * warps);
+    const size_t smem = f32_decode_floats(head_dim, heads, warps) * sizeof(float);
+#define LLMI_LAUNCH_HEADS(NJ, HEADS)                                                                                                    \
+  launch_pdl(PDL_SMALL, attention_f32_decode_kernel<NJ, HEADS>, grid, block, smem, stream, q, ldq, out, ldo, k_cache, v_cache, tok_seq, \
              tok_pos, kv, group, scale, window)
+#define LLMI_LAUNCH(NJ) (heads == 1 ? LLMI_LAUNCH_HEADS(NJ, 1) : heads == 2 ? LLMI_LAUNCH_HEADS(NJ, 2) : LLMI_LAUNCH_HEADS(NJ, F32_HEADS))
     if (head_dim <= 32) return LLMI_LAUNCH(1);
     if (head_dim <= 64) return LLMI_LAUNCH(2);
     return LLMI_LAUNCH(4);
 #undef LLMI_LAUNCH
+#undef LLMI_LAUNCH_HEADS
   }
   const long blocks = (long)(n_tokens / F32_QUERIES + n_seqs) * n_heads;      // at most so many blocks of 32 queries
   if (blocks > 0x7fffffffL) return LLMI_ERR_BAD_SIZE;

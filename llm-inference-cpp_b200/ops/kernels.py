@@ -548,8 +548,19 @@ def attention_f32(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq
     _check("attention_f32", lib().llmi_attention_f32(
         _ptr(q), c_long(q.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(ctx.tok_seq),
         _ptr(ctx.tok_pos), _ptr(seq_pages), c_int(seq_pages.stride(0)), c_int(k_cache.shape[-2]), _ptr(ctx.seq_q_start),
-        c_int(seq_pages.shape[0]), c_int(T), c_int(1 if ctx.decode else 0), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),
-        c_float(scale), c_int(window), _stream()))
+        c_int(seq_pages.shape[0]), c_int(T), c_int(1 if f32_by_token(ctx, T, seq_pages, n_heads, n_kv_heads, window) else 0), c_int(visible_pages(seq_pages.shape[1], window)),
+        c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), _stream()))
+
+
+def f32_by_token(ctx, n_tokens: int, seq_pages, n_heads: int, n_kv_heads: int, window: int) -> bool:
+    """Whether a step of the 32-bit path goes through its attention token by token: decode steps, and prompts of so few tokens a
+    sequence that blocks of 32 queries are all but empty.  (us, blocks of 32 / by token / a warp per query and head as the generic
+    kernel has it; 64 sequences of 2 tokens: 8 x 4 x 128 on 100 positions 189 / 105 / 107, on 1,500 under a window of 100 275 / 125 /
+    123, 1 x 16 x 128 149 / 54 / 84; of 4 tokens under that window 150 / 105 / 106, 8 x 4 x 128 276 / 229 / 223, but 32 x 1 x 64 97 / 137.)"""
+    if ctx.decode:
+        return True
+    blocks, pages, group = sum((n + 31) // 32 for n in ctx.host_q_lens), visible_pages(seq_pages.shape[1], window), n_heads // n_kv_heads
+    return n_tokens <= 65535 and pages >= 2 and (n_tokens <= 2 * blocks or (pages <= 3 and 10 * n_tokens * -(-group // 4) <= 14 * blocks * group))
 
 
 def attention_f32_applies(q: torch.Tensor, out: torch.Tensor, ctx, page_size: int, n_heads: int, n_kv_heads: int, head_dim: int) -> bool:

@@ -173,3 +173,59 @@ def test_products_of_short_k_are_no_slower_than_the_kernel_for_any_rows(M, N, K_
         x, w = (torch.randn(n * K_ + odd, device="cuda")[odd:].view(n, K_) for n in (M, N))
         return _us(lambda: k.linear_simt(x, w, y))
     assert call(0) < 1.15 * call(1)
+
+
+@pytest.mark.parametrize("nkv,group,hd,S,n,q,window", [(32, 1, 64, 64, 100, 1, 0), (1, 16, 128, 1, 40, 1, 0), (1, 8, 64, 1, 60, 1, 0), (8, 4, 128, 64, 100, 1, 0),
+                                                       (8, 4, 128, 64, 100, 2, 0), (1, 16, 128, 64, 1500, 4, 100), (8, 4, 128, 64, 1500, 2, 100)])
+def test_short_sequences_are_no_slower_than_on_the_generic_kernel(nkv, group, hd, S, n, q, window):
+    """Sequences of a page or two, and prompts of a few tokens each, against a warp per query and head (it took 0.3 to 0.8 times as
+    long); the same numbers."""
+    from llmi_b200.engine.runtime import Runtime
+    k = K()
+    torch.manual_seed(n)
+    ctx = _context([q] * S, [n] * S, q == 1)
+    P, nh = (n + 63) // 64, nkv * group
+    pages = torch.randperm(S * P).to(torch.int32).view(S, P).cuda()
+    kc, vc = (torch.randn(S * P, nkv, 64, hd, device="cuda") for _ in range(2))
+    x = torch.randn(S * q, nh * hd, device="cuda")
+    a, b = torch.empty_like(x), torch.empty_like(x)
+    rt = Runtime(torch.float32, "cuda:0")
+    new = _us(lambda: k.attention(x, a, kc, vc, ctx, pages, 64, nh, nkv, hd, hd ** -0.5, window, rt=rt))
+    old = _us(lambda: k.attention_generic(x, b, kc, vc, ctx.tok_seq, ctx.tok_pos, pages, 64, nh, nkv, hd, hd ** -0.5, window))
+    assert float((a - b).norm() / b.norm()) < 1e-6
+    assert new < 1.1 * old
+    k.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(30, 1, 16), (7, 1, 64), (5, 1, 128), (12, 2, 100), (40, 1, 64)])
+def test_attention_f32_many_heads_a_kv_head(nh, nkv, hd):
+    """Heads of a kv head cut over blocks, four, two and one at a time, with a remainder; fewer pages than warps; a prompt token by
+    token and by blocks of 32 queries: the same bits, and 64 bits' result."""
+    from llmi_b200.engine.runtime import Runtime
+    k = K()
+    torch.manual_seed(nh)
+    rt, scale = Runtime(torch.float32, "cuda:0"), hd ** -0.5
+    for S, n, q in ((1, 70, 1), (3, 300, 2), (60, 130, 2), (40, 10, 1)):
+        ctx = _context([q] * S, [n] * S, False)
+        P = (n + 63) // 64
+        pages = torch.randperm(S * P).to(torch.int32).view(S, P).cuda()
+        kc, vc = (torch.randn(S * P, nkv, 64, hd, device="cuda") for _ in range(2))
+        x = torch.randn(S * q, nh * hd, device="cuda")
+        outs = []
+        rule = k.f32_by_token
+        try:
+            for by_token in (True, False):
+                k.f32_by_token = lambda *a: by_token
+                outs.append(torch.full_like(x, 7.0))
+                k.attention(x, outs[-1], kc, vc, ctx, pages, 64, nh, nkv, hd, scale, rt=rt)
+        finally:
+            k.f32_by_token = rule
+        assert torch.equal(outs[0], outs[1])
+        s = 0
+        at = pages[s].long()
+        keys, vals = (c[at].transpose(1, 2).reshape(-1, nkv, hd)[:n].double().repeat_interleave(nh // nkv, 1) for c in (kc, vc))
+        sc = torch.einsum("qhd,khd->hqk", x[:q].double().view(q, nh, hd), keys) * scale
+        sc.masked_fill_(torch.arange(n, device="cuda")[None] > torch.arange(n - q, n, device="cuda")[:, None], -float("inf"))
+        ref = torch.einsum("hqk,khd->qhd", sc.softmax(-1), vals).reshape(q, -1)
+        assert float((outs[0][:q].double() - ref).norm() / ref.norm()) < 1e-6
+    k.check_device_errors("cuda:0")

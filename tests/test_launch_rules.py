@@ -62,3 +62,16 @@ def test_a_cut_prompt_is_weighed_as_one():
     """A step whose lengths are known lets the prompt kernel cut its key ranges: 8 x 8 x 64, one sequence of 4,000, 64 tokens, 24.9 us
     cut and 54.5 whole against 31.7 here."""
     assert K.attention_short_parts(1, 8, 64, 8, 64, 64) == 4 and K.attention_short_parts(1, 8, 64, 8, 64, 64, cut=True) == 0
+
+
+def test_prompts_of_a_few_tokens_in_32_bits():
+    """Token by token where blocks of 32 queries would be all but empty, by blocks otherwise; decode steps always by token."""
+    import torch
+
+    def by_token(q_lens, pages, kv, group, window=0, decode=False):
+        ctx = types.SimpleNamespace(decode=decode, host_q_lens=q_lens)
+        return K.f32_by_token(ctx, sum(q_lens), torch.zeros(len(q_lens), pages), kv * group, kv, window)
+    assert by_token([1] * 8, 1, 4, 1, decode=True)
+    assert by_token([2] * 64, 24, 8, 4) and by_token([2] * 64, 24, 32, 1, 100) and by_token([4] * 64, 24, 1, 16, 100)
+    assert not by_token([4] * 64, 24, 32, 1, 100) and not by_token([4] * 64, 24, 8, 4) and not by_token([30] * 8, 24, 1, 16, 100)
+    assert not by_token([300], 6, 3, 3) and not by_token([2], 1, 8, 4) and not by_token([2] * 40000, 2, 1, 1)
