@@ -374,9 +374,11 @@ delta_recurrence_quad_kernel(const float* __restrict__ prep, long ldp, DeltaDims
   // [k (D) | q (D) | v (CB) | g (D) | beta, 0, 0, 0]; all parts are whole 16-byte pieces
   constexpr int NG = CH ? D : 0;
   const int n16 = (2 * D + CB + NG) / 4, pitch = 2 * D + CB + NG + 4, pieces = n16 + (CH ? 1 : 2);
-  // My copies: piece (threadIdx.x + r blockDim.x) of a batch, counted over its tokens.  (CB = 16, D = 128, CH: 4 x 105 pieces
+  // My copies: piece (threadIdx.x + r blockDim.x) of a batch, counted over its tokens.  (CB = 16, D = 128, CH: 4 x 101 pieces
   // for 128 threads.)
   constexpr int COPIES = 4;
+  static_assert(REC_BATCH * ((2 * D + 16 + NG) / 4 + (CH ? 1 : 2)) <= COPIES * 128 && REC_BATCH * ((2 * D + 32 + NG) / 4 + (CH ? 1 : 2)) <= COPIES * 256,
+                "every piece of a batch is somebody's copy");
   const float* src[COPIES];
   int dst[COPIES], of_token[COPIES];
 #pragma unroll
@@ -504,11 +506,77 @@ delta_recurrence_quad_kernel(const float* __restrict__ prep, long ldp, DeltaDims
   }
 }
 
+// The same for one token a sequence (the same bits): bound by the state's way in and out, so no ring; every vector straight into
+// the registers, beside the state.  With the two kernels before it, 64 sequences, 32
+// heads of 64: 58.9 us in the form above, 46.5 so; 8 of 16 heads of 128 10.7, 9.3.
+template <int D, bool CH>
+__global__ void __launch_bounds__(256)
+delta_recurrence_one_kernel(const float* __restrict__ prep, long ldp, DeltaDims m, float* __restrict__ state,
+                            const int32_t* __restrict__ seq_q_start, const int32_t* __restrict__ seq_slot,
+                            float* __restrict__ o_raw, long ldo, int write_state) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x, seq = blockIdx.y, slot = seq_slot[seq], row = seq_q_start[seq];
+  if (slot < 0 || seq_q_start[seq + 1] <= row) return;
+  constexpr int NI = (D + 63) / 64;
+  const int CB = blockDim.x >> 3, cg = threadIdx.x >> 4, sub = threadIdx.x & 15, col0 = blockIdx.z * CB + 2 * cg, kh = h / (m.H / m.Hk);
+  const bool holds = 4 * sub < D;
+  float* S_g = state + (size_t)slot * m.state_floats() + (size_t)h * D * m.Dv + (size_t)col0 * D;
+  const float* in = prep + (size_t)row * ldp;
+  float2 S_r[2][NI][2];
+  rec_load_state<NI>(S_r, S_g, D, sub, holds);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 kk[NI], qq[NI], gg[NI];
+#pragma unroll
+  for (int c = 0; c < NI; ++c) {
+    qq[c] = holds ? *reinterpret_cast<const float4*>(in + (size_t)kh * D + 64 * c + 4 * sub) : zero;
+    kk[c] = holds ? *reinterpret_cast<const float4*>(in + (size_t)(m.Hk + kh) * D + 64 * c + 4 * sub) : zero;
+    gg[c] = CH && holds ? *reinterpret_cast<const float4*>(in + m.decay_at() + (size_t)h * D + 64 * c + 4 * sub) : zero;
+  }
+  const float2 v = *reinterpret_cast<const float2*>(in + m.n_qk() + (size_t)h * m.Dv + col0);
+  const float beta = in[m.beta_at() + h], g = CH ? 1.0f : in[m.decay_at() + h];
+  float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, o2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int c = 0; c < NI; ++c)
+#pragma unroll
+    for (int col = 0; col < 2; ++col) {
+      if (CH) {
+        S_r[col][c][0] = __fmul2_rn(S_r[col][c][0], make_float2(gg[c].x, gg[c].y));
+        S_r[col][c][1] = __fmul2_rn(S_r[col][c][1], make_float2(gg[c].z, gg[c].w));
+      }
+      acc[col] = __ffma2_rn(S_r[col][c][0], make_float2(kk[c].x, kk[c].y), acc[col]);
+      acc[col] = __ffma2_rn(S_r[col][c][1], make_float2(kk[c].z, kk[c].w), acc[col]);
+    }
+  float skx = pair_sum(acc[0]), sky = pair_sum(acc[1]), none = 0.f, none2 = 0.f;
+  join_four(skx, sky, 0.f, 0.f, sub);
+  const float2 u2[2] = {pair_of(beta * (v.x - (CH ? skx : g * skx))), pair_of(beta * (v.y - (CH ? sky : g * sky)))};
+  const float2 g2 = pair_of(g);
+#pragma unroll
+  for (int c = 0; c < NI; ++c) {
+    const float2 kp[2] = {make_float2(kk[c].x, kk[c].y), make_float2(kk[c].z, kk[c].w)};
+    const float2 qp[2] = {make_float2(qq[c].x, qq[c].y), make_float2(qq[c].z, qq[c].w)};
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int col = 0; col < 2; ++col) {
+        const float2 kept = CH ? S_r[col][c][e] : __fmul2_rn(g2, S_r[col][c][e]);
+        S_r[col][c][e] = __ffma2_rn(kp[e], u2[col], kept);
+        o2[col] = __ffma2_rn(S_r[col][c][e], qp[e], o2[col]);
+      }
+  }
+  if (write_state && holds) rec_store_state<NI>(S_r, S_g, D, sub);
+  const float o = join_four(none, none2, pair_sum(o2[0]), pair_sum(o2[1]), sub);
+  if ((sub & ~1) == 2) o_raw[(size_t)row * ldo + (size_t)h * m.Dv + col0 + (sub & 1)] = o;
+}
+
 template <int D, bool CH>
 int launch_delta_recurrence_quad(const float* prep, long ldp, DeltaDims m, float* state, const int32_t* seq_q_start,
-                                 const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state,
+                                 const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state, int one,
                                  cudaStream_t stream) {
   const int CB = m.Dv % 32 == 0 ? 32 : 16;                   // columns per block
+  if (one)
+    return launch_pdl(PDL_ATTENTION, delta_recurrence_one_kernel<D, CH>, dim3(m.H, n_seqs, m.Dv / CB), dim3(8 * CB), 0, stream, prep, ldp, m,
+                      state, seq_q_start, seq_slot, o_raw, ldo, write_state);
   size_t smem = (size_t)REC_STAGES * REC_BATCH * ((CH ? 3 : 2) * D + CB + 4) * sizeof(float);
   // Few blocks, each a chain over the tokens: two on one SM slow each other down while other SMs stand idle, and that is
   // where they land when they are launched while the kernels before still fill the device (measured, 2,048 tokens, 16 heads
@@ -652,15 +720,15 @@ LLMI_EXPORT int llmi_delta_conv_carry(const float* proj, long ld, int H, int Hk,
 
 LLMI_EXPORT int llmi_delta_recurrence(const float* prep, long ldp, int H, int Hk, int D, int Dv, int taps, float* state,
                                       const int32_t* seq_q_start, const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs,
-                                      int write_state, int channel, cudaStream_t stream) {
-  const DeltaDims m{H, Hk, D, Dv, taps, channel != 0};
+                                      int write_state, int channel, int one, cudaStream_t stream) {
+  const DeltaDims m{H, Hk, D, Dv, taps, channel != 0};      // (one: no sequence brings more than one token)
   if (n_seqs <= 0 || n_seqs > 65535 || !delta_dims_ok(m)) return LLMI_ERR_BAD_SIZE;
   // (16-byte accesses: state rows, o rows and the ring's v entries must be 16-byte aligned)
   if (Dv % 16 == 0 && ldo % 4 == 0 && ldp % 4 == 0 && !((uintptr_t)state & 15) && !((uintptr_t)o_raw & 15) &&
       !((uintptr_t)prep & 15) && DeltaDims{H, Hk, D, Dv, taps}.state_floats() % 4 == 0) {
 #define LLMI_QUAD(DD)                                                                                                                    \
-  return m.channel ? launch_delta_recurrence_quad<DD, true>(prep, ldp, m, state, seq_q_start, seq_slot, o_raw, ldo, n_seqs, write_state, stream) \
-                   : launch_delta_recurrence_quad<DD, false>(prep, ldp, m, state, seq_q_start, seq_slot, o_raw, ldo, n_seqs, write_state, stream)
+  return m.channel ? launch_delta_recurrence_quad<DD, true>(prep, ldp, m, state, seq_q_start, seq_slot, o_raw, ldo, n_seqs, write_state, one, stream) \
+                   : launch_delta_recurrence_quad<DD, false>(prep, ldp, m, state, seq_q_start, seq_slot, o_raw, ldo, n_seqs, write_state, one, stream)
     if (D == 32) LLMI_QUAD(32);
     if (D == 64) LLMI_QUAD(64);
     if (D == 128) LLMI_QUAD(128);

@@ -170,6 +170,7 @@ dplr_recurrence_quad_kernel(const float* __restrict__ proj, long ld, const float
   // My copies: piece (threadIdx.x + r blockDim.x) of a batch, counted over its tokens.  (CB = 16, D = 128: 4 x 164 pieces for
   // 128 threads.)
   constexpr int COPIES = 6;
+  static_assert(REC_BATCH * (5 * Q + 4) <= COPIES * 128 && REC_BATCH * (5 * Q + 8) <= COPIES * 256, "every piece of a batch is somebody's copy");
   const float* src[COPIES];
   int dst[COPIES], of_token[COPIES];
 #pragma unroll
@@ -280,11 +281,73 @@ dplr_recurrence_quad_kernel(const float* __restrict__ proj, long ld, const float
   }
 }
 
+// The same for one token a sequence (the same bits): bound by the state's way in and out, so no ring; every vector straight into
+// the registers, beside the state.  64 sequences, 32 heads of 64: 35.1 us in the form above, 14.8 so; 8 of 16
+// heads of 128 7.0, 4.8.
+template <int D>
+__global__ void __launch_bounds__(256)
+dplr_recurrence_one_kernel(const float* __restrict__ proj, long ld, const float* __restrict__ prep, long ldp, int H, int Dv,
+                           float* __restrict__ state, long state_stride, const int32_t* __restrict__ seq_q_start,
+                           const int32_t* __restrict__ seq_slot, float* __restrict__ o_raw, long ldo, int write_state) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x, seq = blockIdx.y, slot = seq_slot[seq], row = seq_q_start[seq];
+  if (slot < 0 || seq_q_start[seq + 1] <= row) return;
+  constexpr int NI = (D + 63) / 64;
+  const int CB = blockDim.x >> 3, cg = threadIdx.x >> 4, sub = threadIdx.x & 15, col0 = blockIdx.z * CB + 2 * cg, HD = H * D;
+  const bool holds = 4 * sub < D;
+  float* S_g = state + (size_t)slot * state_stride + (size_t)h * D * Dv + (size_t)col0 * D;
+  const float* prow = prep + (size_t)row * ldp + (size_t)h * D + 4 * sub;
+  const float* xrow = proj + (size_t)row * ld;
+  float2 S_r[2][NI][2];
+  rec_load_state<NI>(S_r, S_g, D, sub, holds);
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 ww[NI], pp[NI], mm[NI], kk[NI], rr[NI];
+#pragma unroll
+  for (int c = 0; c < NI; ++c) {
+    ww[c] = holds ? *reinterpret_cast<const float4*>(prow + 64 * c) : zero;
+    pp[c] = holds ? *reinterpret_cast<const float4*>(prow + HD + 64 * c) : zero;
+    mm[c] = holds ? *reinterpret_cast<const float4*>(prow + 2 * (size_t)HD + 64 * c) : zero;
+    rr[c] = holds ? *reinterpret_cast<const float4*>(xrow + (size_t)h * D + 4 * sub + 64 * c) : zero;
+    kk[c] = holds ? *reinterpret_cast<const float4*>(xrow + HD + (size_t)h * D + 4 * sub + 64 * c) : zero;
+  }
+  const float2 v = *reinterpret_cast<const float2*>(xrow + 2 * (size_t)HD + (size_t)h * Dv + col0);
+  float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, o2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+  for (int c = 0; c < NI; ++c)
+#pragma unroll
+    for (int col = 0; col < 2; ++col) {
+      acc[col] = __ffma2_rn(S_r[col][c][0], make_float2(pp[c].x, pp[c].y), acc[col]);
+      acc[col] = __ffma2_rn(S_r[col][c][1], make_float2(pp[c].z, pp[c].w), acc[col]);
+    }
+  float dx = pair_sum(acc[0]), dy = pair_sum(acc[1]), none = 0.f, none2 = 0.f;
+  join_four(dx, dy, 0.f, 0.f, sub);
+  const float2 d2[2] = {pair_of(dx), pair_of(dy)}, v2[2] = {pair_of(v.x), pair_of(v.y)};
+#pragma unroll
+  for (int c = 0; c < NI; ++c) {
+    const float2 wp[2] = {make_float2(ww[c].x, ww[c].y), make_float2(ww[c].z, ww[c].w)}, mp[2] = {make_float2(mm[c].x, mm[c].y), make_float2(mm[c].z, mm[c].w)};
+    const float2 kp[2] = {make_float2(kk[c].x, kk[c].y), make_float2(kk[c].z, kk[c].w)}, rp[2] = {make_float2(rr[c].x, rr[c].y), make_float2(rr[c].z, rr[c].w)};
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int col = 0; col < 2; ++col) {
+        S_r[col][c][e] = __ffma2_rn(kp[e], v2[col], __ffma2_rn(mp[e], d2[col], __fmul2_rn(wp[e], S_r[col][c][e])));
+        o2[col] = __ffma2_rn(S_r[col][c][e], rp[e], o2[col]);
+      }
+  }
+  if (write_state && holds) rec_store_state<NI>(S_r, S_g, D, sub);
+  const float o = join_four(none, none2, pair_sum(o2[0]), pair_sum(o2[1]), sub);
+  if ((sub & ~1) == 2) o_raw[(size_t)row * ldo + (size_t)h * Dv + col0 + (sub & 1)] = o;
+}
+
 template <int D>
 int launch_dplr_quad(const float* proj, long ld, const float* prep, long ldp, int H, int Dv, float* state, long state_stride,
-                     const int32_t* seq_q_start, const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state,
+                     const int32_t* seq_q_start, const int32_t* seq_slot, float* o_raw, long ldo, int n_seqs, int write_state, int one,
                      cudaStream_t stream) {
   const int CB = Dv % 32 == 0 ? 32 : 16;                     // columns per block
+  if (one)
+    return launch_pdl(PDL_ATTENTION, dplr_recurrence_one_kernel<D>, dim3(H, n_seqs, Dv / CB), dim3(8 * CB), 0, stream, proj, ld, prep, ldp, H,
+                      Dv, state, state_stride, seq_q_start, seq_slot, o_raw, ldo, write_state);
   const size_t smem = (size_t)REC_STAGES * REC_BATCH * (5 * D + CB) * sizeof(float);       // (at most 32 KB)
   return launch_pdl(PDL_ATTENTION, dplr_recurrence_quad_kernel<D>, dim3(H, n_seqs, Dv / CB), dim3(8 * CB), smem, stream, proj, ld,
                     prep, ldp, H, Dv, state, state_stride, seq_q_start, seq_slot, o_raw, ldo, write_state);
@@ -318,17 +381,17 @@ LLMI_EXPORT int llmi_tanh_rows(int dtype, const float* src, long ld, void* dst, 
 }
 
 // proj fp32 [T, ld]: r at column 0, k at H*D, v at 2*H*D; prep fp32 [T, ldp]: w at 0, p at H*D, m at 2*H*D;
-// state fp32 [slots, state_stride >= H*D*Dv]; o_raw fp32 [T, ldo] receives Sᵀ r.
+// state fp32 [slots, state_stride >= H*D*Dv]; o_raw fp32 [T, ldo] receives Sᵀ r.  one: no sequence brings more than one token.
 LLMI_EXPORT int llmi_dplr_recurrence(const float* proj, long ld, const float* prep, long ldp, int H, int D, int Dv, float* state,
                                      long state_stride, const int32_t* seq_q_start, const int32_t* seq_slot, float* o_raw,
-                                     long ldo, int n_seqs, int write_state, cudaStream_t stream) {
+                                     long ldo, int n_seqs, int write_state, int one, cudaStream_t stream) {
   if (n_seqs <= 0 || n_seqs > 65535 || H <= 0 || D <= 0 || Dv <= 0 || Dv > 1024) return LLMI_ERR_BAD_SIZE;
   if (Dv % 16 == 0 && ld % 4 == 0 && ldp % 4 == 0 && ldo % 4 == 0 && state_stride % 4 == 0 && !((uintptr_t)state & 15) &&
       !((uintptr_t)o_raw & 15) && !((uintptr_t)prep & 15) && !((uintptr_t)proj & 15)) {
 #define LLMI_QUAD(DD)                                                                                                      \
   if (D == DD)                                                                                                             \
     return launch_dplr_quad<DD>(proj, ld, prep, ldp, H, Dv, state, state_stride, seq_q_start, seq_slot, o_raw, ldo, n_seqs, \
-                                write_state, stream)
+                                write_state, one, stream)
     LLMI_QUAD(32);
     LLMI_QUAD(64);
     LLMI_QUAD(128);

@@ -39,4 +39,25 @@ __device__ __forceinline__ void rec_copy4(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
+// Four entries (64 i + 4 sub ..) of two neighbouring columns, [column][chunk][pair of entries], from or to rows of D entries a column.
+template <int NI>
+__device__ __forceinline__ void rec_load_state(float2 (&S)[2][NI][2], const float* S_g, int D, int sub, bool holds) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const float4 v = holds ? *reinterpret_cast<const float4*>(S_g + c * D + 64 * i + 4 * sub) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[c][i][0] = make_float2(v.x, v.y);
+      S[c][i][1] = make_float2(v.z, v.w);
+    }
+}
+template <int NI>
+__device__ __forceinline__ void rec_store_state(const float2 (&S)[2][NI][2], float* S_g, int D, int sub) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      *reinterpret_cast<float4*>(S_g + c * D + 64 * i + 4 * sub) = make_float4(S[c][i][0].x, S[c][i][0].y, S[c][i][1].x, S[c][i][1].y);
+}
+
 }  // namespace llmi

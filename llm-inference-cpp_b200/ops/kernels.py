@@ -1718,7 +1718,8 @@ def delta_step(proj: torch.Tensor, dims, conv_w, a_log, dt_bias, state: torch.Te
                                                            _ptr(ctx.seq_kv_len), _ptr(ctx.seq_slot), c_int(ctx.n_seqs), _stream()))
     _check("delta_recurrence", l.llmi_delta_recurrence(_ptr(prep), c_long(prep.stride(0)), *d, _ptr(state), _ptr(ctx.seq_q_start),
                                                        _ptr(ctx.seq_slot), _ptr(o_raw), c_long(o_raw.stride(0)), c_int(ctx.n_seqs),
-                                                       c_int(1 if write_state else 0), c_int(1 if z is not None else 0), _stream()))
+                                                       c_int(1 if write_state else 0), c_int(1 if z is not None else 0),
+                                                       c_int(1 if getattr(ctx, "decode", False) else 0), _stream()))
 
 
 GATE_SILU, GATE_SIGMOID = 0, 1
@@ -1834,7 +1835,7 @@ def dplr_recurrence(proj: torch.Tensor, prep: torch.Tensor, H: int, D: int, Dv: 
     _check("dplr_recurrence", lib().llmi_dplr_recurrence(
         _ptr(proj), c_long(proj.stride(0)), _ptr(prep), c_long(prep.stride(0)), c_int(H), c_int(D), c_int(Dv), _ptr(state),
         c_long(state.stride(0)), _ptr(ctx.seq_q_start), _ptr(ctx.seq_slot), _ptr(o_raw), c_long(o_raw.stride(0)),
-        c_int(ctx.n_seqs), c_int(1 if write_state else 0), _stream()))
+        c_int(ctx.n_seqs), c_int(1 if write_state else 0), c_int(1 if getattr(ctx, "decode", False) else 0), _stream()))
 
 
 # ---------------------------------------------------------------------------------------------
