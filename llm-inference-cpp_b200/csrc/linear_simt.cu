@@ -128,8 +128,8 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
 // Many tokens.  Bound by the FMA pipes (128 a clock and SM; 74 TFLOP/s, of which 8 x 8 products out of registers alone reach
 // 55).  800 tokens x 960 -> 5,120: 252 us, 31 TFLOP/s: a block takes 30 us for its 4 segments and the last of 7.03 waves is
 // nearly empty.  (Two blocks of half the stages on an SM: 282 us.)  A block makes a tile of 64 x 64 outputs; its four groups of 64
-// threads take segments 4r, 4r + 1, .. of round r, each thread 8 x 8 outputs in registers (two 16-byte shared loads per 16
-// FMAs where 4 x 4 outputs need four).  With the segments side by side a block keeps four warps' worth of independent chains
+// threads take segments 4r, 4r + 1, .. of round r, each thread 8 x 8 outputs in registers (one 16-byte shared load per 16
+// FMAs where 4 x 4 outputs need two).  With the segments side by side a block keeps two warps of independent chains
 // on every scheduler though its tile is small, and small tiles fill the 148 SMs at the widths of small models (600 tokens x
 // 960 outputs are 150 tiles).  Operands go to shared memory as they lie (rows of 16 k places, 20 floats apart: a quarter
 // warp's 16-byte loads touch 32 different banks) by cp.async, three stages a group.
