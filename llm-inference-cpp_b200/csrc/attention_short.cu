@@ -530,8 +530,6 @@ static int sh_launch_rows(const CUtensorMap& mk, const CUtensorMap& mv, const Sh
 
 using namespace llmi;
 
-LLMI_EXPORT int llmi_attention_short_supported(int head_dim) { return head_dim == 64 || head_dim == 128; }
-
 // q: [tokens, >= n_heads * head_dim] rotated queries, the cache complete; otherwise as llmi_attention_prefill.  max_q: the most
 // tokens a sequence brings; parts: blocks that share a (sequence, kv head, row tile): 1, 2, 4 or 8.
 // fuse = 1 (max_q 1, groups up to 16): a decode step as for llmi_attention_decode_fused — `q` is the step's un-rotated
@@ -544,7 +542,7 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
                                      int write_kv, int wide, int* error_flag, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return LLMI_ERR_BAD_SIZE;
-  if (!llmi_attention_short_supported(head_dim)) return LLMI_ERR_UNSUPPORTED;
+  if (head_dim != 64 && head_dim != 128) return LLMI_ERR_UNSUPPORTED;
   if (((uintptr_t)q & 3) || (ldq & 1) || ((uintptr_t)out & 3) || (ldo & 1) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return LLMI_ERR_ALIGN;
   const int group = n_heads / n_kv_heads;
   if (fuse && (max_q != 1 || group > 16 || (rotary_dim != 0 && (rotary_dim != head_dim || !inv_freq)))) return LLMI_ERR_UNSUPPORTED;

@@ -157,7 +157,6 @@ def lib():
                      "llmi_attention_prefill", "llmi_attention_prefill_supported", "llmi_gemm_skinny",
                      "llmi_gemm_skinny_max_tokens", "llmi_attention_prefill_tc", "llmi_attention_prefill_tc_supported",
                      "llmi_attention_prefill_tc_sizes", "llmi_attention_short",
-                     "llmi_attention_short_supported",
                      "llmi_sm_count", "llmi_dyt", "llmi_dyt_add", "llmi_stream_add", "llmi_linear_simt_batched",
                      "llmi_attention_expanded",
                      "llmi_attention_expanded_supported", "llmi_latent_expand_prepare", "llmi_latent_prepare", "llmi_latent_q_rotate", "llmi_attention_latent", "llmi_delta_prepare",

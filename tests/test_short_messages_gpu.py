@@ -60,8 +60,9 @@ def test_attention_short(hd, group, window):
 @pytest.mark.parametrize("hd,group", [(64, 1), (64, 3), (128, 4), (128, 16)])
 @pytest.mark.parametrize("window,rot,write", [(0, True, True), (200, True, True), (0, False, True), (0, True, False)])
 def test_attention_short_decode_same_bits(hd, group, window, rot, write):
-    """A decode step with the position encoding inside gives, however the pages are shared, the bits and the cache of the
-    kernels it replaces: lengths at the edges of pages, a padding sequence, positions of nobody NaN."""
+    """A decode step with the position encoding inside gives, however the pages are shared, the bits of the same kernel behind the
+    kernel that rotates and appends, and that kernel's cache: lengths at the edges of pages, a padding sequence, positions of
+    nobody NaN.  (Against 64 bits: test_attention_short_small_tiles.)"""
     k = K()
     nkv = 2
     nh, dev = nkv * group, "cuda"
@@ -199,3 +200,48 @@ def test_recorded_messages_of_one_padded_shape(tmp_path, heads, kv_heads, head_d
     assert len(set(g.graphs) - had) == len(plans) and g.replays - before == len(messages) - 2 * len(plans)
     assert len(plans) == (1 if head_dim == 32 or heads == kv_heads else 2)
     kernels.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("group,max_q", [(1, 1), (4, 1), (16, 1), (1, 16), (3, 5), (5, 3), (1, 17), (3, 9), (8, 4), (16, 2), (2, 16)])
+@pytest.mark.parametrize("window", [0, 70])
+def test_attention_short_small_tiles(hd, group, max_q, window):
+    """The tiles of 16 and of 32 rows, whose warps share a page's keys: messages of up to so many tokens (decode steps among them,
+    and the form with 32-bit weights) on histories that end at the edges of pages and of the warps' keys, every way to share
+    the pages, against 64 bits; positions that no query sees are NaN."""
+    k = K()
+    torch.manual_seed(hd + group + max_q + window)
+    nkv, dev = 2, "cuda"
+    nh = nkv * group
+    q_lens = [max_q, 1, max(1, max_q // 2), max_q, max_q, 1, max_q, max_q]
+    held = [0, 15, 16, 31, 63, 64, 700, 1000]
+    S, kv_lens = len(q_lens), [h + q for h, q in zip(held, q_lens)]
+    pages_of = [(n + 63) // 64 for n in kv_lens]
+    table = torch.full((S, max(pages_of) + 1), -1, dtype=torch.int32)
+    order, at = torch.randperm(sum(pages_of)), 0
+    kc = torch.full((sum(pages_of), nkv, 64, hd), float("nan"), device=dev, dtype=torch.bfloat16)
+    vc = kc.clone()
+    starts = np.concatenate([[0], np.cumsum(q_lens)])
+    T, scale = int(starts[-1]), hd ** -0.5
+    q = torch.randn(T, nh * hd, device=dev, dtype=torch.bfloat16)
+    refs = []
+    for i, (ql, kl) in enumerate(zip(q_lens, kv_lens)):
+        keys, vals = (torch.randn(kl, nkv, hd, device=dev).to(torch.bfloat16) for _ in range(2))
+        for p in range(pages_of[i]):
+            table[i, p] = order[at]
+            n = min(64, kl - 64 * p)
+            kc[order[at], :, :n], vc[order[at], :, :n] = keys[64 * p:64 * p + n].transpose(0, 1), vals[64 * p:64 * p + n].transpose(0, 1)
+            at += 1
+        s = torch.einsum("qhd,khd->hqk", q[starts[i]:starts[i + 1]].double().view(ql, nh, hd), keys.double().repeat_interleave(group, 1)) * scale
+        qp, kp = torch.arange(kl - ql, kl, device=dev)[:, None], torch.arange(kl, device=dev)[None]
+        s.masked_fill_((kp > qp) | ((kp <= qp - window) if window else torch.zeros_like(kp > qp)), -float("inf"))
+        refs.append(torch.einsum("hqk,khd->qhd", s.softmax(-1), vals.double().repeat_interleave(group, 1)).reshape(ql, -1))
+    ref = torch.cat(refs)
+    i32 = lambda x: torch.as_tensor(x).to(torch.int32).to(dev)      # noqa: E731
+    for parts in (1, 2, 4, 8):
+        for wide in (False, True) if max_q == 1 and group == 1 and hd == 128 else (False,):
+            out = torch.full((T, nh * hd), 7.0, device=dev, dtype=torch.bfloat16)
+            k.attention_short(q, out, kc, vc, table.to(dev), i32(starts), i32(kv_lens), max_q, nh, nkv, hd, scale, window, parts, wide=wide)
+            # row by row, so that no single row's mistake is lost in the others: weights and output in bf16, 2^-8 at most each
+            assert bool(((out.double() - ref).norm(dim=1) < 2 ** -8 * 2 ** 0.5 * ref.norm(dim=1)).all()), (parts, wide)
+    k.check_device_errors("cuda:0")
