@@ -179,12 +179,11 @@ moe_identity_add_kernel(const T* __restrict__ h, long ldh, const float* __restri
 
 template <int ACT> __device__ __forceinline__ float moe_act(float g) { return expert_act(g, ACT); }
 
-// A warp's dot product of a shared-memory fp32 vector with one weight row, 16 bytes per lane and load.
+// A warp's dot products of a shared-memory fp32 vector with weight rows, 16 bytes per lane and load.
 template <typename T> struct Vec16;
 template <> struct Vec16<__nv_bfloat16> {
   static constexpr int N = 8;
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[8]) {
-    const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  static __device__ __forceinline__ void expand(const uint4& raw, float (&v)[8]) {
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
     for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
@@ -192,23 +191,63 @@ template <> struct Vec16<__nv_bfloat16> {
 };
 template <> struct Vec16<float> {
   static constexpr int N = 4;
-  static __device__ __forceinline__ void load(const float* p, float (&v)[4]) {
-    const float4 f = *reinterpret_cast<const float4*>(p);
-    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+  static __device__ __forceinline__ void expand(const uint4& raw, float (&v)[4]) {
+    v[0] = __uint_as_float(raw.x); v[1] = __uint_as_float(raw.y); v[2] = __uint_as_float(raw.z); v[3] = __uint_as_float(raw.w);
   }
 };
 
-// VEC: rows are 16-byte aligned and a multiple of 16 bytes long.  The order of a row's additions is fixed by (K, VEC).
+// Where entry i of the vector lies in shared memory.  A lane reads N neighbouring entries, 16 bytes at a time; for bf16 rows
+// (N = 8) the fours with even numbers lie in the first half of the buffer and the odd ones in the second, so that the 32 lanes
+// of one read touch 512 neighbouring bytes (in their own order two lanes in eight meet in every bank).
 template <typename T, bool VEC>
-__device__ __forceinline__ float warp_dot(const float* __restrict__ x_s, const T* __restrict__ row, int K, int lane) {
+__device__ __forceinline__ int moe_place(int i, int K) {
+  if (!VEC || Vec16<T>::N == 4) return i;
+  return (i & 4) * (K >> 3) + ((i >> 3) << 2) + (i & 3);
+}
+
+constexpr int MOE_AHEAD = 8;             // loads a lane has in flight: 4 KB of a row per warp
+// Pieces i0, i0 + 32 N, ... of a row; a lane past the row's end reads nothing.
+template <typename T>
+__device__ __forceinline__ void moe_load_row(const T* __restrict__ row, int i0, int K, uint4 (&raw)[MOE_AHEAD]) {
+  constexpr int STEP = 32 * Vec16<T>::N;
+#pragma unroll
+  for (int u = 0; u < MOE_AHEAD; ++u)
+    if (i0 + u * STEP < K) raw[u] = __ldg(reinterpret_cast<const uint4*>(row + i0 + u * STEP));
+}
+template <typename T>
+__device__ __forceinline__ void moe_add_row(const float* __restrict__ x_s, int i0, int K, const uint4 (&raw)[MOE_AHEAD], float& acc) {
+  constexpr int N = Vec16<T>::N, STEP = 32 * N;
+#pragma unroll
+  for (int u = 0; u < MOE_AHEAD; ++u) {
+    const int i = i0 + u * STEP;
+    if (i < K) {
+      float v[N];
+      Vec16<T>::expand(raw[u], v);
+#pragma unroll
+      for (int q = 0; q < N; q += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(x_s + moe_place<T, true>(i + q, K));
+        acc = fmaf(x.x, v[q], acc);
+        acc = fmaf(x.y, v[q + 1], acc);
+        acc = fmaf(x.z, v[q + 2], acc);
+        acc = fmaf(x.w, v[q + 3], acc);
+      }
+    }
+  }
+}
+
+// VEC: rows are 16-byte aligned and a multiple of 16 bytes long.  The order of a row's additions is fixed by (K, VEC).  What
+// bounds these kernels is the latency of the rows' loads: a lane asks for MOE_AHEAD pieces before it uses the first.
+// `raw` holds the row's first pieces already where `loaded` says so.
+template <typename T, bool VEC>
+__device__ __forceinline__ float warp_dot(const float* __restrict__ x_s, const T* __restrict__ row, int K, int lane,
+                                          uint4 (&raw)[MOE_AHEAD], bool loaded) {
   float acc = 0.f;
   if (VEC) {
     constexpr int N = Vec16<T>::N;
-    for (int i = lane * N; i < K; i += 32 * N) {
-      float v[N];
-      Vec16<T>::load(row + i, v);
-#pragma unroll
-      for (int e = 0; e < N; ++e) acc = fmaf(x_s[i + e], v[e], acc);
+    for (int i = lane * N; i < K; i += 32 * N * MOE_AHEAD) {
+      if (!loaded) moe_load_row(row, i, K, raw);
+      loaded = false;
+      moe_add_row<T>(x_s, i, K, raw, acc);
     }
   } else {
     for (int i = lane; i < K; i += 32) acc = fmaf(x_s[i], to_f32(row[i]), acc);
@@ -221,45 +260,72 @@ template <typename T, int ACT, bool VEC>
 __global__ void __launch_bounds__(256)
 moe_up_kernel(const T* __restrict__ h, long ldh, const T* __restrict__ wg, const T* __restrict__ wu, int W, int F, int top,
               const int32_t* __restrict__ idx, float* __restrict__ a) {
-  extern __shared__ float h_s[];
-  pdl_launch_dependents();
+  extern __shared__ __align__(16) float h_s[];
   pdl_wait();
+  // Only behind the wait: moe_down, which may start from here on, then knows that the experts have been chosen.
+  pdl_launch_dependents();
   const int item = blockIdx.x, t = item / top;
   const int e = idx[item];
   if (e < 0) return;
-  for (int i = threadIdx.x; i < W; i += blockDim.x) h_s[i] = to_f32(h[(size_t)t * ldh + i]);
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f = blockIdx.y * 8 + warp;
+  const T* row_u = wu + ((size_t)e * F + f) * W;
+  const T* row_g = wg ? wg + ((size_t)e * F + f) * W : nullptr;
+  uint4 raw_u[MOE_AHEAD], raw_g[MOE_AHEAD];
+  if (VEC && f < F) {
+    moe_load_row(row_u, lane * Vec16<T>::N, W, raw_u);
+    if (row_g) moe_load_row(row_g, lane * Vec16<T>::N, W, raw_g);
+  }
+  for (int i = threadIdx.x; i < W; i += blockDim.x) h_s[moe_place<T, VEC>(i, W)] = to_f32(h[(size_t)t * ldh + i]);
+  __syncthreads();
   if (f >= F) return;
-  const float u = warp_dot<T, VEC>(h_s, wu + ((size_t)e * F + f) * W, W, lane);
+  const float u = warp_dot<T, VEC>(h_s, row_u, W, lane, raw_u, true);
   if (wg == nullptr) {
     if (lane == 0) a[(size_t)item * F + f] = moe_act<ACT>(u);
     return;
   }
-  const float g = warp_dot<T, VEC>(h_s, wg + ((size_t)e * F + f) * W, W, lane);
+  const float g = warp_dot<T, VEC>(h_s, row_g, W, lane, raw_g, true);
   if (lane == 0) a[(size_t)item * F + f] = moe_act<ACT>(g) * u;
 }
 
-// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.
+// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.  `behind_up`: the launch before on the stream is
+// moe_up_kernel with the same idx, whose blocks let this kernel start when the choice and everything before it is done: the
+// first choice's row is then asked for ahead of the wait, and the others' come into L2.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, int F, int top, const int32_t* __restrict__ idx,
-                const float* __restrict__ wt, float* __restrict__ y, long ldy, int add) {
-  extern __shared__ float a_s[];
+                const float* __restrict__ wt, float* __restrict__ y, long ldy, int add, int behind_up) {
+  extern __shared__ __align__(16) float a_s[];
   pdl_launch_dependents();
-  pdl_wait();
   const int t = blockIdx.x;
-  for (int i = threadIdx.x; i < top * F; i += blockDim.x) a_s[i] = a[(size_t)t * top * F + i];
-  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.y * 8 + warp;
+  uint4 raw[MOE_AHEAD];
+  bool loaded = false;
+  if (VEC && behind_up && c < W) {
+    for (int j = 0; j < top; ++j) {
+      const int e = idx[(size_t)t * top + j];
+      if (e < 0) continue;
+      const T* row = wd + ((size_t)e * W + c) * F;
+      if (j == 0) {
+        moe_load_row(row, lane * Vec16<T>::N, F, raw);
+        loaded = true;
+      } else {
+        for (int i = lane * (128 / (int)sizeof(T)); i < F; i += 32 * (128 / (int)sizeof(T)))
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(row + i));
+      }
+    }
+  }
+  pdl_wait();
+  for (int j = 0; j < top; ++j)
+    for (int i = threadIdx.x; i < F; i += blockDim.x) a_s[j * F + moe_place<T, VEC>(i, F)] = a[((size_t)t * top + j) * F + i];
+  __syncthreads();
   if (c >= W) return;
   float total = 0.f;
   for (int j = 0; j < top; ++j) {
     const int e = idx[(size_t)t * top + j];
     if (e < 0) continue;
-    const float s = warp_dot<T, VEC>(a_s + (size_t)j * F, wd + ((size_t)e * W + c) * F, F, lane);
+    const float s = warp_dot<T, VEC>(a_s + (size_t)j * F, wd + ((size_t)e * W + c) * F, F, lane, raw, loaded && j == 0);
     total = fmaf(wt[(size_t)t * top + j], s, total);
   }
   if (lane == 0) y[(size_t)t * ldy + c] = add ? y[(size_t)t * ldy + c] + total : total;
@@ -329,7 +395,7 @@ static int launch_moe_up(const void* h, long ldh, const void* wg, const void* wu
 
 template <typename T, bool VEC>
 static int launch_moe_down(const float* a, const void* wd, int W, int F, int top, const int32_t* idx, const float* wt, float* y, long ldy,
-                           int n_tokens, int add, cudaStream_t stream) {
+                           int n_tokens, int add, int behind_up, cudaStream_t stream) {
   const size_t smem = (size_t)top * F * 4;
   static PerDevice<size_t> allowed;
   if (smem > 48 * 1024 && allowed.here() < smem) {
@@ -338,7 +404,7 @@ static int launch_moe_down(const float* a, const void* wd, int W, int F, int top
     allowed.here() = smem;
   }
   return launch_pdl(PDL_GEMM, moe_down_kernel<T, VEC>, dim3(n_tokens, (W + 7) / 8), dim3(256), smem, stream, a, (const T*)wd, W, F, top,
-                    idx, wt, y, ldy, add);
+                    idx, wt, y, ldy, add, behind_up);
 }
 
 LLMI_EXPORT int llmi_moe_up(int dtype, const void* h, long ldh, const void* wg, const void* wu, int W, int F, int top,
@@ -361,16 +427,18 @@ LLMI_EXPORT int llmi_moe_up(int dtype, const void* h, long ldh, const void* wg, 
   return LLMI_ERR_BAD_DTYPE;
 }
 
+// behind_up: the launch before on this stream is llmi_moe_up with this idx (see moe_down_kernel).
 LLMI_EXPORT int llmi_moe_down(int dtype, const float* a, const void* wd, int W, int F, int top, const int32_t* idx,
-                              const float* wt, float* y, long ldy, int n_tokens, int add, cudaStream_t stream) {
+                              const float* wt, float* y, long ldy, int n_tokens, int add, int behind_up,
+                              cudaStream_t stream) {
   if (n_tokens <= 0 || W <= 0 || F <= 0 || top <= 0 || (size_t)top * F * 4 > 160 * 1024 || (W + 7) / 8 > 65535) return LLMI_ERR_BAD_SIZE;
   const int esz = dtype == LLMI_DTYPE_F32 ? 4 : 2;
   const bool vec = ((size_t)F * esz) % 16 == 0 && !((uintptr_t)wd & 15);
   if (dtype == LLMI_DTYPE_F32)
-    return vec ? launch_moe_down<float, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
-               : launch_moe_down<float, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream);
+    return vec ? launch_moe_down<float, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream)
+               : launch_moe_down<float, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return vec ? launch_moe_down<__nv_bfloat16, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
-               : launch_moe_down<__nv_bfloat16, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream);
+    return vec ? launch_moe_down<__nv_bfloat16, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream)
+               : launch_moe_down<__nv_bfloat16, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream);
   return LLMI_ERR_BAD_DTYPE;
 }

@@ -1908,7 +1908,7 @@ def moe_experts_streamed(h: torch.Tensor, w_gate, w_up, w_down, idx, wt, act: in
     _check("moe_up", l.llmi_moe_up(c_int(_dtype_code(h)), _ptr(h), c_long(h.stride(0)), _ptr(w_gate), _ptr(w_up), c_int(W), c_int(F),
                                    c_int(top), _ptr(idx), _ptr(a), c_int(act), c_int(T), _stream()))
     _check("moe_down", l.llmi_moe_down(c_int(_dtype_code(h)), _ptr(a), _ptr(w_down), c_int(W), c_int(F), c_int(top), _ptr(idx),
-                                       _ptr(wt), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0), _stream()))
+                                       _ptr(wt), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0), c_int(1), _stream()))
 
 
 MOE_GROUPED_MIN_TOKENS = int(os.environ.get("LLMI_MOE_GROUPED_MIN", "4"))
