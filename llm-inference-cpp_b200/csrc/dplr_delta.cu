@@ -77,6 +77,115 @@ gdelta_prepare_kernel(const float* __restrict__ proj, long ld, int H, int D, int
   }
 }
 
+// The same for heads of 32, 64 or 128 entries on 16-byte rows, four entries a thread.  Many tokens (z given): D / 4 threads a head,
+// a token's heads side by side (3,059 tokens of 32 heads of 64: 101 us with a block per token and head and an entry a thread).
+// A few: a block per (token, head) whose 128 threads cut the R rows of W2 into 512 / D segments of equal length, so that a
+// row's loads are not behind one another (one thread walking all R = 128 rows: 17 us for two tokens); the segments' sums are added
+// in ascending order behind w0.
+__device__ __forceinline__ float4 gdelta_four(const float4& k, const float4& a, const float4& b, const float4& z, float inv, float4& u, float4& m) {
+  u = make_float4(k.x * inv, k.y * inv, k.z * inv, k.w * inv);
+  m = make_float4(-sigmoid_f(a.x + b.x) * u.x, -sigmoid_f(a.y + b.y) * u.y, -sigmoid_f(a.z + b.z) * u.z, -sigmoid_f(a.w + b.w) * u.w);
+  const float c = -0.6065306597126334f;
+  return make_float4(expf(c * sigmoid_f(z.x)), expf(c * sigmoid_f(z.y)), expf(c * sigmoid_f(z.z)), expf(c * sigmoid_f(z.w)));
+}
+// 1 / |k| of a head that L = D / 4 neighbouring lanes hold
+template <int L>
+__device__ __forceinline__ float gdelta_inverse(const float4& k) {
+  float ss = fmaf(k.w, k.w, fmaf(k.z, k.z, fmaf(k.y, k.y, k.x * k.x)));
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  return 1.0f / sqrtf(ss + 1e-6f);
+}
+
+template <int D>
+__global__ void __launch_bounds__(256)
+gdelta_prepare_rows_kernel(const float* __restrict__ proj, long ld, int H, int Dv, const float* __restrict__ z_all, long ldz,
+                           const float* __restrict__ w0, const float* __restrict__ a_bias, const int32_t* __restrict__ tok_seq,
+                           float* __restrict__ prep, long ldp) {
+  pdl_launch_dependents();
+  const int t = blockIdx.x, HD = H * D, c = 4 * (blockIdx.y * 256 + threadIdx.x), at = c < HD ? c : 0;
+  pdl_wait();
+  if (tok_seq[t] < 0) return;
+  const float* row = proj + (size_t)t * ld;
+  const float4 k = *reinterpret_cast<const float4*>(row + HD + at);
+  const float4 a = *reinterpret_cast<const float4*>(row + 2 * (size_t)HD + (size_t)H * Dv + at);
+  const float4 zz = *reinterpret_cast<const float4*>(z_all + (size_t)t * ldz + at);
+  const float4 b = *reinterpret_cast<const float4*>(a_bias + at), z0 = *reinterpret_cast<const float4*>(w0 + at);
+  const float inv = gdelta_inverse<D / 4>(k);                 // (every lane takes part; a head's lanes are all in range or all not)
+  if (c >= HD) return;
+  float4 u, m;
+  const float4 w = gdelta_four(k, a, b, make_float4(z0.x + zz.x, z0.y + zz.y, z0.z + zz.z, z0.w + zz.w), inv, u, m);
+  float* out = prep + (size_t)t * ldp + c;
+  *reinterpret_cast<float4*>(out) = w;
+  *reinterpret_cast<float4*>(out + HD) = u;
+  *reinterpret_cast<float4*>(out + 2 * (size_t)HD) = m;
+}
+
+template <int D>
+__global__ void __launch_bounds__(128)
+gdelta_prepare_walk_kernel(const float* __restrict__ proj, long ld, int H, int Dv, int R, const float* __restrict__ w2t,
+                           const float* __restrict__ w0, const float* __restrict__ a_bias, const int32_t* __restrict__ tok_seq,
+                           float* __restrict__ prep, long ldp) {
+  constexpr int L = D / 4, SEGS = 128 / L, AHEAD = 16;
+  extern __shared__ __align__(16) float low_s[];              // tanh of the low-rank path's R entries
+  __shared__ float4 part[SEGS][L];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x, h = blockIdx.y, HD = H * D;
+  if (tok_seq[t] < 0) return;
+  const int lane = threadIdx.x % L, seg = threadIdx.x / L, c = h * D + 4 * lane;
+  const int per = (R + SEGS - 1) / SEGS, j0 = min(R, seg * per), j1 = min(R, j0 + per);
+  const float* row = proj + (size_t)t * ld;
+  const float4 k = *reinterpret_cast<const float4*>(row + HD + c);
+  const float4 a = *reinterpret_cast<const float4*>(row + 2 * (size_t)HD + (size_t)H * Dv + c);
+  const float4 b = *reinterpret_cast<const float4*>(a_bias + c), z0 = *reinterpret_cast<const float4*>(w0 + c);
+  const float* low = row + 3 * (size_t)HD + 2 * (size_t)H * Dv;
+  float4 w[AHEAD];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i)
+    if (j0 + i < j1) w[i] = *reinterpret_cast<const float4*>(w2t + (size_t)(j0 + i) * HD + c);
+  for (int j = threadIdx.x; j < R; j += 128) low_s[j] = tanhf(low[j]);
+  __syncthreads();
+  float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int j = j0; j < j1; j += AHEAD) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (j + i < j1) {
+        const float l = low_s[j + i];
+        z.x = fmaf(w[i].x, l, z.x); z.y = fmaf(w[i].y, l, z.y); z.z = fmaf(w[i].z, l, z.z); z.w = fmaf(w[i].w, l, z.w);
+      }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (j + AHEAD + i < j1) w[i] = *reinterpret_cast<const float4*>(w2t + (size_t)(j + AHEAD + i) * HD + c);
+  }
+  part[seg][lane] = z;
+  __syncthreads();
+  const float inv = gdelta_inverse<L>(k);
+  if (seg > 0) return;
+  z = z0;
+#pragma unroll
+  for (int s = 0; s < SEGS; ++s) {
+    const float4 v = part[s][lane];
+    z = make_float4(z.x + v.x, z.y + v.y, z.z + v.z, z.w + v.w);
+  }
+  float4 u, m;
+  const float4 decay = gdelta_four(k, a, b, z, inv, u, m);
+  float* out = prep + (size_t)t * ldp + c;
+  *reinterpret_cast<float4*>(out) = decay;
+  *reinterpret_cast<float4*>(out + HD) = u;
+  *reinterpret_cast<float4*>(out + 2 * (size_t)HD) = m;
+}
+
+template <int D>
+int launch_gdelta_fours(const float* proj, long ld, int H, int Dv, int R, const float* w2t, const float* z, long ldz, const float* w0,
+                        const float* a_bias, const int32_t* tok_seq, float* prep, long ldp, int n_tokens, cudaStream_t stream) {
+  if (z)
+    return launch_pdl(PDL_SMALL, gdelta_prepare_rows_kernel<D>, dim3(n_tokens, (H * D + 1023) / 1024), dim3(256), 0, stream, proj, ld, H, Dv, z,
+                      ldz, w0, a_bias, tok_seq, prep, ldp);
+  return launch_pdl(PDL_SMALL, gdelta_prepare_walk_kernel<D>, dim3(n_tokens, H), dim3(128), (size_t)R * sizeof(float), stream, proj, ld, H, Dv, R,
+                    w2t, w0, a_bias, tok_seq, prep, ldp);
+}
+
 // The general form: one block per (head, sequence), one thread per column j of S, the column in shared memory
 // (S_s[d][cols]: no two threads share a bank); any D and Dv.  The vectors of the next token are fetched while the
 // current one is computed (two buffers, one barrier per token).
@@ -362,6 +471,12 @@ LLMI_EXPORT int llmi_gdelta_prepare(const float* proj, long ld, int H, int D, in
                                     long ldz, const float* w0, const float* a_bias, const int32_t* tok_seq, float* prep, long ldp,
                                     int n_tokens, cudaStream_t stream) {
   if (n_tokens <= 0 || H <= 0 || H > 65535 || D <= 0 || Dv <= 0 || R <= 0 || R > 8192) return LLMI_ERR_BAD_SIZE;
+  if (ld % 4 == 0 && ldp % 4 == 0 && ldz % 4 == 0 && Dv % 4 == 0 && !((uintptr_t)proj & 15) && !((uintptr_t)prep & 15) && !((uintptr_t)z & 15) &&
+      !((uintptr_t)w2t & 15) && !((uintptr_t)w0 & 15) && !((uintptr_t)a_bias & 15)) {
+    if (D == 32) return launch_gdelta_fours<32>(proj, ld, H, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp, n_tokens, stream);
+    if (D == 64) return launch_gdelta_fours<64>(proj, ld, H, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp, n_tokens, stream);
+    if (D == 128) return launch_gdelta_fours<128>(proj, ld, H, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp, n_tokens, stream);
+  }
   const int threads = D > 64 ? 128 : (D > 32 ? 64 : 32);
   return launch_pdl(PDL_SMALL, gdelta_prepare_kernel, dim3(n_tokens, H), dim3(threads), (size_t)R * sizeof(float), stream, proj, ld,
                     H, D, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp);

@@ -15,7 +15,8 @@
 //   * q is multiplied by a temperature that grows a step every `every` positions: 1 + coef * ln(floor((p + 1) / every) + 1);
 //   * v may be kept as it is for later layers (`v_first`, fp32), or mixed with what an earlier layer kept of the same
 //     token: (1 - lambda) v + lambda v_first; the mixed v is what the cache gets.
-// All arithmetic is fp32; one block per token, or, where no norm ties a part's heads together, one per (token, head).
+// All arithmetic is fp32; one block per token (norms without a rotation: per token and part), or, where no norm ties a part's heads
+// together, one per (token, head).
 #include "common.cuh"
 #include "step_meta.cuh"
 
@@ -260,6 +261,61 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, const float4& v) {
   *reinterpret_cast<uint2*>(o) = u;
 }
 
+// Parts with norms over all their heads and no rotation: a block per (token, part) — q, k, v — with the part's entries in
+// registers between the sum and the store, four a load.  (One block per token that read every entry twice, one at a time: a
+// token of 32 heads of 64 and 2 x 8 key and value heads 20.5 us, the time of its loads one behind the other; 3,059 tokens 40.5.)
+// For parts of up to NORMED_MAX entries; the sum of a part is a thread's entries in ascending order, then block_sum's order.
+constexpr int NORMED_THREADS = 256, NORMED_PER = 4, NORMED_MAX = NORMED_THREADS * 4 * NORMED_PER;
+
+template <typename T>
+__global__ void __launch_bounds__(NORMED_THREADS)
+qkv_prepare_normed_kernel(const float* __restrict__ proj, long ld, int n_q_heads, int n_k_heads, int dk, int n_v_heads, int dv,
+                          const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float eps, int v_from_k,
+                          const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ tok_pos, PagedKV kp, PagedKV vp,
+                          T* __restrict__ k_cache, T* __restrict__ v_cache, T* __restrict__ q_out, long ldq) {
+  __shared__ float scratch[32];
+  pdl_launch_dependents();
+  const int t = blockIdx.x, part = blockIdx.y;
+  const int Nq = n_q_heads * dk, Nk = n_k_heads * dk, n = part == 0 ? Nq : part == 1 ? Nk : n_v_heads * dv;
+  const float* wn = part == 0 ? q_norm_w : part == 1 ? k_norm_w : nullptr;
+  pdl_wait();
+  const int seq = tok_seq[t], pos = tok_pos[t];
+  const float* src = proj + (size_t)t * ld + (part == 0 ? 0 : part == 1 ? Nq : Nq + Nk);
+  float4 x[NORMED_PER], w[NORMED_PER];
+  float ss = 0.f;
+#pragma unroll
+  for (int r = 0; r < NORMED_PER; ++r) {
+    const int i = 4 * (threadIdx.x + r * NORMED_THREADS);
+    x[r] = w[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n && seq >= 0) {
+      x[r] = *reinterpret_cast<const float4*>(src + i);
+      if (wn) w[r] = *reinterpret_cast<const float4*>(wn + i);
+    }
+  }
+  float sc = 1.f;
+  if (wn) {
+#pragma unroll
+    for (int r = 0; r < NORMED_PER; ++r) {
+      ss = fmaf(x[r].x, x[r].x, ss); ss = fmaf(x[r].y, x[r].y, ss); ss = fmaf(x[r].z, x[r].z, ss); ss = fmaf(x[r].w, x[r].w, ss);
+    }
+    sc = 1.0f / sqrtf(block_sum(ss, scratch) / (float)n + eps);
+  }
+#pragma unroll
+  for (int r = 0; r < NORMED_PER; ++r) {
+    const int i = 4 * (threadIdx.x + r * NORMED_THREADS);
+    if (i >= n) break;
+    float4 y = x[r];
+    if (wn) y = make_float4(w[r].x * (x[r].x * sc), w[r].y * (x[r].y * sc), w[r].z * (x[r].z * sc), w[r].w * (x[r].w * sc));
+    if (part == 0) {
+      store4(q_out + (size_t)t * ldq + i, y);                    // (zeros for a row of no sequence)
+    } else if (seq >= 0) {
+      const int size = part == 1 ? dk : dv, hd = i / size, e = i - hd * size;      // (whole fours: within one head)
+      if (part == 1) store4(k_cache + kv_row_offset(kp, seq, pos, hd) + e, y);
+      if (part == 2 || v_from_k) store4(v_cache + kv_row_offset(vp, seq, pos, hd) + e, y);
+    }
+  }
+}
+
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(UP_WARPS * 32)
 qkv_unit_prepare_kernel(const UnitPrepareArgs a, T* __restrict__ k_cache, T* __restrict__ v_cache, T* __restrict__ q_out) {
@@ -393,6 +449,19 @@ LLMI_EXPORT int llmi_qkv_prepare(int dtype, const float* proj, long ld, int n_q_
                                                  amplitude, v_from_k, tok_seq, tok_pos, kp, vp, k_cache, v_cache, q_out, ldq, n_tokens,
                                                  kv, stream);
     return LLMI_ERR_BAD_DTYPE;
+  }
+  const long nq = (long)n_q_heads * dk, nk = has_kv ? (long)n_k_heads * dk : 0, nv = has_kv ? (long)n_v_heads * dv : 0;
+  if (rot_dims == 0 && nq <= NORMED_MAX && nk <= NORMED_MAX && nv <= NORMED_MAX && !(dk % 4) && !(nv > 0 && dv % 4) && !(ld % 4) &&
+      !(ldq % 4) && !((uintptr_t)proj & 15) && !((uintptr_t)q_out & 15) && !((uintptr_t)k_cache & 15) && !((uintptr_t)v_cache & 15) &&
+      !((uintptr_t)q_norm_w & 15) && !((uintptr_t)k_norm_w & 15) && (dtype == LLMI_DTYPE_F32 || dtype == LLMI_DTYPE_BF16)) {
+    const dim3 grid(n_tokens, has_kv && write_kv ? (v_from_k ? 2 : 3) : 1);
+    if (dtype == LLMI_DTYPE_F32)
+      return launch_pdl(PDL_SMALL, qkv_prepare_normed_kernel<float>, grid, dim3(NORMED_THREADS), 0, stream, proj, ld, n_q_heads, n_k_heads, dk,
+                        n_v_heads, dv, q_norm_w, k_norm_w, eps, v_from_k, tok_seq, tok_pos, kp, vp, (float*)k_cache, (float*)v_cache,
+                        (float*)q_out, ldq);
+    return launch_pdl(PDL_SMALL, qkv_prepare_normed_kernel<__nv_bfloat16>, grid, dim3(NORMED_THREADS), 0, stream, proj, ld, n_q_heads,
+                      n_k_heads, dk, n_v_heads, dv, q_norm_w, k_norm_w, eps, v_from_k, tok_seq, tok_pos, kp, vp,
+                      (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (__nv_bfloat16*)q_out, ldq);
   }
   if (dtype == LLMI_DTYPE_F32)
     return launch_pdl(PDL_SMALL, qkv_prepare_kernel<float>, dim3(n_tokens), dim3(128), 0, stream, proj, ld, n_q_heads, n_k_heads,

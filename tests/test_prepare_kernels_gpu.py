@@ -1,0 +1,74 @@
+"""The kernels between a projection and attention or a recurrence, four entries a thread: against 64 bits and the general forms (GPU)."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _ctx(seqs, positions):
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
+    return types.SimpleNamespace(tok_seq=i32(seqs), tok_pos=i32(positions))
+
+
+@pytest.mark.parametrize("H,D,Dv", [(3, 32, 32), (2, 64, 64), (17, 64, 128), (5, 128, 64), (2, 48, 48), (2, 64, 6)])
+@pytest.mark.parametrize("R", [1, 7, 16, 130])
+@pytest.mark.parametrize("walk", [True, False])
+def test_general_delta_vectors(H, D, Dv, R, walk):
+    """W2's rows walked and their product given; a row of no sequence; sizes and pitches that four entries a thread do not take."""
+    from llmi_b200.ops import kernels
+    torch.manual_seed(H * D + R)
+    T, N = 3, H * D
+    for extra in (0, 4, 3):
+        width = 3 * N + 2 * H * Dv + R
+        proj = torch.randn(T, width + extra + (-width) % 4, device="cuda")
+        w2t, w0, ab = torch.randn(R, N, device="cuda") * R ** -0.5, torch.randn(N, device="cuda"), torch.randn(N, device="cuda")
+        low = torch.tanh(proj[:, 3 * N + 2 * H * Dv:width].double())
+        z = low @ w2t.double()
+        prep = torch.full((T, 3 * N + 4), 7.0, device="cuda")
+        kernels.gdelta_prepare(proj, H, D, Dv, w2t, w0, ab, _ctx([0, -1, 1], [5, 0, 9]), prep, None if walk else z.float())
+        k = proj[:, N:2 * N].double().view(T, H, D)
+        u = (k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)).reshape(T, N)
+        at = 2 * N + H * Dv
+        want = torch.cat([torch.exp(-0.6065306597126334 * torch.sigmoid(w0.double() + z)), u,
+                          -torch.sigmoid(proj[:, at:at + N].double() + ab.double()) * u], dim=1)
+        assert (prep[1] == 7.0).all() and (prep[:, 3 * N:] == 7.0).all()
+        # sums of R and D products in 32 bits, then a handful of roundings; every entry is at most 1
+        assert float((prep[[0, 2], :3 * N].double() - want[[0, 2]]).abs().max()) < (R ** 0.5 + D ** 0.5 + 8) * 2.0 ** -23
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nk,dk,nv,dv", [(32, 8, 64, 8, 64), (64, 2, 64, 2, 64), (65, 2, 64, 2, 64), (3, 1, 4, 2, 12), (3, 1, 6, 1, 6), (6, 2, 100, 2, 100)])
+@pytest.mark.parametrize("v_from_k", [False, True])
+def test_norms_over_whole_parts(dtype, nq, nk, dk, nv, dv, v_from_k):
+    """Parts up to the registers' size, one head beyond it, and sizes that whole fours do not divide; one norm, the other, both;
+    keys and values not kept; rows of no sequence."""
+    from llmi_b200.ops import kernels
+    if v_from_k and (nv, dv) != (nk, dk):
+        nv, dv = nk, dk
+    torch.manual_seed(nq + dk)
+    T, page, eps = 4, 64, 1e-5
+    n_v = 0 if v_from_k else nv * dv
+    proj = torch.randn(T, nq * dk + nk * dk + n_v, device="cuda")
+    wq, wk = 1 + 0.2 * torch.randn(nq * dk, device="cuda"), 1 + 0.2 * torch.randn(nk * dk, device="cuda")
+    seqs, at, pages = [0, 1, -1, 1], [3, 70, 0, 71], torch.tensor([[4, 0], [2, 5]], dtype=torch.int32, device="cuda")
+    ctx = _ctx(seqs, at)
+    for uq, uk, write in ((wq, wk, True), (wq, None, True), (None, wk, True), (wq, wk, False)):
+        kc = torch.full((6, nk, page, dk), 7.0, dtype=dtype, device="cuda")
+        vc = torch.full((6, nv, page, dv), 7.0, dtype=dtype, device="cuda")
+        kw, vw, out = kc.double(), vc.double(), torch.full((T, nq * dk), float("nan"), dtype=dtype, device="cuda")
+        kernels.qkv_prepare(proj, nq, nk, dk, nv, dv, uq, uk, eps, None, 0, ctx, pages, page, kc, vc, out, write_kv=write, v_from_k=v_from_k)
+        x = proj.double()
+        q, k, v = x[:, :nq * dk], x[:, nq * dk:nq * dk + nk * dk], x[:, nq * dk + nk * dk:]
+        norm = lambda y, w: y if w is None else y / torch.sqrt((y * y).mean(-1, keepdim=True) + eps) * w.double()      # noqa: E731
+        q, k = norm(q, uq), norm(k, uk)
+        v = k if v_from_k else v
+        q[2] = 0
+        if write:
+            for t in (0, 1, 3):
+                pg = int(pages[seqs[t], at[t] // page])
+                kw[pg, :, at[t] % page], vw[pg, :, at[t] % page] = k[t].view(nk, dk), v[t].view(nv, dv)
+        tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20      # of an entry's own size: the type's rounding, a sum's
+        for got, want in ((out, q), (kc, kw), (vc, vw)):
+            assert bool(((got.double() - want).abs() <= tol * want.abs()).all())
