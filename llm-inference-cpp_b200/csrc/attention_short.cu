@@ -98,14 +98,16 @@ __device__ __forceinline__ void sh_split(float v, float& hi, float& mid, float& 
   lo = __fsub_rn(rest, mid);
 }
 
-// FUSE: one token a sequence; its q is rotated as it is read, its k (rotated) and v are appended to the cache by the block that
-// has the newest page, before it asks for that page (rope_store.cu's arithmetic: the same bits).
+// FUSE: one token a sequence; its q is rotated as it is read, its k (rotated) and v are made, appended to the cache and put into
+// the newest page by the warp that has that row's keys (rope_store.cu's arithmetic: the same bits).  A tile is then 16 rows, and
+// no two warps share keys.
 template <int HD, int ROWS, bool FUSE, bool WIDE>
 __global__ void __launch_bounds__(SH_THREADS, HD == 64 ? 3 : 2)
 attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, ShortParams p) {
   using C = ShCfg<HD>;
   constexpr int WR = ROWS / 16, WK = SH_CONSUMERS / WR;      // row groups, key groups
   constexpr int KEYS = SH_PAGE / WK;                         // keys of a page per warp
+  static_assert(!FUSE || ROWS == 16, "the warp that makes the step's own row has its keys alone");
   extern __shared__ uint8_t smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
@@ -133,6 +135,12 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int pg0 = pg_first + part * per, n_pages = max(0, min(per, n_all - part * per));
   const int32_t* pages = p.seq_pages + (size_t)seq * p.pages_stride;
 
+  // The step's own row of a fused decode step never comes from the cache: the warp that has the row's keys makes it, appends it
+  // and puts it into the page that the copy engine brought.  So no page waits for the kernel before, and nothing for the row's
+  // way out and back (the append, a fence, then the newest page's copy: 0.7 us of a layer of 9 x 64 heads on 340 positions, 1.4 of
+  // eight sequences of 15).  (In attention_decode.cu, whose blocks are bound by the cache's read, the same made eight sequences of
+  // 3,900 positions 15 % slower: their newest pages then compete with the product before.)
+  const bool own_row = FUSE && p.write_kv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ float s_rot[FUSE ? HD : 1];                     // sines, then cosines, of the step's position
   const bool rotate = FUSE && p.rotary_dim > 0;
@@ -152,37 +160,14 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   __syncthreads();
 
   if (warp == SH_CONSUMERS) {
-    // ---- producer (lane 0 asks for the pages; with FUSE the whole warp appends the new k and v) ----
+    // ---- producer (lane 0 asks for the pages) ----
     bool waited = false, ok = true;
     for (int i = 0; i < n_pages && ok; ++i) {
       const int s = i % C::STAGES;
       const int page = pages[pg0 + i];
-      if (!waited && (pg0 + i + 1) * SH_PAGE > pos0) {       // a page with rows of this step: written by the kernel before
+      if (!waited && !own_row && (pg0 + i + 1) * SH_PAGE > pos0) {      // a page with rows of this step: written by a kernel before
         pdl_wait();
         waited = true;
-        if (FUSE && p.write_kv) {                            // (the newest page: the only one that comes here)
-          const __nv_bfloat16* row = p.q + (size_t)q_start * p.ldq;
-          const __nv_bfloat16* ksrc = row + (size_t)(p.n_heads + kvh) * HD;
-          const __nv_bfloat16* vsrc = row + (size_t)(p.n_heads + p.n_kv_heads + kvh) * HD;
-          const size_t dst = (((size_t)page * p.n_kv_heads + kvh) * SH_PAGE + pos0 % SH_PAGE) * HD;
-#pragma unroll
-          for (int j = lane; j < HD / 2; j += 32) {
-            const __nv_bfloat16 a = ksrc[j], b = ksrc[j + HD / 2];
-            if (rotate) {
-              const float fa = __bfloat162float(a), fb = __bfloat162float(b), sn = s_rot[j], cs = s_rot[HD / 2 + j];
-              p.k_cache_w[dst + j] = __float2bfloat16_rn(rot_lo(fa, fb, cs, sn));
-              p.k_cache_w[dst + j + HD / 2] = __float2bfloat16_rn(rot_hi(fa, fb, cs, sn));
-            } else {
-              p.k_cache_w[dst + j] = a;
-              p.k_cache_w[dst + j + HD / 2] = b;
-            }
-            p.v_cache_w[dst + j] = vsrc[j];
-            p.v_cache_w[dst + j + HD / 2] = vsrc[j + HD / 2];
-          }
-          __threadfence();                                    // the copy below reads these rows through the async proxy
-          asm volatile("fence.proxy.async;" ::: "memory");
-          __syncwarp();
-        }
       }
       if (lane == 0) {
         if (i >= C::STAGES && !mbar_wait(empty_bar(s), ((i / C::STAGES) - 1) & 1, p.error_flag, 77)) {
@@ -197,7 +182,6 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           }
         }
       }
-      if (FUSE) __syncwarp();
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     }
   } else {
@@ -205,6 +189,23 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const int wr = warp % WR, wk = warp / WR;
     const int gq = lane >> 2, t = lane & 3;                 // accumulator rows gq and gq + 8, columns 2t and 2t + 1
     pdl_wait();                                             // q comes from the kernel before
+    // the step's own row: entries j and j + HD / 2 of the new key and value, rounded as the cache has them
+    constexpr int NP = HD / 64;
+    const int new_row = pos0 % SH_PAGE, new_page = pos0 / SH_PAGE - pg0;
+    const bool makes_row = own_row && new_page >= 0 && new_page < n_pages && wk == new_row / KEYS;
+    __nv_bfloat16 kn[NP][2], vn[NP][2];
+    if (makes_row) {
+      const __nv_bfloat16* row = p.q + (size_t)q_start * p.ldq;
+      const __nv_bfloat16* ksrc = row + (size_t)(p.n_heads + kvh) * HD;
+      const __nv_bfloat16* vsrc = row + (size_t)(p.n_heads + p.n_kv_heads + kvh) * HD;
+#pragma unroll
+      for (int u = 0; u < NP; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          kn[u][h] = ksrc[lane + 32 * u + HD / 2 * h];
+          vn[u][h] = vsrc[lane + 32 * u + HD / 2 * h];
+        }
+    }
     uint32_t qa[HD / 16][4];
     int qpos[2];
     {
@@ -236,6 +237,23 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           }
       }
     }
+    if (makes_row) {
+      const size_t dst = (((size_t)pages[pg0 + new_page] * p.n_kv_heads + kvh) * SH_PAGE + new_row) * HD;
+#pragma unroll
+      for (int u = 0; u < NP; ++u) {
+        const int j = lane + 32 * u;
+        if (rotate) {
+          const float a = __bfloat162float(kn[u][0]), b = __bfloat162float(kn[u][1]), sn = s_rot[j], cs = s_rot[HD / 2 + j];
+          kn[u][0] = __float2bfloat16_rn(rot_lo(a, b, cs, sn));
+          kn[u][1] = __float2bfloat16_rn(rot_hi(a, b, cs, sn));
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          p.k_cache_w[dst + j + HD / 2 * h] = kn[u][h];
+          p.v_cache_w[dst + j + HD / 2 * h] = vn[u][h];
+        }
+      }
+    }
     float o[HD / 8][4];
 #pragma unroll
     for (int dc = 0; dc < HD / 8; ++dc)
@@ -247,6 +265,18 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       const int s = i % C::STAGES;
       if (!mbar_wait(full_bar(s), (i / C::STAGES) & 1, p.error_flag, 78)) break;
       const uint32_t k_tile = base + s * C::STAGE_BYTES, v_tile = k_tile + C::TILE_BYTES;
+      if (makes_row && i == new_page) {
+#pragma unroll
+        for (int u = 0; u < NP; ++u)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = lane + 32 * u + HD / 2 * h;
+            const uint32_t at = (uint32_t)((j / 64) * C::SUB_BYTES + new_row * 128 + (((j / 8 & 7) ^ (new_row & 7)) << 4) + (j & 7) * 2);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(k_tile + at), "h"(__bfloat16_as_ushort(kn[u][h])) : "memory");
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(v_tile + at), "h"(__bfloat16_as_ushort(vn[u][h])) : "memory");
+          }
+        __syncwarp();
+      }
       const int key0 = (pg0 + i) * SH_PAGE + wk * KEYS;                  // this warp's first key
       const bool inside = key0 + KEYS - 1 <= first_q && (p.window <= 0 || key0 >= last_q - p.window + 1);
       if (key0 + KEYS > kv_len || key0 < lo) {
