@@ -202,6 +202,123 @@ latent_q_rotate_kernel(const T* __restrict__ q, long ldq, int D, T* __restrict__
   }
 }
 
+// The per-head products of a step of a few tokens, out[t, b] = x[t, b] . w[b]^T (bf16, fp32 sums; the queries through the key expansion,
+// the context through the value expansion), and with `q` in the same launch what latent_q_rotate_kernel does.  Such a step is the
+// latency of its loads, so they are all asked for at once, the matrices (where the caller says `early`: a model's weights) ahead of
+// the wait for the kernel before: L lanes a row of K = 8 L CPL entries, RG rows a lane, RG x CPL = 8 pieces of 16 bytes in flight a
+// lane.  A row's sum: a lane's entries ascending, then a butterfly over the lanes; it does not depend on the number of tokens.
+// A request of seven such steps and a prompt, two sequences: with the tensor cores' tiles, a launch for the rotation and attention
+// that waited before its first page 10.86 ms (a map and expert model of 2,048) and 8.35 (channel states, latent rows); 10.55, 8.05.
+struct HeadsArgs {
+  const __nv_bfloat16* x;
+  long ldx, bx;
+  const __nv_bfloat16* w;       // [batch, N, K]
+  __nv_bfloat16* out;
+  long ldo, by;
+  int M, N, early;
+  // the rotation (null: none): q's last R entries of every head into `out` behind the first C
+  const __nv_bfloat16* q;
+  long ldq;
+  int D, C, R;
+  const float* inv_freq;
+  int rot_dims, pairing;
+  float amplitude;
+  const int32_t *tok_seq, *tok_pos;
+};
+constexpr int HEADS_LOADS = 8, HEADS_TOKENS = 4;
+
+template <int L, int CPL>
+__global__ void __launch_bounds__(128)
+heads_token_kernel(const HeadsArgs a) {
+  constexpr int RG = HEADS_LOADS / CPL, K = 8 * L * CPL, GROUPS = 128 / L;      // lane groups of a block
+  pdl_launch_dependents();
+  const int b = blockIdx.y;
+  if (a.q && blockIdx.x == gridDim.x - 1) {
+    pdl_wait();
+    const int half = a.rot_dims / 2 + (a.R - a.rot_dims + 1) / 2;              // the pairs that turn, then the rest two by two
+    for (int idx = threadIdx.x; idx < a.M * half; idx += 128) {
+      const int i = idx % half, t = idx / half;
+      const __nv_bfloat16* src = a.q + (size_t)t * a.ldq + (size_t)b * (a.D + a.R) + a.D;
+      __nv_bfloat16* dst = a.out + (size_t)t * a.ldo + (size_t)b * (a.C + a.R) + a.C;
+      int u = a.rot_dims + 2 * (i - a.rot_dims / 2), v = u + 1;
+      if (i < a.rot_dims / 2) pair_places(i, a.rot_dims, a.pairing, u, v);
+      if (a.tok_seq[t] < 0) {
+        dst[u] = __float2bfloat16_rn(0.f);
+        if (v < a.R) dst[v] = __float2bfloat16_rn(0.f);
+      } else if (i < a.rot_dims / 2) {
+        float s, co;
+        sincosf((float)a.tok_pos[t] * a.inv_freq[i], &s, &co);
+        s *= a.amplitude;
+        co *= a.amplitude;
+        const float x0 = to_f32(src[u]), x1 = to_f32(src[v]);
+        dst[u] = __float2bfloat16_rn(rot_lo(x0, x1, co, s));
+        dst[v] = __float2bfloat16_rn(rot_hi(x0, x1, co, s));
+      } else {
+        dst[u] = src[u];
+        if (v < a.R) dst[v] = src[v];
+      }
+    }
+    return;
+  }
+  const int l = threadIdx.x % L, g = threadIdx.x / L;
+  const int n0 = blockIdx.x * GROUPS * RG + g;                                 // my rows: n0, n0 + GROUPS, ..
+  if (!a.early) pdl_wait();
+  uint4 w[RG][CPL];
+#pragma unroll
+  for (int r = 0; r < RG; ++r)
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      w[r][c] = make_uint4(0u, 0u, 0u, 0u);
+      if (n0 + r * GROUPS < a.N) w[r][c] = *reinterpret_cast<const uint4*>(a.w + ((size_t)b * a.N + n0 + r * GROUPS) * K + 8 * (l + L * c));
+    }
+  if (a.early) pdl_wait();
+  for (int t0 = 0; t0 < a.M; t0 += HEADS_TOKENS) {
+    uint4 x[HEADS_TOKENS][CPL];
+#pragma unroll
+    for (int t = 0; t < HEADS_TOKENS; ++t)
+#pragma unroll
+      for (int c = 0; c < CPL; ++c)
+        x[t][c] = *reinterpret_cast<const uint4*>(a.x + (size_t)min(t0 + t, a.M - 1) * a.ldx + (size_t)b * a.bx + 8 * (l + L * c));
+#pragma unroll
+    for (int t = 0; t < HEADS_TOKENS; ++t) {
+      if (t0 + t >= a.M) break;
+      float sum[RG];
+#pragma unroll
+      for (int r = 0; r < RG; ++r) sum[r] = 0.f;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&x[t][c]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 xf = __bfloat1622float2(xh[e]);
+#pragma unroll
+          for (int r = 0; r < RG; ++r) {
+            const float2 wf = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&w[r][c])[e]);
+            sum[r] = fmaf(wf.x, xf.x, sum[r]);
+            sum[r] = fmaf(wf.y, xf.y, sum[r]);
+          }
+        }
+      }
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < RG; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+      if (l == 0) {
+#pragma unroll
+        for (int r = 0; r < RG; ++r)
+          if (n0 + r * GROUPS < a.N)
+            a.out[(size_t)(t0 + t) * a.ldo + (size_t)b * a.by + n0 + r * GROUPS] = __float2bfloat16_rn(sum[r]);
+      }
+    }
+  }
+}
+
+template <int L, int CPL>
+static int launch_heads_token(const HeadsArgs& a, int batch, cudaStream_t stream) {
+  constexpr int rows = 128 / L * (HEADS_LOADS / CPL);
+  return launch_pdl(PDL_GEMM, heads_token_kernel<L, CPL>, dim3((a.N + rows - 1) / rows + (a.q ? 1 : 0), batch), dim3(128), 0, stream, a);
+}
+
 constexpr int LAT_WARPS = 8;
 
 // One block per (token, group of LAT_WARPS heads), one warp per head.  Keys are taken 32 at a time, in blocks anchored
@@ -396,4 +513,29 @@ LLMI_EXPORT int llmi_attention_latent(int dtype, const void* qa, long ldq, void*
   if (dtype == LLMI_DTYPE_BF16)
     return launch_attention_latent<__nv_bfloat16>(qa, ldq, out, ldo, cache, tok_seq, tok_pos, kv, n_tokens, n_heads, C, scale, window, stream);
   return LLMI_ERR_BAD_DTYPE;
+}
+
+// Row lengths that heads_token_kernel has: 64, 128 and 256 to 2,048 in lane groups of 8, 16 and 32.
+LLMI_EXPORT int llmi_heads_token_supported(int K) { return K == 64 || K == 128 || K == 256 || K == 512 || K == 1024 || K == 2048; }
+
+// `batch` products of a few tokens, one per head: out[:, b*by : b*by + N] = x[:, b*bx : b*bx + K] . w[b]^T (bf16), w [batch, N, K]
+// contiguous; early as llmi_linear_simt.  q (or null): rows [batch][D + R], x == q with bx = D + R and by = C + R, N = C: the last R
+// entries of every head go, rotated as llmi_latent_q_rotate has them, behind its first C outputs.
+LLMI_EXPORT int llmi_heads_token(const void* x, long ldx, long bx, const void* w, void* out, long ldo, long by, int batch, int M, int N,
+                                 int K, int early, const void* q, long ldq, int D, int C, int R, const float* inv_freq, int rot_dims,
+                                 int pairing, float amplitude, const int32_t* tok_seq, const int32_t* tok_pos, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || batch > 65535) return LLMI_ERR_BAD_SIZE;
+  if (!llmi_heads_token_supported(K)) return LLMI_ERR_UNSUPPORTED;
+  if ((ldx % 8) || (bx % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return LLMI_ERR_ALIGN;
+  if (q && (R <= 0 || rot_dims < 0 || (rot_dims & 1) || rot_dims > R || !inv_freq)) return LLMI_ERR_BAD_SIZE;
+  const HeadsArgs a{(const __nv_bfloat16*)x, ldx, bx, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldo, by, M, N, early,
+                    (const __nv_bfloat16*)q, ldq, D, C, R, inv_freq, rot_dims, pairing, amplitude, tok_seq, tok_pos};
+  switch (K) {
+    case 64: return launch_heads_token<8, 1>(a, batch, stream);
+    case 128: return launch_heads_token<16, 1>(a, batch, stream);
+    case 256: return launch_heads_token<32, 1>(a, batch, stream);
+    case 512: return launch_heads_token<32, 2>(a, batch, stream);
+    case 1024: return launch_heads_token<32, 4>(a, batch, stream);
+    default: return launch_heads_token<32, 8>(a, batch, stream);
+  }
 }

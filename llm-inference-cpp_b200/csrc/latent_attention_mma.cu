@@ -48,7 +48,10 @@ template <int NT, int RG>
 __global__ void __launch_bounds__(LM_WARPS * 32 * RG)
 attention_latent_mma_kernel(const LatentMmaArgs a) {
   extern __shared__ __align__(16) unsigned char lm_smem[];
-  pdl_wait();
+  // A step of single tokens (RG == 1): a sequence's rows but its newest are from earlier steps (between two steps lies the copy of
+  // the index block, which waits for all before it), and the first page of them is asked for ahead of the wait for the kernel before.
+  bool waited = RG != 1;
+  if (RG != 1) pdl_wait();
   pdl_launch_dependents();
   const int Dk = a.C + a.R, ldk = Dk + LM_PAD;               // padded pitch: ldmatrix rows fall on different banks
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);                 // [RG * 16][ldk]
@@ -91,6 +94,39 @@ attention_latent_mma_kernel(const LatentMmaArgs a) {
       row_lo[i] = ok ? first_visible(row_pos[i], a.window, 0) : 0;
     }
     const int chunks = Dk / 8;
+    const int n_pages = newest / LM_KEYS + 1;
+    const int first_key = newest < 0 ? 0 : first_visible(oldest, a.window, 0);
+    const int pg_lo = first_key / LM_KEYS + split * a.pages_per_split, pg_hi = min(n_pages, pg_lo + a.pages_per_split);
+
+    // rows `from_row` .. `to_row` - 1 of a page (rows that no query sees: zeros)
+    auto fetch_rows = [&](int pg, int buf, int from_row, int to_row) {
+      const int page = a.seq_pages[(size_t)seq * a.pages_stride + pg];
+      const __nv_bfloat16* src = a.cache + (size_t)page * LM_KEYS * Dk;
+      __nv_bfloat16* dst = k_s + (size_t)buf * LM_KEYS * ldk;
+      for (int r = from_row + (threadIdx.x >> 5); r < to_row; r += RG * LM_WARPS) {      // a warp copies whole rows
+        const bool live = page >= 0 && pg * LM_KEYS + r <= newest && pg * LM_KEYS + r >= first_key;
+        const __nv_bfloat16* from = live ? src + (size_t)r * Dk : a.cache;
+        for (int c8 = lane; c8 < chunks; c8 += 32) cp_async16(dst + r * ldk + 8 * c8, live ? from + 8 * c8 : from, live ? 16 : 0);
+      }
+    };
+    auto fetch = [&](int pg, int buf) {
+      fetch_rows(pg, buf, 0, LM_KEYS);
+      cp_async_commit();
+    };
+    if (RG == 1 && !waited) {
+      const int new_row = pg_lo < pg_hi ? newest - pg_lo * LM_KEYS : LM_KEYS;
+      if (pg_lo < pg_hi) {
+        if (new_row >= LM_KEYS) {
+          fetch_rows(pg_lo, 0, 0, LM_KEYS);
+        } else {
+          fetch_rows(pg_lo, 0, 0, new_row);
+          fetch_rows(pg_lo, 0, new_row + 1, LM_KEYS);
+        }
+      }
+      pdl_wait();
+      if (new_row < LM_KEYS) fetch_rows(pg_lo, 0, new_row, new_row + 1);
+      cp_async_commit();
+    }
     for (int idx = threadIdx.x; idx < RG * LM_ROWS * chunks; idx += blockDim.x) {
       const int r = idx / chunks, c8 = idx - r * chunks;
       const int t = t0 + r / a.heads_per_block, h = h0 + r % a.heads_per_block;
@@ -99,21 +135,6 @@ attention_latent_mma_kernel(const LatentMmaArgs a) {
         v = *reinterpret_cast<const uint4*>(a.qa + (size_t)t * a.ldq + (size_t)h * Dk + 8 * c8);
       *reinterpret_cast<uint4*>(q_s + r * ldk + 8 * c8) = v;
     }
-    const int n_pages = newest / LM_KEYS + 1;
-    const int first_key = newest < 0 ? 0 : first_visible(oldest, a.window, 0);
-    const int pg_lo = first_key / LM_KEYS + split * a.pages_per_split, pg_hi = min(n_pages, pg_lo + a.pages_per_split);
-
-    auto fetch = [&](int pg, int buf) {
-      const int page = a.seq_pages[(size_t)seq * a.pages_stride + pg];
-      const __nv_bfloat16* src = a.cache + (size_t)page * LM_KEYS * Dk;
-      __nv_bfloat16* dst = k_s + (size_t)buf * LM_KEYS * ldk;
-      for (int r = threadIdx.x >> 5; r < LM_KEYS; r += RG * LM_WARPS) {          // a warp copies whole rows
-        const bool live = page >= 0 && pg * LM_KEYS + r <= newest && pg * LM_KEYS + r >= first_key;
-        const __nv_bfloat16* from = live ? src + (size_t)r * Dk : a.cache;
-        for (int c8 = lane; c8 < chunks; c8 += 32) cp_async16(dst + r * ldk + 8 * c8, live ? from + 8 * c8 : from, live ? 16 : 0);
-      }
-      cp_async_commit();
-    };
 
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     float o[NT][4];
@@ -122,7 +143,8 @@ attention_latent_mma_kernel(const LatentMmaArgs a) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
 
-    if (pg_lo < pg_hi) fetch(pg_lo, 0);
+    if (waited && pg_lo < pg_hi) fetch(pg_lo, 0);
+    waited = true;
     for (int pg = pg_lo; pg < pg_hi; ++pg) {
       const int buf = nbuf == 2 ? (pg - pg_lo) & 1 : 0;
       cp_async_wait_all();
@@ -270,6 +292,7 @@ attention_latent_mma_kernel(const LatentMmaArgs a) {
       }
     }
   }
+  if (!waited) pdl_wait();                                     // (no token of a sequence)
   // token rows of no sequence: zeros (one thread group per row)
   if (blockIdx.z == 0)
     for (int t = t0; t <= t_last; ++t)
@@ -287,35 +310,50 @@ attention_latent_join_kernel(const float* __restrict__ ws_o, const float* __rest
                              long ldo, const int32_t* __restrict__ tok_seq, int n_heads, int C, int splits) {
   __shared__ float w_s[LM_MAX_SPLITS];
   __shared__ float red[32];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long item = blockIdx.x;
   const int t = (int)(item / n_heads), h = (int)(item - (long)t * n_heads);
   if (tok_seq[t] < 0) return;                                 // (zeros were written by the first kernel)
-  const float* ml = ws_ml + (size_t)item * splits * 2;
+  // (maximum, sum) of a thread's cuts once, the maxima joined over the block; then sixteen cuts' values on their way at a time
+  const float2* ml = reinterpret_cast<const float2*>(ws_ml) + (size_t)item * splits;
+  constexpr int MINE = (LM_MAX_SPLITS + 127) / 128;
+  float2 v[MINE];
   float M = -INFINITY;
-  for (int s = 0; s < splits; ++s) M = fmaxf(M, ml[2 * s]);   // (the same few words for every thread: served by the cache)
+#pragma unroll
+  for (int u = 0; u < MINE; ++u) {
+    const int s = threadIdx.x + 128 * u;
+    v[u] = s < splits ? ml[s] : make_float2(-INFINITY, 0.f);
+  }
+#pragma unroll
+  for (int u = 0; u < MINE; ++u) M = fmaxf(M, v[u].x);
+  M = warp_max(M);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = M;
+  __syncthreads();
+  M = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
   float part = 0.f;
-  for (int s = threadIdx.x; s < splits; s += blockDim.x) {
-    const float m = ml[2 * s];
-    const float w = m == -INFINITY ? 0.f : expf(m - M);
+#pragma unroll
+  for (int u = 0; u < MINE; ++u) {
+    const int s = threadIdx.x + 128 * u;
+    if (s >= splits) break;
+    const float w = v[u].x == -INFINITY ? 0.f : expf(v[u].x - M);
     w_s[s] = w;
-    part += w * ml[2 * s + 1];
+    part += w * v[u].y;
   }
   const float denom = block_sum(part, red);
   const float inv = 1.0f / denom;
   const float* o = ws_o + (size_t)item * splits * C;
   for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    int s = 0;
-    for (; s + 4 <= splits; s += 4) {
-      a0 = fmaf(w_s[s], o[(size_t)s * C + c], a0);
-      a1 = fmaf(w_s[s + 1], o[(size_t)(s + 1) * C + c], a1);
-      a2 = fmaf(w_s[s + 2], o[(size_t)(s + 2) * C + c], a2);
-      a3 = fmaf(w_s[s + 3], o[(size_t)(s + 3) * C + c], a3);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = 0; s0 < splits; s0 += 16) {
+      float x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = s0 + u < splits ? o[(size_t)(s0 + u) * C + c] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (s0 + u < splits) acc[u & 3] = fmaf(w_s[s0 + u], x[u], acc[u & 3]);
     }
-    for (; s < splits; ++s) a0 = fmaf(w_s[s], o[(size_t)s * C + c], a0);
-    out[(size_t)t * ldo + (size_t)h * C + c] = __float2bfloat16_rn(((a0 + a1) + (a2 + a3)) * inv);
+    out[(size_t)t * ldo + (size_t)h * C + c] = __float2bfloat16_rn(((acc[0] + acc[1]) + (acc[2] + acc[3])) * inv);
   }
 }
 

@@ -168,7 +168,7 @@ def lib():
                      "llmi_moe_identity_add", "llmi_channel_decay", "llmi_rows_activate", "llmi_decay_recurrence",
                      "llmi_normed_pair", "llmi_stream_axpy_norm", "llmi_stream_postnorm", "llmi_softcap_rows", "llmi_moe_table",
                      "llmi_qkv_unit_prepare", "llmi_latent_prepare_direct", "llmi_channel_token_supported",
-                     "llmi_channel_token_prepare", "llmi_channel_token_step", "llmi_cast_rows"):
+                     "llmi_channel_token_prepare", "llmi_channel_token_step", "llmi_cast_rows", "llmi_heads_token", "llmi_heads_token_supported"):
             getattr(l, name).restype = c_int
         l.llmi_gemm_tc_workspace.restype = c_long
         l.llmi_delta_state_floats.restype = c_long
@@ -1486,6 +1486,15 @@ def stream_add(x: torch.Tensor, add: torch.Tensor | None, vec: torch.Tensor | No
 HEADS_MMA_MIN_TOKENS = int(os.environ.get("LLMI_HEADS_MMA_MIN", "1"))      # from here on the per-head products of a step run on the tensor cores (bf16)
 
 
+# Up to here the per-head products of a step go to the kernel that is the latency of its loads, beyond to the tensor cores.
+HEADS_TOKEN_MAX = 8
+
+
+def heads_token_applies(x: torch.Tensor, bx: int, w: torch.Tensor, K: int) -> bool:
+    return bool(x.dtype == torch.bfloat16 and x.shape[0] <= HEADS_TOKEN_MAX and not _FORCE_SIMT and lib().llmi_heads_token_supported(c_int(K))
+                and bx % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
 def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor, by: int, K: int, mode: int = OUT_STORE,
                    early: bool = False) -> None:
     """``w.shape[0]`` products in one launch (one per head): out_b (mode) x_b . w[b]^T with x_b = x[:, b*bx : b*bx + K] and
@@ -1498,6 +1507,12 @@ def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor,
     assert Kw == K and w.is_contiguous() and x.stride(1) == 1 and out.stride(1) == 1 and out.shape[0] == M and x.dtype == w.dtype
     assert (B - 1) * bx + K <= x.shape[1] and (B - 1) * by + N <= out.shape[1]
     assert out.dtype == (x.dtype if mode == OUT_STORE else torch.float32)
+    if mode == OUT_STORE and heads_token_applies(x, bx, w, K):
+        _check("heads_token", lib().llmi_heads_token(
+            _ptr(x), c_long(x.stride(0)), c_long(bx), _ptr(w), _ptr(out), c_long(out.stride(0)), c_long(by), c_int(B), c_int(M), c_int(N),
+            c_int(K), c_int(1 if early else 0), None, c_long(0), c_int(0), c_int(0), c_int(0), None, c_int(0), c_int(0), c_float(1.0),
+            None, None, _stream()))
+        return
     if (x.dtype == torch.bfloat16 and mode == OUT_STORE and M >= HEADS_MMA_MIN_TOKENS and not _FORCE_SIMT and K % 8 == 0
             and bx % 8 == 0 and by % 2 == 0 and x.stride(0) % 8 == 0 and out.stride(0) % 2 == 0 and x.data_ptr() % 16 == 0
             and w.data_ptr() % 16 == 0 and out.data_ptr() % 4 == 0):
@@ -1562,6 +1577,24 @@ def latent_q_rotate(q: torch.Tensor, D: int, qa: torch.Tensor, C: int, R: int, H
     _check("latent_q_rotate", lib().llmi_latent_q_rotate(
         c_int(_dtype_code(q)), _ptr(q), c_long(q.stride(0)), c_int(D), _ptr(qa), c_long(qa.stride(0)), c_int(C), c_int(R), c_int(H),
         _ptr(inv_freq), c_int(rot_dims), _ptr(ctx.tok_seq), _ptr(ctx.tok_pos), c_int(T), c_int(pairing), c_float(amplitude), _stream()))
+
+
+def latent_query(q: torch.Tensor, D: int, w_uk_t: torch.Tensor, qa: torch.Tensor, C: int, R: int, H: int, inv_freq, rot_dims: int, ctx,
+                 pairing: int = 1, amplitude: float = 1.0) -> None:
+    """Every head's query as the latent rows are scored with: [q[:, h, :D] . w_uk_t[h]^T (C) | q[:, h, D:] rotated (R)] into qa
+    [T, H*(C+R)]: :func:`linear_batched` (with a model's weights) and :func:`latent_q_rotate`, for a few tokens in one launch."""
+    assert w_uk_t.shape == (H, C, D) and w_uk_t.is_contiguous() and q.dtype == qa.dtype == w_uk_t.dtype
+    if not R or not heads_token_applies(q, D + R, w_uk_t, D):
+        linear_batched(q, D + R, w_uk_t, qa, C + R, D, early=True)
+        latent_q_rotate(q, D, qa, C, R, H, inv_freq, rot_dims, ctx, pairing, amplitude)
+        return
+    _need_cuda(q, qa, w_uk_t, inv_freq)
+    T = q.shape[0]
+    assert q.stride(1) == 1 and qa.stride(1) == 1 and q.shape[1] == H * (D + R) and qa.shape == (T, H * (C + R))
+    _check("heads_token", lib().llmi_heads_token(
+        _ptr(q), c_long(q.stride(0)), c_long(D + R), _ptr(w_uk_t), _ptr(qa), c_long(qa.stride(0)), c_long(C + R), c_int(H), c_int(T), c_int(C),
+        c_int(D), c_int(1), _ptr(q), c_long(q.stride(0)), c_int(D), c_int(C), c_int(R), _ptr(inv_freq), c_int(rot_dims), c_int(pairing),
+        c_float(amplitude), _ptr(ctx.tok_seq), _ptr(ctx.tok_pos), _stream()))
 
 
 _LATENT_ATTENTION = os.environ.get("LLMI_LATENT_ATTENTION", "mma")      # "generic": the fp32-arithmetic kernel for everything

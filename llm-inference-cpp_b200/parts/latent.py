@@ -132,8 +132,7 @@ class LatentAttention:
                 return kernels.linear(heads, self.w_o, x, None, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,
                                       None if store else then_norm, out_scale)
             qa = rt.scratch("latent_qa", (T, H * (C + R)))
-            kernels.linear_batched(q, D + R, self.w_uk_t, qa, C + R, D, early=True)
-            kernels.latent_q_rotate(q, D, qa, C, R, H, self.inv_freq, self.rot_dims, ctx, self.pairing, self.amplitude)
+            kernels.latent_query(q, D, self.w_uk_t, qa, C, R, H, self.inv_freq, self.rot_dims, ctx, self.pairing, self.amplitude)
         else:
             qa = rt.scratch("latent_qa", (T, H * (C + R)))
             qn = rt.scratch("latent_q", (T, H * D))
