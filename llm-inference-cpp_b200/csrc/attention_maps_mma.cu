@@ -103,7 +103,10 @@ template <int NV, bool PROMPT, bool BIAS>
 __global__ void __launch_bounds__((PROMPT ? AM_PROMPT_WARPS : AM_WARPS) * 32)
 attention_maps_mma_kernel(const MapsArgs a) {
   extern __shared__ __align__(16) unsigned char am_smem[];
-  pdl_wait();
+  // Single tokens: a sequence's rows but its newest are from earlier steps (between two steps lies the copy of the index block,
+  // which waits for all before it), so its first page is asked for ahead of the wait for the kernel before.  (With the join's
+  // sixteen loads at a time a request of seven such steps, eight layers: 9.53 -> 9.45 ms.)
+  if (PROMPT) pdl_wait();
   pdl_launch_dependents();
   constexpr int DV = NV * 16, ROWS = PROMPT ? AM_PROMPT_ROWS : 16, NT2 = PROMPT ? 4 : 1;
   constexpr int NBUF = PROMPT ? 2 : AM_TOKEN_BUFFERS;             // page buffers: NBUF - 1 pages are under way while one is multiplied     // NT2: groups of 16 keys a warp takes per page
@@ -141,6 +144,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
     head0 = kvh * group;
     split = blockIdx.z;
     if (a.seq_kv_len[seq] <= 0 || a.tok_seq[t0] < 0) {
+      pdl_wait();
       if (a.splits == 1)                                        // a sequence of no token: zeros (with cuts, the joining kernel writes them)
         for (int idx = threadIdx.x; idx < group * (NV * 16); idx += blockDim.x) {
           const size_t at = (size_t)t0 * a.ldo + ((size_t)(head0 + idx / (NV * 16)) * a.maps + mp) * (NV * 16) + idx % (NV * 16);
@@ -155,34 +159,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
   const int p_first = a.tok_pos[t0], p_last = p_first + n_rows - 1;
   const int lo_first = first_visible(p_first, a.window, a.chunk);
 
-  // queries into shared memory; rows of no token (or of no head) are zeros
   const int chunks_k = dk / 8;
-  for (int idx = threadIdx.x; idx < ROWS * chunks_k; idx += blockDim.x) {
-    const int r = idx / chunks_k, c8 = idx - r * chunks_k;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (PROMPT) {
-      if (r < n_rows) v = *reinterpret_cast<const uint4*>(a.q + (size_t)(t0 + r) * a.ldq + (size_t)(head0 * a.maps + mp) * dk + 8 * c8);
-    } else {
-      if (r < group) v = *reinterpret_cast<const uint4*>(a.q + (size_t)t0 * a.ldq + (size_t)((head0 + r) * a.maps + mp) * dk + 8 * c8);
-    }
-    *reinterpret_cast<uint4*>(q_s + r * ldk + 8 * c8) = v;
-  }
-
-  // my two rows (g and g + 8 of my warp's 16): position, first visible key, pooled blocks it sees, factor on the scores
-  int row_pos[2], row_lo[2], row_nb[2];
-  float row_scale[2], row_r1[2], row_r2[2];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int r = (PROMPT ? 16 * warp : 0) + g + 8 * i;
-    const bool ok = PROMPT ? r < n_rows : r < group;
-    row_pos[i] = ok ? (PROMPT ? p_first + r : p_first) : -1;
-    row_lo[i] = ok ? first_visible(row_pos[i], a.window, a.chunk) : 0;
-    row_nb[i] = ok ? maps_pooled_visible(row_pos[i], a.window, a.pool) : 0;
-    const int head = PROMPT ? head0 : head0 + (ok ? r : 0);
-    row_scale[i] = a.head_scale ? a.scale_log2 * a.head_scale[head] : a.scale_log2;
-    row_r1[i] = BIAS ? a.r1[head] : 0.f;
-    row_r2[i] = BIAS ? a.r2[head] : 0.f;
-  }
   // what my warp's rows can see at all (a page outside costs my warp nothing)
   int w_hi, w_lo;
   if (PROMPT) {
@@ -215,7 +192,8 @@ attention_maps_mma_kernel(const MapsArgs a) {
     return pg < n_pp ? a.pool_pages[(size_t)seq * a.pool_pages_stride + pg] : a.seq_pages[(size_t)seq * a.pages_stride + tpg_lo + pg - n_pp];
   };
   // `page`: the page's index in the cache, read from the table one iteration ahead of its copies
-  auto fetch = [&](int pg, int buf, int page) {
+  // (`skip`: a row that is left out)
+  auto fetch = [&](int pg, int buf, int page, int skip = -1) {
     const bool pooled = pg < n_pp;
     const __nv_bfloat16* ksrc = (pooled ? a.k_pool : a.k_cache) + ((size_t)(page < 0 ? 0 : page) * (a.G * a.maps) + kh) * AM_PAGE * dk;
     const __nv_bfloat16* vsrc = (pooled ? a.v_pool : a.v_cache) + ((size_t)(page < 0 ? 0 : page) * a.G + kvh) * AM_PAGE * DV;
@@ -225,7 +203,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
     const int live_rows = page < 0 ? 0 : pooled ? n_pool_rows - pg * AM_PAGE : newest - (tpg_lo + pg - n_pp) * AM_PAGE + 1;
     for (int r = kr0, c8 = kc0; r < AM_PAGE;) {
       const bool live = r < live_rows;
-      cp_async16(kd + r * ldk + 8 * c8, live ? ksrc + (size_t)r * dk + 8 * c8 : a.k_cache, live ? 16 : 0);
+      if (r != skip) cp_async16(kd + r * ldk + 8 * c8, live ? ksrc + (size_t)r * dk + 8 * c8 : a.k_cache, live ? 16 : 0);
       r += kr_step;
       c8 += kc_step;
       if (c8 >= chunks_k) { c8 -= chunks_k; ++r; }
@@ -233,9 +211,16 @@ attention_maps_mma_kernel(const MapsArgs a) {
     for (int idx = threadIdx.x; idx < AM_PAGE * chunks_v; idx += blockDim.x) {
       const int r = idx / chunks_v, c8 = idx - r * chunks_v;
       const bool live = r < live_rows;
-      cp_async16(vd + r * ldv + 8 * c8, live ? vsrc + (size_t)r * DV + 8 * c8 : a.v_cache, live ? 16 : 0);
+      if (r != skip) cp_async16(vd + r * ldv + 8 * c8, live ? vsrc + (size_t)r * DV + 8 * c8 : a.v_cache, live ? 16 : 0);
     }
-    cp_async_commit();
+  };
+  auto fetch_row = [&](int buf, int page, int r) {
+    const __nv_bfloat16* ksrc = a.k_cache + (((size_t)page * (a.G * a.maps) + kh) * AM_PAGE + r) * dk;
+    const __nv_bfloat16* vsrc = a.v_cache + (((size_t)page * a.G + kvh) * AM_PAGE + r) * DV;
+    for (int c8 = threadIdx.x; c8 < chunks_k + chunks_v; c8 += blockDim.x) {
+      if (c8 < chunks_k) cp_async16(k_s + (size_t)(buf * AM_PAGE + r) * ldk + 8 * c8, ksrc + 8 * c8, 16);
+      else cp_async16(v_s + (size_t)(buf * AM_PAGE + r) * ldv + 8 * (c8 - chunks_k), vsrc + 8 * (c8 - chunks_k), 16);
+    }
   };
 
   const float inv_cap = a.softcap_log2 > 0.f ? 1.0f / a.softcap_log2 : 0.f;
@@ -248,8 +233,45 @@ attention_maps_mma_kernel(const MapsArgs a) {
 
 #pragma unroll
   for (int ahead = 0; ahead < NBUF - 1; ++ahead) {               // (a group per page, also an empty one: the waits count groups)
-    if (pg_lo + ahead <= pg_hi) fetch(pg_lo + ahead, ahead, page_of(pg_lo + ahead));
-    else cp_async_commit();
+    const int pg = pg_lo + ahead, page = page_of(pg);
+    if (!PROMPT && ahead == 0) {
+      const int new_row = pg <= pg_hi ? newest - (tpg_lo + pg - n_pp) * AM_PAGE : -1;
+      const bool early = pg >= n_pp, has_new = early && new_row >= 0 && new_row < AM_PAGE && page >= 0;
+      if (pg <= pg_hi && early) fetch(pg, 0, page, has_new ? new_row : -1);
+      pdl_wait();
+      if (pg <= pg_hi && !early) fetch(pg, 0, page);      // (pooled rows: this step may have finished one)
+      if (has_new) fetch_row(0, page, new_row);
+    } else if (pg <= pg_hi) {
+      fetch(pg, ahead, page);
+    }
+    cp_async_commit();
+  }
+  // queries into shared memory; rows of no token (or of no head) are zeros
+  for (int idx = threadIdx.x; idx < ROWS * chunks_k; idx += blockDim.x) {
+    const int r = idx / chunks_k, c8 = idx - r * chunks_k;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (PROMPT) {
+      if (r < n_rows) v = *reinterpret_cast<const uint4*>(a.q + (size_t)(t0 + r) * a.ldq + (size_t)(head0 * a.maps + mp) * dk + 8 * c8);
+    } else {
+      if (r < group) v = *reinterpret_cast<const uint4*>(a.q + (size_t)t0 * a.ldq + (size_t)((head0 + r) * a.maps + mp) * dk + 8 * c8);
+    }
+    *reinterpret_cast<uint4*>(q_s + r * ldk + 8 * c8) = v;
+  }
+
+  // my two rows (g and g + 8 of my warp's 16): position, first visible key, pooled blocks it sees, factor on the scores
+  int row_pos[2], row_lo[2], row_nb[2];
+  float row_scale[2], row_r1[2], row_r2[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = (PROMPT ? 16 * warp : 0) + g + 8 * i;
+    const bool ok = PROMPT ? r < n_rows : r < group;
+    row_pos[i] = ok ? (PROMPT ? p_first + r : p_first) : -1;
+    row_lo[i] = ok ? first_visible(row_pos[i], a.window, a.chunk) : 0;
+    row_nb[i] = ok ? maps_pooled_visible(row_pos[i], a.window, a.pool) : 0;
+    const int head = PROMPT ? head0 : head0 + (ok ? r : 0);
+    row_scale[i] = a.head_scale ? a.scale_log2 * a.head_scale[head] : a.scale_log2;
+    row_r1[i] = BIAS ? a.r1[head] : 0.f;
+    row_r2[i] = BIAS ? a.r2[head] : 0.f;
   }
   int page_next = page_of(pg_lo + NBUF - 1);
   const int key_off = PROMPT ? 0 : 16 * warp;                    // my keys within a page
@@ -259,7 +281,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
     cp_async_wait<NBUF - 2>();
     __syncthreads();                                             // this page is here; everyone is done with the page before
     if (pg + NBUF - 1 <= pg_hi) fetch(pg + NBUF - 1, (pg - pg_lo + NBUF - 1) % NBUF, page_next);
-    else cp_async_commit();
+    cp_async_commit();
     page_next = page_of(pg + NBUF);
     const bool pooled = pg < n_pp;
     const int base = (pooled ? pg : tpg_lo + pg - n_pp) * AM_PAGE + key_off;     // the first of my keys: a block's or a position's index
@@ -425,8 +447,8 @@ attention_maps_join_kernel(const float* __restrict__ ws_o, const float* __restri
                            const float* __restrict__ gate, long ldg, int maps, int gate_per, const float* __restrict__ sink) {
   __shared__ float w_s[AM_MAX_PARTS];
   __shared__ float red[32];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const long item = blockIdx.x;
   const int t = (int)(item / per_tok), hm = (int)(item - (long)t * per_tok);
   const size_t at = (size_t)t * ldo + (size_t)hm * dv;
@@ -438,8 +460,13 @@ attention_maps_join_kernel(const float* __restrict__ ws_o, const float* __restri
     return;
   }
   const float* ml = ws_ml + (size_t)item * parts * 2;
+  // the parts' maxima dealt out over the threads, and sixteen parts' values on their way at a time
   float M = -INFINITY;
-  for (int s = 0; s < parts; ++s) M = fmaxf(M, ml[2 * s]);
+  for (int s = threadIdx.x; s < parts; s += blockDim.x) M = fmaxf(M, ml[2 * s]);
+  M = warp_max(M);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = M;
+  __syncthreads();
+  M = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
   float part = 0.f;
   for (int s = threadIdx.x; s < parts; s += blockDim.x) {
     const float m = ml[2 * s];
@@ -452,8 +479,14 @@ attention_maps_join_kernel(const float* __restrict__ ws_o, const float* __restri
   const float* o = ws_o + (size_t)item * parts * dv;
   for (int c = threadIdx.x; c < dv; c += blockDim.x) {
     float acc = 0.f;
-    for (int s = 0; s < parts; ++s)
-      if (w_s[s] != 0.f) acc = fmaf(w_s[s], o[(size_t)s * dv + c], acc);      // (a part that saw no key holds nothing)
+    for (int s0 = 0; s0 < parts; s0 += 16) {
+      float x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = s0 + u < parts ? o[(size_t)(s0 + u) * dv + c] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (s0 + u < parts && w_s[s0 + u] != 0.f) acc = fmaf(w_s[s0 + u], x[u], acc);      // (a part that saw no key holds nothing)
+    }
     float res = acc * inv;
     if (gate && gate_per > 1) res *= 1.0f / (1.0f + __expf(-gate[(size_t)t * ldg + (size_t)hm * dv + c]));
     if (out_f32) ((float*)out)[at + c] = res;
