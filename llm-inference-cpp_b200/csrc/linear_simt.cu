@@ -126,15 +126,20 @@ linear_simt_kernel(const T* __restrict__ x, long ldx, const T* __restrict__ w, l
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Many tokens.  Bound by the FMA pipes (128 a clock and SM; 74 TFLOP/s, of which 8 x 8 products out of registers alone reach
-// 55).  800 tokens x 960 -> 5,120: 252 us, 31 TFLOP/s: a block takes 30 us for its 4 segments and the last of 7.03 waves is
-// nearly empty.  (Two blocks of half the stages on an SM: 282 us.)  A block makes a tile of 64 x 64 outputs; its four groups of 64
+// 55).  800 tokens x 960 -> 5,120: 225 us, 35 TFLOP/s: a block takes 31 us for its 4 segments and the last of 7.03 waves is
+// nearly empty.  (Two blocks of half the stages on an SM were slower, and so were tiles of 64 x 128: as many FMAs a clock, fewer
+// tiles for the SMs.)  A block makes a tile of 64 x 64 outputs; its four groups of 64
 // threads take segments 4r, 4r + 1, .. of round r, each thread 8 x 8 outputs in registers (one 16-byte shared load per 16
 // FMAs where 4 x 4 outputs need two).  With the segments side by side a block keeps two warps of independent chains
 // on every scheduler though its tile is small, and small tiles fill the 148 SMs at the widths of small models (600 tokens x
-// 960 outputs are 150 tiles).  Operands go to shared memory as they lie (rows of 16 k places, 20 floats apart: a quarter
-// warp's 16-byte loads touch 32 different banks) by cp.async, three stages a group.
-constexpr int TILE_STAGES = 3;
-constexpr int TILE_PITCH = BK + 4;
+// 960 outputs are 150 tiles).  Operands go to shared memory as they lie (rows of 32 k places, 36 floats apart: a quarter
+// warp's 16-byte loads touch 32 different banks) by cp.async, two stages a group.  A stage costs a barrier of the group, its copies'
+// addresses and the first loads' latency, which two warps a scheduler do not cover: stages of 16 places, three of them, took 251
+// us for those 800 tokens, and 3 to 11 % more over 65 to 1,500 tokens and the widths of 576 to 5,120 (four requests of the 360M
+// shape in fp32 37.4 -> 35.7 ms).  The same chains: the same bits.
+constexpr int TILE_STAGES = 2;
+constexpr int TILE_BK = 32;            // k places of a stage
+constexpr int TILE_PITCH = TILE_BK + 4;
 constexpr int TILE_STAGE_FLOATS = (BM + BN) * TILE_PITCH;
 constexpr int TOTAL_PITCH = BN + 8;
 constexpr int TILE_SMEM = (4 * TILE_STAGES * TILE_STAGE_FLOATS + BM * TOTAL_PITCH) * (int)sizeof(float);
@@ -164,18 +169,18 @@ linear_f32_tile_kernel(const float* __restrict__ x, long ldx, const float* __res
   for (int round = 0; round * 4 < n_seg; ++round) {
     const int seg = round * 4 + group;
     const int k_begin = seg * SEG, k_end = min(K, k_begin + SEG);
-    const int steps = seg < n_seg ? (k_end - k_begin + BK - 1) / BK : 0;
+    const int steps = seg < n_seg ? (k_end - k_begin + TILE_BK - 1) / TILE_BK : 0;
     auto load = [&](int step) {
       float* s = stages + (step % TILE_STAGES) * TILE_STAGE_FLOATS;
-      const int k = k_begin + step * BK + (t & 3) * 4;
+      const int k = k_begin + step * TILE_BK + (t & 7) * 4;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {              // rows 0..63 of x, then 64 rows of w
-        const int r = (t >> 2) + e * 16;
-        const bool of_x = e < 4;
+      for (int e = 0; e < 16; ++e) {             // rows 0..63 of x, then 64 rows of w
+        const int r = (t >> 3) + e * 8;
+        const bool of_x = e < 8;
         const int row = of_x ? m0 + r : n0 + r - BM;
         const bool real = k < k_end && row < (of_x ? M : N);
         const float* src = of_x ? x + (long)row * ldx + k : w + (long)row * ldw + k;
-        cp_async_16(s + r * TILE_PITCH + (t & 3) * 4, real ? src : x, real);
+        cp_async_16(s + r * TILE_PITCH + (t & 7) * 4, real ? src : x, real);
       }
     };
     float acc[8][8];
@@ -194,8 +199,8 @@ linear_f32_tile_kernel(const float* __restrict__ x, long ldx, const float* __res
       if (step + TILE_STAGES - 1 < steps) load(step + TILE_STAGES - 1);
       asm volatile("cp.async.commit_group;" ::: "memory");
       const float* s = stages + (step % TILE_STAGES) * TILE_STAGE_FLOATS;
-#pragma unroll
-      for (int q = 0; q < BK / 4; ++q) {
+#pragma unroll 2
+      for (int q = 0; q < TILE_BK / 4; ++q) {
         float4 a[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(s + (ty + 8 * i) * TILE_PITCH + 4 * q);
