@@ -74,7 +74,7 @@ struct ShCfg {
   static constexpr int STAGE_BYTES = 2 * TILE_BYTES;
   static constexpr int STAGES = HD == 64 ? 4 : 3;
   static constexpr int OUT_PITCH = HD + 4;      // floats a row of the results: values, maximum, sum
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 16 * STAGES;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 16 * STAGES + 16;
   static_assert(SH_MAX_ROWS * OUT_PITCH * 4 <= STAGES * STAGE_BYTES, "the results lie where the ring was");
 };
 
@@ -99,15 +99,15 @@ __device__ __forceinline__ void sh_split(float v, float& hi, float& mid, float& 
 }
 
 // FUSE: one token a sequence; its q is rotated as it is read, its k (rotated) and v are made, appended to the cache and put into
-// the newest page by the warp that has that row's keys (rope_store.cu's arithmetic: the same bits).  A tile is then 16 rows, and
-// no two warps share keys.
+// the newest page by the block that has that page (rope_store.cu's arithmetic: the same bits).  A tile is then 16 rows, and no two
+// warps share keys.
 template <int HD, int ROWS, bool FUSE, bool WIDE>
 __global__ void __launch_bounds__(SH_THREADS, HD == 64 ? 3 : 2)
 attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, ShortParams p) {
   using C = ShCfg<HD>;
   constexpr int WR = ROWS / 16, WK = SH_CONSUMERS / WR;      // row groups, key groups
   constexpr int KEYS = SH_PAGE / WK;                         // keys of a page per warp
-  static_assert(!FUSE || ROWS == 16, "the warp that makes the step's own row has its keys alone");
+  static_assert(!FUSE || ROWS == 16, "one warp has the keys of the step's own row");
   extern __shared__ uint8_t smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
@@ -116,6 +116,7 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const uint32_t bars = base + C::STAGES * C::STAGE_BYTES;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (C::STAGES + s); };
+  const uint32_t row_bar = bars + 16u * C::STAGES;
   float* results = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));     // [WK][ROWS][OUT_PITCH]
 
   // which (sequence, kv head, row tile); the same for all blocks of a cluster
@@ -135,12 +136,15 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int pg0 = pg_first + part * per, n_pages = max(0, min(per, n_all - part * per));
   const int32_t* pages = p.seq_pages + (size_t)seq * p.pages_stride;
 
-  // The step's own row of a fused decode step never comes from the cache: the warp that has the row's keys makes it, appends it
-  // and puts it into the page that the copy engine brought.  So no page waits for the kernel before, and nothing for the row's
-  // way out and back (the append, a fence, then the newest page's copy: 0.7 us of a layer of 9 x 64 heads on 340 positions, 1.4 of
-  // eight sequences of 15).  (In attention_decode.cu, whose blocks are bound by the cache's read, the same made eight sequences of
-  // 3,900 positions 15 % slower: their newest pages then compete with the product before.)
+  // The step's own row of a fused decode step never comes from the cache: the producer warp, once it has asked for all pages, makes
+  // it, appends it and puts it into the page that the copy engine brought.  So no page waits for the kernel before, and nothing for
+  // the row's way out and back (the append, a fence, then the newest page's copy: 0.7 us of a layer of 9 x 64 heads on 340
+  // positions, 1.4 of eight sequences of 15).  Made by the consumer warp that has the row's keys, it cost 24 sequences of up to
+  // 3,900 positions 1.6 us a layer of 49.  (In attention_decode.cu, whose blocks are bound by the cache's read, the same made eight
+  // sequences of 3,900 positions 15 % slower: their newest pages then compete with the product before.)
   const bool own_row = FUSE && p.write_kv;
+  const int new_row = pos0 % SH_PAGE, new_page = n_all - 1 - part * per;      // (of this part's pages: its last, or none of them)
+  const bool has_newest = own_row && n_pages > 0 && new_page == n_pages - 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __shared__ float s_rot[FUSE ? HD : 1];                     // sines, then cosines, of the step's position
   const bool rotate = FUSE && p.rotary_dim > 0;
@@ -155,6 +159,7 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), SH_CONSUMERS);
     }
+    mbar_init(row_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -184,20 +189,15 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     }
-  } else {
-    // ---- consumers: warp (wr, wk) has rows 16 wr .. and keys KEYS wk .. of every page ----
-    const int wr = warp % WR, wk = warp / WR;
-    const int gq = lane >> 2, t = lane & 3;                 // accumulator rows gq and gq + 8, columns 2t and 2t + 1
-    pdl_wait();                                             // q comes from the kernel before
-    // the step's own row: entries j and j + HD / 2 of the new key and value, rounded as the cache has them
-    constexpr int NP = HD / 64;
-    const int new_row = pos0 % SH_PAGE, new_page = pos0 / SH_PAGE - pg0;
-    const bool makes_row = own_row && new_page >= 0 && new_page < n_pages && wk == new_row / KEYS;
-    __nv_bfloat16 kn[NP][2], vn[NP][2];
-    if (makes_row) {
+    if (has_newest && ok) {
+      // entries j and j + HD / 2 of the new key and value, rounded as the cache has them
+      constexpr int NP = HD / 64;
+      __nv_bfloat16 kn[NP][2], vn[NP][2];
+      pdl_wait();
       const __nv_bfloat16* row = p.q + (size_t)q_start * p.ldq;
       const __nv_bfloat16* ksrc = row + (size_t)(p.n_heads + kvh) * HD;
       const __nv_bfloat16* vsrc = row + (size_t)(p.n_heads + p.n_kv_heads + kvh) * HD;
+      const size_t dst = (((size_t)pages[pg0 + new_page] * p.n_kv_heads + kvh) * SH_PAGE + new_row) * HD;
 #pragma unroll
       for (int u = 0; u < NP; ++u)
 #pragma unroll
@@ -205,7 +205,37 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           kn[u][h] = ksrc[lane + 32 * u + HD / 2 * h];
           vn[u][h] = vsrc[lane + 32 * u + HD / 2 * h];
         }
+      const int s = new_page % C::STAGES;
+      const uint32_t k_tile = base + s * C::STAGE_BYTES, v_tile = k_tile + C::TILE_BYTES;
+      if (mbar_wait(full_bar(s), (new_page / C::STAGES) & 1, p.error_flag, 80)) {
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+          if (rotate) {
+            const int j = lane + 32 * u;
+            const float a = __bfloat162float(kn[u][0]), b = __bfloat162float(kn[u][1]), sn = s_rot[j], cs = s_rot[HD / 2 + j];
+            kn[u][0] = __float2bfloat16_rn(rot_lo(a, b, cs, sn));
+            kn[u][1] = __float2bfloat16_rn(rot_hi(a, b, cs, sn));
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int j = lane + 32 * u + HD / 2 * h;
+            const uint32_t at = (uint32_t)((j / 64) * C::SUB_BYTES + new_row * 128 + (((j / 8 & 7) ^ (new_row & 7)) << 4) + (j & 7) * 2);
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(k_tile + at), "h"(__bfloat16_as_ushort(kn[u][h])) : "memory");
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(v_tile + at), "h"(__bfloat16_as_ushort(vn[u][h])) : "memory");
+            p.k_cache_w[dst + j] = kn[u][h];
+            p.v_cache_w[dst + j] = vn[u][h];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(row_bar);
+      }
     }
+  } else {
+    // ---- consumers: warp (wr, wk) has rows 16 wr .. and keys KEYS wk .. of every page ----
+    const int wr = warp % WR, wk = warp / WR;
+    const int gq = lane >> 2, t = lane & 3;                 // accumulator rows gq and gq + 8, columns 2t and 2t + 1
+    pdl_wait();                                             // q comes from the kernel before
+    const bool has_row = has_newest && wk == new_row / KEYS;      // the step's own row is one of my keys
     uint32_t qa[HD / 16][4];
     int qpos[2];
     {
@@ -237,23 +267,6 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
           }
       }
     }
-    if (makes_row) {
-      const size_t dst = (((size_t)pages[pg0 + new_page] * p.n_kv_heads + kvh) * SH_PAGE + new_row) * HD;
-#pragma unroll
-      for (int u = 0; u < NP; ++u) {
-        const int j = lane + 32 * u;
-        if (rotate) {
-          const float a = __bfloat162float(kn[u][0]), b = __bfloat162float(kn[u][1]), sn = s_rot[j], cs = s_rot[HD / 2 + j];
-          kn[u][0] = __float2bfloat16_rn(rot_lo(a, b, cs, sn));
-          kn[u][1] = __float2bfloat16_rn(rot_hi(a, b, cs, sn));
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          p.k_cache_w[dst + j + HD / 2 * h] = kn[u][h];
-          p.v_cache_w[dst + j + HD / 2 * h] = vn[u][h];
-        }
-      }
-    }
     float o[HD / 8][4];
 #pragma unroll
     for (int dc = 0; dc < HD / 8; ++dc)
@@ -265,18 +278,7 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       const int s = i % C::STAGES;
       if (!mbar_wait(full_bar(s), (i / C::STAGES) & 1, p.error_flag, 78)) break;
       const uint32_t k_tile = base + s * C::STAGE_BYTES, v_tile = k_tile + C::TILE_BYTES;
-      if (makes_row && i == new_page) {
-#pragma unroll
-        for (int u = 0; u < NP; ++u)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int j = lane + 32 * u + HD / 2 * h;
-            const uint32_t at = (uint32_t)((j / 64) * C::SUB_BYTES + new_row * 128 + (((j / 8 & 7) ^ (new_row & 7)) << 4) + (j & 7) * 2);
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(k_tile + at), "h"(__bfloat16_as_ushort(kn[u][h])) : "memory");
-            asm volatile("st.shared.u16 [%0], %1;" ::"r"(v_tile + at), "h"(__bfloat16_as_ushort(vn[u][h])) : "memory");
-          }
-        __syncwarp();
-      }
+      if (has_row && i == new_page && !mbar_wait(row_bar, 0, p.error_flag, 79)) break;      // (the row is in its place)
       const int key0 = (pg0 + i) * SH_PAGE + wk * KEYS;                  // this warp's first key
       const bool inside = key0 + KEYS - 1 <= first_q && (p.window <= 0 || key0 >= last_q - p.window + 1);
       if (key0 + KEYS > kv_len || key0 < lo) {
