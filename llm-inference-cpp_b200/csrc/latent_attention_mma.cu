@@ -38,6 +38,7 @@ struct LatentMmaArgs {
                                 // so that two blocks share an SM and overlap each other instead (steps of single tokens)
   float scale;
   int window;                   // 0: every earlier position
+  int early;                    // single tokens: all rows but the newest were complete before the launch ahead began
   float* ws_o;                  // [T, H, splits, C]   (splits > 1)
   float* ws_ml;                 // [T, H, splits, 2]
 };
@@ -48,10 +49,10 @@ template <int NT, int RG>
 __global__ void __launch_bounds__(LM_WARPS * 32 * RG)
 attention_latent_mma_kernel(const LatentMmaArgs a) {
   extern __shared__ __align__(16) unsigned char lm_smem[];
-  // A step of single tokens (RG == 1): a sequence's rows but its newest are from earlier steps (between two steps lies the copy of
-  // the index block, which waits for all before it), and the first page of them is asked for ahead of the wait for the kernel before.
+  // A step of single tokens (RG == 1): a sequence's rows but its newest are from earlier steps, and where the caller says that those
+  // were complete before the launch ahead began (`early`), the first page of them is asked for ahead of the wait for that launch.
   bool waited = RG != 1;
-  if (RG != 1) pdl_wait();
+  if (RG != 1 || !a.early) pdl_wait();
   pdl_launch_dependents();
   const int Dk = a.C + a.R, ldk = Dk + LM_PAD;               // padded pitch: ldmatrix rows fall on different banks
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);                 // [RG * 16][ldk]
@@ -385,11 +386,13 @@ LLMI_EXPORT long llmi_attention_latent_mma_workspace(int n_tokens, int n_heads, 
   return splits <= 1 ? 0 : (long)n_tokens * n_heads * splits * (C + 2);
 }
 
+// early = 1 (row_groups 1): every row of the step's sequences but the newest was complete before the launch ahead began (a model's
+// step: the copy of its index block lies between), so that it may be read before that launch has ended.
 LLMI_EXPORT int llmi_attention_latent_mma(const void* qa, long ldq, void* out, long ldo, const void* cache,
                                           const int32_t* tok_seq, const int32_t* tok_pos, const int32_t* seq_pages,
                                           int pages_stride, int page_size, int n_tokens, int n_heads, int C, int R, float scale,
                                           int splits, int pages_per_split, int row_groups, float* workspace,
-                                          long workspace_floats, int window, cudaStream_t stream) {
+                                          long workspace_floats, int window, int early, cudaStream_t stream) {
   if (n_tokens <= 0 || n_heads <= 0 || !llmi_attention_latent_mma_supported(C, R, page_size)) return LLMI_ERR_UNSUPPORTED;
   if (splits < 1 || splits > LM_MAX_SPLITS || pages_per_split < 1 || (row_groups != 1 && row_groups != 2) || window < 0) return LLMI_ERR_BAD_SIZE;
   if (((uintptr_t)qa & 15) || ((uintptr_t)cache & 15) || (ldq % 8) || ((uintptr_t)out & 3) || (ldo % 2)) return LLMI_ERR_ALIGN;
@@ -402,7 +405,7 @@ LLMI_EXPORT int llmi_attention_latent_mma(const void* qa, long ldq, void* out, l
   a.tok_seq = tok_seq; a.tok_pos = tok_pos; a.seq_pages = seq_pages; a.pages_stride = pages_stride;
   a.n_tokens = n_tokens; a.n_heads = n_heads; a.C = C; a.R = R;
   a.heads_per_block = hpb; a.tokens_per_block = row_groups * LM_ROWS / hpb;
-  a.splits = splits; a.pages_per_split = pages_per_split; a.scale = scale; a.window = window;
+  a.splits = splits; a.pages_per_split = pages_per_split; a.scale = scale; a.window = window; a.early = early;
   a.page_buffers = row_groups == 1 ? 1 : 2;
   a.ws_o = workspace;
   a.ws_ml = workspace ? workspace + (size_t)n_tokens * n_heads * splits * C : nullptr;

@@ -1623,10 +1623,12 @@ def latent_attention_plan(ctx, n_tokens: int, n_pages: int, H: int, window: int 
 
 
 def attention_latent(qa: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, ctx, seq_pages, page_size: int, H: int, C: int,
-                     R: int, scale: float, rt=None, window: int = 0) -> None:
+                     R: int, scale: float, rt=None, window: int = 0, early: bool = False) -> None:
     """Causal attention of every token's heads over its sequence's latent rows (``window`` > 0: the last ``window`` of them): scores from all C + R entries of a
     row, context from its first C.  qa [T, H*(C+R)], out [T, H*C].  bf16 sizes that the tensor-core kernel takes go
-    there (``rt`` lends the workspace of its cuts); everything else, and the 32-bit path, to the generic kernel."""
+    there (``rt`` lends the workspace of its cuts); everything else, and the 32-bit path, to the generic kernel.
+    ``early``: every row but a single token's newest was complete before the launch ahead began (a model's step: the copy of its
+    index block lies between), so that a step of single tokens may read it before that launch has ended."""
     _need_cuda(qa, out, cache, seq_pages)
     T = qa.shape[0]
     assert qa.dtype == out.dtype == cache.dtype and qa.stride(1) == 1 and out.stride(1) == 1 and cache.is_contiguous()
@@ -1640,7 +1642,8 @@ def attention_latent(qa: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, c
         _check("attention_latent_mma", lib().llmi_attention_latent_mma(
             _ptr(qa), c_long(qa.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(cache), _ptr(ctx.tok_seq), _ptr(ctx.tok_pos),
             _ptr(seq_pages), c_int(seq_pages.stride(0)), c_int(page_size), c_int(T), c_int(H), c_int(C), c_int(R), c_float(scale),
-            c_int(splits), c_int(pps), c_int(1 if ctx.decode else 2), _ptr(ws), c_long(n_ws), c_int(window), _stream()))
+            c_int(splits), c_int(pps), c_int(1 if ctx.decode else 2), _ptr(ws), c_long(n_ws), c_int(window), c_int(1 if early else 0),
+            _stream()))
         return
     _check("attention_latent", lib().llmi_attention_latent(
         c_int(_dtype_code(qa)), _ptr(qa), c_long(qa.stride(0)), _ptr(out), c_long(out.stride(0)), _ptr(cache), _ptr(ctx.tok_seq),

@@ -140,7 +140,8 @@ class LatentAttention:
                                           pages, g.page_size, cache, qn, qa, write_kv=binding.writes, amplitude=self.amplitude)
             kernels.linear_batched(qn, D, self.w_uk_t, qa, C + R, D, early=True)
         lat = rt.scratch("latent_ctx", (T, H * C))
-        kernels.attention_latent(qa, lat, cache, ctx, pages, g.page_size, H, C, R, self.scale, rt=rt, window=self.window)
+        kernels.attention_latent(qa, lat, cache, ctx, pages, g.page_size, H, C, R, self.scale, rt=rt, window=self.window,
+                                 early=True)
         heads = rt.scratch("attn_out", (T, H * Dv))
         kernels.linear_batched(lat, C, self.w_uv, heads, Dv, C, early=True)
         return kernels.linear(heads, self.w_o, x, None, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,

@@ -1,0 +1,82 @@
+"""Kernels that may start before the launch ahead has ended, with that launch still at work (GPU).
+
+Every test puts a launch of two blocks in front that lets the next ones start at once and takes tens of microseconds; the
+kernel that writes the step's own row waits for it, and the reader under test is launched directly behind the writer."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROUNDS = 15
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def _long_launch():
+    from llmi_b200.ops import kernels
+    K = 1 << 17
+    x, w, y = torch.ones(1, K, device="cuda"), torch.ones(16, K, device="cuda"), torch.empty(1, 16, device="cuda")
+    return lambda: kernels.linear_simt(x, w, y)
+
+
+def _token_ctx(positions):
+    """A step in which sequence s brings the token at ``positions[s]``."""
+    S, kv = len(positions), [p + 1 for p in positions]
+    return types.SimpleNamespace(decode=True, n_seqs=S, n_real_seqs=S, tok_seq=_i32(list(range(S))), tok_pos=_i32(positions),
+                                 seq_q_start=_i32(list(range(S + 1))), seq_kv_len=_i32(kv), seq_slot=_i32(list(range(S))),
+                                 host_q_lens=[1] * S, host_kv_lens=kv)
+
+
+def _check(reset, steps):
+    """``steps``: functions of one launch or more each.  Run with the device idle between them, then in a row."""
+    hold = _long_launch()
+    want = []
+    reset()
+    for step in steps:
+        torch.cuda.synchronize()
+        want.append(step().clone())
+    assert all(bool(torch.isfinite(w).all()) for w in want)
+    for _ in range(ROUNDS):
+        reset()
+        hold()
+        got = [step() for step in steps]
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)
+
+
+POSITIONS = [0, 1, 62, 63, 64, 126, 127, 300]
+
+
+@pytest.mark.parametrize("C,R", [(512, 64), (64, 16)])
+@pytest.mark.parametrize("early", [True, False])
+def test_latent_rows(C, R, early):
+    """``early``: the newest row is still to be written when the reader starts.  Without: so is the row before it, which the step
+    before makes in the same row of launches."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels
+    rt = Runtime(torch.bfloat16, "cuda")
+    torch.manual_seed(C)
+    H, Q, S, P, Dk = 16, 128, len(POSITIONS), 6, C + R
+    pages = torch.randperm(S * P, device="cuda").int().view(S, P)
+    full = torch.randn(S * P, 1, 64, Dk, device="cuda").bfloat16()
+    cache = torch.empty_like(full)
+    wq, wc, inv = torch.ones(Q, device="cuda"), torch.ones(C, device="cuda"), torch.rand(R // 2, device="cuda")
+    steps = []
+    for s, p in enumerate(POSITIONS):                    # (what the steps do not write stays no number)
+        for j in range(p, 64 * P):
+            full[pages[s, j // 64], 0, j % 64] = float("nan")
+    for positions in [POSITIONS] if early else [POSITIONS, [p + 1 for p in POSITIONS]]:
+        ctx, down = _token_ctx(positions), torch.randn(S, Q + C + R, device="cuda")
+        cq, qa = torch.empty(S, Q, device="cuda").bfloat16(), (torch.randn(S, H * Dk, device="cuda") * 0.1).bfloat16()
+        out = torch.empty(S, H * C, device="cuda").bfloat16()
+
+        def step(ctx=ctx, down=down, cq=cq, qa=qa, out=out):
+            kernels.latent_prepare(down, Q, C, R, wq, wc, 1e-5, inv, R, ctx, pages, 64, cache, cq)
+            kernels.attention_latent(qa, out, cache, ctx, pages, 64, H, C, R, 0.3, rt=rt, early=early)
+            return out
+        steps.append(step)
+    _check(lambda: cache.copy_(full), steps)
