@@ -76,6 +76,7 @@ struct MapsArgs {
   const float* r1;              // [H] or null: the bias by distance (in base 2: r1 * log2(1 + r2 * d))
   const float* r2;
   const float* sink;            // [H] or null
+  int early;                    // single tokens: all rows but the newest (and pooled ones) were complete before the launch ahead began
 };
 
 __device__ __forceinline__ int maps_pooled_visible(int pos, int window, int pool) {
@@ -103,10 +104,10 @@ template <int NV, bool PROMPT, bool BIAS>
 __global__ void __launch_bounds__((PROMPT ? AM_PROMPT_WARPS : AM_WARPS) * 32)
 attention_maps_mma_kernel(const MapsArgs a) {
   extern __shared__ __align__(16) unsigned char am_smem[];
-  // Single tokens: a sequence's rows but its newest are from earlier steps (between two steps lies the copy of the index block,
-  // which waits for all before it), so its first page is asked for ahead of the wait for the kernel before.  (With the join's
-  // sixteen loads at a time a request of seven such steps, eight layers: 9.53 -> 9.45 ms.)
-  if (PROMPT) pdl_wait();
+  // Single tokens: a sequence's rows but its newest are from earlier steps, and where the caller says that those were complete before
+  // the launch ahead began (`early`), its first page is asked for ahead of the wait for that launch.  (With the join's sixteen
+  // loads at a time a request of seven such steps, eight layers: 9.53 -> 9.45 ms.)
+  if (PROMPT || !a.early) pdl_wait();
   pdl_launch_dependents();
   constexpr int DV = NV * 16, ROWS = PROMPT ? AM_PROMPT_ROWS : 16, NT2 = PROMPT ? 4 : 1;
   constexpr int NBUF = PROMPT ? 2 : AM_TOKEN_BUFFERS;             // page buffers: NBUF - 1 pages are under way while one is multiplied     // NT2: groups of 16 keys a warp takes per page
@@ -526,7 +527,9 @@ LLMI_EXPORT long llmi_attention_maps_mma_workspace(int n_tokens, int n_heads, in
 }
 
 // prompt != 0: n_blocks = an upper bound of the sum over sequences of ceil(tokens / 128).  prompt == 0: every sequence
-// brings one token; `splits` cuts of `pages_per_split` pages over the visible positions.
+// brings one token; `splits` cuts of `pages_per_split` pages over the visible positions.  early = 1 (prompt == 0): every row of the
+// step's sequences but the newest (and the pooled ones) was complete before the launch ahead began (a model's step: the copy of its
+// index block lies between), so that it may be read before that launch has ended.
 LLMI_EXPORT int llmi_attention_maps_mma(const void* q, long ldq, void* out, long ldo, int out_f32, const void* k_cache,
                                         const void* v_cache, const int32_t* tok_seq, const int32_t* tok_pos,
                                         const int32_t* seq_pages, int pages_stride, const int32_t* seq_q_start,
@@ -535,7 +538,7 @@ LLMI_EXPORT int llmi_attention_maps_mma(const void* q, long ldq, void* out, long
                                         int n_blocks, int splits, int pages_per_split, float* workspace, long workspace_floats,
                                         int pool, const void* k_pool, const void* v_pool, const int32_t* pool_pages,
                                         int pool_pages_stride, const float* gate, long ldg, int gate_per, float softcap,
-                                        const float* r1, const float* r2, const float* sink, cudaStream_t stream) {
+                                        const float* r1, const float* r2, const float* sink, int early, cudaStream_t stream) {
   if (gate && gate_per != 1 && (gate_per != dv || maps != 1)) return LLMI_ERR_UNSUPPORTED;
   if (softcap < 0.f || (r1 == nullptr) != (r2 == nullptr)) return LLMI_ERR_BAD_SIZE;
   if (r1 && pool > 0) return LLMI_ERR_UNSUPPORTED;          // a pooled row has no distance
@@ -556,7 +559,7 @@ LLMI_EXPORT int llmi_attention_maps_mma(const void* q, long ldq, void* out, long
   a.pool = pool; a.k_pool = (const __nv_bfloat16*)k_pool; a.v_pool = (const __nv_bfloat16*)v_pool;
   a.pool_pages = pool_pages; a.pool_pages_stride = pool_pages_stride; a.gate = gate; a.ldg = ldg;
   a.gate_per = gate_per; a.softcap_log2 = softcap * 1.4426950408889634f;
-  a.r1 = r1; a.r2 = r2; a.sink = sink;
+  a.r1 = r1; a.r2 = r2; a.sink = sink; a.early = early;
   const int rows = prompt ? AM_PROMPT_ROWS : 16;
   const int nbuf = prompt ? 2 : AM_TOKEN_BUFFERS;
   const size_t smem = ((size_t)(rows + nbuf * AM_PAGE) * (dk + AM_PAD) + (size_t)nbuf * AM_PAGE * (dv + AM_PAD)) * 2;

@@ -1276,10 +1276,12 @@ def pool_rows(k_cache, v_cache, seq_pages, k_pool, v_pool, pool_pages, page_size
 
 def attention_maps(q, out, k_cache, v_cache, ctx, seq_pages, page_size: int, n_heads: int, n_kv_heads: int, maps: int,
                    dk: int, dv: int, scale: float, head_scale=None, window: int = 0, chunk: int = 0, rt=None, pooled=None,
-                   gate=None, softcap: float = 0.0, bias=None, sink=None) -> None:
+                   gate=None, softcap: float = 0.0, bias=None, sink=None, early: bool = False) -> None:
     """The attention of a step in its general form (arguments as :func:`attention_flex`): bf16 sizes that the
     tensor-core kernel takes go there — prompts as blocks of 128 query rows, steps of single tokens cut over the
-    positions (``rt`` lends the workspace of the cuts) —, everything else, and the 32-bit path, to the generic kernel."""
+    positions (``rt`` lends the workspace of the cuts) —, everything else, and the 32-bit path, to the generic kernel.
+    ``early``: every row but a single token's newest (and the pooled ones) was complete before the launch ahead began (a model's
+    step: the copy of its index block lies between), so that a step of single tokens may read it before that launch has ended."""
     gate_per = _gate_per(gate, n_heads, maps, dv)
     plain = maps == 1 and dk == dv                  # more maps, or values of their own size: nothing else beside them
     if (not ctx.decode and (chunk == 0 or seq_pages.shape[1] * 64 <= chunk) and softcap == 0.0 and gate_per == 1 and page_size == 64 and scale > 0
@@ -1336,7 +1338,7 @@ def attention_maps(q, out, k_cache, v_cache, ctx, seq_pages, page_size: int, n_h
             c_int(T // 128 + S), c_int(splits), c_int(pps), _ptr(ws), c_long(n_ws), c_int(pool), _ptr(k_pool), _ptr(v_pool),
             _ptr(pool_pages), c_int(pool_pages.stride(0) if pool else 0), _ptr(gate),
             c_long(gate.stride(0) if gate is not None else 0), c_int(gate_per), c_float(softcap), _ptr(r1), _ptr(r2), _ptr(sink),
-            _stream()))
+            c_int(1 if early else 0), _stream()))
         return
     attention_flex(q, out, k_cache, v_cache, ctx, seq_pages, page_size, n_heads, n_kv_heads, maps, dk, dv, scale, head_scale,
                    window, chunk, pooled, gate, softcap, bias, sink)

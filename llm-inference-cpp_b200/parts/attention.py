@@ -170,7 +170,7 @@ class _MapsAttention:
                             ctx, pages, g.page_size, k_cache, v_cache, q, has_kv=not self.shares_kv, write_kv=binding.writes)
         out = rt.scratch("attn_maps" if M > 1 else "attn_out", (T, H * M * Dv), torch.float32 if M > 1 else None)
         kernels.attention_maps(q, out, k_cache, v_cache, ctx, pages, g.page_size, H, G, M, D, Dv, self.scale, self.head_scale,
-                               self.window, self.chunk, rt=rt)
+                               self.window, self.chunk, rt=rt, early=True)
         return out
 
 
@@ -341,7 +341,7 @@ class WindowPoolAttention(_MapsAttention):
         gate = proj[:, self.n_qkv:] if self.gated else None
         out = rt.scratch("attn_out", (T, H * Dv))
         kernels.attention_maps(q, out, k_cache, v_cache, ctx, pages, g.page_size, H, G, 1, D, Dv, self.scale, None,
-                               self.window, 0, rt=rt, pooled=pooled, gate=gate)
+                               self.window, 0, rt=rt, pooled=pooled, gate=gate, early=True)
         return self._project_out(out, x, store, then_norm)
 
     stores_output = True
@@ -472,7 +472,7 @@ class GatedAttention(_MapsAttention):
         out = rt.scratch("attn_out", (T, H * Dv))
         kernels.attention_maps(q, out, k_cache, v_cache, ctx, pages, g.page_size, H, G, 1, D, Dv, self.scale, None,
                                self.window, self.chunk, rt=rt, gate=proj[:, self.n_qkv:] if self.gated else None,
-                               softcap=self.softcap)
+                               softcap=self.softcap, early=True)
         return kernels.linear(out, self.w_o, x, self.b_o, kernels.OUT_STORE_F32 if store else kernels.OUT_ADD_F32,
                               None if store else then_norm, out_scale)
 
@@ -550,5 +550,5 @@ class DistanceAttention(_MapsAttention):
                                  self.value_mode, self.lam, first, write_kv=binding.writes)
         out = rt.scratch("attn_out", (T, H * Dv))
         kernels.attention_maps(q, out, k_cache, v_cache, ctx, pages, g.page_size, H, G, 1, D, Dv, self.scale, None, self.window, 0,
-                               rt=rt, bias=self.bias, sink=self.sink)
+                               rt=rt, bias=self.bias, sink=self.sink, early=True)
         return self._project_out(out, x, store, then_norm)

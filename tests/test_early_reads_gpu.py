@@ -80,3 +80,35 @@ def test_latent_rows(C, R, early):
             return out
         steps.append(step)
     _check(lambda: cache.copy_(full), steps)
+
+
+@pytest.mark.parametrize("Hq,G,maps,dk,dv,window", [(4, 2, 2, 64, 64, 0), (16, 8, 1, 128, 128, 0), (6, 2, 2, 64, 128, 70)])
+@pytest.mark.parametrize("early", [True, False])
+def test_rows_of_several_maps(Hq, G, maps, dk, dv, window, early):
+    """As above, for keys and values in pages of their own."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels
+    rt = Runtime(torch.bfloat16, "cuda")
+    torch.manual_seed(Hq + dk)
+    S, P, N, Nk, Nv = len(POSITIONS), 6, Hq * maps * dk, G * maps * dk, G * dv
+    pages = torch.randperm(S * P, device="cuda").int().view(S, P)
+    k_full, v_full = torch.randn(S * P, G * maps, 64, dk, device="cuda").bfloat16(), torch.randn(S * P, G, 64, dv, device="cuda").bfloat16()
+    for s, p in enumerate(POSITIONS):
+        for j in range(p, 64 * P):
+            k_full[pages[s, j // 64], :, j % 64] = v_full[pages[s, j // 64], :, j % 64] = float("nan")
+    kc, vc = torch.empty_like(k_full), torch.empty_like(v_full)
+    steps = []
+    for positions in [POSITIONS] if early else [POSITIONS, [p + 1 for p in POSITIONS]]:
+        ctx, proj = _token_ctx(positions), torch.randn(S, N + Nk + Nv, device="cuda")
+        q, out = torch.empty(S, N, device="cuda").bfloat16(), torch.empty(S, Hq * maps * dv, device="cuda").bfloat16()
+
+        def step(ctx=ctx, proj=proj, q=q, out=out):
+            kernels.qkv_prepare(proj, Hq * maps, G * maps, dk, G, dv, None, None, 1e-5, None, 0, ctx, pages, 64, kc, vc, q)
+            kernels.attention_maps(q, out, kc, vc, ctx, pages, 64, Hq, G, maps, dk, dv, dk ** -0.5, None, window, 0, rt=rt, early=early)
+            return out
+        steps.append(step)
+
+    def reset():
+        kc.copy_(k_full)
+        vc.copy_(v_full)
+    _check(reset, steps)
