@@ -6,10 +6,11 @@
 //                               a warp per (token, head of q or k) or 128 channels of v: short convolution from the carried
 //                               inputs, silu, unit norm, and the carried inputs moved on by one (nobody else reads them);
 //                               a warp per token for the write strengths;
+//                               (what the step before left is asked for before the wait on the kernel before, with `early`)
 //                               a block per 64 outputs of the two low-rank products (decay, output gate) for up to 16 tokens:
 //                               fp32 arithmetic, every weight read once per 16 tokens, the decays finished on the spot
 //   llmi_channel_token_step     a cluster per (token, head), a block per 32 columns of S: the state is asked for before the
-//                               wait on the kernel before; update and read-out in registers; the blocks of a cluster
+//                               wait on the kernel before (with `early`); update and read-out in registers; the blocks of a cluster
 //                               exchange their sums of squares, then o / rms(o) * w * logistic(gate) leaves in the compute type
 // Prompts run the general kernels of delta_rule.cu on the same state.
 #include <math.h>
@@ -43,6 +44,7 @@ struct ChannelTokenArgs {
   float* gate;                   // [T, ldg]: the output gate before its logistic function (H*Dv)
   long ldg;
   int n_tokens, write_state;
+  int early;                     // the states were complete before the launch ahead began
   int row_blocks;                // blocks of the first two kinds
   int tiles_a, tiles_g;          // 64-wide tiles of the two products
 };
@@ -62,8 +64,8 @@ __device__ __forceinline__ float ct_conv(const ChannelTokenArgs& a, const float*
   return ct_silu(fmaf(cur, w[K - 1], acc));
 }
 
-// The channels base .. base + n - 1 (n at most 128, up to four taps) of a token, four a lane: what the step before left (done: between
-// two steps lies the copy of the index block) and the weights are asked for ahead of the wait (a channel's seven loads one behind the
+// The channels base .. base + n - 1 (n at most 128, up to four taps) of a token, four a lane: what the step before left and the weights
+// are asked for together, with `early` ahead of the wait (a channel's seven loads one behind the
 // other, four channels a lane: 11 us of a step; a request of seven such steps 8.05 -> 7.93 ms).  `y`: their values; the order of a channel's sum is ct_conv's.
 constexpr int CT_FOUR = CT_V_PIECE / 32;
 __device__ __forceinline__ void ct_conv_piece(const ChannelTokenArgs& a, const float* row, float* carry, int base, int n, int Nc, int lane,
@@ -113,6 +115,7 @@ __device__ __forceinline__ void ct_rows(const ChannelTokenArgs& a, int warp_item
   if (seq < 0) return;
   const int slot = a.seq_slot[seq];
   if (slot < 0) return;
+  if (!a.early) pdl_wait();
   const float* row = a.proj + (size_t)t * a.ld;
   float* carry = a.state + (size_t)slot * a.state_floats + (size_t)a.H * a.D * a.Dv;
   float* out = a.prep + (size_t)t * a.ldp;
@@ -272,6 +275,7 @@ struct ChannelStepArgs {
   long ld_out;
   int slices;                    // blocks of a cluster: ceil(Dv / 32)
   int write_state;
+  int early;                     // the states were complete before the launch ahead of this one's began
 };
 
 // LPC lanes share a column (four entries each, NCH times: entries 4 LPC i + 4 sub + 0..3); a pass covers 256 / LPC columns.
@@ -295,6 +299,7 @@ channel_token_step_kernel(const ChannelStepArgs a, T* __restrict__ out) {
   }
   const int sub = threadIdx.x % LPC, cg = threadIdx.x / LPC;
   float* S_g = a.state + (size_t)slot * a.state_floats + ((size_t)h * Dv + slice * CS_COLS) * D;
+  if (!a.early) pdl_wait();
   float4 S[PASSES][NCH];
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -434,12 +439,14 @@ LLMI_EXPORT int llmi_channel_token_supported(int H, int Hk, int D, int Dv, int t
          taps <= CT_MAX_TAPS && rank_a > 0 && rank_g > 0 && rank_a <= 1024 && rank_g <= 1024;
 }
 
+// Both kernels' `early`: the states of the step's sequences were complete before the launch ahead of llmi_channel_token_prepare began (a
+// model's step: the copy of its index block lies between), so that they may be read before the launch ahead has ended.
 // w_a [rank_a, Na], w_g [rank_g, Ng] (dtype's type), Na and Ng = H*D and H*Dv rounded up to 64, zeros behind.
 LLMI_EXPORT int llmi_channel_token_prepare(int dtype, const float* proj, long ld, int H, int Hk, int D, int Dv, int taps, int low_a,
                                            int rank_a, int low_g, int rank_g, const float* conv_w, const float* a_log,
                                            const float* dt_bias, float* state, const int32_t* tok_seq, const int32_t* seq_slot,
                                            const void* w_a, const void* w_g, float* prep, long ldp, float* gate, long ldg,
-                                           int n_tokens, int write_state, cudaStream_t stream) {
+                                           int n_tokens, int write_state, int early, cudaStream_t stream) {
   if (n_tokens <= 0 || !llmi_channel_token_supported(H, Hk, D, Dv, taps, rank_a, rank_g)) return LLMI_ERR_BAD_SIZE;
   if (((uintptr_t)w_a & 7) || ((uintptr_t)w_g & 7)) return LLMI_ERR_ALIGN;
   ChannelTokenArgs a;
@@ -449,7 +456,7 @@ LLMI_EXPORT int llmi_channel_token_prepare(int dtype, const float* proj, long ld
   a.state = state;
   a.state_floats = (long)H * D * Dv + (long)(taps - 1) * (2 * Hk * D + H * Dv);
   a.tok_seq = tok_seq; a.seq_slot = seq_slot; a.prep = prep; a.ldp = ldp; a.gate = gate; a.ldg = ldg;
-  a.n_tokens = n_tokens; a.write_state = write_state;
+  a.n_tokens = n_tokens; a.write_state = write_state; a.early = early;
   const long items = (long)n_tokens * (2 * Hk + (H * Dv + CT_V_PIECE - 1) / CT_V_PIECE + 1);
   if (items > 0x3fffffffL) return LLMI_ERR_BAD_SIZE;
   a.row_blocks = (int)((items + CT_WARPS - 1) / CT_WARPS);
@@ -470,7 +477,8 @@ LLMI_EXPORT int llmi_channel_token_prepare(int dtype, const float* proj, long ld
 
 LLMI_EXPORT int llmi_channel_token_step(int dtype, const float* prep, long ldp, int H, int Hk, int D, int Dv, int taps, float* state,
                                         const int32_t* tok_seq, const int32_t* seq_slot, const float* gate, long ldg, const float* w,
-                                        float eps, void* out, long ld_out, int n_tokens, int write_state, cudaStream_t stream) {
+                                        float eps, void* out, long ld_out, int n_tokens, int write_state, int early,
+                                        cudaStream_t stream) {
   if (n_tokens <= 0 || n_tokens > 65535 || !llmi_channel_token_supported(H, Hk, D, Dv, taps, 1, 1)) return LLMI_ERR_BAD_SIZE;
   ChannelStepArgs a;
   a.prep = prep; a.ldp = ldp; a.H = H; a.Hk = Hk; a.D = D; a.Dv = Dv; a.state = state;
@@ -479,6 +487,7 @@ LLMI_EXPORT int llmi_channel_token_step(int dtype, const float* prep, long ldp, 
   a.tok_seq = tok_seq; a.seq_slot = seq_slot; a.gate = gate; a.ldg = ldg; a.w = w; a.eps = eps; a.ld_out = ld_out;
   a.slices = (Dv + CS_COLS - 1) / CS_COLS;
   a.write_state = write_state;
+  a.early = early;
   if (dtype == LLMI_DTYPE_F32) return launch_channel_step_sizes<float>(a, out, n_tokens, stream);
   if (dtype == LLMI_DTYPE_BF16) return launch_channel_step_sizes<__nv_bfloat16>(a, out, n_tokens, stream);
   return LLMI_ERR_BAD_DTYPE;

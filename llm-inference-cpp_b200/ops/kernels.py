@@ -1787,13 +1787,14 @@ def channel_token_supported(dims, rank_a: int, rank_g: int) -> bool:
 
 def channel_token(proj: torch.Tensor, dims, low_a: tuple, low_g: tuple, conv_w, a_log, dt_bias, w_a: torch.Tensor, w_g: torch.Tensor,
                   state: torch.Tensor, ctx, prep: torch.Tensor, gate: torch.Tensor, weight, eps: float, out: torch.Tensor,
-                  write_state: bool = True) -> None:
+                  write_state: bool = True, early: bool = False) -> None:
     """For a step in which every sequence brings one token, everything between the two products of a gated-delta-rule mixer
     with a decay per key channel and a logistic output gate through low-rank paths (sizes: :func:`channel_token_supported`).
     ``proj`` fp32 rows [q | k | v | b | ...] with the two low-rank vectors at ``low_a`` and ``low_g`` = (first column, size);
     ``w_a`` [rank_a, H*D up to a multiple of 64], ``w_g`` [rank_g, H*Dv likewise]: the paths' second matrices, transposed,
     zeros behind, in out's type.  ``prep`` fp32 [T, >= 2*Hk*D + H*Dv + H*D + H] (row pitch a multiple of four) and ``gate`` fp32
-    [T, H*Dv] are scratch; ``out`` [T, H*Dv] = o / rms(o) * weight * logistic(gate)."""
+    [T, H*Dv] are scratch; ``out`` [T, H*Dv] = o / rms(o) * weight * logistic(gate).  ``early``: the states were complete before the
+    launch ahead began (a model's step: the copy of its index block lies between), so that they may be read before it has ended."""
     _need_cuda(proj, conv_w, a_log, dt_bias, w_a, w_g, state, prep, gate, weight, out)
     H, Hk, D, Dv, taps = dims
     T = proj.shape[0]
@@ -1806,14 +1807,14 @@ def channel_token(proj: torch.Tensor, dims, low_a: tuple, low_g: tuple, conv_w, 
     assert a_log.numel() == H and dt_bias.numel() == H * D and weight.numel() == Dv and out.shape == (T, H * Dv) and out.stride(1) == 1
     assert state.is_contiguous() and state.shape[-1] == delta_state_floats(H, Hk, D, Dv, taps)
     d = (c_int(H), c_int(Hk), c_int(D), c_int(Dv), c_int(taps))
-    l, code, wr = lib(), c_int(_dtype_code(out)), c_int(1 if write_state else 0)
+    l, code, wr, ahead = lib(), c_int(_dtype_code(out)), c_int(1 if write_state else 0), c_int(1 if early else 0)
     _check("channel_token_prepare", l.llmi_channel_token_prepare(
         code, _ptr(proj), c_long(proj.stride(0)), *d, c_int(low_a[0]), c_int(low_a[1]), c_int(low_g[0]), c_int(low_g[1]), _ptr(conv_w),
         _ptr(a_log), _ptr(dt_bias), _ptr(state), _ptr(ctx.tok_seq), _ptr(ctx.seq_slot), _ptr(w_a), _ptr(w_g), _ptr(prep),
-        c_long(prep.stride(0)), _ptr(gate), c_long(gate.stride(0)), c_int(T), wr, _stream()))
+        c_long(prep.stride(0)), _ptr(gate), c_long(gate.stride(0)), c_int(T), wr, ahead, _stream()))
     _check("channel_token_step", l.llmi_channel_token_step(
         code, _ptr(prep), c_long(prep.stride(0)), *d, _ptr(state), _ptr(ctx.tok_seq), _ptr(ctx.seq_slot), _ptr(gate),
-        c_long(gate.stride(0)), _ptr(weight), c_float(eps), _ptr(out), c_long(out.stride(0)), c_int(T), wr, _stream()))
+        c_long(gate.stride(0)), _ptr(weight), c_float(eps), _ptr(out), c_long(out.stride(0)), c_int(T), wr, ahead, _stream()))
 
 
 def _up64(n: int) -> int:

@@ -190,7 +190,8 @@ class ChannelDeltaRule:
         if ctx.decode and self.single:
             gate = rt.scratch("delta_gate", (T, H * Dv), torch.float32)
             kernels.channel_token(proj, self.dims, self.low_a, self.low_g, self.conv_w, self.a_log, self.dt_bias, *self.w_low_t, state,
-                                  ctx, prep, gate, self.w_norm, self.eps, heads, write_state=binding.writes)
+                                  ctx, prep, gate, self.w_norm, self.eps, heads, write_state=binding.writes,
+                                  early=binding.writes)      # (a call on another call's state: that call has just written it)
         else:
             z = self._low_rank(proj, 0, H * D, "delta_z")
             gate = self._low_rank(proj, 1, H * Dv, "delta_gate")

@@ -112,3 +112,41 @@ def test_rows_of_several_maps(Hq, G, maps, dk, dv, window, early):
         kc.copy_(k_full)
         vc.copy_(v_full)
     _check(reset, steps)
+
+
+@pytest.mark.parametrize("dims,ranks", [((4, 2, 64, 64, 4), (16, 24)), ((3, 3, 160, 96, 3), (8, 8)), ((2, 1, 32, 64, 6), (4, 4))])
+@pytest.mark.parametrize("early", [True, False])
+def test_channel_states(dims, ranks, early):
+    """The row that a step works on is still to be written when it starts; without ``early`` so are the carried inputs and the state,
+    which the step before leaves in the same row of launches."""
+    from llmi_b200.ops import kernels
+    torch.manual_seed(dims[2])
+    H, Hk, D, Dv, taps = dims
+    S, n_conv = 5, 2 * Hk * D + H * Dv
+    at, width = n_conv + H, n_conv + H + sum(ranks)
+    full = torch.randn(S, kernels.delta_state_floats(*dims), device="cuda") * 0.1
+    state, conv = torch.empty_like(full), torch.randn(n_conv, taps, device="cuda") * 0.5
+    a_log, dt_bias, weight = torch.randn(H, device="cuda"), torch.randn(H * D, device="cuda"), torch.ones(Dv, device="cuda")
+    w_a, w_g = (torch.randn(r, -(-n // 64) * 64, device="cuda") * r ** -0.5 for r, n in zip(ranks, (H * D, H * Dv)))
+    ctx, eye, steps = _token_ctx([3, 9, 64, 700, 5]), torch.eye(width, device="cuda"), []
+    eye = torch.nn.functional.pad(eye, (0, -width % 4))
+    proj_a = torch.empty(S, width, device="cuda")
+    for _ in range(1 if early else 3):
+        rows = torch.nn.functional.pad(torch.randn(S, width, device="cuda"), (0, -width % 4))
+        proj, gate, out = torch.empty_like(proj_a), torch.empty(S, H * Dv, device="cuda"), torch.empty(S, H * Dv, device="cuda")
+        pitch = n_conv + H * D + H
+        prep = torch.empty(S, pitch + -pitch % 4, device="cuda")
+
+        def step(rows=rows, proj=proj, gate=gate, out=out, prep=prep):
+            kernels.linear_simt(rows, eye, proj)                         # (the rows as they are: the launch ahead)
+            kernels.channel_token(proj, dims, (at, ranks[0]), (at + ranks[0], ranks[1]), conv, a_log, dt_bias, w_a, w_g, state, ctx,
+                                  prep, gate, weight, 1e-5, out, early=early)
+            return out
+        steps.append(step)
+    projs = [s.__defaults__[1] for s in steps]
+
+    def reset():
+        state.copy_(full)
+        for p in projs:
+            p.fill_(float("nan"))
+    _check(reset, steps)
