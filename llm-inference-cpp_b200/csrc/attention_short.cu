@@ -64,6 +64,7 @@ struct ShortParams {
   int n_heads, write_kv;
   __nv_bfloat16* k_cache_w;
   __nv_bfloat16* v_cache_w;
+  int early;                  // rows of earlier steps were complete before the launch ahead began
 };
 
 template <int HD>
@@ -170,7 +171,8 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     for (int i = 0; i < n_pages && ok; ++i) {
       const int s = i % C::STAGES;
       const int page = pages[pg0 + i];
-      if (!waited && !own_row && (pg0 + i + 1) * SH_PAGE > pos0) {      // a page with rows of this step: written by a kernel before
+      // Where rows of earlier steps may be read ahead, only a page with rows of this step, written by a kernel before, waits.
+      if (!waited && (!p.early || (!own_row && (pg0 + i + 1) * SH_PAGE > pos0))) {
         pdl_wait();
         waited = true;
       }
@@ -567,11 +569,13 @@ using namespace llmi;
 // fuse = 1 (max_q 1, groups up to 16): a decode step as for llmi_attention_decode_fused — `q` is the step's un-rotated
 // [q | k | v] rows, rotary_dim is head_dim or 0, the new k (rotated) and v are appended with write_kv.
 // wide = 1 (max_q 1, ungrouped heads of 128): 32-bit weights.
+// early = 1: what earlier steps left of the step's sequences was complete before the launch ahead began (a model's step: the copy of its
+// index block lies between), so that it may be read before that launch has ended.
 LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ldo, void* k_cache, void* v_cache,
                                      long n_cache_pages, const int32_t* seq_pages, int pages_stride, const int32_t* seq_q_start,
                                      const int32_t* seq_kv_len, int n_seqs, int max_q, int n_heads, int n_kv_heads, int head_dim,
                                      float scale, int window, int parts, int fuse, const float* inv_freq, int rotary_dim,
-                                     int write_kv, int wide, int* error_flag, cudaStream_t stream) {
+                                     int write_kv, int wide, int early, int* error_flag, cudaStream_t stream) {
   if (n_seqs <= 0 || max_q <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_cache_pages <= 0) return LLMI_ERR_BAD_SIZE;
   if (n_heads % n_kv_heads || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return LLMI_ERR_BAD_SIZE;
   if (head_dim != 64 && head_dim != 128) return LLMI_ERR_UNSUPPORTED;
@@ -589,7 +593,7 @@ LLMI_EXPORT int llmi_attention_short(const void* q, long ldq, void* out, long ld
   if (rc != LLMI_OK) return rc;
   ShortParams p{(const __nv_bfloat16*)q, ldq, (__nv_bfloat16*)out, ldo, seq_pages, seq_q_start, seq_kv_len, pages_stride, n_kv_heads,
                 group, (int)tiles, scale * 1.4426950408889634f, window, error_flag, inv_freq, fuse ? rotary_dim : 0, n_heads,
-                write_kv ? 1 : 0, fuse ? (__nv_bfloat16*)k_cache : nullptr, fuse ? (__nv_bfloat16*)v_cache : nullptr};
+                write_kv ? 1 : 0, fuse ? (__nv_bfloat16*)k_cache : nullptr, fuse ? (__nv_bfloat16*)v_cache : nullptr, early};
   const int per_tile = (int)(tile_rows < SH_MAX_ROWS ? tile_rows : SH_MAX_ROWS);
   return head_dim == 64 ? sh_launch_rows<64>(mk, mv, p, (int)items, per_tile, parts, wide != 0, stream)
                         : sh_launch_rows<128>(mk, mv, p, (int)items, per_tile, parts, wide != 0, stream);

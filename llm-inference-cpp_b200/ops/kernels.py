@@ -1017,11 +1017,11 @@ def short_message_plan(ctx, n_seqs: int, n_pages: int, n_kv_heads: int, group: i
 
 def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len, max_q: int,
                     n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: int = 0, parts: int = 1, rope=None,
-                    wide: bool = False) -> None:
+                    wide: bool = False, early: bool = False) -> None:
     """Causal attention of at most ``max_q`` tokens a sequence over its cache pages (bf16, head size 64 or 128, page 64):
     arguments as ``attention_prefill``; ``parts`` blocks (1, 2, 4, 8) share the pages of a sequence and kv head.  ``rope``
     (``max_q`` 1): see :func:`attention_decode_mma`.  ``wide`` (``max_q`` 1, ungrouped heads of 128):
-    the weights meet the values as 32-bit numbers."""
+    the weights meet the values as 32-bit numbers.  ``early``: see :func:`attention`."""
     inv_freq, rotary_dim, write_kv = rope if rope is not None else (None, 0, False)
     assert rotary_dim == 0 or (inv_freq is not None and inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2)
     _need_cuda(q, out, k_cache, v_cache, seq_pages, seq_q_start, seq_kv_len)
@@ -1032,7 +1032,7 @@ def attention_short(q: torch.Tensor, out: torch.Tensor, k_cache, v_cache, seq_pa
         _ptr(seq_pages), c_int(seq_pages.stride(0)), _ptr(seq_q_start), _ptr(seq_kv_len), c_int(seq_pages.shape[0]), c_int(max_q),
         c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_float(scale), c_int(window), c_int(parts),
         c_int(0 if rope is None else 1), _ptr(inv_freq) if rotary_dim else None, c_int(rotary_dim), c_int(1 if write_kv else 0),
-        c_int(1 if wide else 0), _ptr(tc_scratch(q.device).error), _stream()))
+        c_int(1 if wide else 0), c_int(1 if early else 0), _ptr(tc_scratch(q.device).error), _stream()))
 
 
 # Which prompt-attention kernel runs: "tc" (tcgen05: about 43 us for a 2,048-token prompt of 32 heads of 64) or
@@ -1080,13 +1080,16 @@ def attention_fuses_rotation(qkv, ctx, seq_pages, page_size, n_heads, n_kv_heads
 
 
 def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_pages, page_size: int, n_heads: int,
-              n_kv_heads: int, head_dim: int, scale: float, window: int = 0, rt=None, rope=None) -> None:
+              n_kv_heads: int, head_dim: int, scale: float, window: int = 0, rt=None, rope=None, early: bool = False) -> None:
     """Attention of a step's tokens over the cache; q is the first n_heads*head_dim columns of ``qkv``.
 
     In bf16, a decode step goes to the split kernel and a prompt step to the flash kernel when they
     have the head size; the 32-bit path has kernels of its own (``attention_f32``); other head sizes go to the generic kernel.
     ``rope=(inv_freq, rotary_dim, write_kv)``: q, k are not rotated yet and k, v not appended — the kernel
     does it (only where :func:`attention_fuses_rotation` says so).
+    ``early``: what earlier steps left of the step's sequences was complete before the launch ahead began (a model's step: the copy
+    of its index block lies between), so that it may be read before that launch has ended.  (The persistent kernels of a decode
+    step, attention_decode and attention_decode_mma, always take that of the pages ahead of the newest.)
     """
     if _decode_kernel_applies(qkv, ctx, seq_pages, page_size, n_heads, n_kv_heads, head_dim, rt):
         S, P = seq_pages.shape
@@ -1095,7 +1098,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
         if parts:
             # (the kernels it stands in for: ungrouped heads have 32-bit weights, grouped ones bf16)
             attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, 1, n_heads, n_kv_heads, head_dim,
-                            scale, window, parts, rope, wide=n_heads == n_kv_heads)
+                            scale, window, parts, rope, wide=n_heads == n_kv_heads, early=early)
             return
         partials = rt.scratch("attn_partials", (attention_decode_workspace(S, n_heads, head_dim, P, pps),), torch.float32)
         if decode_uses_mma(head_dim, n_heads // n_kv_heads):
@@ -1122,7 +1125,7 @@ def attention(qkv: torch.Tensor, out: torch.Tensor, k_cache, v_cache, ctx, seq_p
             short = decide(ctx, short_message_plan, seq_pages.shape[0], seq_pages.shape[1], n_kv_heads, n_heads // n_kv_heads, head_dim, window)
             if short:
                 attention_short(qkv, out, k_cache, v_cache, seq_pages, ctx.seq_q_start, ctx.seq_kv_len, ctx.short_message, n_heads,
-                                n_kv_heads, head_dim, scale, window, short[0])
+                                n_kv_heads, head_dim, scale, window, short[0], early=early)
                 return
             split = None
             q_lens, kv_lens = getattr(ctx, "host_q_lens", None), getattr(ctx, "host_kv_lens", None)

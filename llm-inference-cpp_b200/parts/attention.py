@@ -93,7 +93,7 @@ class GQAttention:
             rope = None
             self.position.rotate_and_store(qkv, ctx, binding, nh, nkv, hd)
         kernels.attention(qkv, attn, g.k[binding.index], g.v[binding.index], ctx, pages, g.page_size,
-                          nh, nkv, hd, self.scale, self.window, rt=self.rt, rope=rope)
+                          nh, nkv, hd, self.scale, self.window, rt=self.rt, rope=rope, early=True)
         return kernels.linear(attn, self.w_o, x, None, kernels.OUT_ADD_F32, then_norm)
 
 

@@ -150,3 +150,42 @@ def test_channel_states(dims, ranks, early):
         for p in projs:
             p.fill_(float("nan"))
     _check(reset, steps)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window", [(9, 3, 64, 0), (15, 5, 64, 70), (16, 4, 128, 0), (8, 8, 128, 0)])
+@pytest.mark.parametrize("early", [True, False])
+def test_step_that_appends_its_own_row(nh, nkv, hd, window, early):
+    """A decode step whose kernel rotates and appends: its projection is still to be written when it starts; without ``early`` so is
+    the row before it."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels
+    rt = Runtime(torch.bfloat16, "cuda")
+    torch.manual_seed(nh + hd)
+    first = POSITIONS[-4:] if nh == nkv else POSITIONS
+    S, P = len(first), 13 if nh == nkv else 6
+    assert kernels.decode_short_parts(S, nkv, P, hd, nh // nkv, window) > 0
+    pages = torch.randperm(S * P, device="cuda").int().view(S, P)
+    k_full, v_full = (torch.randn(S * P, nkv, 64, hd, device="cuda").bfloat16() for _ in range(2))
+    for s, p in enumerate(first):
+        for j in range(p, 64 * P):
+            k_full[pages[s, j // 64], :, j % 64] = v_full[pages[s, j // 64], :, j % 64] = float("nan")
+    kc, vc, inv = torch.empty_like(k_full), torch.empty_like(v_full), torch.rand(hd // 2, device="cuda")
+    steps, projections = [], []
+    for positions in [first] if early else [first, [p + 1 for p in first]]:
+        ctx, rows = _token_ctx(positions), torch.randn(S, (nh + 2 * nkv) * hd, device="cuda")
+        qkv, out = torch.empty(rows.shape, device="cuda").bfloat16(), torch.empty(S, nh * hd, device="cuda").bfloat16()
+        projections.append(qkv)
+
+        def step(ctx=ctx, rows=rows, qkv=qkv, out=out):
+            kernels.cast_rows(rows, qkv)
+            kernels.attention(qkv, out, kc, vc, ctx, pages, 64, nh, nkv, hd, hd ** -0.5, window, rt=rt, rope=(inv, hd, True), early=early)
+            return out
+        steps.append(step)
+
+    def reset():
+        kc.copy_(k_full)
+        vc.copy_(v_full)
+        for p in projections:
+            p.fill_(float("nan"))
+    _check(reset, steps)
+    kernels.check_device_errors("cuda:0")
