@@ -11,15 +11,17 @@
 //                     is written as index -1 (the product kernels skip it) and the token's summed weight of them to
 //                     `id_wt`, for llmi_moe_identity_add
 //   llmi_moe_table    per token: its experts from a table [vocab, top] by the token's id, each weighted 1 / top (no router)
-//   llmi_moe_up       per (token, choice): a = act(Wg_e h) * (Wu_e h), or a = act(Wu_e h) for experts
+//   llmi_moe_streamed per (token, choice): a = act(Wg_e h) * (Wu_e h), or a = act(Wu_e h) for experts
 //                     without a gate matrix                                                  [T, top, F] fp32
-//   llmi_moe_down     per token: y = sum over its choices, in the order of the choice, of weight * (Wd_e a)   [T, W] fp32
-// The two product kernels stream an expert's rows once per (token, choice): the form for a handful of tokens (a
+//                     per token: y = sum over its choices, in the order of the choice, of weight * (Wd_e a)   [T, W] fp32
+// Its two kernels stream an expert's rows once per (token, choice): the form for a handful of tokens (a
 // decode step), where every chosen expert's weights are read once or a few times anyway.  Each output is one
 // warp's sum in a fixed order, so a token's result does not depend on the batch it is in.
 // Weights are stacked by expert: Wg, Wu [E, F, W], Wd [E, W, F], in the compute type; act: 0 silu, 1 tanh-GELU,
 // 2 the square of relu.
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -288,13 +290,13 @@ moe_up_kernel(const T* __restrict__ h, long ldh, const T* __restrict__ wg, const
   if (lane == 0) a[(size_t)item * F + f] = moe_act<ACT>(g) * u;
 }
 
-// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.  `behind_up`: the launch before on the stream is
-// moe_up_kernel with the same idx, whose blocks let this kernel start when the choice and everything before it is done: the
-// first choice's row is then asked for ahead of the wait, and the others' come into L2.
+// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.  The launch before on the stream is moe_up_kernel with the
+// same idx, whose blocks let this kernel start when the choice and everything before it is done: the first choice's row is asked
+// for ahead of the wait, and the others' come into L2.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, int F, int top, const int32_t* __restrict__ idx,
-                const float* __restrict__ wt, float* __restrict__ y, long ldy, int add, int behind_up) {
+                const float* __restrict__ wt, float* __restrict__ y, long ldy, int add) {
   extern __shared__ __align__(16) float a_s[];
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -302,7 +304,7 @@ moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, in
   const int c = blockIdx.y * 8 + warp;
   uint4 raw[MOE_AHEAD];
   bool loaded = false;
-  if (VEC && behind_up && c < W) {
+  if (VEC && c < W) {
     for (int j = 0; j < top; ++j) {
       const int e = idx[(size_t)t * top + j];
       if (e < 0) continue;
@@ -395,7 +397,7 @@ static int launch_moe_up(const void* h, long ldh, const void* wg, const void* wu
 
 template <typename T, bool VEC>
 static int launch_moe_down(const float* a, const void* wd, int W, int F, int top, const int32_t* idx, const float* wt, float* y, long ldy,
-                           int n_tokens, int add, int behind_up, cudaStream_t stream) {
+                           int n_tokens, int add, cudaStream_t stream) {
   const size_t smem = (size_t)top * F * 4;
   static PerDevice<size_t> allowed;
   if (smem > 48 * 1024 && allowed.here() < smem) {
@@ -404,41 +406,40 @@ static int launch_moe_down(const float* a, const void* wd, int W, int F, int top
     allowed.here() = smem;
   }
   return launch_pdl(PDL_GEMM, moe_down_kernel<T, VEC>, dim3(n_tokens, (W + 7) / 8), dim3(256), smem, stream, a, (const T*)wd, W, F, top,
-                    idx, wt, y, ldy, add, behind_up);
+                    idx, wt, y, ldy, add);
 }
 
-LLMI_EXPORT int llmi_moe_up(int dtype, const void* h, long ldh, const void* wg, const void* wu, int W, int F, int top,
-                            const int32_t* idx, float* a, int act, int n_tokens, cudaStream_t stream) {
-  if (n_tokens <= 0 || W <= 0 || F <= 0 || top <= 0 || (size_t)W * 4 > 160 * 1024 || (F + 7) / 8 > 65535) return LLMI_ERR_BAD_SIZE;
+template <typename T>
+static int launch_moe_streamed(const void* h, long ldh, const void* wg, const void* wu, const void* wd, int W, int F, int top, const int32_t* idx,
+                               const float* wt, int act, float* a, float* y, long ldy, int n_tokens, int add, cudaStream_t stream) {
+  const bool vec_up = ((size_t)W * sizeof(T)) % 16 == 0 && !((uintptr_t)wg & 15) && !((uintptr_t)wu & 15);
+  const bool vec_down = ((size_t)F * sizeof(T)) % 16 == 0 && !((uintptr_t)wd & 15);
+  auto up = [&](auto act_c) {
+    constexpr int ACT = decltype(act_c)::value;
+    return vec_up ? launch_moe_up<T, ACT, true>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream)
+                  : launch_moe_up<T, ACT, false>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream);
+  };
+  const int rc = act == 0   ? up(std::integral_constant<int, 0>())
+                 : act == 1 ? up(std::integral_constant<int, 1>())
+                 : act == 2 ? up(std::integral_constant<int, 2>())
+                            : up(std::integral_constant<int, 3>());
+  if (rc != LLMI_OK) return rc;
+  return vec_down ? launch_moe_down<T, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
+                  : launch_moe_down<T, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream);
+}
+
+// Both products, one launch behind the other: moe_down_kernel reads idx ahead of its wait, which only moe_up_kernel directly before it
+// makes sound.  a: [n_tokens, top, F] scratch.
+LLMI_EXPORT int llmi_moe_streamed(int dtype, const void* h, long ldh, const void* wg, const void* wu, const void* wd, int W, int F, int top,
+                                  const int32_t* idx, const float* wt, int act, float* a, float* y, long ldy, int n_tokens, int add,
+                                  cudaStream_t stream) {
+  if (n_tokens <= 0 || W <= 0 || F <= 0 || top <= 0 || (size_t)W * 4 > 160 * 1024 || (size_t)top * F * 4 > 160 * 1024 ||
+      (F + 7) / 8 > 65535 || (W + 7) / 8 > 65535)
+    return LLMI_ERR_BAD_SIZE;
   if (act < 0 || act > 3) return LLMI_ERR_UNSUPPORTED;
-  const int esz = dtype == LLMI_DTYPE_F32 ? 4 : 2;
-  const bool vec = ((size_t)W * esz) % 16 == 0 && !((uintptr_t)wg & 15) && !((uintptr_t)wu & 15);
-#define LLMI_UP(T, ACT) \
-  return vec ? launch_moe_up<T, ACT, true>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream) \
-             : launch_moe_up<T, ACT, false>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream)
-  if (dtype == LLMI_DTYPE_F32) {
-    if (act == 0) LLMI_UP(float, 0); else if (act == 1) LLMI_UP(float, 1); else if (act == 2) LLMI_UP(float, 2); else LLMI_UP(float, 3);
-  }
-  if (dtype == LLMI_DTYPE_BF16) {
-    if (act == 0) LLMI_UP(__nv_bfloat16, 0); else if (act == 1) LLMI_UP(__nv_bfloat16, 1);
-    else if (act == 2) LLMI_UP(__nv_bfloat16, 2); else LLMI_UP(__nv_bfloat16, 3);
-  }
-#undef LLMI_UP
-  return LLMI_ERR_BAD_DTYPE;
-}
-
-// behind_up: the launch before on this stream is llmi_moe_up with this idx (see moe_down_kernel).
-LLMI_EXPORT int llmi_moe_down(int dtype, const float* a, const void* wd, int W, int F, int top, const int32_t* idx,
-                              const float* wt, float* y, long ldy, int n_tokens, int add, int behind_up,
-                              cudaStream_t stream) {
-  if (n_tokens <= 0 || W <= 0 || F <= 0 || top <= 0 || (size_t)top * F * 4 > 160 * 1024 || (W + 7) / 8 > 65535) return LLMI_ERR_BAD_SIZE;
-  const int esz = dtype == LLMI_DTYPE_F32 ? 4 : 2;
-  const bool vec = ((size_t)F * esz) % 16 == 0 && !((uintptr_t)wd & 15);
   if (dtype == LLMI_DTYPE_F32)
-    return vec ? launch_moe_down<float, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream)
-               : launch_moe_down<float, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream);
+    return launch_moe_streamed<float>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return vec ? launch_moe_down<__nv_bfloat16, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream)
-               : launch_moe_down<__nv_bfloat16, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, behind_up, stream);
+    return launch_moe_streamed<__nv_bfloat16>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, stream);
   return LLMI_ERR_BAD_DTYPE;
 }

@@ -160,8 +160,8 @@ def lib():
                      "llmi_sm_count", "llmi_dyt", "llmi_dyt_add", "llmi_stream_add", "llmi_linear_simt_batched",
                      "llmi_attention_expanded",
                      "llmi_attention_expanded_supported", "llmi_latent_expand_prepare", "llmi_latent_prepare", "llmi_latent_q_rotate", "llmi_attention_latent", "llmi_delta_prepare",
-                     "llmi_delta_conv_carry", "llmi_delta_recurrence", "llmi_delta_finish", "llmi_moe_route", "llmi_moe_up",
-                     "llmi_moe_down", "llmi_moe_grouped", "llmi_linear_heads_mma", "llmi_attention_latent_mma", "llmi_attention_latent_mma_supported",
+                     "llmi_delta_conv_carry", "llmi_delta_recurrence", "llmi_delta_finish", "llmi_moe_route", "llmi_moe_streamed",
+                     "llmi_moe_grouped", "llmi_linear_heads_mma", "llmi_attention_latent_mma", "llmi_attention_latent_mma_supported",
                      "llmi_conv_add", "llmi_conv_carry", "llmi_qkv_prepare", "llmi_attention_flex", "llmi_diff_combine",
                      "llmi_gdelta_prepare", "llmi_dplr_recurrence", "llmi_activate", "llmi_attention_maps_mma", "llmi_attention_maps_mma_supported", "llmi_tanh_rows", "llmi_norm_conv_token",
                      "llmi_layernorm", "llmi_depth_mix", "llmi_gate_rows", "llmi_pool_rows", "llmi_mix_layernorm",
@@ -1946,11 +1946,9 @@ def moe_experts_streamed(h: torch.Tensor, w_gate, w_up, w_down, idx, wt, act: in
     assert h.stride(1) == 1 and h.dtype == w_up.dtype == w_down.dtype and (w_gate is None or w_gate.dtype == h.dtype)
     assert (w_gate is None or (w_gate.is_contiguous() and w_gate.shape == w_up.shape)) and w_up.is_contiguous() and w_down.is_contiguous() and w_down.shape == (E, W, F)
     assert a.dtype == torch.float32 and a.is_contiguous() and a.numel() >= T * top * F and y.dtype == torch.float32 and y.stride(1) == 1
-    l = lib()
-    _check("moe_up", l.llmi_moe_up(c_int(_dtype_code(h)), _ptr(h), c_long(h.stride(0)), _ptr(w_gate), _ptr(w_up), c_int(W), c_int(F),
-                                   c_int(top), _ptr(idx), _ptr(a), c_int(act), c_int(T), _stream()))
-    _check("moe_down", l.llmi_moe_down(c_int(_dtype_code(h)), _ptr(a), _ptr(w_down), c_int(W), c_int(F), c_int(top), _ptr(idx),
-                                       _ptr(wt), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0), c_int(1), _stream()))
+    _check("moe_streamed", lib().llmi_moe_streamed(
+        c_int(_dtype_code(h)), _ptr(h), c_long(h.stride(0)), _ptr(w_gate), _ptr(w_up), _ptr(w_down), c_int(W), c_int(F), c_int(top), _ptr(idx),
+        _ptr(wt), c_int(act), _ptr(a), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0), _stream()))
 
 
 MOE_GROUPED_MIN_TOKENS = int(os.environ.get("LLMI_MOE_GROUPED_MIN", "4"))

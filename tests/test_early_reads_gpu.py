@@ -189,3 +189,29 @@ def test_step_that_appends_its_own_row(nh, nkv, hd, window, early):
             p.fill_(float("nan"))
     _check(reset, steps)
     kernels.check_device_errors("cuda:0")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,top", [(1, 1), (3, 2)])
+def test_experts_chosen_by_the_launch_ahead(dtype, T, top):
+    """The down product asks for weights ahead of its wait, by experts that the router has yet to choose when it is launched."""
+    from llmi_b200.ops import kernels
+    torch.manual_seed(T)
+    E, W, F = 16, 512, 256
+    h, wg, wu = torch.randn(T, W, device="cuda").to(dtype), *(torch.randn(E, F, W, device="cuda").to(dtype) for _ in range(2))
+    wd, ctx = torch.randn(E, W, F, device="cuda").to(dtype), _token_ctx(list(range(T)))
+    router, logits = torch.randn(E, W, device="cuda").to(dtype), torch.empty(T, E, device="cuda")
+    idx, wt = torch.empty(T, top, dtype=torch.int32, device="cuda"), torch.empty(T, top, device="cuda")
+    a, y = torch.empty(T, top, F, device="cuda"), torch.empty(T, W, device="cuda")
+
+    def step():
+        kernels.linear_simt(h, router, logits, mode=kernels.OUT_STORE_F32)
+        kernels.moe_route(logits, top, ctx, idx, wt)
+        kernels.moe_experts_streamed(h, wg, wu, wd, idx, wt, kernels.ACT_SILU, a, y)
+        return y
+
+    def reset():                                         # (other experts, whose rows there are)
+        logits.copy_(torch.rand(T, E, device="cuda"))
+        idx.copy_(torch.randint(0, E, (T, top), device="cuda"))
+        wt.fill_(float("nan"))
+    _check(reset, [step])
