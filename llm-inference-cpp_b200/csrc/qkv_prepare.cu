@@ -305,9 +305,9 @@ qkv_prepare_normed_kernel(const float* __restrict__ proj, long ld, int n_q_heads
     const int i = 4 * (threadIdx.x + r * NORMED_THREADS);
     if (i >= n) break;
     float4 y = x[r];
-    if (wn) y = make_float4(w[r].x * (x[r].x * sc), w[r].y * (x[r].y * sc), w[r].z * (x[r].z * sc), w[r].w * (x[r].w * sc));
+    if (wn && seq >= 0) y = make_float4(w[r].x * (x[r].x * sc), w[r].y * (x[r].y * sc), w[r].z * (x[r].z * sc), w[r].w * (x[r].w * sc));
     if (part == 0) {
-      store4(q_out + (size_t)t * ldq + i, y);                    // (zeros for a row of no sequence)
+      store4(q_out + (size_t)t * ldq + i, y);                    // (zeros for a row of no sequence, whatever eps is)
     } else if (seq >= 0) {
       const int size = part == 1 ? dk : dv, hd = i / size, e = i - hd * size;      // (whole fours: within one head)
       if (part == 1) store4(k_cache + kv_row_offset(kp, seq, pos, hd) + e, y);

@@ -72,3 +72,20 @@ def test_norms_over_whole_parts(dtype, nq, nk, dk, nv, dv, v_from_k):
         tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20      # of an entry's own size: the type's rounding, a sum's
         for got, want in ((out, q), (kc, kw), (vc, vw)):
             assert bool(((got.double() - want).abs() <= tol * want.abs()).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norms_without_an_epsilon(dtype):
+    """eps 0: a row of no sequence has no length to divide by and is zeros all the same; the others are normed."""
+    from llmi_b200.ops import kernels
+    torch.manual_seed(2)
+    T, nq, nk, d = 3, 4, 2, 64
+    proj, wq, wk = torch.randn(T, (nq + 2 * nk) * d, device="cuda"), torch.ones(nq * d, device="cuda"), torch.ones(nk * d, device="cuda")
+    kc, vc = (torch.zeros(2, nk, 64, d, dtype=dtype, device="cuda") for _ in range(2))
+    out, pages = torch.full((T, nq * d), 7.0, dtype=dtype, device="cuda"), torch.tensor([[0], [1]], dtype=torch.int32, device="cuda")
+    kernels.qkv_prepare(proj, nq, nk, d, nk, d, wq, wk, 0.0, None, 0, _ctx([0, -1, 1], [3, 0, 5]), pages, 64, kc, vc, out)
+    q = proj[:, :nq * d].double()
+    want = q / torch.sqrt((q * q).mean(-1, keepdim=True))
+    want[1] = 0
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20         # the type's rounding, a sum's
+    assert bool(((out.double() - want).abs() <= tol * want.abs()).all())
