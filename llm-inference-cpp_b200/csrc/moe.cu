@@ -201,13 +201,17 @@ template <> struct Vec16<float> {
 // Where entry i of the vector lies in shared memory.  A lane reads N neighbouring entries, 16 bytes at a time; for bf16 rows
 // (N = 8) the fours with even numbers lie in the first half of the buffer and the odd ones in the second, so that the 32 lanes
 // of one read touch 512 neighbouring bytes (in their own order two lanes in eight meet in every bank).
-template <typename T, bool VEC>
+template <typename T, bool AHEAD>
 __device__ __forceinline__ int moe_place(int i, int K) {
-  if (!VEC || Vec16<T>::N == 4) return i;
+  if (!AHEAD || Vec16<T>::N == 4) return i;
   return (i & 4) * (K >> 3) + ((i >> 3) << 2) + (i & 3);
 }
 
-constexpr int MOE_AHEAD = 8;             // loads a lane has in flight: 4 KB of a row per warp
+// Loads a lane has in flight: 4 KB of a row per warp.  What bounds a handful of tokens is the latency of the rows' loads (two tokens of two
+// experts, 2,048 x 2,048, bf16: 68 us one load behind the other, 25 so).  With more tokens other blocks cover it, and the
+// registers of the loads cost blocks: 128 tokens of four experts in fp32, 256 x 128, 42 us one behind the other, 70 so.  The
+// caller says which form (ops/kernels.py, moe_streamed_ahead).
+constexpr int MOE_AHEAD = 8;
 // Pieces i0, i0 + 32 N, ... of a row; a lane past the row's end reads nothing.
 template <typename T>
 __device__ __forceinline__ void moe_load_row(const T* __restrict__ row, int i0, int K, uint4 (&raw)[MOE_AHEAD]) {
@@ -237,19 +241,26 @@ __device__ __forceinline__ void moe_add_row(const float* __restrict__ x_s, int i
   }
 }
 
-// VEC: rows are 16-byte aligned and a multiple of 16 bytes long.  The order of a row's additions is fixed by (K, VEC).  What
-// bounds these kernels is the latency of the rows' loads: a lane asks for MOE_AHEAD pieces before it uses the first.
-// `raw` holds the row's first pieces already where `loaded` says so.
-template <typename T, bool VEC>
+// VEC: rows are 16-byte aligned and a multiple of 16 bytes long.  The order of a row's additions is fixed by (K, VEC).  AHEAD (with
+// VEC): a lane asks for MOE_AHEAD pieces before it uses the first; `raw` holds the row's first pieces already where `loaded` says so.
+template <typename T, bool VEC, bool AHEAD>
 __device__ __forceinline__ float warp_dot(const float* __restrict__ x_s, const T* __restrict__ row, int K, int lane,
                                           uint4 (&raw)[MOE_AHEAD], bool loaded) {
   float acc = 0.f;
-  if (VEC) {
+  if (AHEAD) {
     constexpr int N = Vec16<T>::N;
     for (int i = lane * N; i < K; i += 32 * N * MOE_AHEAD) {
       if (!loaded) moe_load_row(row, i, K, raw);
       loaded = false;
       moe_add_row<T>(x_s, i, K, raw, acc);
+    }
+  } else if (VEC) {
+    constexpr int N = Vec16<T>::N;
+    for (int i = lane * N; i < K; i += 32 * N) {
+      float v[N];
+      Vec16<T>::expand(*reinterpret_cast<const uint4*>(row + i), v);
+#pragma unroll
+      for (int e = 0; e < N; ++e) acc = fmaf(x_s[i + e], v[e], acc);
     }
   } else {
     for (int i = lane; i < K; i += 32) acc = fmaf(x_s[i], to_f32(row[i]), acc);
@@ -258,14 +269,15 @@ __device__ __forceinline__ float warp_dot(const float* __restrict__ x_s, const T
 }
 
 // grid (T * top, ceil(F / 8)); 8 warps, one output f per warp.  wg null: experts without a gate matrix, a = act(Wu h).
-template <typename T, int ACT, bool VEC>
+template <typename T, int ACT, bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(256)
 moe_up_kernel(const T* __restrict__ h, long ldh, const T* __restrict__ wg, const T* __restrict__ wu, int W, int F, int top,
-              const int32_t* __restrict__ idx, float* __restrict__ a) {
+              const int32_t* __restrict__ idx, float* __restrict__ a, int down_ahead) {
   extern __shared__ __align__(16) float h_s[];
+  if (!down_ahead) pdl_launch_dependents();
   pdl_wait();
-  // Only behind the wait: moe_down, which may start from here on, then knows that the experts have been chosen.
-  pdl_launch_dependents();
+  // (moe_down with loads ahead of its wait: only here, so that it knows that the experts have been chosen when it starts)
+  if (down_ahead) pdl_launch_dependents();
   const int item = blockIdx.x, t = item / top;
   const int e = idx[item];
   if (e < 0) return;
@@ -274,26 +286,26 @@ moe_up_kernel(const T* __restrict__ h, long ldh, const T* __restrict__ wg, const
   const T* row_u = wu + ((size_t)e * F + f) * W;
   const T* row_g = wg ? wg + ((size_t)e * F + f) * W : nullptr;
   uint4 raw_u[MOE_AHEAD], raw_g[MOE_AHEAD];
-  if (VEC && f < F) {
+  if (AHEAD && f < F) {
     moe_load_row(row_u, lane * Vec16<T>::N, W, raw_u);
     if (row_g) moe_load_row(row_g, lane * Vec16<T>::N, W, raw_g);
   }
-  for (int i = threadIdx.x; i < W; i += blockDim.x) h_s[moe_place<T, VEC>(i, W)] = to_f32(h[(size_t)t * ldh + i]);
+  for (int i = threadIdx.x; i < W; i += blockDim.x) h_s[moe_place<T, AHEAD>(i, W)] = to_f32(h[(size_t)t * ldh + i]);
   __syncthreads();
   if (f >= F) return;
-  const float u = warp_dot<T, VEC>(h_s, row_u, W, lane, raw_u, true);
+  const float u = warp_dot<T, VEC, AHEAD>(h_s, row_u, W, lane, raw_u, true);
   if (wg == nullptr) {
     if (lane == 0) a[(size_t)item * F + f] = moe_act<ACT>(u);
     return;
   }
-  const float g = warp_dot<T, VEC>(h_s, row_g, W, lane, raw_g, true);
+  const float g = warp_dot<T, VEC, AHEAD>(h_s, row_g, W, lane, raw_g, true);
   if (lane == 0) a[(size_t)item * F + f] = moe_act<ACT>(g) * u;
 }
 
-// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.  The launch before on the stream is moe_up_kernel with the
-// same idx, whose blocks let this kernel start when the choice and everything before it is done: the first choice's row is asked
-// for ahead of the wait, and the others' come into L2.
-template <typename T, bool VEC>
+// grid (T, ceil(W / 8)); the token's activations [top, F] in shared memory.  AHEAD (with VEC): the launch before on the stream is
+// moe_up_kernel with the same idx and `down_ahead`, whose blocks let this kernel start when the choice and everything before it is
+// done: the first choice's row is asked for ahead of the wait, and the others' come into L2.
+template <typename T, bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(256)
 moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, int F, int top, const int32_t* __restrict__ idx,
                 const float* __restrict__ wt, float* __restrict__ y, long ldy, int add) {
@@ -304,7 +316,7 @@ moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, in
   const int c = blockIdx.y * 8 + warp;
   uint4 raw[MOE_AHEAD];
   bool loaded = false;
-  if (VEC && c < W) {
+  if (AHEAD && c < W) {
     for (int j = 0; j < top; ++j) {
       const int e = idx[(size_t)t * top + j];
       if (e < 0) continue;
@@ -319,15 +331,17 @@ moe_down_kernel(const float* __restrict__ a, const T* __restrict__ wd, int W, in
     }
   }
   pdl_wait();
-  for (int j = 0; j < top; ++j)
-    for (int i = threadIdx.x; i < F; i += blockDim.x) a_s[j * F + moe_place<T, VEC>(i, F)] = a[((size_t)t * top + j) * F + i];
+  for (int i = threadIdx.x; i < top * F; i += blockDim.x) {
+    const int j = AHEAD ? i / F : 0;                             // (all choices in one loop: their loads side by side)
+    a_s[j * F + moe_place<T, AHEAD>(i - j * F, F)] = a[(size_t)t * top * F + i];
+  }
   __syncthreads();
   if (c >= W) return;
   float total = 0.f;
   for (int j = 0; j < top; ++j) {
     const int e = idx[(size_t)t * top + j];
     if (e < 0) continue;
-    const float s = warp_dot<T, VEC>(a_s + (size_t)j * F, wd + ((size_t)e * W + c) * F, F, lane, raw, loaded && j == 0);
+    const float s = warp_dot<T, VEC, AHEAD>(a_s + (size_t)j * F, wd + ((size_t)e * W + c) * F, F, lane, raw, loaded && j == 0);
     total = fmaf(wt[(size_t)t * top + j], s, total);
   }
   if (lane == 0) y[(size_t)t * ldy + c] = add ? y[(size_t)t * ldy + c] + total : total;
@@ -381,65 +395,69 @@ LLMI_EXPORT int llmi_moe_identity_add(int dtype, const void* h, long ldh, const 
   return LLMI_ERR_BAD_DTYPE;
 }
 
-template <typename T, int ACT, bool VEC>
+template <typename T, int ACT, bool VEC, bool AHEAD>
 static int launch_moe_up(const void* h, long ldh, const void* wg, const void* wu, int W, int F, int top, const int32_t* idx, float* a,
-                         int n_tokens, cudaStream_t stream) {
+                         int n_tokens, int down_ahead, cudaStream_t stream) {
   const size_t smem = (size_t)W * 4;
   static PerDevice<size_t> allowed;
   if (smem > 48 * 1024 && allowed.here() < smem) {
-    if (cudaFuncSetAttribute(moe_up_kernel<T, ACT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(moe_up_kernel<T, ACT, VEC, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return LLMI_ERR_BAD_SIZE;
     allowed.here() = smem;
   }
-  return launch_pdl(PDL_GEMM, moe_up_kernel<T, ACT, VEC>, dim3(n_tokens * top, (F + 7) / 8), dim3(256), smem, stream, (const T*)h, ldh,
-                    (const T*)wg, (const T*)wu, W, F, top, idx, a);
+  return launch_pdl(PDL_GEMM, moe_up_kernel<T, ACT, VEC, AHEAD>, dim3(n_tokens * top, (F + 7) / 8), dim3(256), smem, stream, (const T*)h, ldh,
+                    (const T*)wg, (const T*)wu, W, F, top, idx, a, down_ahead);
 }
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, bool AHEAD>
 static int launch_moe_down(const float* a, const void* wd, int W, int F, int top, const int32_t* idx, const float* wt, float* y, long ldy,
                            int n_tokens, int add, cudaStream_t stream) {
   const size_t smem = (size_t)top * F * 4;
   static PerDevice<size_t> allowed;
   if (smem > 48 * 1024 && allowed.here() < smem) {
-    if (cudaFuncSetAttribute(moe_down_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(moe_down_kernel<T, VEC, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return LLMI_ERR_BAD_SIZE;
     allowed.here() = smem;
   }
-  return launch_pdl(PDL_GEMM, moe_down_kernel<T, VEC>, dim3(n_tokens, (W + 7) / 8), dim3(256), smem, stream, a, (const T*)wd, W, F, top,
+  return launch_pdl(PDL_GEMM, moe_down_kernel<T, VEC, AHEAD>, dim3(n_tokens, (W + 7) / 8), dim3(256), smem, stream, a, (const T*)wd, W, F, top,
                     idx, wt, y, ldy, add);
 }
 
 template <typename T>
 static int launch_moe_streamed(const void* h, long ldh, const void* wg, const void* wu, const void* wd, int W, int F, int top, const int32_t* idx,
-                               const float* wt, int act, float* a, float* y, long ldy, int n_tokens, int add, cudaStream_t stream) {
+                               const float* wt, int act, float* a, float* y, long ldy, int n_tokens, int add, int ahead, cudaStream_t stream) {
   const bool vec_up = ((size_t)W * sizeof(T)) % 16 == 0 && !((uintptr_t)wg & 15) && !((uintptr_t)wu & 15);
   const bool vec_down = ((size_t)F * sizeof(T)) % 16 == 0 && !((uintptr_t)wd & 15);
+  const bool up_ahead = vec_up && (ahead & 1), down_ahead = vec_down && (ahead & 2);
   auto up = [&](auto act_c) {
     constexpr int ACT = decltype(act_c)::value;
-    return vec_up ? launch_moe_up<T, ACT, true>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream)
-                  : launch_moe_up<T, ACT, false>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, stream);
+    return up_ahead ? launch_moe_up<T, ACT, true, true>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, down_ahead, stream)
+           : vec_up ? launch_moe_up<T, ACT, true, false>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, down_ahead, stream)
+                    : launch_moe_up<T, ACT, false, false>(h, ldh, wg, wu, W, F, top, idx, a, n_tokens, down_ahead, stream);
   };
   const int rc = act == 0   ? up(std::integral_constant<int, 0>())
                  : act == 1 ? up(std::integral_constant<int, 1>())
                  : act == 2 ? up(std::integral_constant<int, 2>())
                             : up(std::integral_constant<int, 3>());
   if (rc != LLMI_OK) return rc;
-  return vec_down ? launch_moe_down<T, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
-                  : launch_moe_down<T, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream);
+  return down_ahead ? launch_moe_down<T, true, true>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
+         : vec_down ? launch_moe_down<T, true, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream)
+                    : launch_moe_down<T, false, false>(a, wd, W, F, top, idx, wt, y, ldy, n_tokens, add, stream);
 }
 
-// Both products, one launch behind the other: moe_down_kernel reads idx ahead of its wait, which only moe_up_kernel directly before it
-// makes sound.  a: [n_tokens, top, F] scratch.
+// Both products, one launch behind the other: moe_down_kernel may read idx ahead of its wait, which only moe_up_kernel directly before it
+// makes sound.  a: [n_tokens, top, F] scratch.  ahead: which of them ask for their rows ahead (1 the first, 2 the second; rows that
+// 16-byte loads do not take never do; the same bits in every form).
 LLMI_EXPORT int llmi_moe_streamed(int dtype, const void* h, long ldh, const void* wg, const void* wu, const void* wd, int W, int F, int top,
                                   const int32_t* idx, const float* wt, int act, float* a, float* y, long ldy, int n_tokens, int add,
-                                  cudaStream_t stream) {
+                                  int ahead, cudaStream_t stream) {
   if (n_tokens <= 0 || W <= 0 || F <= 0 || top <= 0 || (size_t)W * 4 > 160 * 1024 || (size_t)top * F * 4 > 160 * 1024 ||
       (F + 7) / 8 > 65535 || (W + 7) / 8 > 65535)
     return LLMI_ERR_BAD_SIZE;
   if (act < 0 || act > 3) return LLMI_ERR_UNSUPPORTED;
   if (dtype == LLMI_DTYPE_F32)
-    return launch_moe_streamed<float>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, stream);
+    return launch_moe_streamed<float>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, ahead, stream);
   if (dtype == LLMI_DTYPE_BF16)
-    return launch_moe_streamed<__nv_bfloat16>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, stream);
+    return launch_moe_streamed<__nv_bfloat16>(h, ldh, wg, wu, wd, W, F, top, idx, wt, act, a, y, ldy, n_tokens, add, ahead, stream);
   return LLMI_ERR_BAD_DTYPE;
 }

@@ -1934,6 +1934,18 @@ def moe_identity_add(h: torch.Tensor, id_wt: torch.Tensor, y: torch.Tensor) -> N
                                                            c_long(y.stride(0)), c_int(W), c_int(T), _stream()))
 
 
+def moe_streamed_ahead(n_tokens: int, W: int, F: int, size: int) -> int:
+    """Which products of :func:`moe_experts_streamed` ask for their rows ahead (1: gate and up, rows of ``W`` entries of ``size`` bytes;
+    2: down, rows of ``F``).  One load behind the other / ahead (us, both products; tokens, experts of each, type, W x F): 1, 2, bf16,
+    2,048 x 2,048 64 / 20; 3, 4, bf16, 512 x 512 32 / 13; 6, 2, fp32, 1,024 x 1,024 27 / 25.  Rows of less than 512 bytes are one load a
+    lane or none (3, 4, bf16, 64 x 64 6.5 / 7.3), short ones beside many rows (6, 8, fp32, 2,048 x 128) 32 / 46, and from 7 tokens on
+    (9 where the second product's rows are the longer part) other blocks cover a load's latency: 32, 2, fp32, 512 x 512 32 / 39.
+    Of 1,287 layouts of 1 to 256 tokens 8 take 5 to 12 % longer by this rule than one behind the other, and all of them 18 % less."""
+    if n_tokens > (8 if F * size >= 2048 and F >= W else 6) or F * size < 512 or (F * size < 1024 and W > 4 * F):
+        return 0
+    return 3 if W * size >= 1024 else 2
+
+
 def moe_experts_streamed(h: torch.Tensor, w_gate, w_up, w_down, idx, wt, act: int, a: torch.Tensor, y: torch.Tensor,
                          add: bool = False) -> None:
     """y = sum over each token's choices of wt * down_e(act(gate_e h) * up_e h); the weight-streaming form.
@@ -1948,7 +1960,8 @@ def moe_experts_streamed(h: torch.Tensor, w_gate, w_up, w_down, idx, wt, act: in
     assert a.dtype == torch.float32 and a.is_contiguous() and a.numel() >= T * top * F and y.dtype == torch.float32 and y.stride(1) == 1
     _check("moe_streamed", lib().llmi_moe_streamed(
         c_int(_dtype_code(h)), _ptr(h), c_long(h.stride(0)), _ptr(w_gate), _ptr(w_up), _ptr(w_down), c_int(W), c_int(F), c_int(top), _ptr(idx),
-        _ptr(wt), c_int(act), _ptr(a), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0), _stream()))
+        _ptr(wt), c_int(act), _ptr(a), _ptr(y), c_long(y.stride(0)), c_int(T), c_int(1 if add else 0),
+        c_int(moe_streamed_ahead(T, W, F, h.element_size())), _stream()))
 
 
 MOE_GROUPED_MIN_TOKENS = int(os.environ.get("LLMI_MOE_GROUPED_MIN", "4"))

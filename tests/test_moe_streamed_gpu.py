@@ -50,3 +50,70 @@ def test_streamed_experts(dtype, W, F, top, gated):
     y, a = torch.full((T, W), float("nan"), device="cuda"), torch.empty(T, top, F, device="cuda")
     kernels.moe_experts_streamed(h, wg, wu, wd, idx, wt, act, a, y)
     assert float((y.double() + start.double() - exact).abs().max()) <= bound * float((size + exact.abs()).max()) and float(y[1].abs().max()) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("W,F", [(64, 64), (256, 128), (2048, 128), (512, 512), (1024, 256), (128, 520)])
+def test_forms_agree(dtype, W, F):
+    """A token's result bit for bit, whichever product asks for its rows ahead, alone, among six tokens and among eight."""
+    from llmi_b200.ops import kernels
+    T, E, top = 8, 6, 3
+    gen = torch.Generator(device="cuda").manual_seed(W + F)
+    h = torch.randn(T, W, generator=gen, device="cuda").to(dtype)
+    wg, wu = ((torch.randn(E, F, W, generator=gen, device="cuda") * W ** -0.5).to(dtype) for _ in range(2))
+    wd = (torch.randn(E, W, F, generator=gen, device="cuda") * F ** -0.5).to(dtype)
+    idx = torch.stack([torch.randperm(E, generator=gen, device="cuda")[:top] for _ in range(T)]).to(torch.int32).contiguous()
+    idx[4], idx[5, 1] = -1, -1
+    wt = torch.rand(T, top, generator=gen, device="cuda")
+
+    def run(lo, hi):
+        y, a = torch.empty(hi - lo, W, device="cuda"), torch.empty(hi - lo, top, F, device="cuda")
+        kernels.moe_experts_streamed(h[lo:hi], wg, wu, wd, idx[lo:hi], wt[lo:hi], kernels.ACT_SILU, a, y)
+        return y
+    want = run(0, T)
+    assert torch.equal(run(0, 6), want[:6]) and all(torch.equal(run(t, t + 1), want[t:t + 1]) for t in range(T))
+    rule = kernels.moe_streamed_ahead
+    try:
+        for form in range(4):
+            kernels.moe_streamed_ahead = lambda *sizes, form=form: form
+            assert torch.equal(run(0, T), want)
+    finally:
+        kernels.moe_streamed_ahead = rule
+
+
+@pytest.mark.parametrize("dtype,T,W,F,top", [(torch.float32, 256, 256, 128, 4), (torch.float32, 128, 64, 64, 2), (torch.float32, 128, 1024, 512, 2),
+                                             (torch.bfloat16, 3, 64, 64, 4)])
+def test_many_tokens_and_short_rows_are_no_slower_than_one_load_behind_the_other(dtype, T, W, F, top):
+    """(They took 1.1 to 2 times as long with their rows asked for ahead.)"""
+    from llmi_b200.ops import kernels
+    E = 16
+    h, wd = torch.randn(T, W, device="cuda").to(dtype), torch.randn(E, W, F, device="cuda").to(dtype)
+    wg, wu = (torch.randn(E, F, W, device="cuda").to(dtype) for _ in range(2))
+    idx = torch.stack([torch.randperm(E, device="cuda")[:top] for _ in range(T)]).to(torch.int32).contiguous()
+    wt, a, y = torch.rand(T, top, device="cuda"), torch.empty(T, top, F, device="cuda"), torch.empty(T, W, device="cuda")
+
+    def us():
+        side, graph, times = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+        run = lambda: kernels.moe_experts_streamed(h, wg, wu, wd, idx, wt, kernels.ACT_SILU, a, y)      # noqa: E731
+        with torch.cuda.stream(side):
+            run()
+            side.synchronize()
+            with torch.cuda.graph(graph, stream=side):
+                for _ in range(20):
+                    run()
+        for _ in range(9):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+    rule = kernels.moe_streamed_ahead
+    mine = us()
+    try:
+        kernels.moe_streamed_ahead = lambda *sizes: 0
+        plain = us()
+    finally:
+        kernels.moe_streamed_ahead = rule
+    assert mine < 1.08 * plain
