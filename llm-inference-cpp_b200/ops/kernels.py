@@ -1491,21 +1491,35 @@ def stream_add(x: torch.Tensor, add: torch.Tensor | None, vec: torch.Tensor | No
 HEADS_MMA_MIN_TOKENS = int(os.environ.get("LLMI_HEADS_MMA_MIN", "1"))      # from here on the per-head products of a step run on the tensor cores (bf16)
 
 
-# Up to here the per-head products of a step go to the kernel that is the latency of its loads, beyond to the tensor cores.
 HEADS_TOKEN_MAX = 8
+HEADS_LAUNCH_US = 1.9       # the rotation's launch, which heads_token does without (see latent_query)
 
 
-def heads_token_applies(x: torch.Tensor, bx: int, w: torch.Tensor, K: int) -> bool:
-    return bool(x.dtype == torch.bfloat16 and x.shape[0] <= HEADS_TOKEN_MAX and not _FORCE_SIMT and lib().llmi_heads_token_supported(c_int(K))
-                and bx % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+def heads_token_faster(n_tokens: int, batch: int, N: int, K: int, saved: float = 0.0) -> bool:
+    """Whether ``batch`` per-head products x [n_tokens, K] . w [N, K]^T take less on the kernel that is the latency of its loads
+    (heads_token) than as tensor-core tiles (``saved``: us of another launch that the kernel does without).  The first costs a token its multiplications on the CUDA cores (16 x 512 x 128, 1 / 2 / 4 / 8
+    tokens: 1.5 / 2.0 / 2.4 / 3.7 us), the second a walk over K and tiles of 64 outputs, whatever the tokens (2.4 us; K = 64 2.0,
+    256 3.1, 512 4.7, 1,024 7.9).  Fitted to 27 layouts of 3 to 128 heads at 1 to 8 tokens (tiles / kernel, us): 16 x 128 x
+    512, 8 tokens 4.7 / 4.3; 32 x 512 x 128, 2 2.8 / 2.4, 4 2.8 / 3.4; 128 x 512 x 128, 2 7.0 / 5.6, 8 7.2 / 11.1.  By this choice none takes
+    4 % longer than as tiles; all of them together take 25 % less, with the kernel for all up to 8 tokens 17 %."""
+    entries = batch * N * K
+    kernel = n_tokens * (0.2 + (0.3e-6 if K > 1024 else 0.2e-6) * entries)
+    tiles = 0.35 + 0.0055 * K + 0.25e-6 * entries + 50e-6 * max(0, batch * N - 30000)      # (both without what they have in common)
+    return n_tokens <= HEADS_TOKEN_MAX and kernel < tiles + saved
+
+
+def heads_token_applies(x: torch.Tensor, bx: int, w: torch.Tensor, K: int, saved: float = 0.0) -> bool:
+    return bool(x.dtype == torch.bfloat16 and heads_token_faster(x.shape[0], w.shape[0], w.shape[1], K, saved) and not _FORCE_SIMT
+                and lib().llmi_heads_token_supported(c_int(K)) and bx % 8 == 0 and x.stride(0) % 8 == 0
+                and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def linear_batched(x: torch.Tensor, bx: int, w: torch.Tensor, out: torch.Tensor, by: int, K: int, mode: int = OUT_STORE,
                    early: bool = False) -> None:
     """``w.shape[0]`` products in one launch (one per head): out_b (mode) x_b . w[b]^T with x_b = x[:, b*bx : b*bx + K] and
-    out_b = out[:, b*by : b*by + N]; w [batch, N, K] contiguous.  fp32 FMA arithmetic for the 32-bit path and for a
-    handful of rows; bf16 products of more rows run as tensor-core tiles (bf16 in, fp32 accumulation).  ``early``: see
-    :func:`linear_simt`."""
+    out_b = out[:, b*by : b*by + N]; w [batch, N, K] contiguous.  fp32 FMA arithmetic for the 32-bit path and, in
+    bf16, for the few rows with which that is the faster one (:func:`heads_token_faster`); other bf16 products run as tensor-core
+    tiles (bf16 in, fp32 accumulation).  ``early``: see :func:`linear_simt`."""
     _need_cuda(x, w, out)
     B, N, Kw = w.shape
     M = x.shape[0]
@@ -1587,9 +1601,10 @@ def latent_q_rotate(q: torch.Tensor, D: int, qa: torch.Tensor, C: int, R: int, H
 def latent_query(q: torch.Tensor, D: int, w_uk_t: torch.Tensor, qa: torch.Tensor, C: int, R: int, H: int, inv_freq, rot_dims: int, ctx,
                  pairing: int = 1, amplitude: float = 1.0) -> None:
     """Every head's query as the latent rows are scored with: [q[:, h, :D] . w_uk_t[h]^T (C) | q[:, h, D:] rotated (R)] into qa
-    [T, H*(C+R)]: :func:`linear_batched` (with a model's weights) and :func:`latent_q_rotate`, for a few tokens in one launch."""
+    [T, H*(C+R)]: :func:`linear_batched` (with a model's weights) and :func:`latent_q_rotate`, for a few tokens in one launch (16 heads of
+    128, rank 512, two launches / one: 1 token 4.1 / 1.8 us, 4 4.1 / 2.7, 7 4.4 / 4.0; 128 heads, 4 9.6 / 7.5, 8 10.0 / 11.7)."""
     assert w_uk_t.shape == (H, C, D) and w_uk_t.is_contiguous() and q.dtype == qa.dtype == w_uk_t.dtype
-    if not R or not heads_token_applies(q, D + R, w_uk_t, D):
+    if not R or not heads_token_applies(q, D + R, w_uk_t, D, HEADS_LAUNCH_US):
         linear_batched(q, D + R, w_uk_t, qa, C + R, D, early=True)
         latent_q_rotate(q, D, qa, C, R, H, inv_freq, rot_dims, ctx, pairing, amplitude)
         return
