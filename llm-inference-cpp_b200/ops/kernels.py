@@ -1488,10 +1488,10 @@ def stream_add(x: torch.Tensor, add: torch.Tensor | None, vec: torch.Tensor | No
     _check("stream_add", lib().llmi_stream_add(_ptr(x), _ptr(add), _ptr(vec), c_int(T), c_int(W), _stream()))
 
 
-HEADS_MMA_MIN_TOKENS = int(os.environ.get("LLMI_HEADS_MMA_MIN", "1"))      # from here on the per-head products of a step run on the tensor cores (bf16)
-
-
-HEADS_TOKEN_MAX = 8
+# LLMI_HEADS_MMA_MIN=n: from n tokens on the per-head products of a step run on the tensor cores (bf16), fewer in fp32 FMA arithmetic
+# (linear_simt.cu).  Without it all of them run on the tensor cores but those that heads_token_faster gives to heads_token.
+HEADS_MMA_MIN_TOKENS = int(os.environ.get("LLMI_HEADS_MMA_MIN", "1"))
+HEADS_TOKEN_MAX = 0 if "LLMI_HEADS_MMA_MIN" in os.environ else 8
 HEADS_LAUNCH_US = 1.9       # the rotation's launch, which heads_token does without (see latent_query)
 
 
