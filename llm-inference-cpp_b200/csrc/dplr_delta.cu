@@ -471,7 +471,11 @@ LLMI_EXPORT int llmi_gdelta_prepare(const float* proj, long ld, int H, int D, in
                                     long ldz, const float* w0, const float* a_bias, const int32_t* tok_seq, float* prep, long ldp,
                                     int n_tokens, cudaStream_t stream) {
   if (n_tokens <= 0 || H <= 0 || H > 65535 || D <= 0 || Dv <= 0 || R <= 0 || R > 8192) return LLMI_ERR_BAD_SIZE;
-  if (ld % 4 == 0 && ldp % 4 == 0 && ldz % 4 == 0 && Dv % 4 == 0 && !((uintptr_t)proj & 15) && !((uintptr_t)prep & 15) && !((uintptr_t)z & 15) &&
+  // Four entries a thread: always behind a product.  Walking W2's rows it pays a barrier and its segments' sum, and blocks of 128 threads
+  // of many registers; the general form walks all R rows one behind the other.  R rows, blocks: general / fours, us: 16, 64 2.9 /
+  // 2.8; 16, 256 3.0 / 3.5; 32, 256 3.4 / 3.4; 64, 512 4.6 / 3.8; 64, 1,024 5.4 / 6.0; 128, 1,024 8.3 / 6.4; 128, 2 6.4 / 2.7; 8, 128 2.6 / 2.9.
+  const bool fours = z || (long)n_tokens * H <= 16L * R - 192;
+  if (fours && ld % 4 == 0 && ldp % 4 == 0 && ldz % 4 == 0 && Dv % 4 == 0 && !((uintptr_t)proj & 15) && !((uintptr_t)prep & 15) && !((uintptr_t)z & 15) &&
       !((uintptr_t)w2t & 15) && !((uintptr_t)w0 & 15) && !((uintptr_t)a_bias & 15)) {
     if (D == 32) return launch_gdelta_fours<32>(proj, ld, H, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp, n_tokens, stream);
     if (D == 64) return launch_gdelta_fours<64>(proj, ld, H, Dv, R, w2t, z, ldz, w0, a_bias, tok_seq, prep, ldp, n_tokens, stream);
