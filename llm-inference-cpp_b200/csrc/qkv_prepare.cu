@@ -451,7 +451,12 @@ LLMI_EXPORT int llmi_qkv_prepare(int dtype, const float* proj, long ld, int n_q_
     return LLMI_ERR_BAD_DTYPE;
   }
   const long nq = (long)n_q_heads * dk, nk = has_kv ? (long)n_k_heads * dk : 0, nv = has_kv ? (long)n_v_heads * dv : 0;
-  if (rot_dims == 0 && nq <= NORMED_MAX && nk <= NORMED_MAX && nv <= NORMED_MAX && !(dk % 4) && !(nv > 0 && dv % 4) && !(ld % 4) &&
+  // Registers for a part: three blocks of 256 threads a token however small it is, where the general form has one of 128 that takes
+  // longer the more entries there are.  Entries of a token, tokens: general / this, us: 256, 400 3.9 / 3.5, 800 4.7 / 5.8, 4,000 10 /
+  // 24; 768, 1,200 8.4 / 8.3, 2,000 10.6 / 12.8; 1,536, 2,000 16.5 / 13.1, 4,000 25.2 / 24.7; 2,304, 4,000 34.8 / 26.0.
+  const long entries = nq + nk + nv;
+  const bool in_registers = n_tokens <= 400 + entries * entries / 800;
+  if (in_registers && rot_dims == 0 && nq <= NORMED_MAX && nk <= NORMED_MAX && nv <= NORMED_MAX && !(dk % 4) && !(nv > 0 && dv % 4) && !(ld % 4) &&
       !(ldq % 4) && !((uintptr_t)proj & 15) && !((uintptr_t)q_out & 15) && !((uintptr_t)k_cache & 15) && !((uintptr_t)v_cache & 15) &&
       !((uintptr_t)q_norm_w & 15) && !((uintptr_t)k_norm_w & 15) && (dtype == LLMI_DTYPE_F32 || dtype == LLMI_DTYPE_BF16)) {
     const dim3 grid(n_tokens, has_kv && write_kv ? (v_from_k ? 2 : 3) : 1);

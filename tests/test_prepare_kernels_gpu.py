@@ -121,3 +121,18 @@ def test_short_walks_are_no_slower_than_in_the_general_form(T, H, D, R):
         proj = torch.randn(T, pitch, device="cuda")
         return _us(lambda: kernels.gdelta_prepare(proj, H, D, D, w2t, w0, ab, ctx, prep))
     assert call(5 * N + R) < 1.08 * call(5 * N + R + 1)
+
+
+@pytest.mark.parametrize("T,nq,nk,dk", [(3000, 4, 2, 32), (4000, 8, 2, 64), (2000, 2, 1, 64), (600, 8, 1, 16), (3000, 2, 1, 8)])
+def test_norms_of_small_parts_are_no_slower_than_in_the_general_form(T, nq, nk, dk):
+    """Rows that whole fours do not divide take the general form (many tokens took 0.4 to 0.9 times as long)."""
+    from llmi_b200.ops import kernels
+    wq, wk = torch.ones(nq * dk, device="cuda"), torch.ones(nk * dk, device="cuda")
+    kc, vc = (torch.zeros(T // 64 + 1, nk, 64, dk, device="cuda").bfloat16() for _ in range(2))
+    out, pages = torch.empty(T, nq * dk, device="cuda").bfloat16(), torch.arange(T // 64 + 1, device="cuda").int().view(1, -1)
+    ctx = _ctx([0] * T, list(range(T)))
+
+    def call(pitch):
+        proj = torch.randn(T, pitch, device="cuda")
+        return _us(lambda: kernels.qkv_prepare(proj, nq, nk, dk, nk, dk, wq, wk, 1e-5, None, 0, ctx, pages, 64, kc, vc, out))
+    assert call((nq + 2 * nk) * dk) < 1.08 * call((nq + 2 * nk) * dk + 1)
