@@ -106,7 +106,7 @@ attention_maps_mma_kernel(const MapsArgs a) {
   extern __shared__ __align__(16) unsigned char am_smem[];
   // Single tokens: a sequence's rows but its newest are from earlier steps, and where the caller says that those were complete before
   // the launch ahead began (`early`), its first page is asked for ahead of the wait for that launch.  (With the join's sixteen
-  // loads at a time a request of seven such steps, eight layers: 9.53 -> 9.45 ms.)
+  // loads at a time, us, 32 heads of 64 over 8, one sequence of 100, 2,000, 8,000: 7.3, 10.8, 17.3 -> 6.3, 7.9, 14.2.)
   // The next launch may start behind that wait only (see latent_attention_mma.cu).
   if (PROMPT || !a.early) {
     pdl_wait();

@@ -139,10 +139,11 @@ attention_short_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
   // The step's own row of a fused decode step never comes from the cache: the producer warp, once it has asked for all pages, makes
   // it, appends it and puts it into the page that the copy engine brought.  So no page waits for the kernel before, and nothing for
-  // the row's way out and back (the append, a fence, then the newest page's copy: 0.7 us of a layer of 9 x 64 heads on 340
-  // positions, 1.4 of eight sequences of 15).  Made by the consumer warp that has the row's keys, it cost 24 sequences of up to
-  // 3,900 positions 1.6 us a layer of 49.  (In attention_decode.cu, whose blocks are bound by the cache's read, the same made eight
-  // sequences of 3,900 positions 15 % slower: their newest pages then compete with the product before.)
+  // the row's way out and back (the append, a fence, then the newest page's copy).  A token step, us a layer less: 9 heads of 64
+  // over 3, one sequence of 100, 340, 1,000 positions 0.5, 0.5, 0.1; 15 over 5, eight sequences of 100, 340, 1,000 1.1, 0.7, 0.9; from
+  // 3,900 positions on the same within 0.1.  Made by the consumer warp that has the row's keys, it cost 24 sequences of up to 3,900
+  // positions 1.6 us a layer of 49.  (In attention_decode.cu, whose blocks are bound by the cache's read, a turn of eight sequences of
+  // 3,900 positions took 36.9 ms instead of 31.4 so: their newest pages then compete with the product before.)
   const bool own_row = FUSE && p.write_kv;
   const int new_row = pos0 % SH_PAGE, new_page = n_all - 1 - part * per;      // (of this part's pages: its last, or none of them)
   const bool has_newest = own_row && n_pages > 0 && new_page == n_pages - 1;

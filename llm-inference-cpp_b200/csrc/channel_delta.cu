@@ -65,8 +65,9 @@ __device__ __forceinline__ float ct_conv(const ChannelTokenArgs& a, const float*
 }
 
 // The channels base .. base + n - 1 (n at most 128, up to four taps) of a token, four a lane: what the step before left and the weights
-// are asked for together, with `early` ahead of the wait (a channel's seven loads one behind the
-// other, four channels a lane: 11 us of a step; a request of seven such steps 8.05 -> 7.93 ms).  `y`: their values; the order of a channel's sum is ct_conv's.
+// are asked for together, with `early` ahead of the wait (a channel's seven loads came one behind the other, four channels a lane;
+// 16 heads of 128, us with the step's kernel: 1 sequence 7.9 -> 7.5, 8 10.1 -> 9.4, 64 40.4 -> 38.4).  `y`: their values; the order of
+// a channel's sum is ct_conv's.
 constexpr int CT_FOUR = CT_V_PIECE / 32;
 __device__ __forceinline__ void ct_conv_piece(const ChannelTokenArgs& a, const float* row, float* carry, int base, int n, int Nc, int lane,
                                               float (&y)[CT_FOUR]) {

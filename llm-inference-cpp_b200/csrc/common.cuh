@@ -190,13 +190,28 @@ inline int launch_status() { return cudaPeekAtLastError() == cudaSuccess ? LLMI_
 // kernel after it start early in turn.  Both are no-ops in a kernel launched the plain way.  A decode
 // step is a chain of hundreds of few-microsecond kernels: this overlaps each kernel's launch and
 // set-up (and, in the matrix product, its first weight loads) with the tail of the one before.
+//
+// What a kernel may read AHEAD of its wait.  Behind it everything launched before is complete.  Ahead of it nothing is
+// that any kernel of the chain wrote, not only the one before: kernels that let the next one start ahead of their own wait
+// stand in a row of any length.  So only what was complete before the chain began, that is before the last launch or copy
+// that waits for all before it and is waited for by all behind it:
+//   * weights (products; where a caller may hand over a matrix that the launch ahead writes, only if it says `early`);
+//   * the step's index block, whose copy lies between two steps of a model;
+//   * with `early`, by which the caller says that such a copy lies between two steps on the same cache or states, what
+//     earlier steps left of the step's sequences: latent_attention_mma.cu and attention_maps_mma.cu (the first page of single
+//     tokens, all rows but the newest), attention_short.cu (pages without a row of the step; where the kernel makes the
+//     step's own row, the newest page too), channel_delta.cu (carried inputs and states);
+//   * attention_decode.cu and attention_decode_mma.cu take that for granted of the pages ahead of the newest.
+// One read rests on the kernel before instead: moe_down_kernel's of the chosen experts, because moe_up_kernel, always
+// directly before it, then lets it start only behind its own wait (moe.cu).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // LLMI_PDL is a bit mask of the kernel kinds that launch this way (default: all).  One rule came from
 // measurement: the decode attention kernel must not start while the product before the rotary kernel
 // still runs (batch 16: 3.86 ms a step against 3.18 ms; batch 64: 13.6 against 10.5), so the rotary
-// kernel signals its dependents only after its own wait, where every other kernel signals at once.
+// kernel signals its dependents only after its own wait, where most kernels signal at once.  (Others that wait first: attention
+// over latent rows and maps, the recurrences, the grouped experts, moe_up_kernel ahead of a moe_down_kernel that reads early.)
 constexpr int PDL_SMALL = 1, PDL_GEMM = 2, PDL_ATTENTION = 4, PDL_ROPE = 8;
 inline bool pdl_enabled(int kind) {
   static int mask = -1;

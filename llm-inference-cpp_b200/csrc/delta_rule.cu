@@ -50,7 +50,8 @@ constexpr int DELTA_V_PIECE = 256;
 
 __device__ __forceinline__ float delta_conv_one(const float* __restrict__ proj, long ld, const float* __restrict__ carry,
                                                 const float* __restrict__ conv_w, int ch, int Nc, int K, int pos, int p0, int r0) {
-  // four taps at a time, oldest first: their loads ahead of the sum (one behind the other, a token took 6.5 us)
+  // four taps at a time, oldest first: their loads ahead of the sum (a token of 16 heads of 128 with its
+  // recurrence 5.0 us, 5.9 one behind the other)
   float acc = 0.f;
   for (int d0 = K - 1; d0 >= 0; d0 -= 4) {
     float x[4], w[4];

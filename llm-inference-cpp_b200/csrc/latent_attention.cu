@@ -10,6 +10,7 @@
 //   llmi_latent_prepare_direct  the same for a layer whose queries come straight from its input: per token and head the
 //                           plain part of the query in the compute type and its rotated part, and the cache row
 //   llmi_latent_q_rotate    the rotated part of every head's query into its row [q~ | qrot]
+//   llmi_heads_token        the per-head products of a few tokens (q~ = Ukᵀ q, with that rotation; out = Uv context), bf16
 //   llmi_attention_latent   scores, softmax and context of every (token, head), any sizes, fp32 arithmetic; serves
 //                           prompts and single tokens, both types; optionally over a window of the last positions only
 // Rotation: pairs turned by the angle float(pos) * inv_freq[i], computed in fp32 with sincosf — neighbours (2i, 2i+1)
@@ -206,9 +207,10 @@ latent_q_rotate_kernel(const T* __restrict__ q, long ldq, int D, T* __restrict__
 // the context through the value expansion), and with `q` in the same launch what latent_q_rotate_kernel does.  Such a step is the
 // latency of its loads, so they are all asked for at once, the matrices (where the caller says `early`: a model's weights) ahead of
 // the wait for the kernel before: L lanes a row of K = 8 L CPL entries, RG rows a lane, RG x CPL = 8 pieces of 16 bytes in flight a
-// lane.  A row's sum: a lane's entries ascending, then a butterfly over the lanes; it does not depend on the number of tokens.
-// A request of seven such steps and a prompt, two sequences: with the tensor cores' tiles, a launch for the rotation and attention
-// that waited before its first page 10.86 ms (a map and expert model of 2,048) and 8.35 (channel states, latent rows); 10.55, 8.05.
+// lane.  A row's sum: a lane's entries ascending, then a butterfly over the lanes; in this kernel it does not depend on the number
+// of tokens.  16 heads of 512 x 128, us on the tensor cores' tiles / here: 1 token 2.4 / 1.5, 2 2.4 / 2.0, 4 2.4 / 2.4, 8 2.4 / 3.7; 128 x
+// 512, 1 4.7 / 1.6, 8 4.7 / 4.3; with the rotation, which the tiles leave to a launch of its own, 1 4.1 / 1.8, 4 4.1 / 2.7, 8 4.5 / 4.2.
+// Each token costs its multiplications on the CUDA cores; the caller chooses (ops/kernels.py, heads_token_faster).
 struct HeadsArgs {
   const __nv_bfloat16* x;
   long ldx, bx;
@@ -515,7 +517,7 @@ LLMI_EXPORT int llmi_attention_latent(int dtype, const void* qa, long ldq, void*
   return LLMI_ERR_BAD_DTYPE;
 }
 
-// Row lengths that heads_token_kernel has: 64, 128 and 256 to 2,048 in lane groups of 8, 16 and 32.
+// Row lengths that heads_token_kernel has (the powers of two from 64 to 2,048; others stay with the tiles): lane groups of 8, 16 and 32.
 LLMI_EXPORT int llmi_heads_token_supported(int K) { return K == 64 || K == 128 || K == 256 || K == 512 || K == 1024 || K == 2048; }
 
 // `batch` products of a few tokens, one per head: out[:, b*by : b*by + N] = x[:, b*bx : b*bx + K] . w[b]^T (bf16), w [batch, N, K]

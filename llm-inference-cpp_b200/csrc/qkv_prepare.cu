@@ -263,7 +263,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* o, const float4& v) {
 
 // Parts with norms over all their heads and no rotation: a block per (token, part) — q, k, v — with the part's entries in
 // registers between the sum and the store, four a load.  (One block per token that read every entry twice, one at a time: a
-// token of 32 heads of 64 and 2 x 8 key and value heads 20.5 us, the time of its loads one behind the other; 3,059 tokens 40.5.)
+// token of 32 heads of 64 and 2 x 8 key and value heads 13.1 us, the time of its loads one behind the other, 1.9 so; 3,000 tokens
+// 34.8 and 20.5.)
 // For parts of up to NORMED_MAX entries; the sum of a part is a thread's entries in ascending order, then pairs of lanes and pairs of
 // warps (eight warps one behind the other, as block_sum adds them, left the scale of 1,536 entries 5 % further from 64 bits than the
 // general form's four).

@@ -741,10 +741,11 @@ def decode_short_parts(n_live: int, n_kv_heads: int, n_pages: int, head_dim: int
     do ungrouped heads of 64, whose kernel gives its softmax 32-bit weights as this one does for heads of 128: with them
     this one is between 5 % faster and 30 % slower (32 heads, sequences of 2,200: 20 65.4 -> 70.3, 28 88.8 -> 102, 32 95.5 -> 106, 64 190 ->
     181, 96 273 -> 278).  Under a window the pages are those that it spans (planned by the whole
-    history, 32 sequences of 4,000 under a window of 128, 3 x 3 x 64, took 7.7 us, the persistent kernel 6.6; by the window 5.5).  Measured, persistent -> this (us, with the position encoding; kv heads x
-    group x size, sequences, positions): 3 x 3 x 64, 1, 1,000 8.0 -> 5.1, 8, 4,000 11.2 -> 10.0, 1, 8,000 10.4 -> 10.6; 8 x 4 x
-    128, 1, 1,000 9.8 -> 6.1, 1, 200 in one part 5.6 -> 5.0, in two 5.8, 24, 2,200 39.5 -> 38.5; 16 x 128, 1, 2,000 9.7 -> 10.2, 1, 4,000 15.1
-    -> 13.8, 4, 4,000 33.8 -> 26.4, 64, 2,200 229 -> 180."""
+    history, 32 sequences of 4,000 under a window of 128, 3 x 3 x 64, took longer than on the persistent kernel).  Measured, persistent
+    -> this (us, with the position encoding, launches in a row; kv heads x group x size, sequences, positions): 3 x 3 x 64, 1, 1,000
+    8.1 -> 5.1, 8, 4,000 10.0 -> 8.9, 32, 4,000 under a window of 128 5.3 -> 3.8; 8 x 4 x 128, 1, 1,000 9.5 -> 6.2, 1, 200 5.4 -> 5.0, 24,
+    2,200 39.6 -> 37.0; 16 x 128, 1, 2,000 7.9 -> 10.9, 1, 4,000 12.2 -> 12.5, 4, 4,000 31.9 -> 24.1, 64, 2,200 228 -> 174.  Of 343 layouts
+    the choice is more than 6 % from the better one in 12, 10 of them ungrouped heads of 128 (one sequence of 1,000: 6.2 -> 7.4)."""
     if group > 16 or head_dim not in (64, 128) or _DECODE_ATTENTION != "mma" or (group == 1 and head_dim == 64):
         return 0
     n_pages = visible_pages(n_pages, window)

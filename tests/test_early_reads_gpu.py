@@ -1,7 +1,8 @@
 """Kernels that may start before the launch ahead has ended, with that launch still at work (GPU).
 
-Every test puts a launch of two blocks in front that lets the next ones start at once and takes tens of microseconds; the
-kernel that writes the step's own row waits for it, and the reader under test is launched directly behind the writer."""
+Every test puts a launch of two blocks in front that lets the next ones start at once and takes longer than the host needs to
+launch them all (half a millisecond); the kernel that writes the step's own row waits for it, and the reader under test is
+launched directly behind the writer."""
 import types
 
 import pytest
@@ -18,7 +19,7 @@ def _i32(x):
 
 def _long_launch():
     from llmi_b200.ops import kernels
-    K = 1 << 17
+    K = 1 << 19
     x, w, y = torch.ones(1, K, device="cuda"), torch.ones(16, K, device="cuda"), torch.empty(1, 16, device="cuda")
     return lambda: kernels.linear_simt(x, w, y)
 
