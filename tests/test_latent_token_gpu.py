@@ -116,3 +116,23 @@ def test_reading_ahead_is_no_slower(H, C, R, S, n):
             times.append(start.elapsed_time(end) * 50.0)
         return min(times)
     assert us(True) < 1.05 * us(False)
+
+
+@pytest.mark.parametrize("K", [64, 128, 256, 1024, 2048])
+@pytest.mark.parametrize("N,M", [(13, 4), (130, 5), (64, 8), (2, 7)])
+@pytest.mark.parametrize("token", [True, False])
+def test_per_head_products_on_either_kernel(K, N, M, token, monkeypatch):
+    """The kernel of a few tokens and the tensor cores' tiles, whichever the choice by sizes is: around the former's batch of four."""
+    from llmi_b200.ops import kernels
+    monkeypatch.setattr(kernels, "heads_token_faster", lambda *sizes: token)
+    torch.manual_seed(K + N + M)
+    B, bx, by = 3, K + 8, N + N % 2 + 2
+    x, w = torch.randn(M, B * bx, device="cuda").bfloat16(), (torch.randn(B, N, K, device="cuda") * K ** -0.5).bfloat16()
+    out = torch.full((M, B * by), 7.0, device="cuda").bfloat16()
+    kernels.linear_batched(x, bx, w, out, by, K, early=True)
+    for b in range(B):
+        want, got = x[:, b * bx:b * bx + K].double() @ w[b].double().T, out[:, b * by:b * by + N].double()
+        size = x[:, b * bx:b * bx + K].double().abs() @ w[b].double().abs().T
+        # the result's rounding, and a sum of K exact products in 32 bits
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + K ** 0.5 * 2.0 ** -23 * size).all())
+        assert bool((out[:, b * by + N + N % 2:(b + 1) * by] == 7.0).all())
